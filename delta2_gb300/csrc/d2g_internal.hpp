@@ -162,12 +162,13 @@ struct Engine {
     DBuf<double> flt;
     // sequential-impulse solve
     DBuf<unsigned long long> sv_keys, sv_keys_out;
-    DBuf<int32_t> sv_vals, sv_order, sv_wave_idx, sv_wave_off, sv_wave_cursor;
-    DBuf<double> sv_static_imp, sv_sdelta;
-    DBuf<int32_t> sv_scon, sv_list, sv_grid, sv_cl_flags;
+    DBuf<int32_t> sv_vals, sv_order, sv_slot, sv_part_int, sv_con_int, sv_tcon, sv_tl;
+    DBuf<double> sv_sdelta;
+    DBuf<int32_t> sv_list, sv_grid, sv_cl_flags;
+    bool sv_smem_set = false;  // the solve kernels' shared memory limit was raised
     int sv_cl_fit[4] = {-1, -1, -1, -1};  // resident thread-block clusters of 16, 8, 4, 2 solve blocks
     int sv_layout[4] = {0, 0, 0, 0};  // the last solve call's layout (d2g_ctx_solve_layout)
-    DBuf<unsigned char> sv_bw_raw, sv_cw_raw;
+    DBuf<unsigned char> sv_bg_raw, sv_bs_raw, sv_cg_raw, sv_cs_raw;
     // GPU broad phase (d2g_broadphase.cu)
     DBuf<float> bp_box;
     DBuf<unsigned long long> bp_key, bp_key_s;

@@ -5,15 +5,16 @@
 // de-duplication of contact midpoints.
 //
 // SequentialImpulses::solve (strategies/contact_force/sequential_impulses.cpp:
-// 104-638): one block per cluster.  The reference's Gauss-Seidel sweep visits
-// the contacts in sorted order and integrates both bodies after each one; a
-// contact only reads and writes its own two bodies, so contacts are grouped
-// into waves: a contact's wave is one past the last wave that touched either
-// of its moving bodies.  Within a wave the bodies are disjoint and the
-// contacts run in parallel; every body still sees its contacts in sorted
-// order, so every floating-point operation happens in the reference's order
-// (static bodies are never integrated; the impulse sum the convergence test
-// reads for them is accumulated from per-contact deltas in sorted order).
+// 104-638): one block, a thread-block cluster or a grid per cluster.  The
+// reference's Gauss-Seidel sweep visits the contacts in sorted order and
+// integrates both bodies after each one; a contact only reads and writes its
+// own two bodies, so contacts are grouped into waves: a contact's wave is one
+// past the last wave that touched either of its moving bodies.  Within a wave
+// the bodies are disjoint and the contacts run in parallel; every body still
+// sees its contacts in sorted order, so every floating-point operation happens
+// in the reference's order (static bodies are never integrated; the impulse
+// sum the convergence test reads for them is accumulated from per-contact
+// deltas in sorted order).
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -31,7 +32,9 @@ constexpr int kSolveBlock = 256;
 constexpr int kGridMinContacts = 128;    // a cluster this large may take a cooperative grid
 constexpr int kGridMaxClusters = 8;      // ... with more parts than D2G_TUNE_GRID_MIN_PARTS,
                                          // when at most this many clusters qualify
-constexpr int kClusterMinContacts = 32;  // a cluster this large takes a thread-block cluster
+constexpr int kClusterMinContacts = 32;  // a cluster this large may take a thread-block cluster
+constexpr int kPartsPerBlock = 32;       // particles of a cluster per block of its thread-block cluster
+constexpr int kSolveSmemMax = 200 * 1024;  // dynamic shared memory of a solve block at most
 inline int nblocks(long long n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
 // ------------------------------------------------------------ filtering ---
@@ -127,26 +130,62 @@ __global__ void k_filter_offsets(int n, const int32_t* __restrict__ off, const i
 }
 
 // ---------------------------------------------------------------- solve ---
-// Per-body working state (indexed by global body id; moving bodies belong to
-// one cluster only).
-struct BodyWork {
-    double FS[14], FSf[14];
-    double T_FS[12], T_FSf[12], T_cur[12];
-    double Iinv[9];  // R(fut.q) * ii * R(fut.q)^T, constant during a solve
-    double imp[3], rimp[3], ioff[3], roff[3], last_imp[3];
-    double rmass;  // 1 / mass, for m_div_recip
-    int last_level;
+// What a sweep of the reference really recomputes.  updateState
+// (sequential_impulses.cpp:46-70) integrates a body's state from its impulse
+// sums: v from imp, x from ioff, L from rimp, and q from roff.  roff only ever
+// receives the friction loop's zero updates, so q, the rotation and with it
+// R * local of every contact are constants of a solve; updateStateImmediate's
+// state is read by nothing that reaches a result.  A contact's update is
+// therefore two short chains: a position half (x, ioff, the offset impulse
+// and the penetration test) that reads nothing of the other, and a velocity
+// half (v, L, imp, rimp, the normal impulse) that reads the position half's
+// lever arms and test.  Every value is produced by the reference's operations
+// in the reference's order.
+//
+// The halves run on different warps, the position half one wave ahead:
+// GB300 issues an FP64 warp instruction every 64 cycles per SM sub-partition
+// whatever the number of active lanes, so a wave costs the longest warp's
+// FP64 instruction count, 28 for the velocity half and 20 for the position
+// half, against ~143 when one warp formed both with the quaternion integration
+// of two states.  A contact takes eight lanes of each (side A or B, component).
+// Bodies live in shared memory (spread over the blocks of a thread-block
+// cluster, read and written through distributed shared memory) and a contact
+// in the shared memory of the block that always processes it, both in global
+// memory where they do not fit or the blocks form a cooperative grid.
+//
+// A wave of one contact in one block takes 1.3 us (7.2 before); the table at
+// run_solve has the layouts.
+
+struct BodyS {  // one body's working state
+    double x[3], v[3], w[3];  // position, velocity, body inverse inertia * L
+    double imp[3], rimp[3], ioff[3], last_imp[3];
+    double fx[3], fv[3], fL[3];  // the input future state
+    double ii[9], m, rm;  // rm = 1 / m, for div_by
+    int32_t is_static, rbad;  // rbad: friction iteration (1-based) whose lever arm was not finite, 0 = none
 };
 
-// Per-contact working state (indexed by the contact's position in the call).
-struct ConWork {
-    double local_A[3], local_B[3], n[3];
-    double start_dist, mass_eff, outer, impulse, impulse_offset;
-    double slop, damp_m;  // per-solve constants of the normal loop: its slop and damp * mass_eff
-    double rcnt;          // 1 / pair_cnt, for m_div_recip
-    double last_fi[3], last_rot_A[3], last_rot_B[3], upd_total[3];
-    int a, b, level, pair_cnt;
-    int spos;  // position among the contacts touching a static body, -1 if none
+struct ConS {  // one contact's working state in the normal loop
+    double rl[2][3], n[3];  // R * local per side, the normal
+    double r[2][3];         // lever arms p1 - x, from the position half to the velocity half
+    double imp, off, outer, m, slop, damp_m;
+    BodyS* body[2];
+    double* sd;          // where its impulse delta on a static body goes, or null
+    int32_t ci;          // the contact in sorted order, -1: an unused place
+    int16_t near_, sneg;  // d1 < outer (position half); the delta is -u (the static body is b)
+};
+
+struct BodyG {  // per body, written once per solve (global memory)
+    double Ti[16];     // inverse transform of the input future state
+    double R0[9];      // its rotation
+    double q[4], R[9];  // the solved state's quaternion and rotation
+};
+
+struct ConG {  // per contact in sorted order (global memory)
+    double local[2][3], n[3], outer, mass_eff, slop, damp_m, impulse;
+    double rl[2][3], rF[2][3];  // R * local; contact point - input position
+    double u[3], rf[2][2][3], lf[3];  // body update, torques (by iteration parity and side), friction impulse
+    double mu, cnt, rcnt;
+    int32_t a, b;  // particle indices within the cluster
 };
 
 __device__ __forceinline__ V3 ld3(const double* p) { return mk(p[0], p[1], p[2]); }
@@ -155,48 +194,46 @@ __device__ __forceinline__ void st3(double* p, V3 v) {
     p[1] = v.y;
     p[2] = v.z;
 }
-__device__ __forceinline__ void rigid12(const State& s, double* T12) {
-    double T[16];
-    transformation(s.q, s.x, T);
-    for (int k = 0; k < 12; k++) T12[k] = T[k];
-}
 __device__ __forceinline__ V3 calc_torque(V3 force, V3 point, V3 com) { return cross(-force, point - com); }
-
-// sequential_impulses.cpp:46-70 updateState (variant 0, FS) or :72-96
-// updateStateImmediate (variant 1, FSf) of one body, with R(fut.q) * ii *
-// R(fut.q)^T precomputed (it only depends on fut).  Both forms are evaluated
-// and the variant's selected, so lanes integrating different variants do
-// not diverge.
-__device__ void integrate_one(BodyWork& w, const double* fut, double mass, double t, int variant) {
-    const State f = load_state(fut);
-    const V3 imp = ld3(w.imp), ioff = ld3(w.ioff), rimp = ld3(w.rimp), roff = ld3(w.roff);
-    State u = f;
-    const V3 im = mk(m_div_recip(imp.x, mass, w.rmass), m_div_recip(imp.y, mass, w.rmass),
-                     m_div_recip(imp.z, mass, w.rmass));
-    u.v = f.v + im;
-    const V3 xa = f.x + mk(m_div_recip(ioff.x, mass, w.rmass), m_div_recip(ioff.y, mass, w.rmass),
-                           m_div_recip(ioff.z, mass, w.rmass)) * t;
-    const V3 xb = xa + im * t;
-    u.x = variant ? xb : xa;
-    u.L = f.L + rimp;
-    const V3 La = f.L + t * roff;
-    const V3 Lb = La + t * rimp;
-    const V3 omega = m3_vec(w.Iinv, variant ? Lb : La);
-    u.q = qmul(qexp((0.5 * omega) * t), f.q);
-    store_state(variant ? w.FSf : w.FS, u);
-    rigid12(u, variant ? w.T_FSf : w.T_FS);
-}
-
 __device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ V3 shfl3(V3 v, int src) { return mk(shfl_d(v.x, src), shfl_d(v.y, src), shfl_d(v.z, src)); }
-
-__device__ __forceinline__ V3 xf12(V3 p, const double* T) {
-    return mk(((T[0] * p.x + T[1] * p.y) + T[2] * p.z) + T[3] * 1.0,
-              ((T[4] * p.x + T[5] * p.y) + T[6] * p.z) + T[7] * 1.0,
-              ((T[8] * p.x + T[9] * p.y) + T[10] * p.z) + T[11] * 1.0);
+// v with its sign flipped where f (an integer operation)
+__device__ __forceinline__ double neg_if(double v, bool f) {
+    return __hiloint2double(__double2hiint(v) ^ (f ? (int)0x80000000 : 0), __double2loint(v));
+}
+// Comparisons of the hot loops on bit patterns: the FP64 pipe takes a
+// comparison at the price of an addition.
+__device__ __forceinline__ bool is_pos(double v) {  // v > 0 (false for NaN)
+    const long long b = __double_as_longlong(v);
+    return b > 0 && b <= 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ double max0(double v) {  // dmax(v, 0.0): v unless v < 0
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull ? 0.0 : v;
+}
+// sqrt(s) > 1e-6 and sqrt(s) > 1e-4 for s >= 0 without the root: the rounded
+// square root is monotone, and these are the largest doubles whose root does
+// not pass the bound (false for NaN).
+constexpr double kSqMax1e6 = 1e-12, kSqMax1e4 = 1.0000000000000002e-08;
+__device__ __forceinline__ bool sq_above(double s, double lim) {
+    const long long b = __double_as_longlong(s);
+    return b > __double_as_longlong(lim) && b <= 0x7ff0000000000000ll;
 }
 
-__device__ __forceinline__ bool block_any(bool v) { return __syncthreads_or(v ? 1 : 0) != 0; }
+// x / y given ry = 1 / y: m_div_recip (same result), its three operations
+// issued ahead of the range checks, which run beside them.
+__device__ __forceinline__ double div_by(double x, double y, double ry) {
+    const double q = x * ry;
+    const double r = fma(-q, y, x);
+    double res = fma(r, ry, q);
+    const bool yok = (unsigned)(m_exp_field(y) - 573) <= 900u;
+    if (!(yok && (unsigned)(m_exp_field(q) - 573) <= 900u)) {
+        if (yok && m_is_zero(x))
+            res = q;
+        else
+            res = x / y;
+    }
+    return res;
+}
 
 // Synchronisation of one cluster's solve: the threads of one block, the
 // blocks of a thread-block cluster (the hardware cluster barrier), or every
@@ -208,11 +245,14 @@ __device__ __forceinline__ bool block_any(bool v) { return __syncthreads_or(v ? 
 // so the kernel can stop and report it.
 enum SyncMode : int { kSyncBlock = 0, kSyncGrid = 1, kSyncCluster = 2 };
 
+// A cluster's small integers (shared memory of a block, else global memory
+// zeroed before the launch).
+enum { kFlFail = 0, kFlLevels, kFlTasks, kFlAny0, kFlAny1, kFlSpin, kFlStatics, kFlCursor, kFlags };
+
 struct SolveSync {
-    int mode;
     unsigned long long* count;  // grid barrier arrivals (monotonic within a launch)
     unsigned long long* passed;  // grid: the block's barriers passed so far (shared memory)
-    int32_t* flags;       // [0] fail, [1] levels, [2] static contacts, [3], [4] "moved" by parity, [5] spin error
+    int32_t* flags;
     unsigned int spin_limit;  // polls before a grid barrier wait gives up
 };
 
@@ -240,12 +280,14 @@ __device__ __forceinline__ void cluster_barrier() {
 // until every block has arrived as often as it has, then __syncthreads
 // hands the acquired writes to the block.  The barriers passed so far are
 // counted per block in shared memory (every block passes the same ones).
-__device__ bool solve_sync(const SolveSync& S) {
-    if (S.mode == kSyncBlock) {
+template <int MODE>
+__device__ __forceinline__ bool solve_sync(const SolveSync& S) {
+    if (MODE == kSyncBlock) {
         __syncthreads();
         return true;
     }
-    if (S.mode == kSyncCluster) {
+    if (MODE == kSyncCluster) {
+        __syncwarp();
         cluster_barrier();
         return true;
     }
@@ -258,7 +300,7 @@ __device__ bool solve_sync(const SolveSync& S) {
         unsigned int spins = 0;
         while (ld_acquire_u64(S.count) < target) {
             if (++spins > S.spin_limit) {  // seconds at the default: the other blocks are gone
-                atomicExch(S.flags + 5, 1);
+                atomicExch(S.flags + kFlSpin, 1);
                 ok = 0;
                 break;
             }
@@ -269,16 +311,17 @@ __device__ bool solve_sync(const SolveSync& S) {
     return s_ok != 0;
 }
 
-// true when any thread of the cluster's solve passes v; slot 3 or 4 by the
-// iteration's parity (the other slot is cleared for the next iteration by
-// the first block, gb = 0).
-__device__ bool solve_any(const SolveSync& S, bool v, int parity, int gb, bool* ok) {
-    if (S.mode == kSyncBlock) return block_any(v);
+// true when any thread of the cluster's solve passes v; flag 0 or 1 by the
+// call's parity (the other one is cleared for the next call by the first
+// block, gb = 0).
+template <int MODE>
+__device__ __forceinline__ bool solve_any(const SolveSync& S, bool v, int parity, int gb, bool* ok) {
     const bool blk = __syncthreads_or(v ? 1 : 0) != 0;
-    if (threadIdx.x == 0 && blk) atomicOr(S.flags + 3 + parity, 1);
-    *ok = solve_sync(S) && *ok;
-    const bool r = ld_relaxed_i32(S.flags + 3 + parity) != 0;
-    if (gb == 0 && threadIdx.x == 0) S.flags[3 + (parity ^ 1)] = 0;
+    if (MODE == kSyncBlock) return blk;
+    if (threadIdx.x == 0 && blk) atomicOr(S.flags + kFlAny0 + parity, 1);
+    *ok = solve_sync<MODE>(S) && *ok;
+    const bool r = ld_relaxed_i32(S.flags + kFlAny0 + parity) != 0;
+    if (gb == 0 && threadIdx.x == 0) S.flags[kFlAny0 + (parity ^ 1)] = 0;
     return r;
 }
 
@@ -289,660 +332,675 @@ struct SolveArgs {
     const int32_t* pair_cnt;
     const double *warm, *cl_step;
     const uint8_t* is_static;
-    const double *mass, *ii, *mu, *cur;
+    const double *mass, *ii, *mu;
     double* fut;
     double gravity_z;
-    BodyWork* bw;
-    ConWork* cw;
-    int32_t *wave_idx, *wave_off, *wave_cursor, *scon;
-    double* sdelta;  // per contact touching a static body: its impulse delta on that body
-    double* static_imp;
+    // work arrays: per particle of the call, per contact, and the waves' tasks
+    BodyG* bg;
+    BodyS* bs;    // bodies that are not in shared memory
+    ConG* cg;
+    ConS* cs;     // contacts that are not in shared memory (four places per contact)
+    int32_t *slot, *deg, *boff, *statics;  // per body; per particle
+    int2* ab;          // contacts' particles, bit 30 marks a static one
+    int32_t *blist, *lpos, *prev, *level;  // two per contact (level: one)
+    int32_t *tcon, *tl;  // contacts of the waves' tasks, first task of every wave
+    double* sdelta;      // per entry of blist: a contact's impulse delta on a static body
     int32_t *status, *iters;
     double* out_impulse;
     int32_t* out_ab;
     const int32_t* con_pair;
     double* pair_warm;
-    int lanes;  // normal-loop lanes per contact: 0 = by wave width, 4 or 16
+    int smem;  // dynamic shared memory, bytes
 };
 
-// This lane's contact (index within its cluster) and body in the warp's
-// first task of a sixteen-lane wave [n0, n1), or (-1, -1) when the warp has
-// no task in it.  Loaded before the barrier that precedes the wave (the
-// schedule does not change during the loop), so the wave starts with one
-// round of loads instead of three dependent ones.
-__device__ __forceinline__ int2 wave16_first(int n0, int n1, const int32_t* __restrict__ widx, int c0, int G,
-                                             int gb, const SolveArgs& a) {
-    const int lane = threadIdx.x & 31, side = lane & 1;
-    const int wslot = (int)(threadIdx.x >> 5) * G + gb;
-    if (wslot >= (n1 - n0 + 1) >> 1) return make_int2(-1, -1);
-    const int q = n0 + 2 * wslot + (lane >> 4);
-    const int ci = widx[q < n1 ? q : n0];
-    return make_int2(ci, side ? a.cw[c0 + ci].b : a.cw[c0 + ci].a);
+constexpr int kStaticBit = 1 << 30;
+
+// Body p of the cluster: block p % G's shared memory, or global memory.
+template <int MODE>
+__device__ __forceinline__ BodyS* body_at(int p, BodyS* sm, BodyS* gl, bool in_smem, int G) {
+    if (!in_smem) return gl + p;
+    if (MODE == kSyncBlock) return sm + p;
+    unsigned long long out;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"((unsigned long long)(sm + p / G)), "r"(p % G));
+    return (BodyS*)out;
 }
 
-// One wave of the normal loop (sequential_impulses.cpp:239-378: per contact
-// the normal and offset impulses, then updateState :46-70 and
-// updateStateImmediate :72-96 of both bodies) with sixteen lanes per
-// contact: lane bit 0 picks the body side (A, B) and bit 1 the integrated
-// state (FS, FSf) as in the four-lane form, bits 2-3 a component (x, y, z
-// of the vectors and rows of the matrices; the fourth lane carries the
-// quaternions' w).  Every value
-// is the four-lane form's, operation for operation: vector and matrix work
-// is spread over the component lanes and gathered with shuffles, the
-// d1 / v1 dot products run on the FS / FSf lanes and sin / cos of the
-// quaternion exponential on even / odd component lanes, which halves the
-// FP64 instructions of a contact's dependent chain.  Each warp takes two
-// contacts; warps are dealt to SMs first, then to the SMs' sub-partitions,
-// as in the four-lane form.
-__device__ __forceinline__ void normal_wave16(int n0, int n1, const int32_t* __restrict__ widx, int c0, int G,
-                                              int gb, double t, double rt, int2 pre, const SolveArgs& a) {
-    const int lane = threadIdx.x & 31;
-    const int side = lane & 1, variant = (lane >> 1) & 1, c = (lane >> 2) & 3;
-    const int cc = c < 3 ? c : 0;   // the w lane repeats component x in vector work
-    const int grp = lane & ~12;     // component 0 of this lane's (side, state)
-    const int s1 = grp | ((cc == 2 ? 0 : cc + 1) << 2), s2 = grp | ((cc == 0 ? 2 : cc - 1) << 2);
-    const int tasks = (n1 - n0 + 1) >> 1;
-    const int wslot = (int)(threadIdx.x >> 5) * G + gb, nwarps = (int)(blockDim.x >> 5) * G;
-    for (int task = wslot; task < tasks; task += nwarps) {
-        const int q = n0 + 2 * task + (lane >> 4);
-        const bool act = q < n1;
-        int ci, g;
-        if (task == wslot && pre.x >= 0) {  // loaded before the barrier
-            ci = pre.x;
-            g = pre.y;
-        } else {
-            ci = widx[act ? q : n0];
-            g = side ? a.cw[c0 + ci].b : a.cw[c0 + ci].a;
+// The position half of one contact (sequential_impulses.cpp:239-378): eight
+// lanes, side = lane bit 2, component = lane bits 0-1 (the fourth lane repeats
+// x and writes nothing).
+__device__ __forceinline__ void position_half(ConS& C, bool act, int side, int c, double t, double rt) {
+    const int lane = threadIdx.x & 31, cc = c < 3 ? c : 0, base = lane & ~3;
+    BodyS& B = *C.body[side];
+    const double x = B.x[cc], ioff = B.ioff[cc], fx = B.fx[cc], m = B.m, rm = B.rm;
+    const double n = C.n[cc];
+    const bool st = B.is_static != 0;
+    const double p1 = C.rl[side][cc] + x;
+    const double r = p1 - x;
+    const double pr = p1 * n;
+    const double dv = (shfl_d(pr, base) + shfl_d(pr, base | 1)) + shfl_d(pr, base | 2);
+    const double ot = shfl_d(dv, lane ^ 4);
+    const double d1 = (side ? dv : ot) - (side ? ot : dv);  // n.p1B - n.p1A
+    const double pen = C.outer - d1;
+    const bool near_ = is_pos(pen);  // d1 < outer
+    const double e = pen - C.slop;
+    const double off0 = C.off;
+    const double dn = div_by(C.damp_m * (is_pos(e) ? e : 0.0), t, rt);
+    const double off1 = max0(off0 + (near_ ? dn : neg_if(off0, true)));
+    const double uo = neg_if(n, true) * (off1 - off0);
+    const double io = ioff + neg_if(uo, side);
+    const double xn = fx + div_by(io, m, rm) * t;
+    __syncwarp();
+    if (act && c < 3) {
+        C.r[side][c] = r;
+        if (!st) {
+            B.ioff[c] = io;
+            B.x[c] = xn;
         }
-        ConWork& C = a.cw[c0 + ci];
-        BodyWork& W = a.bw[g];
-        const bool st = a.is_static[g];
-        // this side's contact point p1 = T_FS local and its velocity
-        // v1 = v + (ii L) x (p1 - x) (State::pointVelocity), component cc
-        // (p1 on the FS lanes and ii L on the FSf lanes in one instruction
-        // stream, each with its own operations in its order, then swapped)
-        const double* lp = side ? C.local_B : C.local_A;
-        const double* Tr = W.T_FS + 4 * cc;
-        const double* Ir = a.ii + 9 * (size_t)g + 3 * cc;
-        const double* X = variant ? Ir : Tr;
-        const double* Y = variant ? W.FS + 5 : lp;
-        const double dot3 = (X[0] * Y[0] + X[1] * Y[1]) + X[2] * Y[2];
-        const double mine = variant ? dot3 : dot3 + Tr[3] * 1.0;
-        const double other = shfl_d(mine, lane ^ 2);
-        const double p1 = variant ? other : mine;
-        const double wv = variant ? mine : other;
-        const double r = p1 - W.FS[8 + cc];
-        const double w1 = shfl_d(wv, s1), w2 = shfl_d(wv, s2), r1 = shfl_d(r, s1), r2 = shfl_d(r, s2);
-        const double v1s = W.FS[11 + cc] + (w1 * r2 - w2 * r1);
-        const double pA = shfl_d(p1, lane & ~1), pB = shfl_d(p1, lane | 1);
-        const double vA = shfl_d(v1s, lane & ~1), vB = shfl_d(v1s, lane | 1);
-        // d1 = n.p1B - n.p1A on the FS lanes, v1 = n.v1A - n.v1B on the FSf lanes
-        const double ncc = C.n[cc];
-        const double PX = (variant ? vA : pB) * ncc, PY = (variant ? vB : pA) * ncc;
-        const double dd = ((shfl_d(PX, grp) + shfl_d(PX, grp | 4)) + shfl_d(PX, grp | 8)) -
-                          ((shfl_d(PY, grp) + shfl_d(PY, grp | 4)) + shfl_d(PY, grp | 8));
-        const double d1 = shfl_d(dd, lane & ~2), v1 = shfl_d(dd, lane | 2);
-        const double outer = C.outer, m = C.mass_eff, damp = 0.1;
-        const double imp0 = C.impulse, off0 = C.impulse_offset;
-        const double dimp = d1 < outer ? (v1 * m) * damp : -imp0;
-        const double imp1 = dmax(imp0 + dimp, 0.0);
-        const double u = (-ncc) * (imp1 - imp0);
-        const double pen = outer - d1;
-        const double doff = d1 < outer ? m_div_recip(C.damp_m * dmax(0.0, pen - C.slop), t, rt) : -off0;
-        const double off1 = dmax(off0 + doff, 0.0);
-        const double uo = (-ncc) * (off1 - off0);
-        // this side's impulse sums after the contact: imp + us,
-        // rimp + (-us) x (p1 - x), ioff + uso (us, uso: u, uo or their negatives)
-        const double us = side ? -u : u;
-        const double nus = -us;
-        const double imp = W.imp[cc] + us;
-        const double rimp = W.rimp[cc] + (shfl_d(nus, s1) * r2 - shfl_d(nus, s2) * r1);
-        const double ioff = W.ioff[cc] + (side ? -uo : uo);
-        // integrate_one on these sums, component cc
-        const double* F = a.fut + 14 * (size_t)g;
-        const double ms = a.mass[g];
-        // imp / ms on the FS lanes, ioff / ms on the FSf lanes, then swapped
-        const double qm = m_div_recip(variant ? ioff : imp, ms, W.rmass);
-        const double qm2 = shfl_d(qm, lane ^ 2);
-        const double im = variant ? qm2 : qm, iom = variant ? qm : qm2;
-        const double vnew = F[11 + cc] + im;
-        const double xa = F[8 + cc] + iom * t;
-        const double xb = xa + im * t;
-        const double xnew = variant ? xb : xa;
-        const double Lnew = F[5 + cc] + rimp;
-        const double La = F[5 + cc] + t * W.roff[cc];
-        const double Lb = La + t * rimp;
-        const double Ls = variant ? Lb : La;
-        const double* Ii = W.Iinv + 3 * cc;
-        const double om = (Ii[0] * shfl_d(Ls, grp) + Ii[1] * shfl_d(Ls, grp | 4)) + Ii[2] * shfl_d(Ls, grp | 8);
-        const double d = (0.5 * om) * t;
-        // qexp(d) = (cos |d|, (d / |d|) sin |d|), the identity for |d| = 0
-        const double dq = d * d;
-        const double nrm = sqrt((shfl_d(dq, grp) + shfl_d(dq, grp | 4)) + shfl_d(dq, grp | 8));
-        const bool finite_arg = (nrm < 0.0 ? -nrm : nrm) < 1e9;
-        double rr;
-        int qd;
-        m_reduce(finite_arg ? nrm : 0.0, rr, qd);
-        const double kk = m_kernel_sincos(rr, (c & 1) != 0);
-        const double ks = shfl_d(kk, grp), kc = shfl_d(kk, grp | 4);
-        double sn = qd == 0 ? ks : (qd == 1 ? kc : (qd == 2 ? -ks : -kc));  // m_sin
-        double cs = qd == 0 ? kc : (qd == 1 ? -ks : (qd == 2 ? -kc : ks));  // m_cos
-        if (!finite_arg) sn = cs = nrm - nrm;
-        const bool ident = nrm == 0.0;
-        const double ew = ident ? 1.0 : cs;
-        const double ev = ident ? 0.0 : (d / nrm) * sn;
-        // u.q = qmul(e, f.q), component c (w on the fourth lane):
-        // w = ((ew bw - ex bx) - ey by) - ez bz, x = ((ew bx + ex bw) + ey bz) - ez by, ...
-        const double ex = shfl_d(ev, grp), ey = shfl_d(ev, grp | 4), ez = shfl_d(ev, grp | 8);
-        const double fw = F[1], fx = F[2], fy = F[3], fz = F[4];
-        const bool wl = c == 3;
-        const double b1 = wl ? fw : (c == 0 ? fx : (c == 1 ? fy : fz));
-        const double a2 = wl ? ex : (c == 0 ? ex : (c == 1 ? ey : ez));
-        const double b2 = wl ? fx : fw;
-        const double a3 = wl ? ey : (c == 0 ? ey : (c == 1 ? ez : ex));
-        const double b3 = wl ? fy : (c == 0 ? fz : (c == 1 ? fx : fy));
-        const double a4 = wl ? ez : (c == 0 ? ez : (c == 1 ? ex : ey));
-        const double b4 = wl ? fz : (c == 0 ? fy : (c == 1 ? fz : fx));
-        const double P1 = ew * b1, P2 = a2 * b2, P3 = a3 * b3, P4 = a4 * b4;
-        const double qn = ((P1 + (wl ? -P2 : P2)) + (wl ? -P3 : P3)) - P4;
-        // rigid12 of the new state: row cc of R(q) (qmat), then x
-        const double qw = shfl_d(qn, grp | 12), qx = shfl_d(qn, grp), qy = shfl_d(qn, grp | 4),
-                     qz = shfl_d(qn, grp | 8);
-        const double tc = 2.0 * qn;
-        const double tx = shfl_d(tc, grp), ty = shfl_d(tc, grp | 4), tz = shfl_d(tc, grp | 8);
-        // row 0: 1 - (tyy + tzz), txy - twz, txz + twy
-        // row 1: txy + twz, 1 - (txx + tzz), tyz - twx
-        // row 2: txz - twy, tyz + twx, 1 - (txx + tyy)
-        const double Pd = (cc == 0 ? ty : tx) * (cc == 0 ? qy : qx);
-        const double Qd = (cc == 2 ? ty : tz) * (cc == 2 ? qy : qz);
-        const double A1 = (cc == 2 ? tz : ty) * qx;
-        const double B1 = (cc == 2 ? ty : tz) * qw;
-        const double A2 = tz * (cc == 0 ? qx : qy);
-        const double B2 = (cc == 0 ? ty : tx) * qw;
-        const double diag = 1.0 - (Pd + Qd);
-        const double o1 = A1 + (cc == 1 ? B1 : -B1);
-        const double o2 = A2 + (cc == 1 ? -B2 : B2);
-        __syncwarp();
-        if (act && variant == 0 && c < 3) {
-            if (!st) {
-                W.imp[c] = imp;
-                W.rimp[c] = rimp;
-                W.ioff[c] = ioff;
-            }
-            if (side == 0) {
-                if (C.spos >= 0) a.sdelta[3 * (size_t)(c0 + C.spos) + c] = a.is_static[C.a] ? u : -u;
-                if (c == 0) {
-                    C.impulse = imp1;
-                    C.impulse_offset = off1;
-                }
-            }
-        }
-        if (act && !st) {
-            double* S = variant ? W.FSf : W.FS;
-            double* T = (variant ? W.T_FSf : W.T_FS) + 4 * cc;
-            if (wl) {
-                S[1] = qn;
-            } else {
-                if (c == 0) S[0] = F[0];
-                S[2 + c] = qn;
-                S[5 + c] = Lnew;
-                S[8 + c] = xnew;
-                S[11 + c] = vnew;
-                T[c] = diag;
-                T[c == 0 ? 1 : 0] = o1;
-                T[c == 2 ? 1 : 2] = o2;
-                T[3] = xnew;
-            }
+        if ((side | c) == 0) {
+            C.off = off1;
+            C.near_ = near_ ? 1 : 0;
         }
     }
+}
+
+// The velocity half, lanes as above, with the lever arms and the test that
+// the position half left in the contact.
+__device__ __forceinline__ void velocity_half(ConS& C, bool act, int side, int c) {
+    const int lane = threadIdx.x & 31, cc = c < 3 ? c : 0, base = lane & ~3;
+    const int c1 = cc == 2 ? 0 : cc + 1, c2 = cc == 0 ? 2 : cc - 1;
+    BodyS& B = *C.body[side];
+    const double w1 = B.w[c1], w2 = B.w[c2], r1 = C.r[side][c1], r2 = C.r[side][c2];
+    const double v = B.v[cc], n = C.n[cc];
+    const double imp_b = B.imp[cc], rimp_b = B.rimp[cc], fv = B.fv[cc], fL = B.fL[cc], m = B.m, rm = B.rm;
+    const double i0 = B.ii[3 * cc], i1 = B.ii[3 * cc + 1], i2 = B.ii[3 * cc + 2];
+    const bool st = B.is_static != 0;
+    const double vs = v + (w1 * r2 - w2 * r1);  // v + (ii L) x (p1 - x)
+    const double pr = vs * n;
+    const double dv = (shfl_d(pr, base) + shfl_d(pr, base | 1)) + shfl_d(pr, base | 2);
+    const double ot = shfl_d(dv, lane ^ 4);
+    const double v1 = (side ? ot : dv) - (side ? dv : ot);  // n.v1A - n.v1B
+    const double imp0 = C.imp;
+    const double dn = (v1 * C.m) * 0.1;
+    const double imp1 = max0(imp0 + (C.near_ ? dn : neg_if(imp0, true)));
+    const double u = neg_if(n, true) * (imp1 - imp0);
+    const double us = neg_if(u, side);
+    const double nus = neg_if(us, true);
+    const double n1 = shfl_d(nus, base | c1), n2 = shfl_d(nus, base | c2);
+    const double rimp = rimp_b + (n1 * r2 - n2 * r1);
+    const double L = fL + rimp;
+    const double imp = imp_b + us;
+    const double L0 = shfl_d(L, base), L1 = shfl_d(L, base | 1), L2 = shfl_d(L, base | 2);
+    const double vn = fv + div_by(imp, m, rm);
+    const double w = (i0 * L0 + i1 * L1) + i2 * L2;
+    __syncwarp();
+    if (act && c < 3) {
+        if (!st) {
+            B.imp[c] = imp;
+            B.rimp[c] = rimp;
+            B.v[c] = vn;
+            B.w[c] = w;
+        }
+        if (side == 0) {
+            if (C.sd) C.sd[c] = neg_if(u, C.sneg != 0);
+            if (c == 0) C.imp = imp1;
+        }
+    }
+}
+
+// Body p's impulse sums over its contacts in sorted order
+// (sequential_impulses.cpp:193-215 and :560-607: imp +- u, rimp - last + new),
+// then updateState: eight lanes, lane bit 2 picks imp or rimp, bits 0-1 the
+// component.  par: the torques' parity; the other one holds the last ones.
+// The list's entries are loaded eight at a time: their latency, not the two
+// additions of an entry, would be the cost.
+__device__ __forceinline__ void accumulate_body(BodyS& B, const int32_t* __restrict__ list, int n, const ConG* cg,
+                                                int par, bool act, bool with_x, double t) {
+    constexpr int kChunk = 8;
+    const int lane = threadIdx.x & 31, kind = (lane >> 2) & 1, c = lane & 3, cc = c < 3 ? c : 0, base = lane & ~3;
+    double acc = kind ? B.rimp[cc] : B.imp[cc];
+    if (!act) n = 0;
+    for (int k = 0; k < n; k += kChunk) {
+        int e[kChunk];
+        double s1[kChunk], s2[kChunk];
+#pragma unroll
+        for (int q = 0; q < kChunk; q++) e[q] = k + q < n ? list[k + q] : -1;
+#pragma unroll
+        for (int q = 0; q < kChunk; q++) {
+            if (e[q] < 0) continue;
+            const ConG& C = cg[e[q] >> 1];
+            const int role = e[q] & 1;
+            s1[q] = kind ? neg_if(C.rf[par ^ 1][role][cc], true) : neg_if(C.u[cc], role != 0);
+            s2[q] = C.rf[par][role][cc];
+        }
+#pragma unroll
+        for (int q = 0; q < kChunk; q++) {
+            if (e[q] < 0) continue;
+            acc = acc + s1[q];
+            if (kind) acc = acc + s2[q];
+        }
+    }
+    __syncwarp();
+    const double L = B.fL[cc] + acc;  // rimp lanes
+    const double L0 = shfl_d(L, base), L1 = shfl_d(L, base | 1), L2 = shfl_d(L, base | 2);
+    if (act && c < 3) {
+        if (kind) {
+            B.rimp[c] = acc;
+            B.w[c] = (B.ii[3 * c] * L0 + B.ii[3 * c + 1] * L1) + B.ii[3 * c + 2] * L2;
+        } else {
+            B.imp[c] = acc;
+            B.v[c] = B.fv[c] + div_by(acc, B.m, B.rm);
+            if (with_x) B.x[c] = B.fx[c] + div_by(B.ioff[c], B.m, B.rm) * t;
+        }
+    }
+}
+
+// A static body's impulse sum: s plus n deltas in order, one warp; lane c < 3
+// returns component c.  get(k, d) loads delta k.  A zero delta changes
+// nothing but a zero's sign, which no test reads.
+template <class F>
+__device__ __forceinline__ double static_sum(double s, int n, F get) {
+    const int lane = threadIdx.x & 31;
+    for (int b = 0; b < n; b += 32) {
+        double d[3] = {0.0, 0.0, 0.0};
+        if (b + lane < n) get(b + lane, d);
+        unsigned live =
+            __ballot_sync(0xffffffffu, !(m_is_zero(d[0]) && m_is_zero(d[1]) && m_is_zero(d[2])));
+        while (live) {
+            const int k = __ffs(live) - 1;
+            live &= live - 1;
+            const double a = shfl_d(d[0], k), e = shfl_d(d[1], k), f = shfl_d(d[2], k);
+            s = s + (lane == 0 ? a : (lane == 1 ? e : f));
+        }
+    }
+    return s;
 }
 
 #define SYNC()                           \
     do {                                 \
-        if (!solve_sync(S)) {            \
-            if (tid == 0) status[k] = 3; \
+        if (!solve_sync<MODE>(S)) {      \
+            if (tid == 0) a.status[k] = 3; \
             return;                      \
         }                                \
     } while (0)
 
-// One chunk of a wave of the friction loop's ordered accumulation
-// (sequential_impulses.cpp:560-607) with four lanes per contact: lane bits
-// 0-1 pick the component (x, y, z; the fourth lane repeats x and writes
-// nothing), eight contacts per warp.  Each lane evaluates its component of
-// the reference's vector expressions operation for operation; the cross
-// products and norms gather the other components with shuffles.
-// Returns whether a contact of this lane's quad changed an impulse by more
-// than 1e-4 (the loop's convergence test).
-__device__ __forceinline__ bool friction_accumulate4(int base, int end4, const int32_t* __restrict__ widx,
-                                                     int w0, int c0, const SolveArgs& a) {
-    const int lane = threadIdx.x & 31, quad = lane & ~3, c = lane & 3;
-    const int cc = c < 3 ? c : 0;
-    const int c1 = cc == 2 ? 0 : cc + 1, c2 = cc == 0 ? 2 : cc - 1;  // cross: a[c1] b[c2] - a[c2] b[c1]
-    const int qq = base + lane;
-    const bool act = qq < end4;
-    ConWork& C = a.cw[c0 + widx[act ? (qq >> 2) : w0]];
-    BodyWork &A = a.bw[C.a], &B = a.bw[C.b];
-    const bool sa = a.is_static[C.a], sb = a.is_static[C.b];
-    const double cnt = (double)C.pair_cnt;
-    const double* TA = A.T_FS + 4 * cc;
-    const double* TB = B.T_FS + 4 * cc;
-    const double p1A = ((TA[0] * C.local_A[0] + TA[1] * C.local_A[1]) + TA[2] * C.local_A[2]) + TA[3] * 1.0;
-    const double p1B = ((TB[0] * C.local_B[0] + TB[1] * C.local_B[1]) + TB[2] * C.local_B[2]) + TB[3] * 1.0;
-    const double lf = C.upd_total[cc];
-    const double u = m_div_recip(lf - C.last_fi[cc], cnt, C.rcnt);
-    const double ux = shfl_d(u, quad), uy = shfl_d(u, quad | 1), uz = shfl_d(u, quad | 2);
-    const double nu = sqrt((ux * ux + uy * uy) + uz * uz);
-    // rfA = (-lf) x (p1A - xA), rfB = lf x (p1B - xB) (calc_torque with -lf)
-    const double rA = p1A - A.FS[8 + cc], rB = p1B - B.FS[8 + cc];
-    const double nlf = -lf;
-    const double rA1 = shfl_d(rA, quad | c1), rA2 = shfl_d(rA, quad | c2);
-    const double rB1 = shfl_d(rB, quad | c1), rB2 = shfl_d(rB, quad | c2);
-    const double nlf1 = shfl_d(nlf, quad | c1), nlf2 = shfl_d(nlf, quad | c2);
-    const double lf1 = shfl_d(lf, quad | c1), lf2 = shfl_d(lf, quad | c2);
-    const double rfA = nlf1 * rA2 - nlf2 * rA1;
-    const double rfB = lf1 * rB2 - lf2 * rB1;
-    const double uo = m_div_recip(0.0 - 0.0, cnt, C.rcnt);
-    const double uox = shfl_d(uo, quad), uoy = shfl_d(uo, quad | 1), uoz = shfl_d(uo, quad | 2);
-    const double nuo = sqrt((uox * uox + uoy * uoy) + uoz * uoz);
-    // roff: (-uo) x (p1A - xA) for A, uo x (p1B - xB) for B (calc_torque with uo, -uo)
-    const double nuo_ = -uo;
-    const double nuo1 = shfl_d(nuo_, quad | c1), nuo2 = shfl_d(nuo_, quad | c2);
-    const double uo1 = shfl_d(uo, quad | c1), uo2 = shfl_d(uo, quad | c2);
-    const double roA = nuo1 * rA2 - nuo2 * rA1;
-    const double roB = uo1 * rB2 - uo2 * rB1;
-    __syncwarp();
-    if (act && c < 3) {
-        C.last_fi[c] = lf;
-        double sd = 0.0;
-        if (!sa)
-            A.imp[c] = A.imp[c] + u;
-        else
-            sd = u;
-        if (!sb)
-            B.imp[c] = B.imp[c] - u;
-        else
-            sd = -u;
-        if (C.spos >= 0) a.sdelta[3 * (size_t)(c0 + C.spos) + c] = sd;
-        if (!sa) A.rimp[c] = (A.rimp[c] - C.last_rot_A[c]) + rfA;
-        if (!sb) B.rimp[c] = (B.rimp[c] - C.last_rot_B[c]) + rfB;
-        C.last_rot_A[c] = rfA;
-        C.last_rot_B[c] = rfB;
-        if (!sa) A.ioff[c] = A.ioff[c] + uo;
-        if (!sb) B.ioff[c] = B.ioff[c] - uo;
-        if (!sa) A.roff[c] = A.roff[c] + roA;
-        if (!sb) B.roff[c] = B.roff[c] + roB;
-    }
-    return act && (nu > 1e-4 || nuo > 1e-4);
-}
-
-// SequentialImpulses::solve of cluster k.  tid / nt: this thread's index
-// among the cluster's threads and their count; G blocks cooperate (G = 1 for
-// one block), gb is this block's index among them.  In a grid the indices
-// interleave the blocks, so consecutive bodies, contacts and warps of a wave
-// land on different SMs.  shv: three ints shared by those threads.
-__device__ void solve_body(int k, int tid, int nt, int gb, int G, int* shv, const SolveSync& S,
-                           const SolveArgs& a) {
-    const int32_t *cl_part_off = a.cl_part_off, *cl_parts = a.cl_parts, *cl_con_off = a.cl_con_off,
-                  *order = a.order, *pair_cnt = a.pair_cnt, *con_pair = a.con_pair;
-    const double *rec = a.rec, *warm = a.warm, *cl_step = a.cl_step, *mass = a.mass, *ii = a.ii, *mu = a.mu,
-                 *cur = a.cur;
-    const uint8_t* is_static = a.is_static;
-    double* fut = a.fut;
-    const double gravity_z = a.gravity_z;
-    BodyWork* bw = a.bw;
-    ConWork* cw = a.cw;
-    int32_t *wave_idx = a.wave_idx, *wave_off = a.wave_off, *wave_cursor = a.wave_cursor, *scon = a.scon;
-    double* sdelta = a.sdelta;
-    double* static_imp = a.static_imp;
-    int32_t *status = a.status, *iters = a.iters, *out_ab = a.out_ab;
-    double *out_impulse = a.out_impulse, *pair_warm = a.pair_warm;
-    const int p0 = cl_part_off[k], p1 = cl_part_off[k + 1];
-    const int c0 = cl_con_off[k], c1 = cl_con_off[k + 1];
-    const int nc = c1 - c0;
-    const double t = cl_step[k];
-    const double rt = 1.0 / t;  // for m_div_recip
+// SequentialImpulses::solve of cluster k by G blocks of kSolveBlock threads;
+// gb is this block's index among them.  Thread, body and task indices
+// interleave the blocks.
+template <int MODE>
+__device__ void solve_body(int k, int gb, int G, const SolveSync& S, const SolveArgs& a) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    const int tid = (int)threadIdx.x * G + gb, nt = kSolveBlock * G;
+    const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5);
+    const int p0 = a.cl_part_off[k], np = a.cl_part_off[k + 1] - p0;
+    const int c0 = a.cl_con_off[k], nc = a.cl_con_off[k + 1] - c0;
+    const double t = a.cl_step[k];
+    const double rt = 1.0 / t;  // for div_by
     bool ok = true;
+    const int32_t* parts = a.cl_parts + p0;
+    volatile int32_t* fl = S.flags;
+    ConG* cg = a.cg + c0;
+    const int nloc = np > gb ? (np - gb + G - 1) / G : 0;  // bodies of this block
+    const size_t body_bytes = sizeof(BodyS) * (size_t)((np + G - 1) / G);
+    const bool bodies_in = MODE != kSyncGrid && 2 * body_bytes <= (size_t)a.smem;
+    BodyS* bsm = (BodyS*)dyn;
+    BodyS* bgl = a.bs + p0;
+    unsigned char* rest = dyn + (bodies_in ? body_bytes : 0);
+    const size_t rest_bytes = (size_t)a.smem - (bodies_in ? body_bytes : 0);
+    auto body = [&](int p) { return body_at<MODE>(p, bsm, bgl, bodies_in, G); };
+    auto own_body = [&](int s) { return bodies_in ? bsm + s : bgl + (s * G + gb); };
 
-    // ---- contacts in sorted order: local frames, normal mass, failure test (:109-168)
-    if (tid == 0) shv[0] = 0;
-    SYNC();
-    for (int i = tid; i < nc; i += nt) {
-        ConWork& C = cw[c0 + i];
-        const double* h = rec + 14 * (size_t)order[c0 + i];
-        const V3 A = ld3(h), B = ld3(h + 3);
-        C.a = (int)h[11];
-        C.b = (int)h[12];
-        C.pair_cnt = pair_cnt[order[c0 + i]];
-        C.rcnt = 1.0 / (double)C.pair_cnt;
-        C.start_dist = norm(A - B);
-        if (C.start_dist < 1e-6 && t > 1e-4) atomicExch(&shv[0], 1);
-        double T[16], Ti[16];
-        const State fa = load_state(fut + 14 * (size_t)C.a), fb = load_state(fut + 14 * (size_t)C.b);
-        transformation(fa.q, fa.x, T);
-        mat_inverse(T, Ti);
-        st3(C.local_A, xform_general(A, Ti));
-        transformation(fb.q, fb.x, T);
-        mat_inverse(T, Ti);
-        st3(C.local_B, xform_general(B, Ti));
-        const V3 gn = (B - A) / 2.0;
-        st3(C.n, normalized(gn));
-        const V3 rnA = cross(A - fa.x, gn), rnB = cross(B - fb.x, gn);
-        double kn = 0.0;
-        if (!is_static[C.a]) kn += 1.0 / mass[C.a] + quad_form(rnA, ii + 9 * (size_t)C.a);
-        if (!is_static[C.b]) kn += 1.0 / mass[C.b] + quad_form(rnB, ii + 9 * (size_t)C.b);
-        C.mass_eff = kn < 1e-6 ? 0.0 : 1.0 / kn;
-        C.outer = (h[6] + h[7]) * 0.25;
-        // the normal loop's slop and damp * m (sequential_impulses.cpp:
-        // 260-287) depend on the contact alone
-        C.slop = lerp1(dmax(C.outer * 0.2, C.outer - C.start_dist), C.outer * 0.2, 0.3);
-        C.damp_m = 0.1 * C.mass_eff;
-        C.impulse = warm[order[c0 + i]] == warm[order[c0 + i]] ? warm[order[c0 + i]] * 0.75 : 0.0;
-        C.impulse_offset = 0.0;
-        for (int q = 0; q < 3; q++) C.last_fi[q] = C.last_rot_A[q] = C.last_rot_B[q] = 0.0;
+    // ---- bodies (:178-188), the inverse transforms on the first half of the
+    // block's warps, the integrated orientation on the second
+    if (MODE == kSyncBlock) {
+        if (threadIdx.x < kFlags) S.flags[threadIdx.x] = 0;
+        __syncthreads();
+    }
+    for (int s = threadIdx.x & (kSolveBlock / 2 - 1); s < nloc; s += kSolveBlock / 2) {
+        const int p = s * G + gb, g = parts[p];
+        const double* F = a.fut + 14 * (size_t)g;
+        BodyG& W = a.bg[p0 + p];
+        const bool st = a.is_static[g] != 0;
+        const State f = load_state(F);
+        if (threadIdx.x < kSolveBlock / 2) {
+            double T[16];
+            transformation(f.q, f.x, T);
+            mat_inverse(T, W.Ti);
+            for (int r = 0; r < 3; r++)
+                for (int q = 0; q < 3; q++) W.R0[3 * r + q] = T[4 * r + q];
+            a.deg[p0 + p] = 0;
+            if (st)
+                a.statics[p0 + atomicAdd(S.flags + kFlStatics, 1)] = p;
+            else
+                a.slot[g] = p;
+        } else {
+            BodyS& B = *own_body(s);
+            const double m = a.mass[g];
+            const double* ii = a.ii + 9 * (size_t)g;
+            B.m = m;
+            B.rm = 1.0 / m;
+            B.is_static = st ? 1 : 0;
+            B.rbad = 0;
+            for (int q = 0; q < 9; q++) B.ii[q] = ii[q];
+            st3(B.fx, f.x);
+            st3(B.fv, f.v);
+            st3(B.fL, f.L);
+            st3(B.x, f.x);
+            st3(B.v, f.v);
+            st3(B.w, m3_vec(ii, f.L));
+            st3(B.imp, mk(m * 0.0, m * 0.0, m * a.gravity_z) * t);
+            for (int q = 0; q < 3; q++) B.rimp[q] = B.ioff[q] = 0.0;
+            Quat q = f.q;
+            if (!st) {
+                double Iinv[9];
+                world_inv_inertia(f.q, ii, Iinv);
+                const V3 omega = m3_vec(Iinv, f.L + t * mk(0.0, 0.0, 0.0));  // roff = 0
+                q = qmul(qexp((0.5 * omega) * t), f.q);
+            }
+            W.q[0] = q.w;
+            W.q[1] = q.x;
+            W.q[2] = q.y;
+            W.q[3] = q.z;
+            qmat(q, W.R);
+        }
     }
     SYNC();
-    if (((volatile int*)shv)[0]) {
-        if (tid == 0) status[k] = 1;
+    const int n_static = fl[kFlStatics];
+    // ---- contacts in sorted order: local frames, normal mass, failure test
+    // (:109-168) and warm-start impulses (:193-215), two lanes per contact
+    for (int b2 = 32 * (warp * G + gb); b2 < 2 * nc; b2 += nt) {
+        const int i = (b2 + lane) >> 1, side = lane & 1;
+        const bool act = i < nc;
+        double term = 0.0;
+        int p = 0;
+        bool st = false;
+        V3 gn = mk(0, 0, 0), A = gn, Bp = gn;
+        const double* h = nullptr;
+        int oi = 0, g = 0;
+        if (act) {
+            ConG& C = cg[i];
+            oi = a.order[c0 + i];
+            h = a.rec + 14 * (size_t)oi;
+            A = ld3(h);
+            Bp = ld3(h + 3);
+            g = (int)h[11 + side];
+            st = a.is_static[g] != 0;
+            if (st) {
+                for (int q = 0; q < n_static; q++) {
+                    const int cand = a.statics[p0 + q];
+                    if (parts[cand] == g) {
+                        p = cand;
+                        break;
+                    }
+                }
+            } else {
+                p = a.slot[g];
+            }
+            const BodyG& W = a.bg[p0 + p];
+            const double* F = a.fut + 14 * (size_t)g;
+            const V3 P = side ? Bp : A, fx = ld3(F + 8);
+            const V3 loc = xform_general(P, W.Ti);
+            st3(C.local[side], loc);
+            const V3 rF = P - fx;
+            st3(C.rF[side], rF);
+            gn = (Bp - A) / 2.0;
+            const V3 rn = cross(rF, gn);
+            term = 1.0 / a.mass[g] + quad_form(rn, a.ii + 9 * (size_t)g);
+            const double wv = a.warm[oi];
+            const double impulse = wv == wv ? wv * 0.75 : 0.0;
+            const V3 n = normalized(gn);
+            const V3 u = (-n) * impulse;
+            // p1 = T_FS local with the input future state's transform
+            const V3 p1 = mk(((W.R0[0] * loc.x + W.R0[1] * loc.y) + W.R0[2] * loc.z) + fx.x * 1.0,
+                             ((W.R0[3] * loc.x + W.R0[4] * loc.y) + W.R0[5] * loc.z) + fx.y * 1.0,
+                             ((W.R0[6] * loc.x + W.R0[7] * loc.y) + W.R0[8] * loc.z) + fx.z * 1.0);
+            st3(C.rf[0][side], calc_torque(side ? -u : u, p1, fx));
+            for (int q = 0; q < 3; q++) C.rf[1][side][q] = 0.0;
+            a.prev[2 * (c0 + i) + side] = -1;
+            if (side == 0) {
+                st3(C.u, u);
+                st3(C.n, n);
+                C.impulse = impulse;
+                for (int q = 0; q < 3; q++) C.lf[q] = 0.0;
+                const int cnt = a.pair_cnt[oi];
+                C.cnt = (double)cnt;
+                C.rcnt = 1.0 / (double)cnt;
+                C.outer = (h[6] + h[7]) * 0.25;
+                // the normal loop's slop and damp * m (:260-287) depend on the contact alone
+                const double start_dist = norm(A - Bp);
+                if (start_dist < 1e-6 && t > 1e-4) atomicExch(S.flags + kFlFail, 1);
+                C.slop = lerp1(dmax(C.outer * 0.2, C.outer - start_dist), C.outer * 0.2, 0.3);
+            }
+        }
+        const double tB = shfl_d(term, lane | 1);
+        const int pB = __shfl_sync(0xffffffffu, p, lane | 1), gB = __shfl_sync(0xffffffffu, g, lane | 1);
+        const bool sB = __shfl_sync(0xffffffffu, st ? 1 : 0, lane | 1) != 0;
+        if (act && side == 0) {
+            ConG& C = cg[i];
+            double kn = 0.0;
+            if (!st) kn += term;
+            if (!sB) kn += tB;
+            C.mass_eff = kn < 1e-6 ? 0.0 : 1.0 / kn;
+            C.damp_m = 0.1 * C.mass_eff;
+            C.mu = dmin(a.mu[g], a.mu[gB]);
+            C.a = p;
+            C.b = pB;
+            a.ab[c0 + i] = make_int2(p | (st ? kStaticBit : 0), pB | (sB ? kStaticBit : 0));
+            // lists: a moving body has every contact that names it, a static one
+            // those of which it is a, or b beside a moving a
+            atomicAdd(a.deg + p0 + p, 1);
+            if ((!sB && pB != p) || (sB && !st)) atomicAdd(a.deg + p0 + pB, 1);
+        }
+    }
+    SYNC();
+    if (fl[kFlFail]) {
+        if (tid == 0) a.status[k] = 1;
         return;
     }
-    // ---- bodies: gravity impulse, states (:178-188)
-    for (int i = p0 + tid; i < p1; i += nt) {
-        const int g = cl_parts[i];
-        BodyWork& W = bw[g];
-        const double m = mass[g];
-        W.rmass = 1.0 / m;
-        const V3 f = mk(m * 0.0, m * 0.0, m * gravity_z);
-        st3(W.imp, f * t);
-        for (int q = 0; q < 3; q++) W.rimp[q] = W.ioff[q] = W.roff[q] = 0.0;
-        for (int q = 0; q < 14; q++) W.FS[q] = W.FSf[q] = fut[14 * (size_t)g + q];
-        const State fs = load_state(fut + 14 * (size_t)g);
-        rigid12(fs, W.T_FS);
-        rigid12(fs, W.T_FSf);
-        rigid12(load_state(cur + 14 * (size_t)g), W.T_cur);
-        world_inv_inertia(fs.q, ii + 9 * (size_t)g, W.Iinv);
-        W.last_level = -1;
-        if (is_static[g]) st3(static_imp + 3 * (size_t)i, f * t);
+    // ---- every body's contacts in sorted order, a warp per body: a warp reads
+    // all of the cluster's contacts (a few thousand coalesced 8-byte loads),
+    // which needs neither a sort nor an order of arrival
+    for (int p = warp * G + gb; p < np; p += (kSolveBlock / 32) * G) {
+        const int n = a.deg[p0 + p];
+        int base = 0;
+        if (lane == 0) base = atomicAdd(S.flags + kFlCursor, n);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (lane == 0) a.boff[p0 + p] = base;
+        const bool st = a.is_static[parts[p]] != 0;
+        int cnt = 0, carry = -1;
+        for (int b = 0; b < nc && cnt < n; b += 32) {
+            const int i = b + lane;
+            const int2 q = i < nc ? a.ab[c0 + i] : make_int2(-1, -1);
+            const bool isa = i < nc && (q.x & ~kStaticBit) == p, isb = i < nc && (q.y & ~kStaticBit) == p;
+            const bool in = st ? isa || (isb && !(q.x & kStaticBit)) : isa || isb;
+            const unsigned m = __ballot_sync(0xffffffffu, in), low = m & ((1u << lane) - 1u);
+            if (in) {
+                const int role = isa ? 0 : 1, at = base + cnt + __popc(low);
+                a.blist[2 * c0 + at] = 2 * i + role;
+                a.lpos[2 * (c0 + i) + role] = at;
+                if (!st) a.prev[2 * (c0 + i) + role] = low ? b + 31 - __clz(low) : carry;
+            }
+            if (m) carry = b + 31 - __clz(m);
+            cnt += __popc(m);
+        }
     }
     SYNC();
-    // ---- wave schedule (sequential, integer work only)
-    if (tid == 0) {
-        int levels = 0;
-        for (int i = 0; i < nc; i++) {
-            ConWork& C = cw[c0 + i];
-            int lv = 0;
-            if (!is_static[C.a]) lv = max(lv, bw[C.a].last_level + 1);
-            if (!is_static[C.b]) lv = max(lv, bw[C.b].last_level + 1);
-            C.level = lv;
-            if (!is_static[C.a]) bw[C.a].last_level = lv;
-            if (!is_static[C.b]) bw[C.b].last_level = lv;
-            levels = max(levels, lv + 1);
-        }
-        for (int l = 0; l <= levels; l++) wave_off[c0 + k + l] = 0;
-        for (int i = 0; i < nc; i++) wave_off[c0 + k + cw[c0 + i].level + 1]++;
-        for (int l = 0; l < levels; l++) wave_off[c0 + k + l + 1] += wave_off[c0 + k + l];
-        // stable scatter: contacts of each wave in sorted order
-        int32_t* cursor = wave_cursor + c0 + k;
-        for (int l = 0; l < levels; l++) cursor[l] = wave_off[c0 + k + l];
-        for (int i = 0; i < nc; i++) wave_idx[c0 + cursor[cw[c0 + i].level]++] = i;
-        // the contacts touching a static body, in sorted order, for its impulse
-        // sums: each writes its delta at its position, scon holds the body
-        int ns = 0;
-        for (int i = 0; i < nc; i++) {
-            ConWork& C = cw[c0 + i];
-            const bool sa = is_static[C.a], sb = is_static[C.b];
-            C.spos = (sa || sb) ? ns : -1;
-            if (sa || sb) scon[c0 + ns++] = sa ? C.a : C.b;
-        }
-        shv[1] = levels;
-        shv[2] = ns;
-    }
-    SYNC();
-    const int levels = ((volatile int*)shv)[1];
-    const int n_scon = ((volatile int*)shv)[2];
-    const int* woff = wave_off + c0 + k;
-    const int* widx = wave_idx + c0;
-
-    // Static impulse sums: add the contacts' deltas in sorted order.
-    auto static_sum = [&]() {
-        for (int i = p0 + tid; i < p1; i += nt) {
-            const int g = cl_parts[i];
-            if (!is_static[g]) continue;
-            V3 s = ld3(static_imp + 3 * (size_t)i);
-            for (int q = 0; q < n_scon; q++)
-                if (scon[c0 + q] == g) s = s + ld3(sdelta + 3 * (size_t)(c0 + q));
-            st3(static_imp + 3 * (size_t)i, s);
+    // ---- the warm-start sums of every body, then updateState
+    auto accumulate = [&](int par, bool with_x) {
+        const int grp = (int)threadIdx.x >> 3;
+        for (int s0 = 0; s0 < nloc; s0 += kSolveBlock / 8) {
+            if (s0 + (warp << 2) >= nloc) break;  // uniform per warp
+            const int s = s0 + grp;
+            const bool in = s < nloc;
+            BodyS& B = *own_body(in ? s : s0 + (warp << 2));
+            const int p = in ? s * G + gb : gb;
+            accumulate_body(B, a.blist + 2 * (size_t)c0 + a.boff[p0 + p], a.deg[p0 + p], cg, par,
+                            in && !B.is_static, with_x, t);
         }
     };
-
-    // ---- warm-start impulses (:193-215), in waves
-    for (int l = 0; l < levels; l++) {
-        for (int q = woff[l] + tid; q < woff[l + 1]; q += nt) {
-            ConWork& C = cw[c0 + widx[q]];
-            BodyWork &A = bw[C.a], &B = bw[C.b];
-            const V3 n = ld3(C.n);
-            const V3 p1A = xf12(ld3(C.local_A), A.T_FS), p1B = xf12(ld3(C.local_B), B.T_FS);
-            const V3 u = (-n) * C.impulse;
-            V3 sd = mk(0, 0, 0);
-            if (!is_static[C.a]) {
-                st3(A.imp, ld3(A.imp) + u);
-                st3(A.rimp, ld3(A.rimp) + calc_torque(u, p1A, ld3(A.FS + 8)));
-            } else {
-                sd = u;
+    accumulate(0, true);
+    for (int q = gb; q < n_static; q += G) {  // static bodies' running sums, by their block's first warp
+        const int p = a.statics[p0 + q];
+        if (warp != 0) continue;
+        double* imp = body(p)->imp;
+        const int32_t* list = a.blist + 2 * (size_t)c0 + a.boff[p0 + p];
+        const double s = static_sum(lane < 3 ? imp[lane] : 0.0, a.deg[p0 + p], [&](int j, double* d) {
+            const int i = list[j] >> 1;
+            const bool neg = (a.ab[c0 + i].y & kStaticBit) != 0;  // -u on a static b
+            for (int e = 0; e < 3; e++) d[e] = neg_if(cg[i].u[e], neg);
+        });
+        if (lane < 3) imp[lane] = s;
+    }
+    // ---- wave schedule, by the first block: round l takes the contacts whose
+    // predecessors on both moving bodies lie in earlier rounds; a wave's
+    // contacts are dealt to tasks of four
+    if (gb == 0 && nc > 0) {
+        __shared__ int s_cnt;
+        const bool in = 12 * (size_t)nc <= rest_bytes;
+        int32_t* lv = in ? (int32_t*)rest : a.level + c0;
+        const int32_t* pv = in ? (int32_t*)rest + nc : a.prev + 2 * (size_t)c0;
+        for (int i = threadIdx.x; i < nc; i += kSolveBlock) {
+            lv[i] = -1;
+            if (in) {
+                ((int32_t*)rest)[nc + 2 * i] = a.prev[2 * (c0 + i)];
+                ((int32_t*)rest)[nc + 2 * i + 1] = a.prev[2 * (c0 + i) + 1];
             }
-            if (!is_static[C.b]) {
-                st3(B.imp, ld3(B.imp) - u);
-                st3(B.rimp, ld3(B.rimp) + calc_torque(-u, p1B, ld3(B.FS + 8)));
-            } else {
-                sd = -u;
-            }
-            if (C.spos >= 0) st3(sdelta + 3 * (size_t)(c0 + C.spos), sd);
         }
-        SYNC();
+        int total = 0, l = 0, T = 0;
+        volatile int32_t* vlv = lv;
+        while (total < nc) {
+            if (threadIdx.x == 0) s_cnt = 0;
+            __syncthreads();
+            for (int i = threadIdx.x; i < nc; i += kSolveBlock) {
+                if (vlv[i] >= 0) continue;
+                const int pa = pv[2 * i], pb = pv[2 * i + 1];
+                const int la = pa < 0 ? -2 : vlv[pa], lb = pb < 0 ? -2 : vlv[pb];
+                if (la == -1 || la >= l || lb == -1 || lb >= l) continue;
+                vlv[i] = l;
+                a.tcon[4 * (size_t)(c0 + T) + atomicAdd(&s_cnt, 1)] = i;
+            }
+            __syncthreads();
+            const int w = s_cnt, tasks = (w + 3) >> 2;
+            if (w == 0) break;  // (every round takes at least the first contact left)
+            if (threadIdx.x < 4 && w + (int)threadIdx.x < 4 * tasks)
+                a.tcon[4 * (size_t)(c0 + T) + w + threadIdx.x] = -1;
+            if (threadIdx.x == 0) a.tl[c0 + k + l] = T;
+            T += tasks;
+            total += w;
+            l++;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            a.tl[c0 + k + l] = T;
+            fl[kFlLevels] = l;
+            fl[kFlTasks] = T;
+        }
     }
-    static_sum();
     SYNC();
-    for (int k2 = tid; k2 < 2 * (p1 - p0); k2 += nt) {  // two lanes per body: FS, FSf
-        const int g = cl_parts[p0 + (k2 >> 1)];
-        if (!is_static[g]) integrate_one(bw[g], fut + 14 * (size_t)g, mass[g], t, k2 & 1);
-    }
-    SYNC();
-
     int it_n = 0, it_f = 0;
     if (nc > 0) {
-        // ---- normal loop (:230-395)
-        bool converged = false;
+        const int levels = fl[kFlLevels], tasks = fl[kFlTasks];
+        const int32_t* tl = a.tl + c0 + k;
+        const bool cons_in = sizeof(ConS) * 4 * (size_t)((tasks + G - 1) / G) <= rest_bytes;
+        ConS* cs = cons_in ? (ConS*)rest : a.cs + 4 * (size_t)c0;
+        // place of task gt's first contact: tasks gb, gb + G, ... are this block's
+        auto place = [&](int gt) { return cons_in ? 4 * (gt / G) : 4 * gt; };
+        const int n_tasks = tasks > gb ? (tasks - gb + G - 1) / G : 0;
+        for (int s = threadIdx.x; s < 8 * n_tasks; s += kSolveBlock) {
+            const int gt = (s >> 3) * G + gb, q = (s >> 1) & 3, side = s & 1;
+            const int i = a.tcon[4 * (size_t)c0 + 4 * (size_t)gt + q];
+            ConS& C = cs[place(gt) + q];
+            if (side == 0) C.ci = i;
+            if (i < 0) continue;
+            ConG& g = cg[i];
+            const int2 ab = a.ab[c0 + i];
+            const int pw = side ? ab.y : ab.x, p = pw & ~kStaticBit;
+            const double* R = a.bg[p0 + p].R;
+            const double lx = g.local[side][0], ly = g.local[side][1], lz = g.local[side][2];
+            for (int r = 0; r < 3; r++) {
+                const double v = (R[3 * r] * lx + R[3 * r + 1] * ly) + R[3 * r + 2] * lz;
+                C.rl[side][r] = v;
+                g.rl[side][r] = v;
+            }
+            C.body[side] = body(p);
+            if (side == 0) {
+                for (int r = 0; r < 3; r++) C.n[r] = g.n[r];
+                C.imp = g.impulse;
+                C.off = 0.0;
+                C.outer = g.outer;
+                C.m = g.mass_eff;
+                C.slop = g.slop;
+                C.damp_m = g.damp_m;
+                const bool sa = (ab.x & kStaticBit) != 0, sb = (ab.y & kStaticBit) != 0;
+                C.sd = sa || sb ? a.sdelta + 3 * (2 * (size_t)c0 + a.lpos[2 * (c0 + i) + (sa ? 0 : 1)]) : nullptr;
+                C.sneg = sa ? 0 : 1;
+                C.near_ = 0;
+            }
+        }
         // every iteration compares the moving bodies' impulses with their values
         // at its start (kept in last_imp, refreshed by the convergence test);
-        // static bodies keep their running sums in static_imp
-        for (int i = p0 + tid; i < p1; i += nt) {
-            const int g = cl_parts[i];
-            if (!is_static[g])
-                for (int q = 0; q < 3; q++) bw[g].last_imp[q] = bw[g].imp[q];
+        // static bodies keep their running sums
+        for (int s = threadIdx.x; s < nloc; s += kSolveBlock) {
+            BodyS& B = *own_body(s);
+            for (int q = 0; q < 3; q++) B.last_imp[q] = B.imp[q];
         }
         SYNC();
-        // Narrow waves (a warp of two contacts per SM sub-partition) take
-        // sixteen lanes per contact, wider ones four.  The next wave's bounds
-        // and first sixteen-lane task are loaded before each barrier.
-        auto lanes16 = [&](int w0, int w1) { return a.lanes == 16 || (a.lanes == 0 && (w1 - w0 + 1) / 2 <= 4 * G); };
-        int n0 = woff[0], n1 = woff[1];
-        int2 pre = lanes16(n0, n1) ? wave16_first(n0, n1, widx, c0, G, gb, a) : make_int2(-1, -1);
+        // ---- normal loop (:230-395).  Warps 0, 1, 4, 5 take velocity halves,
+        // 2, 3, 6, 7 position halves: a block's first two tasks put one warp
+        // on each sub-partition.
+        const bool vel = (warp & 2) == 0;
+        const int rank = (warp & 1) | ((warp >> 1) & 2);
+        const int grp = lane >> 3, side = (lane >> 2) & 1, c = lane & 3;
+        bool converged = false;
         while (!converged && it_n < 1000) {
-            for (int l = 0; l < levels; l++) {
-                const int w0 = n0, w1 = n1;
-                const int ln = l + 1 < levels ? l + 1 : 0;
-                n0 = woff[ln];
-                n1 = woff[ln + 1];
-                if (lanes16(w0, w1)) {
-                    // the next wave's first task, loaded while this wave computes
-                    const int2 pre_next =
-                        lanes16(n0, n1) ? wave16_first(n0, n1, widx, c0, G, gb, a) : make_int2(-1, -1);
-                    normal_wave16(w0, w1, widx, c0, G, gb, t, rt, pre, a);
-                    pre = pre_next;
-                    SYNC();
-                    continue;
+            int t0 = 0, t1 = tl[0], t2 = tl[1];
+            for (int j = 0; j <= levels; j++) {
+                // position halves of wave j [t1, t2), velocity halves of wave j - 1 [t0, t1)
+                const int lo = vel ? t0 : t1, hi = vel ? t1 : t2;
+                const int t3 = j + 2 <= levels ? tl[j + 2] : t2;
+                int gt = lo + (gb - lo % G + G) % G + rank * G;
+                for (; gt < hi; gt += 4 * G) {
+                    ConS* C = cs + place(gt);
+                    const bool act = C[grp].ci >= 0;
+                    ConS& Cg = C[act ? grp : 0];
+                    if (vel)
+                        velocity_half(Cg, act, side, c);
+                    else
+                        position_half(Cg, act, side, c, t, rt);
                 }
-                // Four lanes per contact, one warp instruction stream: lane bit 0
-                // picks the body side (A, B), bit 1 the integrated state (FS,
-                // FSf).  FP64 latency, not lane count, bounds a wave, so the
-                // sides and the four integrations run side by side.
-                const int end4 = 4 * w1;
-                const int wslot = (int)(threadIdx.x >> 5) * G + gb, nwarps = (int)(blockDim.x >> 5) * G;
-                for (int base = 4 * w0 + 32 * wslot; base < end4; base += 32 * nwarps) {
-                    const int lane = threadIdx.x & 31, quad = lane & ~3, side = lane & 1, variant = (lane >> 1) & 1;
-                    const int qq = base + lane;
-                    const bool act = qq < end4;
-                    ConWork& C = cw[c0 + widx[act ? (qq >> 2) : w0]];
-                    const int g = side ? C.b : C.a;
-                    BodyWork& W = bw[g];
-                    const bool st = is_static[g];
-                    // this side's contact point and its velocity (State::pointVelocity)
-                    const V3 p1 = xf12(ld3(side ? C.local_B : C.local_A), W.T_FS);
-                    const V3 x = ld3(W.FS + 8);
-                    const V3 v1s = ld3(W.FS + 11) + cross(m3_vec(ii + 9 * (size_t)g, ld3(W.FS + 5)), p1 - x);
-                    const V3 p1A = shfl3(p1, quad), p1B = shfl3(p1, quad + 1);
-                    const V3 v1A = shfl3(v1s, quad), v1B = shfl3(v1s, quad + 1);
-                    const bool sa = is_static[C.a];
-                    const V3 n = ld3(C.n);
-                    const double outer = C.outer;
-                    const double d1 = dot(p1B, n) - dot(p1A, n);
-                    const double v1 = dot(v1A, n) - dot(v1B, n);
-                    const double m = C.mass_eff;
-                    const double damp = 0.1;
-                    const double imp0 = C.impulse, off0 = C.impulse_offset;
-                    const double dimp = d1 < outer ? (v1 * m) * damp : -imp0;
-                    const double imp1 = dmax(imp0 + dimp, 0.0);
-                    const V3 u = (-n) * (imp1 - imp0);
-                    const double pen = outer - d1;
-                    const double doff = d1 < outer ? m_div_recip(C.damp_m * dmax(0.0, pen - C.slop), t, rt) : -off0;
-                    const double off1 = dmax(off0 + doff, 0.0);
-                    const V3 uo = (-n) * (off1 - off0);
-                    __syncwarp();
-                    if (act && variant == 0) {
-                        if (!st) {  // imp[b] - u is imp[b] + (-u) in IEEE arithmetic
-                            const V3 us = side ? -u : u;
-                            st3(W.imp, ld3(W.imp) + us);
-                            st3(W.rimp, ld3(W.rimp) + calc_torque(us, p1, x));
-                            st3(W.ioff, ld3(W.ioff) + (side ? -uo : uo));
-                        }
-                        if (side == 0) {
-                            C.impulse = imp1;
-                            C.impulse_offset = off1;
-                            if (C.spos >= 0) st3(sdelta + 3 * (size_t)(c0 + C.spos), sa ? u : -u);
-                        }
-                    }
-                    __syncwarp();
-                    if (act && !st) integrate_one(W, fut + 14 * (size_t)g, mass[g], t, variant);
-                }
-                pre = lanes16(n0, n1) ? wave16_first(n0, n1, widx, c0, G, gb, a) : make_int2(-1, -1);
+                t0 = t1;
+                t1 = t2;
+                t2 = t3;
                 SYNC();
             }
             // convergence over every particle of the cluster (:380-387)
             bool moved = false;
-            for (int i = p0 + tid; i < p1; i += nt) {
-                const int g = cl_parts[i];
-                if (is_static[g]) {
-                    const V3 before = ld3(static_imp + 3 * (size_t)i);
-                    V3 s = before;
-                    for (int q = 0; q < n_scon; q++)
-                        if (scon[c0 + q] == g) s = s + ld3(sdelta + 3 * (size_t)(c0 + q));
-                    st3(static_imp + 3 * (size_t)i, s);
-                    if (norm(s - before) > 1e-6) moved = true;
-                } else {
-                    const V3 now = ld3(bw[g].imp);
-                    if (norm(now - ld3(bw[g].last_imp)) > 1e-6) moved = true;
-                    st3(bw[g].last_imp, now);
-                }
+            for (int s = threadIdx.x; s < nloc; s += kSolveBlock) {
+                BodyS& B = *own_body(s);
+                if (B.is_static) continue;
+                const V3 now = ld3(B.imp), d = now - ld3(B.last_imp);
+                moved = moved || sq_above(dot(d, d), kSqMax1e6);
+                st3(B.last_imp, now);
             }
-            converged = !solve_any(S, moved, it_n & 1, gb, &ok);
+            for (int q = gb; q < n_static; q += G) {
+                const int p = a.statics[p0 + q];
+                if (warp != kSolveBlock / 32 - 1) continue;
+                double* imp = body(p)->imp;
+                const double* sd = a.sdelta + 3 * (2 * (size_t)c0 + a.boff[p0 + p]);
+                const double before = lane < 3 ? imp[lane] : 0.0;
+                const double s = static_sum(before, a.deg[p0 + p], [&](int j, double* d) {
+                    for (int e = 0; e < 3; e++) d[e] = sd[3 * (size_t)j + e];
+                });
+                const double d = s - before, d2 = d * d;
+                const double sq = (shfl_d(d2, 0) + shfl_d(d2, 1)) + shfl_d(d2, 2);
+                moved = moved || sq_above(sq, kSqMax1e6);
+                if (lane < 3) imp[lane] = s;
+            }
+            converged = !solve_any<MODE>(S, moved, it_n & 1, gb, &ok);
             if (!ok) {
-                if (tid == 0) status[k] = 3;
+                if (tid == 0) a.status[k] = 3;
                 return;
             }
             it_n++;
         }
-        // ---- friction loop (:397-607)
+        for (int s = threadIdx.x; s < 4 * n_tasks; s += kSolveBlock) {
+            const ConS& C = cs[place((s >> 2) * G + gb) + (s & 3)];
+            if (C.ci >= 0) cg[C.ci].impulse = C.imp;
+        }
+        SYNC();
+        // ---- friction loop (:397-607): every contact's update reads the state
+        // at the iteration's start, then each body adds its own in sorted order
         converged = false;
         while (!converged && it_f < 100) {
-            for (int i = tid; i < nc; i += nt) {  // pass 1: every contact reads, none writes bodies
-                ConWork& C = cw[c0 + i];
-                const BodyWork &A = bw[C.a], &B = bw[C.b];
-                const bool sa = is_static[C.a], sb = is_static[C.b];
-                const double* h = rec + 14 * (size_t)order[c0 + i];
-                const V3 n = ld3(C.n);
-                const V3 p1A = xf12(ld3(C.local_A), A.T_FS), p1B = xf12(ld3(C.local_B), B.T_FS);
-                const V3 v1A = sa ? mk(0, 0, 0)
-                                  : ld3(A.FS + 11) + cross(m3_vec(ii + 9 * (size_t)C.a, ld3(A.FS + 5)), p1A - ld3(A.FS + 8));
-                const V3 v1B = sb ? mk(0, 0, 0)
-                                  : ld3(B.FS + 11) + cross(m3_vec(ii + 9 * (size_t)C.b, ld3(B.FS + 5)), p1B - ld3(B.FS + 8));
-                const V3 lpA = xf12(ld3(C.local_A), A.T_cur), fpA = xf12(ld3(C.local_A), A.T_FSf);
-                const V3 vdA = (fpA - lpA) / t;
-                const V3 lpB = xf12(ld3(C.local_B), B.T_cur), fpB = xf12(ld3(C.local_B), B.T_FSf);
-                const V3 vdB = (fpB - lpB) / t;
+            bool big = false;
+            const int par = it_f & 1;
+            for (int i = tid; i < nc; i += nt) {
+                ConG& C = cg[i];
+                BodyS &A = *body(C.a), &B = *body(C.b);
+                const bool sa = A.is_static != 0, sb = B.is_static != 0;
+                const V3 n = ld3(C.n), xA = ld3(A.x), xB = ld3(B.x);
+                V3 lA = ld3(C.rl[0]), lB = ld3(C.rl[1]);
+                // a lever arm that is not finite makes the body's roff, and so its
+                // rotation, NaN from the next iteration on
+                const double nan = __longlong_as_double(0x7ff8000000000000ll);
+                if (A.rbad && A.rbad <= it_f) lA = mk(nan, nan, nan);
+                if (B.rbad && B.rbad <= it_f) lB = mk(nan, nan, nan);
+                const V3 rA = (lA + xA) - xA, rB = (lB + xB) - xB;
+                auto bad = [](V3 r) {
+                    return m_exp_field(r.x) == 2047 || m_exp_field(r.y) == 2047 || m_exp_field(r.z) == 2047;
+                };
+                if (!sa && bad(rA) && !A.rbad) A.rbad = it_f + 1;
+                if (!sb && bad(rB) && !B.rbad) B.rbad = it_f + 1;
+                const V3 v1A = sa ? mk(0, 0, 0) : ld3(A.v) + cross(ld3(A.w), rA);
+                const V3 v1B = sb ? mk(0, 0, 0) : ld3(B.v) + cross(ld3(B.w), rB);
                 const V3 vAB = v1A - v1B;
-                const V3 vABd = vdA - vdB;
                 const V3 vt = vAB - dot(vAB, n) * n;
-                (void)vABd;
-                const double mu_ = dmin(mu[C.a], mu[C.b]);
-                const double max_force = (C.impulse * mu_) * 10;
-                const V3 rA = ld3(h) - ld3(fut + 14 * (size_t)C.a + 8);
-                const V3 rB = ld3(h + 3) - ld3(fut + 14 * (size_t)C.b + 8);
+                const double max_force = (C.impulse * C.mu) * 10;
                 const V3 tan = normalized(vt);
                 double kt = 0.0;
-                if (!sa) kt += A.rmass + quad_form(cross(rA, tan), ii + 9 * (size_t)C.a);  // 1.0 / mass
-                if (!sb) kt += B.rmass + quad_form(cross(rB, tan), ii + 9 * (size_t)C.b);
+                if (!sa) kt += A.rm + quad_form(cross(ld3(C.rF[0]), tan), A.ii);
+                if (!sb) kt += B.rm + quad_form(cross(ld3(C.rF[1]), tan), B.ii);
                 const double mit = kt < 1e-6 ? 0.0 : 1.0 / kt;
                 const V3 dfi = ((-vt) * mit) * 0.9;
-                V3 total = ld3(C.last_fi) + dfi;
+                const V3 last = ld3(C.lf);
+                V3 total = last + dfi;
                 total = normalized(total) * dclamp(norm(total), 0.0, max_force);
-                st3(C.upd_total, total);
+                st3(C.lf, total);
+                const V3 d = total - last;
+                const V3 u = mk(div_by(d.x, C.cnt, C.rcnt), div_by(d.y, C.cnt, C.rcnt), div_by(d.z, C.cnt, C.rcnt));
+                st3(C.u, u);
+                big = big || sq_above(dot(u, u), kSqMax1e4);
+                st3(C.rf[par][0], cross(-total, rA));
+                st3(C.rf[par][1], cross(total, rB));
             }
             SYNC();
-            bool big = false;
-            for (int l = 0; l < levels; l++) {  // pass 2: ordered accumulation, wave by wave
-                const int end4 = 4 * woff[l + 1];
-                const int wslot = (int)(threadIdx.x >> 5) * G + gb, nwarps = (int)(blockDim.x >> 5) * G;
-                for (int base = 4 * woff[l] + 32 * wslot; base < end4; base += 32 * nwarps)
-                    big = friction_accumulate4(base, end4, widx, woff[l], c0, a) || big;
-                SYNC();
-            }
+            accumulate(par, false);
             // (the static bodies' impulse sums are read only by the normal loop's test)
-            for (int k2 = tid; k2 < 2 * (p1 - p0); k2 += nt) {  // two lanes per body: FS, FSf
-                const int g = cl_parts[p0 + (k2 >> 1)];
-                if (!is_static[g]) integrate_one(bw[g], fut + 14 * (size_t)g, mass[g], t, k2 & 1);
-            }
-            converged = !solve_any(S, big, (it_n + it_f) & 1, gb, &ok);
+            converged = !solve_any<MODE>(S, big, (it_n + it_f) & 1, gb, &ok);
             if (!ok) {
-                if (tid == 0) status[k] = 3;
+                if (tid == 0) a.status[k] = 3;
                 return;
             }
             it_f++;
         }
     }
-    SYNC();
     // ---- write back (:622-624) and the contacts' impulses for the warm start
-    for (int i = p0 + tid; i < p1; i += nt) {
-        const int g = cl_parts[i];
-        if (!is_static[g])
-            for (int q = 0; q < 14; q++) fut[14 * (size_t)g + q] = bw[g].FS[q];
+    for (int s = threadIdx.x; s < nloc; s += kSolveBlock) {
+        const BodyS& B = *own_body(s);
+        if (B.is_static) continue;
+        const int p = s * G + gb;
+        double* F = a.fut + 14 * (size_t)parts[p];
+        const double* q = a.bg[p0 + p].q;
+        for (int e = 0; e < 4; e++) F[1 + e] = B.rbad ? __longlong_as_double(0x7ff8000000000000ll) : q[e];
+        for (int e = 0; e < 3; e++) {
+            F[5 + e] = B.fL[e] + B.rimp[e];
+            F[8 + e] = B.x[e];
+            F[11 + e] = B.v[e];
+        }
     }
     for (int i = tid; i < nc; i += nt) {
-        out_impulse[c0 + i] = cw[c0 + i].impulse;
-        out_ab[2 * (c0 + i)] = cw[c0 + i].a;
-        out_ab[2 * (c0 + i) + 1] = cw[c0 + i].b;
-    }
-    if (tid == 0) {
-        status[k] = 0;
-        iters[2 * k] = it_n;
-        iters[2 * k + 1] = it_f;
+        const ConG& C = cg[i];
+        a.out_impulse[c0 + i] = C.impulse;
+        a.out_ab[2 * (c0 + i)] = parts[C.a];
+        a.out_ab[2 * (c0 + i) + 1] = parts[C.b];
         // Warm-start store (sequential_impulses_warm_start.cpp:28-54): each
         // body pair keeps the impulse of its last contact in sorted order;
         // a pair's first contact enters as 0.0 + impulse.
-        if (pair_warm)
-            for (int i = 0; i < nc; i++) {
-                const int oi = order[c0 + i];
-                pair_warm[con_pair[oi]] = pair_cnt[oi] == 1 ? 0.0 + cw[c0 + i].impulse : cw[c0 + i].impulse;
-            }
+        if (a.pair_warm) {
+            const int oi = a.order[c0 + i], pr = a.con_pair[oi];
+            const int role = (a.ab[c0 + i].x & kStaticBit) && !(a.ab[c0 + i].y & kStaticBit) ? 1 : 0;
+            const int p = role ? C.b : C.a, end = a.boff[p0 + p] + a.deg[p0 + p];
+            bool last = true;
+            for (int e = a.lpos[2 * (c0 + i) + role] + 1; e < end && last; e++)
+                last = a.con_pair[a.order[c0 + (a.blist[2 * c0 + e] >> 1)]] != pr;
+            if (last) a.pair_warm[pr] = a.pair_cnt[oi] == 1 ? 0.0 + C.impulse : C.impulse;
+        }
     }
+    if (tid == 0) {
+        a.status[k] = 0;
+        a.iters[2 * k] = it_n;
+        a.iters[2 * k + 1] = it_f;
+    }
+    if (MODE == kSyncCluster) cluster_barrier();  // no block leaves while another reads its shared memory
 }
 
 #undef SYNC
@@ -950,9 +1008,9 @@ __device__ void solve_body(int k, int tid, int nt, int gb, int G, int* shv, cons
 // One block per cluster (clusters cl_list[b], or b when cl_list is null).
 __global__ void __launch_bounds__(kSolveBlock) k_solve(int n_list, const int32_t* __restrict__ cl_list, SolveArgs a) {
     if ((int)blockIdx.x >= n_list) return;
-    __shared__ int s_local[3];
-    const SolveSync S{kSyncBlock, nullptr, nullptr, nullptr, 0u};
-    solve_body(cl_list ? cl_list[blockIdx.x] : (int)blockIdx.x, threadIdx.x, blockDim.x, 0, 1, s_local, S, a);
+    __shared__ int32_t s_flags[kFlags];
+    const SolveSync S{nullptr, nullptr, s_flags, 0u};
+    solve_body<kSyncBlock>(cl_list ? cl_list[blockIdx.x] : (int)blockIdx.x, 0, 1, S, a);
 }
 
 // Every block of a cooperative grid on cluster k (all blocks resident).
@@ -961,8 +1019,7 @@ __global__ void __launch_bounds__(kSolveBlock) k_solve_grid(int k, SolveSync S, 
     if (threadIdx.x == 0) s_passed = 0;
     __syncthreads();
     S.passed = &s_passed;
-    solve_body(k, threadIdx.x * gridDim.x + blockIdx.x, gridDim.x * blockDim.x, blockIdx.x, gridDim.x, S.flags, S,
-               a);
+    solve_body<kSyncGrid>(k, (int)blockIdx.x, (int)gridDim.x, S, a);
 }
 
 // The blocks of thread-block cluster c solve cluster cl_list[c] together
@@ -974,9 +1031,8 @@ __global__ void __launch_bounds__(kSolveBlock) k_solve_cl(const int32_t* __restr
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(nrank));
     asm("mov.u32 %0, %%clusterid.x;" : "=r"(cid));
-    int32_t* f = flags + 16 * (size_t)cid;
-    const SolveSync S{kSyncCluster, nullptr, nullptr, f, 0u};
-    solve_body(cl_list[cid], threadIdx.x * nrank + rank, (int)(nrank * blockDim.x), (int)rank, (int)nrank, f, S, a);
+    const SolveSync S{nullptr, nullptr, flags + 16 * (size_t)cid, 0u};
+    solve_body<kSyncCluster>(cl_list[cid], (int)rank, (int)nrank, S, a);
 }
 
 // Sort key of Contact::operator< (contact.h:17-21) as orderable bits
@@ -1067,24 +1123,52 @@ int run_filter(d2g_ctx* ctx, const int32_t* d_off, const double* d_rec, int n_pa
     return D2G_OK;
 }
 
+// Dynamic shared memory of a solve block: its share of np bodies and nc
+// contacts (a wave's tasks of four leave places empty, hence the factor), at
+// most `cap`; a block whose cluster needs more keeps the contacts, then the
+// bodies, in global memory.
+int solve_smem(int np, int nc, int G, int cap) {
+    const long long want = (long long)sizeof(BodyS) * ((np + G - 1) / G) * (np > 0 ? 1 : 0) +
+                           std::max(12LL * nc, (long long)sizeof(ConS) * (2LL * nc / G + 64));
+    return (int)std::min<long long>((want + 1023) / 1024 * 1024, cap);
+}
+
+// The solve kernels' largest dynamic shared memory, allowed once per context.
+int allow_solve_smem(d2g_ctx* ctx) {
+    Engine& E = ctx->eng;
+    if (E.sv_smem_set) return D2G_OK;
+    D2G_CUDA(cudaFuncSetAttribute((const void*)k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmemMax));
+    D2G_CUDA(cudaFuncSetAttribute((const void*)k_solve_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmemMax));
+    D2G_CUDA(cudaFuncSetAttribute((const void*)k_solve_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kSolveSmemMax));
+    D2G_CUDA(cudaFuncSetAttribute((const void*)k_solve_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    E.sv_smem_set = true;
+    return D2G_OK;
+}
+
+void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int cs, int n, int smem, cudaStream_t st) {
+    cfg = {};
+    cfg.gridDim = dim3((unsigned)(n * cs));
+    cfg.blockDim = dim3(kSolveBlock);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+}
+
 // Thread-block clusters of `cs` solve blocks that can be resident at once
 // (cached per context).
 int max_solve_clusters(d2g_ctx* ctx, int cs, int* out) {
     Engine& E = ctx->eng;
     const int slot = cs == 16 ? 0 : cs == 8 ? 1 : cs == 4 ? 2 : 3;
     if (E.sv_cl_fit[slot] < 0) {
-        if (cs > 8)
-            D2G_CUDA(cudaFuncSetAttribute((const void*)k_solve_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(kSolveBlock);
+        cudaLaunchConfig_t cfg;
         cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cs;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
+        cluster_config(cfg, at, cs, 1, kSolveSmemMax, nullptr);
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, (const void*)k_solve_cl, &cfg) != cudaSuccess) {
             (void)cudaGetLastError();  // this size is not available: never chosen
@@ -1099,22 +1183,21 @@ int max_solve_clusters(d2g_ctx* ctx, int cs, int* out) {
 // k_solve_cl over n clusters (list d_list), cs blocks each.
 int launch_solve_cl(d2g_ctx* ctx, int cs, int n, const int32_t* d_list, int32_t* d_flags, const SolveArgs& a,
                     cudaStream_t st) {
-    if (cs > 8)
-        D2G_CUDA(cudaFuncSetAttribute((const void*)k_solve_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n * cs));
-    cfg.blockDim = dim3(kSolveBlock);
-    cfg.stream = st;
+    cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cs;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cluster_config(cfg, at, cs, n, a.smem, st);
     D2G_CUDA(cudaLaunchKernelEx(&cfg, k_solve_cl, d_list, d_flags, a));
     ctx->eng.launches++;
     return D2G_OK;
+}
+
+// Blocks that serve a cluster of np particles best: a wave holds a seventh to
+// a quarter as many contacts as the cluster has particles, four to a task, and
+// a block runs two tasks at full rate (measured: the table in run_solve).
+int best_cluster_size(int np) {
+    int cs = 1;
+    while (cs < 16 && cs * kPartsPerBlock < np) cs *= 2;
+    return cs;
 }
 
 // Solve clusters.  Contacts (14-double records in the reference's hit order,
@@ -1128,20 +1211,22 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
               const int32_t* h_con_off, const int32_t* h_part_off) {
     Engine& E = ctx->eng;
     cudaStream_t s = ctx->stream;
-    RC(E.sv_scon.ensure(n_con + 1));
-    RC(E.sv_sdelta.ensure(3 * (size_t)n_con + 3));
-    RC(E.sv_keys.ensure(n_con + 1));
-    RC(E.sv_keys_out.ensure(n_con + 1));
-    RC(E.sv_vals.ensure(n_con + 1));
-    RC(E.sv_order.ensure(n_con + 1));
-    RC(E.sv_bw_raw.ensure(sizeof(BodyWork) * ((size_t)ctx->n_bodies + 1)));
-    RC(E.sv_cw_raw.ensure(sizeof(ConWork) * ((size_t)n_con + 1)));
-    BodyWork* bw = (BodyWork*)E.sv_bw_raw.p;
-    ConWork* cw = (ConWork*)E.sv_cw_raw.p;
-    RC(E.sv_wave_idx.ensure(n_con + 1));
-    RC(E.sv_wave_off.ensure(n_con + n_clusters + 2));
-    RC(E.sv_wave_cursor.ensure(n_con + n_clusters + 2));
-    RC(E.sv_static_imp.ensure(3 * (size_t)n_parts + 3));
+    const size_t n1 = (size_t)n_con + 1, np1 = (size_t)n_parts + 1;
+    RC(E.sv_keys.ensure(n1));
+    RC(E.sv_keys_out.ensure(n1));
+    RC(E.sv_vals.ensure(n1));
+    RC(E.sv_order.ensure(n1));
+    RC(E.sv_bg_raw.ensure(sizeof(BodyG) * np1));
+    RC(E.sv_bs_raw.ensure(sizeof(BodyS) * np1));
+    RC(E.sv_cg_raw.ensure(sizeof(ConG) * n1));
+    RC(E.sv_cs_raw.ensure(sizeof(ConS) * 4 * n1));
+    RC(E.sv_slot.ensure((size_t)ctx->n_bodies + 1));
+    RC(E.sv_part_int.ensure(3 * np1));
+    RC(E.sv_con_int.ensure(9 * n1 + 1));
+    RC(E.sv_tcon.ensure(4 * n1));
+    RC(E.sv_tl.ensure(n_con + n_clusters + 2));
+    RC(E.sv_sdelta.ensure(6 * n1));
+    RC(allow_solve_smem(ctx));
     if (n_con > 0) {
         VLAUNCH(k_prop_keys, n_con, n_con, d_rec, E.sv_keys.p, E.sv_vals.p);
         size_t bytes = 0;
@@ -1167,38 +1252,50 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
         a.mass = ctx->mass.p;
         a.ii = ctx->inv_inertia.p;
         a.mu = ctx->mu.p;
-        a.cur = ctx->cur.p;
         a.fut = ctx->fut.p;
         a.gravity_z = gravity_z;
-        a.bw = bw;
-        a.cw = cw;
-        a.wave_idx = E.sv_wave_idx.p;
-        a.wave_off = E.sv_wave_off.p;
-        a.wave_cursor = E.sv_wave_cursor.p;
-        a.scon = E.sv_scon.p;
+        a.bg = (BodyG*)E.sv_bg_raw.p;
+        a.bs = (BodyS*)E.sv_bs_raw.p;
+        a.cg = (ConG*)E.sv_cg_raw.p;
+        a.cs = (ConS*)E.sv_cs_raw.p;
+        a.slot = E.sv_slot.p;
+        a.deg = E.sv_part_int.p;
+        a.boff = a.deg + np1;
+        a.statics = a.boff + np1;
+        a.ab = (int2*)E.sv_con_int.p;
+        a.blist = E.sv_con_int.p + 2 * n1;
+        a.lpos = a.blist + 2 * n1;
+        a.prev = a.lpos + 2 * n1;
+        a.level = a.prev + 2 * n1;
+        a.tcon = E.sv_tcon.p;
+        a.tl = E.sv_tl.p;
         a.sdelta = E.sv_sdelta.p;
-        a.static_imp = E.sv_static_imp.p;
         a.status = d_status;
         a.iters = d_iters;
         a.out_impulse = d_out_impulse;
         a.out_ab = d_out_ab;
         a.con_pair = d_con_pair;
         a.pair_warm = d_pair_warm;
-        a.lanes = E.tune[D2G_TUNE_SOLVE_LANES];
-        // Where each cluster is solved.  A wave holds at most one contact per
-        // moving body and lasts about one contact's dependent FP64 chain when
-        // its warps each have an SM sub-partition to themselves: a block runs
-        // waves of up to eight contacts that way, a thread-block cluster of
-        // 16 blocks up to 128 (with a hardware barrier, ~0.2 us, between
-        // waves), a cooperative grid over all SMs any width (~1.5 us per
-        // grid barrier).  So a cluster with at least 128 contacts and more
-        // than D2G_TUNE_GRID_MIN_PARTS parts takes a grid when at most 8
-        // clusters of the call qualify (grids run one after another); any
-        // other cluster of at least 32 contacts takes a thread-block cluster
-        // (D2G_TUNE_SOLVE_CLUSTER blocks, or the most that lets every such
-        // cluster be resident at once); the rest one block each.  Blocks and
-        // thread-block clusters run side by side on two streams, the grids
-        // after them.
+        // Where each cluster is solved (us per iteration on GB300, normal and
+        // friction; one block / thread-block cluster of 4 / 8 / 16 / grid):
+        //     8 cubes, 46 waves of 2.2 contacts     61 /   88 /   88 /  88 /    -
+        //    27 cubes, 89 waves of 5.0             123 /  167 /  166 / 166 /  240
+        //   100 cubes, one layer                   310 /  176 /  165 / 164 /  219
+        //   512 hulls, 24 waves of 71              353 /  113 /   82 /  71 /   85
+        // 1,024 hulls, 23 waves of 142             671 /  213 /  125 /  88 /   90
+        // 2,304 hulls                             1530 /  481 /  289 / 178 /  135
+        // 5,120 hulls                             3646 / 1115 /  683 / 467 /  268
+        // (before: 331 us for the 8 cubes, 257 for the 1,024 hulls).  A block
+        // barrier costs ~0.1 us, the cluster barrier with distributed shared
+        // memory ~0.5 us more, a grid barrier ~1.5 us, and a block runs two
+        // tasks at full rate: so one block up to kPartsPerBlock particles, then
+        // twice as many for every doubling (best_cluster_size) as long as all
+        // such clusters of the call are resident at once, and a cooperative
+        // grid for a cluster with at least kGridMinContacts contacts and more
+        // than D2G_TUNE_GRID_MIN_PARTS parts when at most kGridMaxClusters
+        // qualify (grids run one after another).  D2G_TUNE_SOLVE_CLUSTER fixes
+        // the cluster's size.  Blocks and thread-block clusters run side by
+        // side on two streams, the grids after them.
         const int cl_setting = E.tune[D2G_TUNE_SOLVE_CLUSTER];
         std::vector<int32_t> small, mid, big;
         if (h_con_off && h_part_off)
@@ -1213,7 +1310,9 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
                 continue;
             }
             const int nck = h_con_off ? h_con_off[c + 1] - h_con_off[c] : 0;
-            if (h_con_off && cl_setting != 1 && nck >= kClusterMinContacts)
+            const int npk = h_con_off && h_part_off ? h_part_off[c + 1] - h_part_off[c] : 0;
+            const bool wide = cl_setting > 1 || (cl_setting == 0 && best_cluster_size(npk) > 1);
+            if (h_con_off && wide && nck >= kClusterMinContacts)
                 mid.push_back(c);
             else
                 small.push_back(c);
@@ -1223,7 +1322,10 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
             if (cl_setting > 1) {
                 cs = cl_setting;
             } else {
+                int most = 1;
+                for (int c : mid) most = std::max(most, best_cluster_size(h_part_off[c + 1] - h_part_off[c]));
                 for (int cand : {16, 8, 4, 2}) {
+                    if (cand > most) continue;
                     int fit = 0;
                     RC(max_solve_clusters(ctx, cand, &fit));
                     if (fit >= (int)mid.size()) {
@@ -1238,6 +1340,14 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
                 mid.clear();
             }
         }
+        auto smem_of = [&](const std::vector<int32_t>& list, int G, int cap) {
+            int m = 0;
+            for (int c : list)
+                m = std::max(m, h_con_off && h_part_off ? solve_smem(h_part_off[c + 1] - h_part_off[c],
+                                                                     h_con_off[c + 1] - h_con_off[c], G, cap)
+                                                        : cap);
+            return m;
+        };
         const bool all_small = mid.empty() && big.empty();
         E.sv_layout[0] = (int)small.size();
         E.sv_layout[1] = (int)mid.size();
@@ -1252,7 +1362,9 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
                                          cudaMemcpyHostToDevice, s));
                 d_list = E.sv_list.p;
             }
-            k_solve<<<(int)small.size(), kSolveBlock, 0, s>>>((int)small.size(), d_list, a);
+            // one block alone on its SM may take all of its shared memory
+            a.smem = smem_of(small, 1, small.size() <= 128 ? kSolveSmemMax : kSolveSmemMax / 2);
+            k_solve<<<(int)small.size(), kSolveBlock, a.smem, s>>>((int)small.size(), d_list, a);
             ctx->eng.launches++;
         }
         if (!mid.empty()) {
@@ -1263,6 +1375,7 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
             D2G_CUDA(cudaMemsetAsync(E.sv_cl_flags.p, 0, (16 * mid.size() + 16) * sizeof(int32_t), s));
             D2G_CUDA(cudaEventRecord(ctx->ev_fork, s));
             D2G_CUDA(cudaStreamWaitEvent(ctx->stream2, ctx->ev_fork, 0));
+            a.smem = smem_of(mid, cs, kSolveSmemMax);
             RC(launch_solve_cl(ctx, cs, (int)mid.size(), d_mid, E.sv_cl_flags.p, a, ctx->stream2));
             D2G_CUDA(cudaEventRecord(ctx->ev_join, ctx->stream2));
             D2G_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
@@ -1270,13 +1383,13 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
         if (!big.empty()) {
             int dev_sms = 0, per_sm = 0;
             D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
-            D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_grid, kSolveBlock, 0));
+            a.smem = kSolveSmemMax;
+            D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_grid, kSolveBlock, a.smem));
             const int G_max = std::max(1, std::min(dev_sms, dev_sms * per_sm));
             RC(E.sv_grid.ensure(16 * big.size() + 16));
             D2G_CUDA(cudaMemsetAsync(E.sv_grid.p, 0, (16 * big.size() + 16) * sizeof(int32_t), s));
             for (size_t b = 0; b < big.size(); b++) {
                 SolveSync S;
-                S.mode = kSyncGrid;
                 S.count = (unsigned long long*)(E.sv_grid.p + 16 * b);  // 8-byte aligned: 16 ints per cluster
                 S.passed = nullptr;
                 S.flags = E.sv_grid.p + 16 * b + 4;
@@ -1287,8 +1400,8 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
                 const int nck = h_con_off[k + 1] - h_con_off[k];
                 const int G = std::max(1, std::min(G_max, std::max(8, nck / E.tune[D2G_TUNE_GRID_CONTACTS])));
                 void* args[] = {&k, &S, &a};
-                D2G_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve_grid, dim3(G), dim3(kSolveBlock), args, 0,
-                                                     s));
+                D2G_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve_grid, dim3(G), dim3(kSolveBlock), args,
+                                                     (size_t)a.smem, s));
                 ctx->eng.launches++;
             }
         }

@@ -247,9 +247,8 @@ int d2g_ctx_ccd_stats(d2g_ctx* ctx, int32_t reset, int64_t* stats, int32_t n);
  *   D2G_TUNE_GRID_MIN_PARTS (default 512, >= 0): a cluster with at least
  *     128 contacts and more parts than this is solved by a cooperative grid
  *     over the SMs, when at most 8 clusters of the solve call qualify.
- *   D2G_TUNE_SOLVE_LANES (default 0; 0, 4 or 16): lanes per contact in the
- *     solve's normal-impulse waves; 0 takes sixteen for a wave narrow enough
- *     that its warps each have an SM sub-partition to themselves, else four.
+ *   D2G_TUNE_SOLVE_LANES (default 0; 0, 4 or 16): has no effect any more (the
+ *     solve's waves have one form); kept so that settings files still apply.
  *   D2G_TUNE_SPIN_LIMIT (default 33554432, >= 1): polls a block of the
  *     cooperative-grid solve makes at a grid barrier before it gives up
  *     (several seconds at the default); a call whose barrier gave up returns
@@ -263,9 +262,10 @@ int d2g_ctx_ccd_stats(d2g_ctx* ctx, int32_t reset, int64_t* stats, int32_t n);
  *   D2G_TUNE_SOLVE_CLUSTER (default 0; 0, 1, 2, 4, 8 or 16): a cluster with
  *     at least 32 contacts that does not take a grid is solved by a
  *     thread-block cluster of this many blocks (waves between them on the
- *     hardware cluster barrier); 0 takes the largest size at which every
- *     such cluster of the call is resident at once (one block each when
- *     none is), 1 solves them with one block each.
+ *     hardware cluster barrier); 0 chooses the size from the clusters'
+ *     particles (one block up to 32, then doubling) as far as every such
+ *     cluster of the call is resident at once (one block each when none is),
+ *     1 solves them with one block each.
  * delta2_gb300/autotune.py measures candidate values on a workload and
  * writes them to a file that the Python layer applies. */
 #define D2G_TUNE_EE_FIRST_ITERS 0

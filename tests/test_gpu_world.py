@@ -443,3 +443,24 @@ def test_world_obj_scene_matches_oracle(ctx, tmp_path):
     s = b.finish()
     st = run_world(ctx, s, 80)
     assert st["np_contacts"] > 0
+
+
+@pytest.mark.parametrize("cluster", [0, 2, 1], ids=["auto", "cluster2", "block"])
+@pytest.mark.parametrize("nx, ny, nz", [(1, 1, 1), (2, 1, 1), (3, 2, 1), (3, 3, 2)])
+def test_solve_sizes_match_oracle(ctx, nx, ny, nz, cluster):
+    """Clusters around the solve's task and block sizes (waves of one to a
+    dozen contacts, four to a task; fewer bodies than blocks): touching,
+    slightly turned cubes on the ground, bit for bit against the oracle."""
+    s = D.make_scene(1, nx=nx, ny=ny, nz=nz, spacing=1.02, speed_sigma=0.0)
+    rng = np.random.default_rng(100 * nx + 10 * ny + nz)
+    q = np.concatenate([np.ones((nx * ny * nz, 1)), 0.004 * rng.standard_normal((nx * ny * nz, 3))], axis=1)
+    s.cur[1:, 1:5] = q / np.linalg.norm(q, axis=1)[:, None]
+    s.cur[1:, 10] += 0.53 - s.cur[1:, 10].min()
+    s.cur[1:, 11:14] = 0.3 * rng.standard_normal((nx * ny * nz, 3))
+    s.fut[1:] = s.cur[1:]
+    s.last[1:] = s.cur[1:]
+    ctx.set_tuning(D.TUNE_SOLVE_CLUSTER, cluster)
+    try:
+        solve_against_oracle(ctx, s.copy(), s)
+    finally:
+        ctx.set_tuning(D.TUNE_SOLVE_CLUSTER, 0)
