@@ -24,6 +24,7 @@
 
 #include "d2g_geom.cuh"
 #include "d2g_internal.hpp"
+#include "d2g_prune.cuh"
 
 namespace d2g {
 
@@ -1320,8 +1321,6 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 }
 
 // ----------------------------------------------------------- discrete -----
-// All 64 slots of a node pair: triangle distance at the future poses and the
-// hit test dist < float(search) + eps_a + eps_b (comparison_dist.h:223-236).
 // Candidate slots of the discrete narrow phase.  A (node pair, ta, tb) slot
 // can only hit (comparison_dist.h:231-233) when the triangles are closer than
 // thr = search + eps_a + eps_b.  Lower bounds on that distance: the bounding
@@ -1333,22 +1332,61 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // (1 mm plus 4e-6 of the magnitudes involved) far above the FP32 rounding of
 // the bound and the FP64 rounding of the exact test, so every slot that hits
 // survives.  Dropped slots produce nothing in the reference
-// either.  One thread per slot; per warp a survivor mask and count.  The valid
-// slots (ta < ntris_a, tb < ntris_b) are counted for the statistics.
+// either.  One thread per slot; per warp a survivor mask and count.
+//
+// A node pair with an inner node emits nothing: all the traversal needs of it
+// is whether some slot hits.  The exact distance is at most that of any edge
+// pair, so a slot whose vertices, or else edges, are closer than thr by the
+// same margin certainly hits; its node pair is marked and none of its slots
+// goes on to the FP64 test (`nodes` null: every slot's hit is wanted).
+__device__ __forceinline__ float vv_min(const float (&wa)[3][3], const float (&wb)[3][3]) {
+    float m = 3.4e38f;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const float dx = wa[i][0] - wb[j][0], dy = wa[i][1] - wb[j][1], dz = wa[i][2] - wb[j][2];
+            m = fminf(m, dx * dx + dy * dy + dz * dz);
+        }
+    return sqrtf(m);
+}
+__device__ __forceinline__ float ee_min(const float (&wa)[3][3], const float (&wb)[3][3]) {
+    float m = 3.4e38f;
+    F3 A[3], B[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        A[i] = f3(wa[i][0], wa[i][1], wa[i][2]);
+        B[i] = f3(wb[i][0], wb[i][1], wb[i][2]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            float d2;
+            seg_vector(A[i], A[(i + 1) % 3], B[j], B[(j + 1) % 3], d2);
+            m = fminf(m, d2);  // NaN (a degenerate edge) is passed over
+        }
+    return sqrtf(m);
+}
+
 __global__ void __launch_bounds__(kBlock) k_np_mask(int n_slots, const Entry* __restrict__ front,
                                                     const float* __restrict__ pm32, const int32_t* __restrict__ ntris,
                                                     const float4* __restrict__ sph, const float* __restrict__ tri32,
                                                     const float* __restrict__ eps_up,
-                                                    const float* __restrict__ search, uint32_t* __restrict__ mask,
-                                                    int32_t* __restrict__ cnt, int32_t* __restrict__ tri_pairs,
-                                                    int use_bounds) {
+                                                    const float* __restrict__ search, const int4* __restrict__ nodes,
+                                                    uint32_t* __restrict__ mask, int32_t* __restrict__ cnt,
+                                                    int32_t* __restrict__ entry_hits, int use_bounds) {
+    __shared__ int s_hit[kBlock / 64];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool valid = false, keep = false;
+    if (threadIdx.x < kBlock / 64) s_hit[threadIdx.x] = 0;
+    bool keep = false, inner = false;
+    float room = 0.f;  // thr less the margin
+    float wa[3][3], wb[3][3];  // [vertex][axis]
     if (i < n_slots) {
         const Entry e = front[i >> 6];
         const int ta = (i >> 3) & 7, tb = i & 7;
-        valid = ta < ntris[e.na] && tb < ntris[e.nb];
-        if (valid) {
+        inner = nodes && use_bounds && (ld_node(nodes, e.na).z || ld_node(nodes, e.nb).z);
+        if (ta < ntris[e.na] && tb < ntris[e.nb]) {
             const float* A = pm32 + 24 * (size_t)e.pair;
             const float* B = A + 12;
             const float4 sa = sph[(size_t)e.na * 8 + ta], sb = sph[(size_t)e.nb * 8 + tb];
@@ -1363,81 +1401,113 @@ __global__ void __launch_bounds__(kBlock) k_np_mask(int n_slots, const Entry* __
                               fabsf(sa.x) + fabsf(sa.y) + fabsf(sa.z) + fabsf(sb.x) + fabsf(sb.y) + fabsf(sb.z) +
                               sa.w + sb.w + thr;
             float lb = sqrtf(dx * dx + dy * dy + dz * dz) - sa.w - sb.w;
-            // the gap between the transformed triangles' boxes is a second lower bound
-            const float* va = tri32 + ((size_t)e.na * 8 + ta) * 9;
-            const float* vb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
-            float wa[3][3], wb[3][3];  // [vertex][axis]
-#pragma unroll
-            for (int v = 0; v < 3; v++)
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    wa[v][r] = A[4 * r] * va[3 * v] + A[4 * r + 1] * va[3 * v + 1] + A[4 * r + 2] * va[3 * v + 2] +
-                               A[4 * r + 3];
-                    wb[v][r] = B[4 * r] * vb[3 * v] + B[4 * r + 1] * vb[3 * v + 1] + B[4 * r + 2] * vb[3 * v + 2] +
-                               B[4 * r + 3];
-                }
-            float gap2 = 0.f;
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const float alo = fminf(fminf(wa[0][r], wa[1][r]), wa[2][r]);
-                const float ahi = fmaxf(fmaxf(wa[0][r], wa[1][r]), wa[2][r]);
-                const float blo = fminf(fminf(wb[0][r], wb[1][r]), wb[2][r]);
-                const float bhi = fmaxf(fmaxf(wb[0][r], wb[1][r]), wb[2][r]);
-                const float g = fmaxf(blo - ahi, alo - bhi);
-                if (g > 0.f) gap2 += g * g;
-            }
-            lb = fmaxf(lb, sqrtf(gap2));
             const float lim = thr + (1e-3f + 4e-6f * mag);
-            if (!(lb > lim)) {
-                // Separating axes: along any direction n the distance is at
-                // least the gap between the projections divided by |n|,
-                // whatever n is, so n computed in FP32 still bounds; the two
-                // face normals and the nine edge-edge cross products.
-                auto axis_gap = [&](float nx, float ny, float nz) {
-                    const float nn = sqrtf(nx * nx + ny * ny + nz * nz);
-                    if (!(nn > 1e-20f)) return 0.f;
-                    float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
+            keep = !use_bounds || !(lb > lim);  // NaN keeps the slot
+            if (keep) {
+                const float* va = tri32 + ((size_t)e.na * 8 + ta) * 9;
+                const float* vb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
 #pragma unroll
-                    for (int v = 0; v < 3; v++) {
-                        const float pa = wa[v][0] * nx + wa[v][1] * ny + wa[v][2] * nz;
-                        const float pb = wb[v][0] * nx + wb[v][1] * ny + wb[v][2] * nz;
-                        a0 = fminf(a0, pa);
-                        a1 = fmaxf(a1, pa);
-                        b0 = fminf(b0, pb);
-                        b1 = fmaxf(b1, pb);
-                    }
-                    return fmaxf(b0 - a1, a0 - b1) / nn;
-                };
-                float ea[3][3], eb[3][3];
-#pragma unroll
-                for (int k = 0; k < 3; k++)
+                for (int v = 0; v < 3; v++)
 #pragma unroll
                     for (int r = 0; r < 3; r++) {
-                        ea[k][r] = wa[(k + 1) % 3][r] - wa[k][r];
-                        eb[k][r] = wb[(k + 1) % 3][r] - wb[k][r];
+                        wa[v][r] = A[4 * r] * va[3 * v] + A[4 * r + 1] * va[3 * v + 1] + A[4 * r + 2] * va[3 * v + 2] +
+                                   A[4 * r + 3];
+                        wb[v][r] = B[4 * r] * vb[3 * v] + B[4 * r + 1] * vb[3 * v + 1] + B[4 * r + 2] * vb[3 * v + 2] +
+                                   B[4 * r + 3];
                     }
-                lb = fmaxf(lb, axis_gap(ea[0][1] * ea[1][2] - ea[0][2] * ea[1][1], ea[0][2] * ea[1][0] - ea[0][0] * ea[1][2],
-                                        ea[0][0] * ea[1][1] - ea[0][1] * ea[1][0]));
-                lb = fmaxf(lb, axis_gap(eb[0][1] * eb[1][2] - eb[0][2] * eb[1][1], eb[0][2] * eb[1][0] - eb[0][0] * eb[1][2],
-                                        eb[0][0] * eb[1][1] - eb[0][1] * eb[1][0]));
+                if (use_bounds) {
+                    // the gap between the transformed triangles' boxes
+                    float gap2 = 0.f;
 #pragma unroll
-                for (int x = 0; x < 3; x++)
+                    for (int r = 0; r < 3; r++) {
+                        const float alo = fminf(fminf(wa[0][r], wa[1][r]), wa[2][r]);
+                        const float ahi = fmaxf(fmaxf(wa[0][r], wa[1][r]), wa[2][r]);
+                        const float blo = fminf(fminf(wb[0][r], wb[1][r]), wb[2][r]);
+                        const float bhi = fmaxf(fmaxf(wb[0][r], wb[1][r]), wb[2][r]);
+                        const float g = fmaxf(blo - ahi, alo - bhi);
+                        if (g > 0.f) gap2 += g * g;
+                    }
+                    keep = !(sqrtf(gap2) > lim);
+                }
+                room = thr - (1e-3f + 4e-6f * mag);
+                if (keep && use_bounds && !(inner && vv_min(wa, wb) < room)) {
+                    // Separating axes: along any direction n the distance is at
+                    // least the gap between the projections divided by |n|,
+                    // whatever n is, so n computed in FP32 still bounds; the two
+                    // face normals and the nine edge-edge cross products.
+                    lb = 0.f;
+                    auto axis_gap = [&](float nx, float ny, float nz) {
+                        const float nn = sqrtf(nx * nx + ny * ny + nz * nz);
+                        if (!(nn > 1e-20f)) return 0.f;
+                        float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
 #pragma unroll
-                    for (int y = 0; y < 3; y++)
-                        lb = fmaxf(lb, axis_gap(ea[x][1] * eb[y][2] - ea[x][2] * eb[y][1],
-                                                ea[x][2] * eb[y][0] - ea[x][0] * eb[y][2],
-                                                ea[x][0] * eb[y][1] - ea[x][1] * eb[y][0]));
+                        for (int v = 0; v < 3; v++) {
+                            const float pa = wa[v][0] * nx + wa[v][1] * ny + wa[v][2] * nz;
+                            const float pb = wb[v][0] * nx + wb[v][1] * ny + wb[v][2] * nz;
+                            a0 = fminf(a0, pa);
+                            a1 = fmaxf(a1, pa);
+                            b0 = fminf(b0, pb);
+                            b1 = fmaxf(b1, pb);
+                        }
+                        return fmaxf(b0 - a1, a0 - b1) / nn;
+                    };
+                    float ea[3][3], eb[3][3];
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+#pragma unroll
+                        for (int r = 0; r < 3; r++) {
+                            ea[k][r] = wa[(k + 1) % 3][r] - wa[k][r];
+                            eb[k][r] = wb[(k + 1) % 3][r] - wb[k][r];
+                        }
+                    lb = fmaxf(lb, axis_gap(ea[0][1] * ea[1][2] - ea[0][2] * ea[1][1],
+                                            ea[0][2] * ea[1][0] - ea[0][0] * ea[1][2],
+                                            ea[0][0] * ea[1][1] - ea[0][1] * ea[1][0]));
+                    lb = fmaxf(lb, axis_gap(eb[0][1] * eb[1][2] - eb[0][2] * eb[1][1],
+                                            eb[0][2] * eb[1][0] - eb[0][0] * eb[1][2],
+                                            eb[0][0] * eb[1][1] - eb[0][1] * eb[1][0]));
+#pragma unroll
+                    for (int x = 0; x < 3; x++)
+#pragma unroll
+                        for (int y = 0; y < 3; y++)
+                            lb = fmaxf(lb, axis_gap(ea[x][1] * eb[y][2] - ea[x][2] * eb[y][1],
+                                                    ea[x][2] * eb[y][0] - ea[x][0] * eb[y][2],
+                                                    ea[x][0] * eb[y][1] - ea[x][1] * eb[y][0]));
+                    keep = !(lb > lim);
+                }
             }
-            keep = !use_bounds || !(lb > lim);  // NaN keeps the slot
         }
     }
+    // node pairs that certainly hit: by the vertices, else by the edges
+    __syncthreads();
+    int* const hit = s_hit + (threadIdx.x >> 6);
+    if (keep && inner && vv_min(wa, wb) < room) *hit = 1;
+    __syncthreads();
+    const bool open = !*(volatile int*)hit;
+    __syncthreads();
+    if (open && keep && inner && ee_min(wa, wb) < room) *hit = 1;
+    __syncthreads();
+    if (*hit) {
+        keep = false;
+        if ((threadIdx.x & 63) == 0) entry_hits[i >> 6] = 1;
+    }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
-    const unsigned v = __ballot_sync(0xffffffffu, valid);
     if ((threadIdx.x & 31) == 0 && i < n_slots) {
         mask[i >> 5] = m;
         cnt[i >> 5] = __popc(m);
-        if (tri_pairs && v) atomicAdd(tri_pairs, __popc(v));  // statistics only
     }
+}
+
+// The valid slots (ta < ntris_a, tb < ntris_b) of a level, for the statistics.
+__global__ void k_count_slots(int n, const Entry* __restrict__ front, const int32_t* __restrict__ ntris,
+                              int32_t* __restrict__ total) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int v = 0;
+    if (i < n) {
+        const Entry e = front[i];
+        v = ntris[e.na] * ntris[e.nb];
+    }
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(total, v);
 }
 
 // Ordered compaction of the surviving slots (slot order = the reference's
@@ -1451,6 +1521,10 @@ __global__ void k_np_items(int n_slots, const uint32_t* __restrict__ mask, const
     if ((m >> lane) & 1u) items[off[i >> 5] + __popc(m & ((1u << lane) - 1u))] = i;
 }
 
+// One surviving slot a thread: the FP64 triangle distance and the hit test.
+// Bound by the FP64 pipe; tri_tri_dist_below evaluates 2 to 3 of the 21
+// features (1,024 packed hulls: 825 us a level with all of them, the whole
+// call 5.60 -> 2.35 ms with that and the node pairs marked by k_np_mask).
 __global__ void __launch_bounds__(kBlock) k_np(int n_slots, const Entry* __restrict__ front,
                                                const int32_t* __restrict__ pairs, const double* __restrict__ pm,
                                                const int32_t* __restrict__ ntris, const double* __restrict__ tris,
@@ -1459,15 +1533,11 @@ __global__ void __launch_bounds__(kBlock) k_np(int n_slots, const Entry* __restr
                                                const float* __restrict__ search, PrimResult* __restrict__ res,
                                                double* __restrict__ res_eps, int32_t* __restrict__ hit,
                                                int32_t* __restrict__ entry_hits, const int32_t* __restrict__ items,
-                                               const int32_t* __restrict__ n_items) {
+                                               int use_bounds) {
     // Work item k tests slot items[k] (all slots when items is null); results
     // are stored per item.
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n_slots) return;
-    if (n_items && k >= *n_items) {
-        hit[k] = 0;
-        return;
-    }
     const int i = items ? items[k] : k;
     const Entry e = front[i >> 6];
     const int ta = (i >> 3) & 7, tb = i & 7;
@@ -1477,9 +1547,10 @@ __global__ void __launch_bounds__(kBlock) k_np(int n_slots, const Entry* __restr
         const Tri A = tri_xform_rigid(load_tri(tris + (size_t)e.na * 72 + ta * 9), M);
         const Tri B = tri_xform_rigid(load_tri(tris + (size_t)e.nb * 72 + tb * 9), M + 16);
         V3 P, Q;
-        const double d = tri_tri_dist(A, B, P, Q);
         const double ea = eps[(size_t)e.na * 8 + ta], eb = eps[(size_t)e.nb * 8 + tb];
-        h = d < ((double)search[e.pair] + ea) + eb ? 1 : 0;
+        const double thr = ((double)search[e.pair] + ea) + eb;
+        const double d = use_bounds ? tri_tri_dist_below(A, B, thr, P, Q) : tri_tri_dist(A, B, P, Q);
+        h = d < thr ? 1 : 0;
         if (h) {
             const int a = pairs[2 * e.pair], b = pairs[2 * e.pair + 1];
             put_result(res[k], d, P, Q, 0.0);
@@ -2363,7 +2434,8 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
         RC(E.np_off.ensure(n_words + 1));
         RC(E.items.ensure(n_slots + 1));
         LAUNCH(k_np_mask, n_slots, n_slots, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p,
-               E.search.p, E.np_mask.p, E.np_cnt.p, E.np_tri.p, E.fp32_bounds ? 1 : 0);
+               E.search.p, ctx->nodes.p, E.np_mask.p, E.np_cnt.p, E.entry_hits.p, E.fp32_bounds ? 1 : 0);
+        LAUNCH(k_count_slots, n, n, E.soup.p, ctx->ntris.p, E.np_tri.p);
         RC(scan(ctx, E.np_cnt.p, E.np_off.p, n_words));
         LAUNCH(k_np_items, n_slots, n_slots, E.np_mask.p, E.np_off.p, E.items.p);
         // the survivors' count sizes every later kernel of the level
@@ -2376,7 +2448,7 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
             const int pf = prof_begin(ctx, PROF_NP, n_slots);
             LAUNCH(k_np, n_items, n_items, E.soup.p, d_pairs, E.pm.p, ctx->ntris.p, ctx->tris.p, ctx->eps.p,
                    ctx->inner_eps.p, ctx->geo_eps.p, E.search.p, E.res.p, res_eps.p, E.hit.p, E.entry_hits.p,
-                   E.items.p, (const int32_t*)nullptr);
+                   E.items.p, E.fp32_bounds ? 1 : 0);
             prof_end(ctx, pf);
             LAUNCH(k_final_flags, n_items, n_items, E.items.p, E.soup.p, ctx->nodes.p, E.hit.p, E.flags.p);
         }
@@ -2473,7 +2545,8 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
     RC(E.np_off.ensure(n_words + 1));
     RC(E.items.ensure(n_slots + 1));
     LAUNCH(k_np_mask, n_slots, n_slots, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p,
-           ctx->eps_up.p, E.search.p, E.np_mask.p, E.np_cnt.p, E.np_tri.p, E.fp32_bounds ? 1 : 0);
+           ctx->eps_up.p, E.search.p, (const int4*)nullptr, E.np_mask.p, E.np_cnt.p, E.entry_hits.p,
+           E.fp32_bounds ? 1 : 0);
     RC(scan(ctx, E.np_cnt.p, E.np_off.p, n_words));
     LAUNCH(k_np_items, n_slots, n_slots, E.np_mask.p, E.np_off.p, E.items.p);
     int32_t n_items = 0;
@@ -2485,7 +2558,7 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
         const int pf = prof_begin(ctx, PROF_NP, n_slots);
         LAUNCH(k_np, n_items, n_items, E.soup.p, d_pair, E.pm.p, ctx->ntris.p, ctx->tris.p, ctx->eps.p,
                ctx->inner_eps.p, ctx->geo_eps.p, E.search.p, E.res.p, res_eps.p, E.hit.p, E.entry_hits.p, E.items.p,
-               (const int32_t*)nullptr);
+               E.fp32_bounds ? 1 : 0);
         prof_end(ctx, pf);
     }
     RC(E.flag_off.ensure(n_items + 1));
@@ -2700,7 +2773,7 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
         const int n_slots = 64 * n;
         D2G_CUDA(cudaMemsetAsync(entry_hits, 0, sizeof(int32_t) * n, s));
         NA_LAUNCH(k_np, n_slots, n_slots, front, d_pairs, pm, sc->ntris, sc->tris, sc->eps, sc->inner_eps,
-                  sc->geo_eps, search, res, res_eps, hit, entry_hits, nullptr, nullptr);
+                  sc->geo_eps, search, res, res_eps, hit, entry_hits, nullptr, 1);
         NA_LAUNCH(k_final_flags, n_slots, n_slots, nullptr, front, nodes, hit, flags);
         if (int rc = noalloc_scan(s, tmp, tmp_bytes, flags, flag_off, n_slots)) return rc;
         int32_t tot = 0;
