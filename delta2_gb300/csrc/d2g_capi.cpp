@@ -437,7 +437,6 @@ void d2g_ctx_destroy(d2g_ctx* c) {
     E.cflag_off.release();
     E.nn_cnt.release();
     E.nn_off.release();
-    E.citem_off.release();
     E.st_mt.release();
     E.st_new_dt.release();
     E.st_step.release();
@@ -457,7 +456,6 @@ void d2g_ctx_destroy(d2g_ctx* c) {
     E.rec_idx.release();
     E.rec_idx_sorted.release();
     E.out_off.release();
-    E.pair_cnt.release();
     E.d_pairs.release();
     E.d_max_time.release();
     E.cub_tmp.release();

@@ -6,15 +6,14 @@
 // holds the node pairs of ALL body pairs, sorted by body pair and, within a
 // pair, in the reference's order; every expansion is an ordered compaction
 // (prefix sums), so the contacts of each pair come out in exactly the order
-// the reference's sequential loops produce them.  Each level of each stage
-// is three kinds of launches:
-//   1. a cheap filter over all primitive slots (swept boxes in the CCD soup
-//      stage), compacted into a dense work list;
-//   2. one thread per primitive test (triangle-triangle CCD, point-triangle
-//      CCD, edge-edge CCD or discrete triangle distance) writing its result
-//      and hit flag;
-//   3. ordered compaction of the contacts of leaf-leaf node pairs and
-//      expansion of the node pairs that hit into the next frontiers.
+// the reference's sequential loops produce them.
+//
+// The descent only needs to know which node pairs have a hit; leaf pairs end
+// it.  So a level decides its node pairs (FP32 where the answer is certain,
+// the FP64 tests until the first hit where it is not) and puts the leaf pairs
+// it opens onto one list, and all leaf pairs of the call are tested in FP64 at
+// once after the last level: one chain of the slowest tests instead of one per
+// level, and enough tests to fill the GPU.
 // All arithmetic is FP64 with -fmad=false, in the order declared in
 // d2g_geom.cuh, so results equal the CPU restatement bit for bit.
 #include <cub/cub.cuh>
@@ -146,22 +145,13 @@ __global__ void k_conn_nn(int n, const Entry* __restrict__ conn, const int32_t* 
     cnt[i] = ntris[e.na] * ntris[e.nb];
 }
 
-__global__ void k_scale(int n, const int32_t* __restrict__ in, int32_t m, int32_t* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = m * in[i];
-}
-
-// Last entry e with m*off[e] <= k (off[0] == 0).
-__device__ __forceinline__ int find_entry(const int32_t* __restrict__ off, int n_entries, int m, int k) {
-    int lo = 0, hi = n_entries;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (m * off[mid] <= k)
-            lo = mid;
-        else
-            hi = mid;
-    }
-    return lo;
+// The leaf pair of every leaf-pair triangle pair: tp[off[e] .. off[e + 1]) = e,
+// a warp per leaf pair.  Test j of a list with m tests per triangle pair
+// belongs to leaf pair tp[j / m] (a search of off in every test kernel before).
+__global__ void k_tp_fill(int n, const int32_t* __restrict__ off, int32_t* __restrict__ tp) {
+    const int e = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    if (e >= n) return;
+    for (int k = off[e] + (threadIdx.x & 31); k < off[e + 1]; k += 32) tp[k] = e;
 }
 
 __device__ __forceinline__ void store_prim(PrimResult* __restrict__ r, double dist, V3 A, V3 B, double toc) {
@@ -231,7 +221,17 @@ __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restri
 }
 
 // The swept-AABB prefilter of every (triangle of a, triangle of b) slot of a
-// soup node pair (continuous_comparison.h:804-812), one warp per node pair:
+// soup node pair (continuous_comparison.h:804-812), one warp per node pair, and
+// what the descent needs of the pair.  A node pair of the soup stage has an
+// inner node, emits nothing and is opened when any of its triangle pairs has a
+// test with a distance below the search distance.  Every edge-edge test
+// returns at most its distance at the start (edgeEdgeCCD evaluates it first)
+// or at most 1e-8, so a slot whose triangles' vertices, or else edges, are
+// closer than the search distance there by a margin (1 mm plus 4e-6 of the
+// coordinates, FP32) certainly hits: the node pair is marked and done.  The
+// slots of the others go onto `list` for k_soup_tests.  Two bodies that are
+// single leaves meet at the root: their slots are counted (`lc`) and tested
+// with the leaf pairs (k_soup_filter).  The box stage:
 // lanes 0-7 form the swept boxes of a's triangles, lanes 8-15 those of b's,
 // once each, and every lane then tests two of the 64 slots from shuffled
 // boxes.  flags[64 * entry + 8 * ta + tb] = 1 where the boxes overlap.  The
@@ -240,23 +240,15 @@ __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restri
 // largest coordinate, far above the FP32 rounding of the box edges) has the
 // answer the FP64 boxes give; a warp with any slot inside the margin (or a
 // NaN) forms the FP64 boxes and decides those slots exactly.
-__global__ void k_soup_filter(int n_soup, const Entry* __restrict__ soup, const int32_t* __restrict__ pairs,
-                              const double* __restrict__ pm, const float* __restrict__ pm32,
-                              const int32_t* __restrict__ ntris, const double* __restrict__ tris,
-                              const float* __restrict__ tri32, const double* __restrict__ geo_eps,
-                              const uint8_t* __restrict__ skip, const uint8_t* __restrict__ eskip,
-                              int32_t* __restrict__ flags) {
-    const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+// res[h]: the swept boxes of slot lane + 32 h overlap.  verts: the warp's 16
+// triangles (a's, then b's) in FP32 at the start, [16][9]; mag: the largest
+// coordinate of each, for the margins.
+__device__ __forceinline__ void swept_slots(const Entry& e, const int32_t* __restrict__ pairs,
+                                            const double* __restrict__ pm, const float* __restrict__ pm32,
+                                            const int32_t* __restrict__ ntris, const double* __restrict__ tris,
+                                            const float* __restrict__ tri32, const double* __restrict__ geo_eps,
+                                            int (&res)[2], float (*verts)[9], float* mags) {
     const int lane = threadIdx.x & 31;
-    if (w >= n_soup) return;  // uniform per warp
-    const Entry e = soup[w];
-    // a pair the root certificate proved contact-free, or a node pair its
-    // separation witness proved clear: no slot goes on
-    if ((skip && skip[e.pair]) || (eskip && eskip[w])) {
-        flags[64 * (size_t)w + lane] = 0;
-        flags[64 * (size_t)w + lane + 32] = 0;
-        return;
-    }
     const int na = ntris[e.na], nb = ntris[e.nb];
     const bool side_b = lane >= 8;
     const int t = lane & 7;
@@ -270,11 +262,16 @@ __global__ void k_soup_filter(int n_soup, const Entry* __restrict__ soup, const 
         const float* tv = tri32 + ((size_t)node * 8 + t) * 9;
         const float* MS = pm32_of(pm32, e.pair, side_b ? P32_BS : P32_AS);
         const float* ME = pm32_of(pm32, e.pair, side_b ? P32_BE : P32_AE);
-        float o[3];
+        float o[3], oe[3][3];
 #pragma unroll
         for (int v = 0; v < 3; v++) {
             box_add(b32, MS, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
-            box_add(b32, ME, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
+            if (verts) {
+                verts[lane][3 * v] = o[0];
+                verts[lane][3 * v + 1] = o[1];
+                verts[lane][3 * v + 2] = o[2];
+            }
+            box_add(b32, ME, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], oe[v], mag);
         }
         const float e32 = (float)geo_eps[body];
 #pragma unroll
@@ -283,8 +280,27 @@ __global__ void k_soup_filter(int n_soup, const Entry* __restrict__ soup, const 
             b32.hi[k] += e32;
         }
         mag += e32;
+        if (mags) {
+            // a distance is certain to be returned only while none of the
+            // triangle's edges can vanish on its way: no edge is shorter than
+            // 0.1 mm or changes by more than half
+            const float* q = verts[lane];
+            bool steady = true;
+#pragma unroll
+            for (int v = 0; v < 3; v++) {
+                const int v1 = (v + 1) % 3;
+                float l2 = 0.f, c2 = 0.f;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const float l = q[3 * v1 + k] - q[3 * v + k], c = (oe[v1][k] - oe[v][k]) - l;
+                    l2 += l * l;
+                    c2 += c * c;
+                }
+                steady = steady && l2 > 1e-8f && c2 < 0.2f * l2;
+            }
+            mags[lane] = steady ? mag : 3.4e38f;
+        }
     }
-    int res[2];
     bool border = false;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -334,6 +350,108 @@ __global__ void k_soup_filter(int n_soup, const Entry* __restrict__ soup, const 
             if (res[h] == 2) res[h] = box_overlap(A, B) ? 1 : 0;
         }
     }
+}
+
+// Counters of a traversal, on the device.
+enum { LC_LIST = 0, LC_NEXT, LC_LEAF, LC_ROOT, LC_TRI = 8, LC_TRI_N = 32, LC_SIZE = LC_TRI + LC_TRI_N };
+
+__device__ __forceinline__ void warp_append(int j, bool keep, int32_t* list, int32_t* count);
+
+__device__ __forceinline__ float vert_min(const float* a, const float* b) {
+    float m = 3.4e38f;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const float dx = a[3 * i] - b[3 * j], dy = a[3 * i + 1] - b[3 * j + 1], dz = a[3 * i + 2] - b[3 * j + 2];
+            m = fminf(m, dx * dx + dy * dy + dz * dz);
+        }
+    return sqrtf(m);
+}
+__device__ __forceinline__ float edge_min(const float* a, const float* b) {
+    float m = 3.4e38f;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int i1 = (i + 1) % 3, j1 = (j + 1) % 3;
+            float d2;
+            seg_vector(f3(a[3 * i], a[3 * i + 1], a[3 * i + 2]), f3(a[3 * i1], a[3 * i1 + 1], a[3 * i1 + 2]),
+                       f3(b[3 * j], b[3 * j + 1], b[3 * j + 2]), f3(b[3 * j1], b[3 * j1 + 1], b[3 * j1 + 2]), d2);
+            m = fminf(m, d2);
+        }
+    return sqrtf(m);
+}
+
+__global__ void __launch_bounds__(kBlock) k_ccd_level(
+    int n_soup, const Entry* __restrict__ soup, const int32_t* __restrict__ pairs, const double* __restrict__ pm,
+    const float* __restrict__ pm32, const int32_t* __restrict__ ntris, const double* __restrict__ tris,
+    const float* __restrict__ tri32, const double* __restrict__ geo_eps, const float* __restrict__ search,
+    const int4* __restrict__ nodes, const uint8_t* __restrict__ skip, const uint8_t* __restrict__ eskip,
+    int use_bounds, int32_t* __restrict__ entry_hits, int32_t* __restrict__ list, int32_t* __restrict__ lc) {
+    __shared__ float s_verts[kBlock / 32][16][9];
+    __shared__ float s_mag[kBlock / 32][16];
+    const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    if (w >= n_soup) return;  // uniform per warp
+    const Entry e = soup[w];
+    // a pair the root certificate proved contact-free, or a node pair its
+    // separation witness proved clear: no slot goes on
+    if ((skip && skip[e.pair]) || (eskip && eskip[w])) {
+        if (lane == 0) entry_hits[w] = 0;
+        return;
+    }
+    int res[2];
+    swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, s_verts[wi], s_mag[wi]);
+    const int k = __popc(__ballot_sync(0xffffffffu, res[0])) + __popc(__ballot_sync(0xffffffffu, res[1]));
+    if (lane == 0 && k) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), k);
+    bool sure = false;
+    if (ld_node(nodes, e.na).z || ld_node(nodes, e.nb).z) {
+        __syncwarp();
+        const float thr = search[e.pair];
+        float room[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
+            room[h] = -1.f;
+            if (!res[h] || !use_bounds || !(thr > 1e-6f)) continue;
+            room[h] = thr - (1e-3f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
+            sure = sure || vert_min(s_verts[wi][ta], s_verts[wi][8 + tb]) < room[h];
+        }
+        sure = __any_sync(0xffffffffu, sure);
+        if (!sure) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
+                if (room[h] > 0.f) sure = sure || edge_min(s_verts[wi][ta], s_verts[wi][8 + tb]) < room[h];
+            }
+            sure = __any_sync(0xffffffffu, sure);
+        }
+        if (!sure) {
+            warp_append(64 * w + lane, res[0] != 0, list, lc + LC_LIST);
+            warp_append(64 * w + lane + 32, res[1] != 0, list, lc + LC_LIST);
+        }
+    } else if (lane == 0 && k) {
+        atomicAdd(lc + LC_ROOT, 1);
+    }
+    if (lane == 0) entry_hits[w] = sure ? 1 : 0;
+}
+
+// The swept-box flags of the root node pairs that are two leaves (the soup
+// stage's only emitting ones); 0 for every other node pair's slots.
+__global__ void k_soup_filter(int n_soup, const Entry* __restrict__ soup, const int32_t* __restrict__ pairs,
+                              const double* __restrict__ pm, const float* __restrict__ pm32,
+                              const int32_t* __restrict__ ntris, const double* __restrict__ tris,
+                              const float* __restrict__ tri32, const double* __restrict__ geo_eps,
+                              const int4* __restrict__ nodes, const uint8_t* __restrict__ skip,
+                              int32_t* __restrict__ flags) {
+    const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (w >= n_soup) return;  // uniform per warp
+    const Entry e = soup[w];
+    int res[2] = {0, 0};
+    if (!(skip && skip[e.pair]) && !ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z)
+        swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, nullptr, nullptr);
     flags[64 * (size_t)w + lane] = res[0];
     flags[64 * (size_t)w + lane + 32] = res[1];
 }
@@ -724,7 +842,7 @@ struct PtWork {
     int32_t* hit;
 };
 __device__ __forceinline__ PtWork decode_pt(int j, int n_tp, const int32_t* items, const Entry* soup,
-                                            const Entry* conn, const int32_t* nn_off, int n_conn,
+                                            const Entry* conn, const int32_t* nn_off, const int32_t* tp,
                                             const int32_t* ntris, PrimResult* sub, PrimResult* cres, int32_t* chit) {
     PtWork w;
     w.hit = nullptr;
@@ -746,7 +864,7 @@ __device__ __forceinline__ PtWork decode_pt(int j, int n_tp, const int32_t* item
         return w;
     }
     const int jp = j - 6 * n_tp;
-    const int ei = find_entry(nn_off, n_conn, 6, jp);
+    const int ei = tp[jp / 6];
     const Entry e = conn[ei];
     const int l = jp - 6 * nn_off[ei];
     const int na = ntris[e.na], nb = ntris[e.nb];
@@ -775,7 +893,7 @@ struct EeWork {
     int32_t* hit;
 };
 __device__ __forceinline__ EeWork decode_ee(int j, int n_tp, const int32_t* items, const Entry* soup,
-                                            const Entry* conn, const int32_t* nn_off, int n_conn,
+                                            const Entry* conn, const int32_t* nn_off, const int32_t* tp,
                                             const int32_t* ntris, PrimResult* sub, PrimResult* cres, int32_t* chit) {
     EeWork w;
     w.hit = nullptr;
@@ -791,7 +909,7 @@ __device__ __forceinline__ EeWork decode_ee(int j, int n_tp, const int32_t* item
         w.out = sub + 15 * (size_t)k + 5 * w.aEdge + 2 + w.bEdge;
     } else {
         const int jp = j - 9 * n_tp;
-        const int ei = find_entry(nn_off, n_conn, 9, jp);
+        const int ei = tp[jp / 9];
         e = conn[ei];
         const int m = jp - 9 * nn_off[ei];
         const int na = ntris[e.na], nb = ntris[e.nb];
@@ -828,9 +946,32 @@ __device__ __forceinline__ void warp_append(int j, bool keep, int32_t* list, int
     if (keep) list[base + __popc(m & ((1u << lane) - 1u))] = j;
 }
 
+// The FP32 box bound of a point-triangle test: certainly farther apart than thr.
+__device__ __forceinline__ bool pt_box_gap(const float* __restrict__ pm32, int pair, int mC, int mT, const float* pt,
+                                           const float* tv, float thr) {
+    const float *Cs = pm32_of(pm32, pair, mC), *Ce = pm32_of(pm32, pair, mC + 1);
+    const float *tS = pm32_of(pm32, pair, mT), *tE = pm32_of(pm32, pair, mT + 1);
+    float mag = 0.f, ps[3], pe[3], o[3];
+    Box32 bp, bq, scratch;
+    box_init(bp);
+    box_init(bq);
+    box_init(scratch);
+    box_add(scratch, Cs, pt[0], pt[1], pt[2], ps, mag);
+    box_add(scratch, Ce, pt[0], pt[1], pt[2], pe, mag);
+    box_add(bp, tS, ps[0], ps[1], ps[2], o, mag);
+    box_add(bp, tS, pe[0], pe[1], pe[2], o, mag);
+    box_add(bp, tE, ps[0], ps[1], ps[2], o, mag);
+    box_add(bp, tE, pe[0], pe[1], pe[2], o, mag);
+    for (int v = 0; v < 3; v++) {
+        box_add(bq, tS, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
+        box_add(bq, tE, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
+    }
+    return box_gap(bp, bq) > thr + (1e-3f + 4e-6f * (mag + thr));  // NaN: not certain
+}
+
 __global__ void __launch_bounds__(kBlock) k_ccd_mask_pt(int n_tp, int n_total, const int32_t* __restrict__ items,
                                                         const Entry* __restrict__ soup, const Entry* __restrict__ conn,
-                                                        const int32_t* __restrict__ nn_off, int n_conn,
+                                                        const int32_t* __restrict__ nn_off, const int32_t* __restrict__ tp,
                                                         const float* __restrict__ pm32,
                                                         const int32_t* __restrict__ ntris,
                                                         const float* __restrict__ tri32,
@@ -841,28 +982,10 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_pt(int n_tp, int n_total, c
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     bool keep = false;
     if (j < n_total) {
-        const PtWork w = decode_pt(j, n_tp, items, soup, conn, nn_off, n_conn, ntris, sub, cres, chit);
+        const PtWork w = decode_pt(j, n_tp, items, soup, conn, nn_off, tp, ntris, sub, cres, chit);
         const float* pt = tri32 + ((size_t)w.pt_node * 8 + w.pt_tri) * 9 + 3 * w.pt_vert;
         const float* tv = tri32 + ((size_t)w.tri_node * 8 + w.tri_idx) * 9;
-        const float *Cs = pm32_of(pm32, w.pair, w.mC), *Ce = pm32_of(pm32, w.pair, w.mC + 1);
-        const float *tS = pm32_of(pm32, w.pair, w.mT), *tE = pm32_of(pm32, w.pair, w.mT + 1);
-        float mag = 0.f, ps[3], pe[3], o[3];
-        Box32 bp, bq, scratch;
-        box_init(bp);
-        box_init(bq);
-        box_init(scratch);
-        box_add(scratch, Cs, pt[0], pt[1], pt[2], ps, mag);
-        box_add(scratch, Ce, pt[0], pt[1], pt[2], pe, mag);
-        box_add(bp, tS, ps[0], ps[1], ps[2], o, mag);
-        box_add(bp, tS, pe[0], pe[1], pe[2], o, mag);
-        box_add(bp, tE, ps[0], ps[1], ps[2], o, mag);
-        box_add(bp, tE, pe[0], pe[1], pe[2], o, mag);
-        for (int v = 0; v < 3; v++) {
-            box_add(bq, tS, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
-            box_add(bq, tE, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
-        }
-        const float thr = search[w.pair];
-        keep = !use_bounds || !(box_gap(bp, bq) > thr + (1e-3f + 4e-6f * (mag + thr)));  // NaN keeps the test
+        keep = !use_bounds || !pt_box_gap(pm32, w.pair, w.mC, w.mT, pt, tv, search[w.pair]);
         if (!keep) record_no_contact(w.out, w.hit);
     }
     warp_append(j, keep, list, count);
@@ -870,7 +993,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_pt(int n_tp, int n_total, c
 
 __global__ void __launch_bounds__(kBlock) k_ccd_mask_ee(int n_tp, int n_total, const int32_t* __restrict__ items,
                                                         const Entry* __restrict__ soup, const Entry* __restrict__ conn,
-                                                        const int32_t* __restrict__ nn_off, int n_conn,
+                                                        const int32_t* __restrict__ nn_off, const int32_t* __restrict__ tp,
                                                         const float* __restrict__ pm32,
                                                         const int32_t* __restrict__ ntris,
                                                         const float* __restrict__ tri32,
@@ -881,7 +1004,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_ee(int n_tp, int n_total, c
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     bool keep = false;
     if (j < n_total) {
-        const EeWork w = decode_ee(j, n_tp, items, soup, conn, nn_off, n_conn, ntris, sub, cres, chit);
+        const EeWork w = decode_ee(j, n_tp, items, soup, conn, nn_off, tp, ntris, sub, cres, chit);
         const float* ta = tri32 + ((size_t)w.na * 8 + w.aTri) * 9;
         const float* tb = tri32 + ((size_t)w.nb * 8 + w.bTri) * 9;
         const int a0 = w.aEdge, a1 = w.aEdge == 2 ? 0 : w.aEdge + 1;
@@ -907,7 +1030,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_ee(int n_tp, int n_total, c
 
 __global__ void __launch_bounds__(kPrimBlock) k_prim_pt(int n_tp, int n_total, const int32_t* __restrict__ items,
                                                         const Entry* __restrict__ soup, const Entry* __restrict__ conn,
-                                                        const int32_t* __restrict__ nn_off, int n_conn,
+                                                        const int32_t* __restrict__ nn_off, const int32_t* __restrict__ tp,
                                                         const double* __restrict__ pm,
                                                         const int32_t* __restrict__ ntris,
                                                         const double* __restrict__ tris,
@@ -933,7 +1056,7 @@ __global__ void __launch_bounds__(kPrimBlock) k_prim_pt(int n_tp, int n_total, c
         return;
     }
     const int jp = j - 6 * n_tp;
-    const int ei = find_entry(nn_off, n_conn, 6, jp);
+    const int ei = tp[jp / 6];
     const Entry e = conn[ei];
     const int l = jp - 6 * nn_off[ei];
     const int na = ntris[e.na], nb = ntris[e.nb];
@@ -980,11 +1103,12 @@ __global__ void __launch_bounds__(kPrimBlock) k_prim_pt(int n_tp, int n_total, c
 // The first pass's iteration cap is the context setting D2G_TUNE_EE_FIRST_ITERS (default 2).
 constexpr int kEeRec = 10;  // saved test: t, min_dist, P, Q, toc, iterations done (the edges are recomputed)
 struct EeArgs {
-    int n_tp, n_conn;
+    int n_tp;
     const int32_t* items;
     const Entry* soup;
     const Entry* conn;
     const int32_t* nn_off;
+    const int32_t* tp;
     const int32_t* ntris;
     const float* search;
     PrimResult* sub;
@@ -1027,6 +1151,131 @@ __device__ __forceinline__ void ee_store_at(const EeArgs& a, int o, float thr, c
     }
 }
 
+// No point of the motion shortens the edge to nothing: its change is less than
+// half of it.
+__device__ __forceinline__ bool ee_steady(const Edge& S, const Edge& E) {
+    const V3 v = S.B - S.A, w = (E.B - E.A) - v;
+    return dot(w, w) < 0.25 * dot(v, v);
+}
+
+// The undecided slots of a level (list of node pair * 64 + slot): whether any
+// of their 15 sub-tests (continuous_comparison.h:692-777) returns a distance
+// below the search distance; a hit marks the node pair and ends its other
+// tests.  A thread a test, edge-edge tests first, in grid-stride order over
+// the list's device count.  FP32 bounds as in k_ccd_mask_pt / ee drop most
+// tests, and for edges also the gap along the closest points' direction at
+// the start, the smaller of the start's and the end's (the gap of linearly
+// moving points is concave in time).  An edge-edge test's distance at the
+// start decides it when it is a hit, or when it is beyond the search distance
+// by more than the motion (ee_motion_bound); only the rest runs edgeEdgeCCD.
+__global__ void __launch_bounds__(kPrimBlock) k_soup_tests(
+    const int32_t* __restrict__ list, const int32_t* __restrict__ n_list, const Entry* __restrict__ soup,
+    const double* __restrict__ pm, const float* __restrict__ pm32, const double* __restrict__ tris,
+    const float* __restrict__ tri32, const float* __restrict__ search, int32_t* entry_hits, int use_bounds,
+    int certificates, unsigned long long* ca_stats) {
+    const int n = *n_list;
+    const long long n_ee = 9LL * n, total = 15LL * n;
+    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < total;
+         j += (long long)gridDim.x * blockDim.x) {
+        const bool ee = j < n_ee;
+        const int k = (int)(ee ? j / 9 : (j - n_ee) / 6), q = (int)(ee ? j % 9 : (j - n_ee) % 6);
+        const int slot = list[k];
+        if (((volatile int32_t*)entry_hits)[slot >> 6]) continue;
+        const Entry e = soup[slot >> 6];
+        const int ta = (slot >> 3) & 7, tb = slot & 7;
+        const float thr = search[e.pair];
+        const float* fa = tri32 + ((size_t)e.na * 8 + ta) * 9;
+        const float* fb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
+        const double* M = pm + (size_t)PM_SIZE * e.pair;
+        const double* da = tris + (size_t)e.na * 72 + ta * 9;
+        const double* db = tris + (size_t)e.nb * 72 + tb * 9;
+        bool hit = false;
+        if (ee) {
+            const int ia = q / 3, ib = q % 3;
+            if (use_bounds) {
+                const int a1 = ia == 2 ? 0 : ia + 1, b1 = ib == 2 ? 0 : ib + 1;
+                float mag = 0.f, o[2][4][3];  // [start, end][a0 a1 b0 b1]
+                Box32 ba, bb;
+                box_init(ba);
+                box_init(bb);
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    const float* MA = pm32_of(pm32, e.pair, P32_AS + m);
+                    const float* MB = pm32_of(pm32, e.pair, P32_BS + m);
+                    box_add(ba, MA, fa[3 * ia], fa[3 * ia + 1], fa[3 * ia + 2], o[m][0], mag);
+                    box_add(ba, MA, fa[3 * a1], fa[3 * a1 + 1], fa[3 * a1 + 2], o[m][1], mag);
+                    box_add(bb, MB, fb[3 * ib], fb[3 * ib + 1], fb[3 * ib + 2], o[m][2], mag);
+                    box_add(bb, MB, fb[3 * b1], fb[3 * b1 + 1], fb[3 * b1 + 2], o[m][3], mag);
+                }
+                const float lim = thr + (1e-3f + 4e-6f * (mag + thr));
+                if (box_gap(ba, bb) > lim) continue;  // NaN keeps the test
+                auto at = [&](int m, int v) { return f3(o[m][v][0], o[m][v][1], o[m][v][2]); };
+                float d2;
+                const F3 d = seg_vector(at(0, 0), at(0, 1), at(0, 2), at(0, 3), d2);
+                const float g0 = fminf(dot3(d, at(0, 2)), dot3(d, at(0, 3))) - fmaxf(dot3(d, at(0, 0)), dot3(d, at(0, 1)));
+                const float g1 = fminf(dot3(d, at(1, 2)), dot3(d, at(1, 3))) - fmaxf(dot3(d, at(1, 0)), dot3(d, at(1, 1)));
+                if (fminf(g0, g1) > lim * sqrtf(d2)) continue;
+            }
+            const Edge ea = tedge(load_tri(da), ia), eb = tedge(load_tri(db), ib);
+            Edge aS, aE, bS, bE;
+            aS.A = xform_rigid(ea.A, M + PM_AS);
+            aS.B = xform_rigid(ea.B, M + PM_AS);
+            bS.A = xform_rigid(eb.A, M + PM_BS);
+            bS.B = xform_rigid(eb.B, M + PM_BS);
+            aE.A = xform_rigid(ea.A, M + PM_AE);
+            aE.B = xform_rigid(ea.B, M + PM_AE);
+            bE.A = xform_rigid(eb.A, M + PM_BE);
+            bE.B = xform_rigid(eb.B, M + PM_BE);
+            // while no edge can vanish on its way every distance is a number
+            if (thr > 1e-6f && ee_steady(aS, aE) && ee_steady(bS, bE)) {
+                V3 P, Q;
+                const double d0 = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q), lim = (double)thr;
+                hit = d0 < lim;
+                bool open = !hit;
+                if (open && certificates) {
+                    const V3 d = Q - P;
+                    const double g0 = fmin(dot(d, bS.A), dot(d, bS.B)) - fmax(dot(d, aS.A), dot(d, aS.B));
+                    const double g1 = fmin(dot(d, bE.A), dot(d, bE.B)) - fmax(dot(d, aE.A), dot(d, aE.B));
+                    const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
+                                            fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
+                    if (fmin(g0, g1) >= ((lim + 1e-6) + 1e-9 * mag) * d0) {
+                        open = false;
+                        atomicAdd(ca_stats, 1ull);
+                        atomicAdd(ca_stats + 1, (unsigned long long)(kEeNewtonIters - 1));
+                    }
+                }
+                if (open) {  // edgeEdgeCCD up to its first distance below the limit
+                    Ccd r;
+                    const double dot_start = ee_coplanarity(aS, bS);
+                    double best = DBL_MAX, t = 0.0;
+                    if (dot_start * ee_coplanarity(aE, bE) < 0.0) best = ee_bisect(aS, aE, bS, bE, dot_start, r);
+                    hit = best < lim;
+                    for (int iter = 0; iter < kEeNewtonIters && !hit && best > 1e-8; iter++) {
+                        const bool last = ee_newton_iter(aS, aE, bS, bE, t, best, r);
+                        hit = best < lim;
+                        if (last) break;
+                    }
+                }
+            } else {
+                hit = edge_edge_ccd(aS, aE, bS, bE).dist < (double)thr;
+            }
+        } else {
+            const int i = q >> 1;
+            const bool pb = (q & 1) != 0;  // a vertex of b against a, else of a against b
+            if (use_bounds) {
+                const float* pt = (pb ? fb : fa) + 3 * i;
+                const float* tv = pb ? fa : fb;
+                if (pt_box_gap(pm32, e.pair, pb ? P32_BAS : P32_ABS, pb ? P32_AS : P32_BS, pt, tv, thr)) continue;
+            }
+            const Tri A = load_tri(da), B = load_tri(db);
+            const Ccd r = pb ? point_tri_ccd(tvert(B, i), M + PM_BAS, M + PM_BAE, A, M + PM_AS, M + PM_AE)
+                             : point_tri_ccd(tvert(A, i), M + PM_ABS, M + PM_ABE, B, M + PM_BS, M + PM_BE);
+            hit = r.dist < (double)thr;
+        }
+        if (hit) entry_hits[slot >> 6] = 1;
+    }
+}
+
 __global__ void __launch_bounds__(kPrimBlock) k_ee_first(int n_total, const int32_t* __restrict__ list,
                                                          const int32_t* __restrict__ n_list,
                                                          const double* __restrict__ pm,
@@ -1041,7 +1290,7 @@ __global__ void __launch_bounds__(kPrimBlock) k_ee_first(int n_total, const int3
     int iters = 0;
     if (kk < n_total && kk < *n_list) {
         const int j = list[kk];
-        const EeWork w = decode_ee(j, a.n_tp, a.items, a.soup, a.conn, a.nn_off, a.n_conn, a.ntris, a.sub, a.cres,
+        const EeWork w = decode_ee(j, a.n_tp, a.items, a.soup, a.conn, a.nn_off, a.tp, a.ntris, a.sub, a.cres,
                                    a.chit);
         o = w.hit ? -1 - (int)(w.out - a.cres) : (int)(w.out - a.sub);
         thr = a.search[w.pair];
@@ -1219,7 +1468,7 @@ __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
     const int n_quads = (gridDim.x * blockDim.x) >> 2;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; i < n; i += n_quads) {
         const double* R = a.rec + (size_t)kEeRec * i;
-        const EeWork w = decode_ee(a.work[i], a.n_tp, a.items, a.soup, a.conn, a.nn_off, a.n_conn, a.ntris, a.sub,
+        const EeWork w = decode_ee(a.work[i], a.n_tp, a.items, a.soup, a.conn, a.nn_off, a.tp, a.ntris, a.sub,
                                    a.cres, a.chit);
         // this lane's component of the edges' endpoints at start and end
         // (xform_rigid's row `comp`, the same operations in the same order)
@@ -1293,13 +1542,10 @@ __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
 }
 
 // triTriCCDLinear's sequential (dist, toc) selection over its 15 sub-tests
-// (continuous_comparison.h:682-778), then the soup hit test (:817) and the
-// final-contact flag (a hit between two leaves, as k_final_flags sets it).
+// (continuous_comparison.h:682-778), then the soup hit test (:817).
 __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entry* __restrict__ soup,
                             const PrimResult* __restrict__ sub, const float* __restrict__ search,
-                            PrimResult* __restrict__ res, int32_t* __restrict__ hit,
-                            int32_t* __restrict__ entry_hits, const int4* __restrict__ nodes,
-                            int32_t* __restrict__ flags) {
+                            PrimResult* __restrict__ res, int32_t* __restrict__ hit) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
     PrimResult best;
@@ -1312,12 +1558,8 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
         if (c.dist < best.dist || (c.dist == best.dist && c.toc < best.toc)) best = c;
     }
     res[k] = best;
-    const int slot = items[k];
-    const Entry e = soup[slot >> 6];
-    const int h = best.dist < (double)search[e.pair] ? 1 : 0;
-    hit[k] = h;
-    if (h) atomicAdd(&entry_hits[slot >> 6], 1);
-    flags[k] = (h && !ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z) ? 1 : 0;
+    const Entry e = soup[items[k] >> 6];
+    hit[k] = best.dist < (double)search[e.pair] ? 1 : 0;
 }
 
 // ----------------------------------------------------------- discrete -----
@@ -1364,7 +1606,7 @@ __device__ __forceinline__ float ee_min(const float (&wa)[3][3], const float (&w
         for (int j = 0; j < 3; j++) {
             float d2;
             seg_vector(A[i], A[(i + 1) % 3], B[j], B[(j + 1) % 3], d2);
-            m = fminf(m, d2);  // NaN (a degenerate edge) is passed over
+            m = fminf(m, d2);
         }
     return sqrtf(m);
 }
@@ -1429,7 +1671,14 @@ __global__ void __launch_bounds__(kBlock) k_np_mask(int n_slots, const Entry* __
                     }
                     keep = !(sqrtf(gap2) > lim);
                 }
-                room = thr - (1e-3f + 4e-6f * mag);
+                // (a triangle that is almost a point has no edge that certainly returns a distance)
+                auto extent = [](const float(&q)[3][3]) {
+                    float m = 0.f;
+#pragma unroll
+                    for (int r = 0; r < 3; r++) m = fmaxf(m, fmaxf(fabsf(q[1][r] - q[0][r]), fabsf(q[2][r] - q[0][r])));
+                    return m;
+                };
+                room = extent(wa) > 1e-5f && extent(wb) > 1e-5f ? thr - (1e-3f + 4e-6f * mag) : -1.f;
                 if (keep && use_bounds && !(inner && vv_min(wa, wb) < room)) {
                     // Separating axes: along any direction n the distance is at
                     // least the gap between the projections divided by |n|,
@@ -1596,26 +1845,13 @@ __global__ void k_final_flags(int n, const int32_t* __restrict__ items, const En
 // Append flagged results as contact records (collision_detection/contact.h).
 __global__ void k_emit(int n, const int32_t* __restrict__ flags, const int32_t* __restrict__ off,
                        const int32_t* __restrict__ items, int slot_shift, const Entry* __restrict__ front,
-                       const int32_t* __restrict__ conn_off, int n_conn, const int32_t* __restrict__ pairs,
+                       const int32_t* __restrict__ tp, const int32_t* __restrict__ pairs,
                        const PrimResult* __restrict__ res, const double* __restrict__ res_eps,
                        const double* __restrict__ geo_eps, double* __restrict__ rec, int32_t* __restrict__ rec_pair,
                        int base) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || !flags[k]) return;
-    int ei;
-    if (conn_off) {
-        int lo = 0, hi = n_conn;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (conn_off[mid] <= k)
-                lo = mid;
-            else
-                hi = mid;
-        }
-        ei = lo;
-    } else {
-        ei = (items ? items[k] : k) >> slot_shift;
-    }
+    const int ei = tp ? tp[k / 15] : (items ? items[k] : k) >> slot_shift;
     const Entry e = front[ei];
     const int a = pairs[2 * e.pair], b = pairs[2 * e.pair + 1];
     const PrimResult& r = res[k];
@@ -1716,17 +1952,129 @@ __global__ void k_expand_write(int n, const Entry* __restrict__ front, const int
     }
 }
 
+// k_expand_count, its prefix sums and k_expand_write in one block for a level
+// of up to kExpandOneBlock node pairs (a launch instead of three; 6 us against
+// 18 at 2,700 node pairs): each thread takes a run of consecutive node pairs.
+// Children with an inner node go to next[0 ..), leaf pairs to leaf[lc[LC_LEAF]
+// ..); the totals go to lc and the level's list is emptied for the next one.
+constexpr int kExpandThreads = 1024, kExpandOneBlock = 24576;
+__device__ __forceinline__ int expand_rule(int4 A, int4 B) {  // 1: open a, 2: open b, 0: two leaves
+    if (!A.z && !B.z) return 0;
+    if (!A.z) return 2;
+    if (!B.z) return 1;
+    return A.w < B.w ? 1 : 2;
+}
+__global__ void __launch_bounds__(kExpandThreads) k_expand_level(int n, const Entry* __restrict__ front,
+                                                                 const int32_t* __restrict__ entry_hits,
+                                                                 const int4* __restrict__ nodes,
+                                                                 Entry* __restrict__ next, Entry* __restrict__ leaf,
+                                                                 int32_t* __restrict__ lc) {
+    __shared__ int2 wsum[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int per = (n + kExpandThreads - 1) / kExpandThreads;
+    const int i0 = min(n, tid * per), i1 = min(n, i0 + per);
+    int s = 0, c = 0;
+    auto open = [&](int i, Entry& e, int4& P, int& rule) {
+        if (entry_hits[i] <= 0) return false;
+        e = front[i];
+        const int4 A = ld_node(nodes, e.na), B = ld_node(nodes, e.nb);
+        rule = expand_rule(A, B);
+        P = rule == 1 ? A : B;
+        return rule != 0;
+    };
+    auto child = [&](const Entry& e, const int4& P, int rule, int ch) {
+        Entry x;
+        x.pair = e.pair;
+        x.na = rule == 1 ? P.x + ch : e.na;
+        x.nb = rule == 1 ? e.nb : P.x + ch;
+        return x;
+    };
+    for (int i = i0; i < i1; i++) {
+        Entry e;
+        int4 P;
+        int rule;
+        if (!open(i, e, P, rule)) continue;
+        for (int ch = 0; ch < P.y; ch++) {
+            const Entry x = child(e, P, rule, ch);
+            if (ld_node(nodes, x.na).z || ld_node(nodes, x.nb).z)
+                s++;
+            else
+                c++;
+        }
+    }
+    int xs = s, xc = c;  // inclusive warp scans
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int ys = __shfl_up_sync(0xffffffffu, xs, o), yc = __shfl_up_sync(0xffffffffu, xc, o);
+        if (lane >= o) {
+            xs += ys;
+            xc += yc;
+        }
+    }
+    if (lane == 31) wsum[w] = make_int2(xs, xc);
+    const int leaf0 = lc[LC_LEAF];
+    __syncthreads();
+    if (w == 0) {
+        int zs = wsum[lane].x, zc = wsum[lane].y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int ys = __shfl_up_sync(0xffffffffu, zs, o), yc = __shfl_up_sync(0xffffffffu, zc, o);
+            if (lane >= o) {
+                zs += ys;
+                zc += yc;
+            }
+        }
+        wsum[lane] = make_int2(zs, zc);
+    }
+    __syncthreads();
+    int os = xs - s + (w ? wsum[w - 1].x : 0), oc = leaf0 + xc - c + (w ? wsum[w - 1].y : 0);
+    for (int i = i0; i < i1; i++) {
+        Entry e;
+        int4 P;
+        int rule;
+        if (!open(i, e, P, rule)) continue;
+        for (int ch = 0; ch < P.y; ch++) {
+            const Entry x = child(e, P, rule, ch);
+            if (ld_node(nodes, x.na).z || ld_node(nodes, x.nb).z)
+                next[os++] = x;
+            else
+                leaf[oc++] = x;
+        }
+    }
+    if (tid == 0) {
+        lc[LC_LIST] = 0;
+        lc[LC_NEXT] = wsum[31].x;
+        lc[LC_LEAF] = leaf0 + wsum[31].y;
+    }
+}
+
+// The totals of a larger level's prefix sums, as k_expand_level leaves them.
+__global__ void k_expand_totals(const int32_t* __restrict__ n_next, const int32_t* __restrict__ n_leaf,
+                                int32_t* __restrict__ lc) {
+    lc[LC_LIST] = 0;
+    lc[LC_NEXT] = *n_next;
+    lc[LC_LEAF] += *n_leaf;
+}
+
 // ---------------------------------------------------------- output sort ----
 __global__ void k_iota(int n, int32_t* __restrict__ v) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) v[i] = i;
 }
-__global__ void k_count_pairs(int n, int p0, int n_pairs, const int32_t* __restrict__ rec_pair,
-                              int32_t* __restrict__ cnt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int p = rec_pair[i] - p0;
-    if (p >= 0 && p < n_pairs) atomicAdd(&cnt[p], 1);
+// First record of every pair in the sorted pair ids: out[p] for p in [0, n_pairs].
+__global__ void k_pair_offsets(int n, int p0, int n_pairs, const int32_t* __restrict__ rec_pair,
+                               int32_t* __restrict__ out) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p > n_pairs) return;
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (rec_pair[mid] < p0 + p)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    out[p] = lo;
 }
 __global__ void k_gather(int n, const int32_t* __restrict__ idx, const double* __restrict__ in,
                          double* __restrict__ out) {
@@ -1816,10 +2164,10 @@ void prof_collect(d2g_ctx* ctx) {
 constexpr int kScanThreads = 1024, kScanPer = 8, kScanChunk = kScanThreads * kScanPer;
 static_assert(kScanThreads == 32 * 32, "the warp-sum scan assumes 32 warps");
 constexpr int kScanOneBlock = 4 * kScanChunk;  // larger arrays go to cub
-struct ScanSeg {  // up to four independent scans, one block each
-    const int32_t* in[4];
-    int32_t* out[4];
-    int n[4];
+struct ScanSeg {  // up to two independent scans, one block each
+    const int32_t* in[2];
+    int32_t* out[2];
+    int n[2];
 };
 __global__ void __launch_bounds__(kScanThreads) k_scan1(ScanSeg sg) {
     __shared__ int32_t buf[kScanChunk];
@@ -1910,26 +2258,6 @@ int scan2(d2g_ctx* ctx, const int32_t* in0, int32_t* out0, int n0, const int32_t
     return scan(ctx, in1, out1, n1);
 }
 
-// Four scans in one launch when each fits one block, else one by one.
-int scan4(d2g_ctx* ctx, const int32_t* const* in, int32_t* const* out, const int* n) {
-    ScanSeg sg;
-    bool one = true;
-    for (int i = 0; i < 4; i++) {
-        sg.in[i] = in[i];
-        sg.out[i] = out[i];
-        sg.n[i] = n[i];
-        one = one && n[i] <= kScanOneBlock;
-    }
-    if (one) {
-        k_scan1<<<4, kScanThreads, 0, ctx->stream>>>(sg);
-        ctx->eng.launches++;
-        return D2G_OK;
-    }
-    for (int i = 0; i < 4; i++)
-        if (int rc = scan(ctx, in[i], out[i], n[i])) return rc;
-    return D2G_OK;
-}
-
 // Read k device int32 scalars (after the stream's pending work).
 int read_scalars(d2g_ctx* ctx, const int32_t* const* src, int k, int32_t* dst) {
     for (int i = 0; i < k; i++)
@@ -1951,9 +2279,7 @@ int read_scalars(d2g_ctx* ctx, const int32_t* const* src, int k, int32_t* dst) {
 int finish_records(d2g_ctx* ctx, int n_pairs, int n_rec, int p0 = 0) {
     Engine& E = ctx->eng;
     RC(E.out_off.ensure(n_pairs + 1));
-    RC(E.pair_cnt.ensure(n_pairs + 1));
     RC(E.rec_sorted.ensure(14 * (size_t)n_rec + 14));
-    D2G_CUDA(cudaMemsetAsync(E.pair_cnt.p, 0, sizeof(int32_t) * (n_pairs + 1), ctx->stream));
     if (n_rec > 0) {
         RC(E.rec_idx.ensure(n_rec));
         RC(E.rec_idx_sorted.ensure(n_rec));
@@ -1968,9 +2294,8 @@ int finish_records(d2g_ctx* ctx, int n_pairs, int n_rec, int p0 = 0) {
         D2G_CUDA(cub::DeviceRadixSort::SortPairs(E.cub_tmp.p, bytes, E.rec_pair.p, E.rec_pair_sorted.p, E.rec_idx.p,
                                                  E.rec_idx_sorted.p, n_rec, 0, bits, ctx->stream));
         LAUNCH(k_gather, n_rec, n_rec, E.rec_idx_sorted.p, E.rec.p, E.rec_sorted.p);
-        LAUNCH(k_count_pairs, n_rec, n_rec, p0, n_pairs, E.rec_pair.p, E.pair_cnt.p);
     }
-    RC(scan(ctx, E.pair_cnt.p, E.out_off.p, n_pairs));
+    LAUNCH(k_pair_offsets, n_pairs + 1, n_rec, p0, n_pairs, E.rec_pair_sorted.p, E.out_off.p);
     return D2G_OK;
 }
 
@@ -1990,10 +2315,9 @@ void prof_mark_collect(d2g_ctx* ctx) { prof_collect(ctx); }
 
 // Append flagged results (already scanned into `off`) as contact records at `base`.
 void emit_records(d2g_ctx* ctx, int n, const int32_t* flags, const int32_t* off, const int32_t* items, int shift,
-                  const Entry* front, const int32_t* conn_off, int n_conn, const int32_t* d_pairs,
-                  const PrimResult* res, int base) {
+                  const Entry* front, const int32_t* tp, const int32_t* d_pairs, const PrimResult* res, int base) {
     Engine& E = ctx->eng;
-    LAUNCH(k_emit, n, n, flags, off, items, shift, front, conn_off, n_conn, d_pairs, res, nullptr, ctx->geo_eps.p,
+    LAUNCH(k_emit, n, n, flags, off, items, shift, front, tp, d_pairs, res, nullptr, ctx->geo_eps.p,
            E.rec.p, E.rec_pair.p, base);
 }
 
@@ -2009,6 +2333,19 @@ int ee_grid_size(d2g_ctx* ctx, int* grid) {
         E.ee_grid = std::max(1, dev_sms * std::max(1, per_sm));
     }
     *grid = E.ee_grid;
+    return D2G_OK;
+}
+
+// Grid of k_soup_tests, which reads its list's length from device memory too.
+int soup_grid_size(d2g_ctx* ctx, int* grid) {
+    Engine& E = ctx->eng;
+    if (E.soup_grid == 0) {
+        int dev_sms = 0, per_sm = 0;
+        D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
+        D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_soup_tests, kPrimBlock, 0));
+        E.soup_grid = std::max(1, dev_sms * std::max(1, per_sm));
+    }
+    *grid = E.soup_grid;
     return D2G_OK;
 }
 
@@ -2099,6 +2436,215 @@ int read_ccd_stats(d2g_ctx* ctx, int64_t* out, int n, bool reset) {
     return D2G_OK;
 }
 
+// A descent's outcome: whether it passed the byte budget, the node pairs
+// and swept (or valid) triangle pairs it saw, its levels and the leaf pairs it
+// left in E.conn, in level order.
+struct Traversal {
+    bool abandon = false;
+    double peak = 0.0;
+    int64_t nodes = 0, tri = 0, levels = 0;
+    int n_leaf = 0, n_root = 0;  // n_root: root pairs of two leaves with candidate slots
+};
+
+// Descends from the n node pairs in E.soup: per level `decide` marks the node
+// pairs with a hit in E.entry_hits, and their children go to the next level
+// or, two leaves, onto E.conn.  One read of the counts per level.
+template <class F>
+int descend(d2g_ctx* ctx, int n, double budget, bool may_abandon, Traversal& T, F decide) {
+    Engine& E = ctx->eng;
+    cudaStream_t s = ctx->stream;
+    RC(E.lc.ensure(LC_SIZE));
+    D2G_CUDA(cudaMemsetAsync(E.lc.p, 0, sizeof(int32_t) * LC_SIZE, s));
+    int new_leaf = 0;
+    while (n > 0) {
+        // past the budget (768 bytes a node pair: its slot list and its
+        // children), or past 32-bit slot indices (64 slots per node pair)
+        const double need = 64.0 * 8.0 * 1.5 * n;
+        if ((need > budget || 64LL * n > (long long)INT32_MAX / 2) && may_abandon) {
+            T.abandon = true;
+            return D2G_OK;
+        }
+        T.peak = std::max(T.peak, need / budget);
+        T.levels++;
+        T.nodes += n;
+        RC(E.entry_hits.ensure(n + 1));
+        RC(decide(n));
+        RC(E.soup_next.ensure(8 * (size_t)n + 1));  // a node has at most 8 children
+        RC(E.conn.ensure_keep((size_t)T.n_leaf + 8 * (size_t)n + 1, (size_t)T.n_leaf, s));
+        if (n <= kExpandOneBlock) {
+            k_expand_level<<<1, kExpandThreads, 0, s>>>(n, E.soup.p, E.entry_hits.p, ctx->nodes.p, E.soup_next.p,
+                                                        E.conn.p, E.lc.p);
+            E.launches++;
+        } else {
+            RC(E.cnt_a.ensure(n));
+            RC(E.cnt_b.ensure(n));
+            RC(E.off_a.ensure(n + 1));
+            RC(E.off_b.ensure(n + 1));
+            LAUNCH(k_expand_count, n, n, E.soup.p, E.entry_hits.p, ctx->nodes.p, 1, E.cnt_a.p, E.cnt_b.p);
+            RC(scan2(ctx, E.cnt_a.p, E.off_a.p, n, E.cnt_b.p, E.off_b.p, n));
+            LAUNCH(k_expand_write, n, n, E.soup.p, E.entry_hits.p, ctx->nodes.p, 1, E.off_a.p, E.off_b.p,
+                   E.soup_next.p, E.conn.p + T.n_leaf);
+            k_expand_totals<<<1, 1, 0, s>>>(E.off_a.p + n, E.off_b.p + n, E.lc.p);
+            E.launches++;
+        }
+        D2G_CUDA(cudaMemcpyAsync(ctx->h_pinned, E.lc.p, sizeof(int32_t) * LC_SIZE, cudaMemcpyDeviceToHost, s));
+        D2G_CUDA(cudaStreamSynchronize(s));
+        prof_collect(ctx);
+        std::swap(E.soup, E.soup_next);
+        n = ctx->h_pinned[LC_NEXT];
+        new_leaf = ctx->h_pinned[LC_LEAF] - T.n_leaf;
+        T.n_leaf = ctx->h_pinned[LC_LEAF];
+        T.n_root = ctx->h_pinned[LC_ROOT];
+        for (int k = 0; k < LC_TRI_N; k++) T.tri += (uint32_t)ctx->h_pinned[LC_TRI + k];
+        D2G_CUDA(cudaMemsetAsync(E.lc.p + LC_TRI, 0, sizeof(int32_t) * LC_TRI_N, s));
+    }
+    if (new_leaf > 0) T.levels++;  // the last level's leaf pairs are a level of the reference's
+    return D2G_OK;
+}
+
+// The FP64 tests of the descent's leaf pairs (E.conn, in level order), and of
+// the chunk's root pairs that are two leaves (soup stage: the best of a
+// triangle pair's 15 tests); their contacts are appended to E.rec.  Large lists
+// run in ranges that keep the test buffers within the budget.
+int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, int p0, int p1, const Traversal& T,
+                   double budget, int* n_rec_io, long long* n_pp, bool* abandon) {
+    Engine& E = ctx->eng;
+    cudaStream_t s = ctx->stream;
+    int ee_grid = 0;
+    RC(ee_grid_size(ctx, &ee_grid));
+    int n_rec = *n_rec_io;
+    // ~1900 bytes of test buffers per triangle pair (x1.5 growth slack), at most 64 in a leaf pair
+    const int range = (int)std::min(1.0e6, std::max(256.0, budget / (1.5 * 1900.0 * 64.0)));
+    for (int c0 = T.n_root > 0 ? -1 : 0; c0 < T.n_leaf; c0 = c0 < 0 ? 0 : c0 + range) {
+        // c0 = -1: the roots; else the leaf pairs [c0, c0 + n_conn)
+        const int n_soup = c0 < 0 ? p1 - p0 : 0, n_conn = c0 < 0 ? 0 : std::min(range, T.n_leaf - c0);
+        const Entry* soup = E.roots.p + p0;
+        const Entry* conn = E.conn.p + (c0 < 0 ? 0 : c0);
+        const int n_slots = 64 * n_soup;
+        int K = 0, P = 0;  // soup triangle pairs, leaf-pair triangle pairs
+        if (n_soup > 0) {
+            if (64LL * n_soup > (long long)INT32_MAX / 2 && p1 - p0 > 1) {
+                *abandon = true;
+                return D2G_OK;
+            }
+            RC(E.flags.ensure(n_slots + 1));
+            RC(E.flag_off.ensure(n_slots + 1));
+            LAUNCH(k_soup_filter, 32LL * n_soup, n_soup, soup, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p,
+                   ctx->tri32.p, ctx->geo_eps.p, ctx->nodes.p, skip, E.flags.p);
+            RC(scan(ctx, E.flags.p, E.flag_off.p, n_slots));
+            const int32_t* src = E.flag_off.p + n_slots;
+            RC(read_scalars(ctx, &src, 1, &K));
+        } else {
+            RC(E.nn_cnt.ensure(n_conn + 1));
+            RC(E.nn_off.ensure(n_conn + 1));
+            LAUNCH(k_conn_nn, n_conn, n_conn, conn, ctx->ntris.p, E.nn_cnt.p);
+            RC(scan(ctx, E.nn_cnt.p, E.nn_off.p, n_conn));
+            const int32_t* src = E.nn_off.p + n_conn;
+            RC(read_scalars(ctx, &src, 1, &P));
+            RC(E.tp.ensure((size_t)P + 1));
+            LAUNCH(k_tp_fill, 32LL * n_conn, n_conn, E.nn_off.p, E.tp.p);
+            *n_pp += P;
+        }
+        if (15LL * K + 15LL * P > (long long)INT32_MAX || 1.5 * 1900.0 * (double)K > budget) {
+            if (p1 - p0 > 1) {  // test indices are 32-bit; the budget
+                *abandon = true;
+                return D2G_OK;
+            }
+            if (15LL * K + 15LL * P > (long long)INT32_MAX) {
+                set_error("CCD call with " + std::to_string(K) + " + " + std::to_string(P) +
+                          " triangle pairs in one body pair exceeds the 32-bit test index range");
+                return D2G_ERR_INVALID;
+            }
+        }
+        if (K + P == 0) continue;
+        RC(E.items.ensure(K + 1));
+        RC(E.sub.ensure(15 * (size_t)K + 1));
+        RC(E.res.ensure(K + 1));
+        RC(E.hit.ensure(K + 1));
+        RC(E.cres.ensure(15 * (size_t)P + 1));
+        RC(E.chit.ensure(15 * (size_t)P + 1));
+        RC(E.cflag_off.ensure(15 * (size_t)P + 1));
+        RC(E.tp.ensure((size_t)P + 1));
+        if (n_soup > 0) LAUNCH(k_compact, n_slots, n_slots, E.flags.p, E.flag_off.p, E.items.p);
+        const int n_pt = 6 * K + 6 * P, n_ee = 9 * K + 9 * P;
+        // FP32 bounds drop the tests that cannot hit; the FP64 kernels run on
+        // the survivors, which the bound kernels append to their lists
+        RC(E.ccd_cnt.ensure(3));
+        RC(E.ccd_list.ensure((size_t)n_pt + n_ee + 2));
+        int32_t* cnt_pt = E.ccd_cnt.p;
+        int32_t* cnt_ee = E.ccd_cnt.p + 1;
+        int32_t* cnt_rest = E.ccd_cnt.p + 2;  // edge-edge tests continued by k_ee_rest4
+        int32_t* list_pt = E.ccd_list.p;
+        int32_t* list_ee = E.ccd_list.p + n_pt;
+        D2G_CUDA(cudaMemsetAsync(E.ccd_cnt.p, 0, 3 * sizeof(int32_t), s));
+        RC(E.ee_rec.ensure((size_t)kEeRec * n_ee));
+        RC(E.ee_work.ensure(n_ee));
+        // The point-triangle and edge-edge chains touch disjoint outputs: the
+        // edge-edge chain runs on the second stream beside the other.
+        cudaStream_t s_ee = ctx->stream2;
+        D2G_CUDA(cudaEventRecord(ctx->ev_fork, s));
+        D2G_CUDA(cudaStreamWaitEvent(s_ee, ctx->ev_fork, 0));
+        k_ccd_mask_ee<<<nblocks(n_ee), kBlock, 0, s_ee>>>(K, n_ee, E.items.p, soup, conn, E.nn_off.p, E.tp.p,
+                                                          E.pm32c.p, ctx->ntris.p, ctx->tri32.p, E.search.p, E.sub.p,
+                                                          E.cres.p, E.chit.p, list_ee, cnt_ee, E.fp32_bounds ? 1 : 0);
+        const int pfe = prof_begin(ctx, PROF_CONN, n_ee, s_ee);
+        EeArgs ea;
+        ea.n_tp = K;
+        ea.items = E.items.p;
+        ea.soup = soup;
+        ea.conn = conn;
+        ea.nn_off = E.nn_off.p;
+        ea.tp = E.tp.p;
+        ea.ntris = ctx->ntris.p;
+        ea.search = E.search.p;
+        ea.sub = E.sub.p;
+        ea.cres = E.cres.p;
+        ea.chit = E.chit.p;
+        ea.pm = E.pm.p;
+        ea.tris = ctx->tris.p;
+        ea.rec = E.ee_rec.p;
+        ea.work = E.ee_work.p;
+        ea.count = cnt_rest;
+        ea.first_iters = E.tune[D2G_TUNE_EE_FIRST_ITERS];
+        ea.certificates = E.certificates ? 1 : 0;
+        ea.ca_stats = E.ccd_stats.p;
+        k_ee_first<<<nblocks(n_ee, kPrimBlock), kPrimBlock, 0, s_ee>>>(n_ee, list_ee, cnt_ee, E.pm.p, ctx->tris.p,
+                                                                      ea);
+        k_ee_rest4<<<ee_grid, kBlock, 0, s_ee>>>(ea);
+        ctx->eng.launches += 3;
+        prof_end(ctx, pfe, s_ee);
+        LAUNCH(k_ccd_mask_pt, n_pt, K, n_pt, E.items.p, soup, conn, E.nn_off.p, E.tp.p, E.pm32c.p, ctx->ntris.p,
+               ctx->tri32.p, E.search.p, E.sub.p, E.cres.p, E.chit.p, list_pt, cnt_pt, E.fp32_bounds ? 1 : 0);
+        const int pfp = prof_begin(ctx, PROF_SOUP_CCD, n_pt);
+        LAUNCHB(k_prim_pt, n_pt, kPrimBlock, K, n_pt, E.items.p, soup, conn, E.nn_off.p, E.tp.p, E.pm.p, ctx->ntris.p,
+                ctx->tris.p, E.search.p, E.sub.p, E.cres.p, E.chit.p, list_pt, cnt_pt);
+        prof_end(ctx, pfp);
+        D2G_CUDA(cudaEventRecord(ctx->ev_join, s_ee));
+        D2G_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
+        // contacts, in order
+        int32_t fin = 0;
+        const int32_t* src;
+        if (n_soup > 0) {
+            LAUNCH(k_soup_fold, K, K, E.items.p, soup, E.sub.p, E.search.p, E.res.p, E.hit.p);
+            RC(scan(ctx, E.hit.p, E.flag_off.p, K));
+            src = E.flag_off.p + K;
+        } else {
+            RC(scan(ctx, E.chit.p, E.cflag_off.p, 15 * P));
+            src = E.cflag_off.p + 15 * P;
+        }
+        RC(read_scalars(ctx, &src, 1, &fin));
+        RC(E.rec.ensure_keep(14 * (size_t)(n_rec + fin + 1), 14 * (size_t)n_rec, s));
+        RC(E.rec_pair.ensure_keep((size_t)(n_rec + fin + 1), (size_t)n_rec, s));
+        if (fin > 0 && n_soup > 0)
+            emit_records(ctx, K, E.hit.p, E.flag_off.p, E.items.p, 6, soup, nullptr, d_pairs, E.res.p, n_rec);
+        else if (fin > 0)
+            emit_records(ctx, 15 * P, E.chit.p, E.cflag_off.p, nullptr, 0, conn, E.tp.p, d_pairs, E.cres.p, n_rec);
+        n_rec += fin;
+    }
+    *n_rec_io = n_rec;
+    return D2G_OK;
+}
+
 int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int n_pairs, int* n_out,
             int64_t* counters, const CcdSink* sink) {
     Engine& E = ctx->eng;
@@ -2110,8 +2656,8 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
     RC(E.pfut.ensure(28 * (size_t)n_pairs + 1));
     RC(E.search.ensure(n_pairs + 1));
     RC(E.soup.ensure(n_pairs + 1));
-    int ee_grid = 0;
-    RC(ee_grid_size(ctx, &ee_grid));
+    int test_grid = 0;
+    RC(soup_grid_size(ctx, &test_grid));
     int n_rec = 0;
     long long n_streamed = 0;  // records handed to the sink
     if (n_pairs > 0)
@@ -2152,213 +2698,59 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
     int chunk = E.ccd_chunk > 0 ? std::min(n_pairs, E.ccd_chunk) : n_pairs;
     double peak = 0.0;  // largest level need / budget among finished chunks
     for (int p0 = 0; p0 < n_pairs;) {
-    const int p1 = std::min(n_pairs, p0 + chunk);
-    const int rec_start = n_rec;
-    int64_t k_node = 0, k_tri = 0, k_leaf = 0, k_levels = 0;
-    bool abandon = false;
-    double chunk_peak = 0.0;
-    RC(E.soup.ensure((size_t)(p1 - p0) + 1));  // the frontiers swap every level: this one may be the smaller
-    D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
-    int n_soup = p1 - p0, n_conn = 0;
-    while (n_soup > 0 || n_conn > 0) {
-        // past the budget, or past 32-bit slot indices (64 slots per node pair)
-        if ((64.0 * 8.0 * 1.5 * n_soup > budget || 64LL * n_soup > (long long)INT32_MAX / 2) && p1 - p0 > 1) {
-            abandon = true;
-            break;
-        }
-        chunk_peak = std::max(chunk_peak, 64.0 * 8.0 * 1.5 * n_soup / budget);
-        k_levels++;
-        k_node += n_soup + n_conn;
-        k_leaf += n_conn;
-        // (1) soup swept-box filter and leaf-pair sizes, one synchronisation
-        const int n_slots = 64 * n_soup;
-        RC(E.flags.ensure(n_slots + 1));
-        RC(E.flag_off.ensure(n_slots + 1));
-        RC(E.entry_hits.ensure(n_soup + 1));
-        RC(E.nn_cnt.ensure(n_conn + 1));
-        RC(E.nn_off.ensure(n_conn + 1));
-        RC(E.citem_off.ensure(n_conn + 1));
-        if (n_soup > 0) {
-            D2G_CUDA(cudaMemsetAsync(E.entry_hits.p, 0, sizeof(int32_t) * n_soup, s));
-            const int pff = prof_begin(ctx, PROF_SOUP_FILTER, n_slots);
+        const int p1 = std::min(n_pairs, p0 + chunk);
+        const int rec_start = n_rec;
+        Traversal T;
+        RC(E.soup.ensure((size_t)(p1 - p0) + 1));  // the frontiers swap every level: this one may be the smaller
+        D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
+        RC(descend(ctx, p1 - p0, budget, p1 - p0 > 1, T, [&](int n_soup) -> int {
+            RC(E.ccd_list.ensure(64 * (size_t)n_soup));
+            const int pff = prof_begin(ctx, PROF_SOUP_FILTER, 64LL * n_soup);
             const uint8_t* eskip = nullptr;
             if (E.witnesses) {
                 RC(E.wt_flag.ensure(n_soup + 1));
                 LAUNCH(k_witness_check, 32LL * n_soup, n_soup, E.soup.p, d_pairs, E.pm.p, E.pm32c.p, ctx->tri32.p,
-                       ctx->mesh.p,
-                       ctx->mesh_node_off.p, ctx->ntris.p, ctx->tris.p, ctx->geo_eps.p, E.search.p, E.wt_table.p,
-                       E.wt_log2cap, E.wt_flag.p, E.ccd_stats.p);
+                       ctx->mesh.p, ctx->mesh_node_off.p, ctx->ntris.p, ctx->tris.p, ctx->geo_eps.p, E.search.p,
+                       E.wt_table.p, E.wt_log2cap, E.wt_flag.p, E.ccd_stats.p);
                 eskip = E.wt_flag.p;
             }
-            LAUNCH(k_soup_filter, 32LL * n_soup, n_soup, E.soup.p, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p,
-                   ctx->tris.p, ctx->tri32.p, ctx->geo_eps.p, skip, eskip, E.flags.p);
+            LAUNCH(k_ccd_level, 32LL * n_soup, n_soup, E.soup.p, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p,
+                   ctx->tri32.p, ctx->geo_eps.p, E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0,
+                   E.entry_hits.p, E.ccd_list.p, E.lc.p);
             prof_end(ctx, pff);
-        }
-        if (n_conn > 0) LAUNCH(k_conn_nn, n_conn, n_conn, E.conn.p, ctx->ntris.p, E.nn_cnt.p);
-        RC(scan2(ctx, E.flags.p, E.flag_off.p, n_slots, E.nn_cnt.p, E.nn_off.p, n_conn));
-        int32_t tot1[2];
-        const int32_t* src1[2] = {E.flag_off.p + n_slots, E.nn_off.p + n_conn};
-        RC(read_scalars(ctx, src1, 2, tot1));
-        const int K = tot1[0], P = tot1[1];  // soup triangle pairs, leaf-pair triangle pairs
-        if (15LL * K + 15LL * P > (long long)INT32_MAX) {  // test indices are 32-bit
-            if (p1 - p0 > 1) {
-                abandon = true;
-                break;
+            k_soup_tests<<<test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p, E.pm32c.p,
+                                                          ctx->tris.p, ctx->tri32.p, E.search.p, E.entry_hits.p,
+                                                          E.fp32_bounds ? 1 : 0, E.certificates ? 1 : 0,
+                                                          E.ccd_stats.p);
+            E.launches++;
+            if (E.witnesses) {
+                LAUNCH(k_witness_make, 32LL * n_soup, n_soup, E.soup.p, E.entry_hits.p, E.wt_flag.p, skip, d_pairs,
+                       E.pm.p, E.pm32c.p, ctx->tri32.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->ntris.p, ctx->tris.p,
+                       ctx->geo_eps.p, E.search.p, E.wt_table.p, E.wt_log2cap, E.ccd_stats.p);
+                E.wt_inserts += n_soup;
             }
-            set_error("CCD level with " + std::to_string(K) + " + " + std::to_string(P) +
-                      " triangle pairs exceeds the 32-bit test index range");
-            return D2G_ERR_INVALID;
+            return D2G_OK;
+        }));
+        bool abandon = T.abandon;
+        long long n_pp = 0;  // leaf pairs' triangle pairs
+        if (!abandon) RC(ccd_leaf_tests(ctx, d_pairs, skip, p0, p1, T, budget, &n_rec, &n_pp, &abandon));
+        if (abandon) {
+            n_rec = rec_start;
+            chunk = std::max(1, (p1 - p0) / 2);
+            continue;
         }
-        // bytes of the level's test buffers (x1.5 for the buffers' growth slack)
-        if (1.5 * 1900.0 * ((double)K + (double)P) > budget && p1 - p0 > 1) {
-            abandon = true;
-            break;
+        c_node += T.nodes + T.n_leaf;
+        c_tri += T.tri + 15 * n_pp;
+        c_leaf += T.n_leaf;
+        c_levels += T.levels;
+        peak = std::max(peak, T.peak);
+        if (sink) {  // the chunk's records, sorted by pair, go to the consumer and are dropped
+            RC(finish_records(ctx, p1 - p0, n_rec, p0));
+            RC(sink->consume(ctx, sink->user, p0, p1));
+            n_streamed += n_rec;
+            n_rec = 0;
         }
-        chunk_peak = std::max(chunk_peak, 1.5 * 1900.0 * ((double)K + (double)P) / budget);
-        k_tri += (int64_t)K + 15 * (int64_t)P;
-        // (2) all primitive tests of the level
-        RC(E.items.ensure(K + 1));
-        RC(E.sub.ensure(15 * (size_t)K + 1));
-        RC(E.res.ensure(K + 1));
-        RC(E.hit.ensure(K + 1));
-        RC(E.cres.ensure(15 * (size_t)P + 1));
-        RC(E.chit.ensure(15 * (size_t)P + 1));
-        RC(E.cflag_off.ensure(15 * (size_t)P + 1));
-        if (n_soup > 0) LAUNCH(k_compact, n_slots, n_slots, E.flags.p, E.flag_off.p, E.items.p);
-        const int n_pt = 6 * K + 6 * P, n_ee = 9 * K + 9 * P;
-        // FP32 bounds drop the tests that cannot hit; the FP64 kernels run on
-        // the survivors, which the bound kernels append to their lists
-        RC(E.ccd_cnt.ensure(3));
-        RC(E.ccd_list.ensure((size_t)n_pt + n_ee + 2));
-        int32_t* cnt_pt = E.ccd_cnt.p;
-        int32_t* cnt_ee = E.ccd_cnt.p + 1;
-        int32_t* cnt_rest = E.ccd_cnt.p + 2;  // edge-edge tests continued by k_ee_rest4
-        int32_t* list_pt = E.ccd_list.p;
-        int32_t* list_ee = E.ccd_list.p + n_pt;
-        D2G_CUDA(cudaMemsetAsync(E.ccd_cnt.p, 0, 3 * sizeof(int32_t), s));
-        if (n_ee > 0) {
-            RC(E.ee_rec.ensure((size_t)kEeRec * n_ee));
-            RC(E.ee_work.ensure(n_ee));
-        }
-        // The point-triangle and edge-edge chains touch disjoint outputs: the
-        // edge-edge chain runs on the second stream beside the other.
-        const bool fork = n_pt > 0 && n_ee > 0;
-        cudaStream_t s_ee = fork ? ctx->stream2 : s;
-        if (fork) {
-            D2G_CUDA(cudaEventRecord(ctx->ev_fork, s));
-            D2G_CUDA(cudaStreamWaitEvent(s_ee, ctx->ev_fork, 0));
-        }
-        if (n_ee > 0) {
-            k_ccd_mask_ee<<<nblocks(n_ee), kBlock, 0, s_ee>>>(K, n_ee, E.items.p, E.soup.p, E.conn.p, E.nn_off.p,
-                                                            n_conn, E.pm32c.p, ctx->ntris.p, ctx->tri32.p,
-                                                            E.search.p, E.sub.p, E.cres.p, E.chit.p, list_ee,
-                                                            cnt_ee, E.fp32_bounds ? 1 : 0);
-            const int pf = prof_begin(ctx, PROF_CONN, n_ee, s_ee);
-            EeArgs ea;
-            ea.n_tp = K;
-            ea.n_conn = n_conn;
-            ea.items = E.items.p;
-            ea.soup = E.soup.p;
-            ea.conn = E.conn.p;
-            ea.nn_off = E.nn_off.p;
-            ea.ntris = ctx->ntris.p;
-            ea.search = E.search.p;
-            ea.sub = E.sub.p;
-            ea.cres = E.cres.p;
-            ea.chit = E.chit.p;
-            ea.pm = E.pm.p;
-            ea.tris = ctx->tris.p;
-            ea.rec = E.ee_rec.p;
-            ea.work = E.ee_work.p;
-            ea.count = cnt_rest;
-            ea.first_iters = E.tune[D2G_TUNE_EE_FIRST_ITERS];
-            ea.certificates = E.certificates ? 1 : 0;
-            ea.ca_stats = E.ccd_stats.p;
-            k_ee_first<<<nblocks(n_ee, kPrimBlock), kPrimBlock, 0, s_ee>>>(n_ee, list_ee, cnt_ee, E.pm.p,
-                                                                          ctx->tris.p, ea);
-            k_ee_rest4<<<ee_grid, kBlock, 0, s_ee>>>(ea);
-            ctx->eng.launches += 2;
-            prof_end(ctx, pf, s_ee);
-            ctx->eng.launches += 1;  // the bound kernel
-        }
-        if (n_pt > 0) {
-            LAUNCH(k_ccd_mask_pt, n_pt, K, n_pt, E.items.p, E.soup.p, E.conn.p, E.nn_off.p, n_conn, E.pm32c.p,
-                   ctx->ntris.p, ctx->tri32.p, E.search.p, E.sub.p, E.cres.p, E.chit.p, list_pt, cnt_pt,
-                   E.fp32_bounds ? 1 : 0);
-            const int pf = prof_begin(ctx, PROF_SOUP_CCD, n_pt);
-            LAUNCHB(k_prim_pt, n_pt, kPrimBlock, K, n_pt, E.items.p, E.soup.p, E.conn.p, E.nn_off.p, n_conn, E.pm.p,
-                    ctx->ntris.p, ctx->tris.p, E.search.p, E.sub.p, E.cres.p, E.chit.p, list_pt, cnt_pt);
-            prof_end(ctx, pf);
-        }
-        if (fork) {
-            D2G_CUDA(cudaEventRecord(ctx->ev_join, s_ee));
-            D2G_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
-        }
-        // (3) soup fold and finals, leaf-pair finals, expansion; one synchronisation
-        if (K > 0) {
-            LAUNCH(k_soup_fold, K, K, E.items.p, E.soup.p, E.sub.p, E.search.p, E.res.p, E.hit.p, E.entry_hits.p,
-                   ctx->nodes.p, E.flags.p);
-        }
-        RC(E.cnt_a.ensure(n_soup + 1));
-        RC(E.cnt_b.ensure(n_soup + 1));
-        RC(E.off_a.ensure(n_soup + 1));
-        RC(E.off_b.ensure(n_soup + 1));
-        if (n_soup > 0 && E.witnesses) {
-            LAUNCH(k_witness_make, 32LL * n_soup, n_soup, E.soup.p, E.entry_hits.p, E.wt_flag.p, skip, d_pairs,
-                   E.pm.p, E.pm32c.p, ctx->tri32.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->ntris.p, ctx->tris.p, ctx->geo_eps.p, E.search.p,
-                   E.wt_table.p, E.wt_log2cap, E.ccd_stats.p);
-            E.wt_inserts += n_soup;
-        }
-        if (n_soup > 0)
-            LAUNCH(k_expand_count, n_soup, n_soup, E.soup.p, E.entry_hits.p, ctx->nodes.p, 1, E.cnt_a.p, E.cnt_b.p);
-        {  // final flags of soup and leaf-pair tests, children of soup node pairs: one launch
-            const int32_t* sin[4] = {E.flags.p, E.chit.p, E.cnt_a.p, E.cnt_b.p};
-            int32_t* sout[4] = {E.flag_off.p, E.cflag_off.p, E.off_a.p, E.off_b.p};
-            const int sn[4] = {K, 15 * P, n_soup, n_soup};
-            RC(scan4(ctx, sin, sout, sn));
-        }
-        int32_t tot2[4];
-        const int32_t* src2[4] = {E.flag_off.p + K, E.cflag_off.p + 15 * P, E.off_a.p + n_soup, E.off_b.p + n_soup};
-        RC(read_scalars(ctx, src2, 4, tot2));
-        const int fin_soup = tot2[0], fin_conn = tot2[1];
-        RC(E.rec.ensure_keep(14 * (size_t)(n_rec + fin_soup + fin_conn + 1), 14 * (size_t)n_rec, s));
-        RC(E.rec_pair.ensure_keep((size_t)(n_rec + fin_soup + fin_conn + 1), (size_t)n_rec, s));
-        if (fin_soup > 0)
-            emit_records(ctx, K, E.flags.p, E.flag_off.p, E.items.p, 6, E.soup.p, nullptr, 0, d_pairs, E.res.p, n_rec);
-        n_rec += fin_soup;
-        if (fin_conn > 0) {
-            LAUNCH(k_scale, n_conn + 1, n_conn + 1, E.nn_off.p, 15, E.citem_off.p);
-            emit_records(ctx, 15 * P, E.chit.p, E.cflag_off.p, nullptr, 0, E.conn.p, E.citem_off.p, n_conn, d_pairs,
-                         E.cres.p, n_rec);
-        }
-        n_rec += fin_conn;
-        RC(E.soup_next.ensure(tot2[2] + 1));
-        RC(E.conn_next.ensure(tot2[3] + 1));
-        if (n_soup > 0)
-            LAUNCH(k_expand_write, n_soup, n_soup, E.soup.p, E.entry_hits.p, ctx->nodes.p, 1, E.off_a.p, E.off_b.p,
-                   E.soup_next.p, E.conn_next.p);
-        std::swap(E.soup, E.soup_next);
-        std::swap(E.conn, E.conn_next);
-        n_soup = tot2[2];
-        n_conn = tot2[3];
-    }
-    if (abandon) {
-        n_rec = rec_start;
-        chunk = std::max(1, (p1 - p0) / 2);
-        continue;
-    }
-    c_node += k_node;
-    c_tri += k_tri;
-    c_leaf += k_leaf;
-    c_levels += k_levels;
-    peak = std::max(peak, chunk_peak);
-    if (sink) {  // the chunk's records, sorted by pair, go to the consumer and are dropped
-        RC(finish_records(ctx, p1 - p0, n_rec, p0));
-        RC(sink->consume(ctx, sink->user, p0, p1));
-        n_streamed += n_rec;
-        n_rec = 0;
-    }
-    p0 = p1;
+        p0 = p1;
     }
     if (n_pairs > 0) E.ccd_chunk = chunk >= n_pairs ? 0 : (peak < 1.0 / 3.0 ? 2 * chunk : chunk);
     if (!sink) RC(finish_records(ctx, n_pairs, n_rec));
@@ -2459,7 +2851,7 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
         RC(E.rec_pair.ensure_keep((size_t)(n_rec + n_items + 1), (size_t)n_rec, s));
         if (n_items > 0)
             LAUNCH(k_emit, n_items, n_items, E.flags.p, E.flag_off.p, E.items.p, 6, E.soup.p, (const int32_t*)nullptr,
-                   0, d_pairs, E.res.p, res_eps.p, ctx->geo_eps.p, E.rec.p, E.rec_pair.p, n_rec);
+                   d_pairs, E.res.p, res_eps.p, ctx->geo_eps.p, E.rec.p, E.rec_pair.p, n_rec);
         RC(E.cnt_a.ensure(n));
         RC(E.cnt_b.ensure(n));
         RC(E.off_a.ensure(n + 1));
@@ -2572,7 +2964,7 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
     RC(E.rec.ensure(14 * (size_t)tot + 14));
     RC(E.rec_pair.ensure((size_t)tot + 1));
     if (tot > 0)
-        LAUNCH(k_emit, n_items, n_items, E.hit.p, E.flag_off.p, E.items.p, 6, E.soup.p, (const int32_t*)nullptr, 0,
+        LAUNCH(k_emit, n_items, n_items, E.hit.p, E.flag_off.p, E.items.p, 6, E.soup.p, (const int32_t*)nullptr,
                d_pair, E.res.p, res_eps.p, ctx->geo_eps.p, E.rec.p, E.rec_pair.p, 0);
     D2G_CUDA(cudaGetLastError());
     *n_hits = tot;
@@ -2740,7 +3132,6 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
     int32_t* rec_pair_sorted = cv.take<int32_t>(MR);
     int32_t* rec_idx = cv.take<int32_t>(MR);
     int32_t* rec_idx_sorted = cv.take<int32_t>(MR);
-    int32_t* pair_cnt = cv.take<int32_t>(MP + 1);
     int32_t* err = cv.take<int32_t>(1);
     const size_t tmp_bytes = kNoAllocBytes - ((cv.used + 255) & ~(size_t)255) - 256;
     void* tmp = cv.take<unsigned char>(tmp_bytes);
@@ -2783,7 +3174,7 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
             return D2G_ERR_INVALID;
         }
         if (tot > 0)
-            NA_LAUNCH(k_emit, n_slots, n_slots, flags, flag_off, nullptr, 6, front, nullptr, 0, d_pairs, res, res_eps,
+            NA_LAUNCH(k_emit, n_slots, n_slots, flags, flag_off, nullptr, 6, front, nullptr, d_pairs, res, res_eps,
                       sc->geo_eps, rec, rec_pair, n_rec);
         n_rec += tot;
         NA_LAUNCH(k_expand_count, n, n, front, entry_hits, nodes, 0, cnt_a, cnt_b);
@@ -2803,7 +3194,6 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
         n = nn;
         level++;
     }
-    D2G_CUDA(cudaMemsetAsync(pair_cnt, 0, sizeof(int32_t) * (n_pairs + 1), s));
     if (n_rec > 0) {
         NA_LAUNCH(k_iota, n_rec, n_rec, rec_idx);
         int bits = 1;
@@ -2819,9 +3209,8 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
         D2G_CUDA(cub::DeviceRadixSort::SortPairs(tmp, avail, rec_pair, rec_pair_sorted, rec_idx, rec_idx_sorted,
                                                  n_rec, 0, bits, s));
         if (n_rec <= capacity) NA_LAUNCH(k_gather, n_rec, n_rec, rec_idx_sorted, rec, d_contacts);
-        NA_LAUNCH(k_count_pairs, n_rec, n_rec, 0, n_pairs, rec_pair, pair_cnt);
     }
-    if (int rc = noalloc_scan(s, tmp, tmp_bytes, pair_cnt, d_offsets, n_pairs)) return rc;
+    NA_LAUNCH(k_pair_offsets, n_pairs + 1, n_rec, 0, n_pairs, rec_pair_sorted, d_offsets);
     D2G_CUDA(cudaGetLastError());
     D2G_CUDA(cudaStreamSynchronize(s));
     *n_contacts = n_rec;

@@ -144,7 +144,7 @@ struct Engine {
     // flattened primitive tests of a CCD level: soup sub-test results, leaf-pair
     // results, their hit flags and offsets
     DBuf<PrimResult> sub, cres;
-    DBuf<int32_t> chit, cflag_off, nn_cnt, nn_off, citem_off;
+    DBuf<int32_t> chit, cflag_off, nn_cnt, nn_off, tp, lc;  // tp: leaf pair of a triangle pair; lc: level counters
     // time-step selection
     DBuf<double> st_mt, st_new_dt, st_step, st_out;
     DBuf<int32_t> st_has, st_cl_pair_off, st_cl_part_off, st_cl_parts, st_loc;
@@ -194,7 +194,7 @@ struct Engine {
     DBuf<int32_t> last_pair;
     // results (processing order) and the sorted output
     DBuf<double> rec, rec_sorted;
-    DBuf<int32_t> rec_pair, rec_pair_sorted, rec_idx, rec_idx_sorted, out_off, pair_cnt;
+    DBuf<int32_t> rec_pair, rec_pair_sorted, rec_idx, rec_idx_sorted, out_off;
     DBuf<int32_t> d_pairs, bucket_nodes;
     // mesh sets of d2g_mass_properties
     DBuf<double> ms_V, ms_out;
@@ -205,7 +205,7 @@ struct Engine {
     // phased edge-edge CCD (d2g_engine.cu)
     DBuf<double> ee_rec;
     DBuf<int32_t> ee_work;
-    int ee_grid = 0;  // k_ee_rest4 grid (every block resident)
+    int ee_grid = 0, soup_grid = 0;  // k_ee_rest4 and k_soup_tests grids (every block resident)
     // traversal chunking: root entries of the call's pairs; a byte budget for
     // a level's buffers (0: a third of the device memory)
     DBuf<Entry> roots;
