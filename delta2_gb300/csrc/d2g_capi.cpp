@@ -422,10 +422,7 @@ void d2g_ctx_destroy(d2g_ctx* c) {
     E.soup_next.release();
     E.conn_next.release();
     E.entry_hits.release();
-    E.cnt_a.release();
-    E.cnt_b.release();
     E.off_a.release();
-    E.off_b.release();
     E.flags.release();
     E.flag_off.release();
     E.items.release();

@@ -1574,200 +1574,213 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // (1 mm plus 4e-6 of the magnitudes involved) far above the FP32 rounding of
 // the bound and the FP64 rounding of the exact test, so every slot that hits
 // survives.  Dropped slots produce nothing in the reference
-// either.  One thread per slot; per warp a survivor mask and count.
+// either.
 //
-// A node pair with an inner node emits nothing: all the traversal needs of it
-// is whether some slot hits.  The exact distance is at most that of any edge
-// pair, so a slot whose vertices, or else edges, are closer than thr by the
-// same margin certainly hits; its node pair is marked and none of its slots
-// goes on to the FP64 test (`nodes` null: every slot's hit is wanted).
-__device__ __forceinline__ float vv_min(const float (&wa)[3][3], const float (&wb)[3][3]) {
-    float m = 3.4e38f;
+// A warp per node pair: lanes 0-7 transform a's triangles, 8-15 b's, once each
+// into shared memory, and every lane takes two of the 64 slots (a thread per
+// slot transformed both triangles of each: 870 us of a 1,024-hull call).
+//
+// LEAF: the node pair's contacts are wanted; the survivors as two mask words
+// and counts.  Otherwise the pair has an inner node and emits nothing: all the
+// descent needs of it is whether some slot hits.  The exact distance is at most
+// that of any edge pair, so a slot whose vertices, or else edges, are closer
+// than thr by the same margin certainly hits (unless a triangle is almost a
+// point, whose edges return no distance); the pair is marked and done, and only
+// the survivors of the others go onto `list` for k_np_level_tests.
+__device__ __forceinline__ float sat_gap(const float* a, const float* b) {
+    // Separating axes: along any direction n the distance is at least the gap
+    // between the projections divided by |n|, whatever n is, so n computed in
+    // FP32 still bounds; the two face normals and the nine edge-edge cross
+    // products.
+    float wa[3][3], wb[3][3], ea[3][3], eb[3][3];
 #pragma unroll
-    for (int i = 0; i < 3; i++)
+    for (int v = 0; v < 3; v++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) {
-            const float dx = wa[i][0] - wb[j][0], dy = wa[i][1] - wb[j][1], dz = wa[i][2] - wb[j][2];
-            m = fminf(m, dx * dx + dy * dy + dz * dz);
+        for (int r = 0; r < 3; r++) {
+            wa[v][r] = a[3 * v + r];
+            wb[v][r] = b[3 * v + r];
         }
-    return sqrtf(m);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            ea[k][r] = wa[(k + 1) % 3][r] - wa[k][r];
+            eb[k][r] = wb[(k + 1) % 3][r] - wb[k][r];
+        }
+    auto axis_gap = [&](float nx, float ny, float nz) {
+        const float nn = sqrtf(nx * nx + ny * ny + nz * nz);
+        if (!(nn > 1e-20f)) return 0.f;
+        float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
+#pragma unroll
+        for (int v = 0; v < 3; v++) {
+            const float pa = wa[v][0] * nx + wa[v][1] * ny + wa[v][2] * nz;
+            const float pb = wb[v][0] * nx + wb[v][1] * ny + wb[v][2] * nz;
+            a0 = fminf(a0, pa);
+            a1 = fmaxf(a1, pa);
+            b0 = fminf(b0, pb);
+            b1 = fmaxf(b1, pb);
+        }
+        return fmaxf(b0 - a1, a0 - b1) / nn;
+    };
+    auto cross_gap = [&](const float(&u)[3], const float(&v)[3]) {
+        return axis_gap(u[1] * v[2] - u[2] * v[1], u[2] * v[0] - u[0] * v[2], u[0] * v[1] - u[1] * v[0]);
+    };
+    float lb = fmaxf(cross_gap(ea[0], ea[1]), cross_gap(eb[0], eb[1]));
+#pragma unroll
+    for (int x = 0; x < 3; x++)
+#pragma unroll
+        for (int y = 0; y < 3; y++) lb = fmaxf(lb, cross_gap(ea[x], eb[y]));
+    return lb;
 }
-__device__ __forceinline__ float ee_min(const float (&wa)[3][3], const float (&wb)[3][3]) {
-    float m = 3.4e38f;
-    F3 A[3], B[3];
+__device__ __forceinline__ float box_gap9(const float* a, const float* b) {
+    float gap2 = 0.f;
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-        A[i] = f3(wa[i][0], wa[i][1], wa[i][2]);
-        B[i] = f3(wb[i][0], wb[i][1], wb[i][2]);
+    for (int r = 0; r < 3; r++) {
+        const float alo = fminf(fminf(a[r], a[3 + r]), a[6 + r]), ahi = fmaxf(fmaxf(a[r], a[3 + r]), a[6 + r]);
+        const float blo = fminf(fminf(b[r], b[3 + r]), b[6 + r]), bhi = fmaxf(fmaxf(b[r], b[3 + r]), b[6 + r]);
+        const float g = fmaxf(blo - ahi, alo - bhi);
+        if (g > 0.f) gap2 += g * g;
     }
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            float d2;
-            seg_vector(A[i], A[(i + 1) % 3], B[j], B[(j + 1) % 3], d2);
-            m = fminf(m, d2);
-        }
-    return sqrtf(m);
+    return sqrtf(gap2);
 }
 
-__global__ void __launch_bounds__(kBlock) k_np_mask(int n_slots, const Entry* __restrict__ front,
-                                                    const float* __restrict__ pm32, const int32_t* __restrict__ ntris,
-                                                    const float4* __restrict__ sph, const float* __restrict__ tri32,
-                                                    const float* __restrict__ eps_up,
-                                                    const float* __restrict__ search, const int4* __restrict__ nodes,
-                                                    uint32_t* __restrict__ mask, int32_t* __restrict__ cnt,
-                                                    int32_t* __restrict__ entry_hits, int use_bounds) {
-    __shared__ int s_hit[kBlock / 64];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (threadIdx.x < kBlock / 64) s_hit[threadIdx.x] = 0;
-    bool keep = false, inner = false;
-    float room = 0.f;  // thr less the margin
-    float wa[3][3], wb[3][3];  // [vertex][axis]
-    if (i < n_slots) {
-        const Entry e = front[i >> 6];
-        const int ta = (i >> 3) & 7, tb = i & 7;
-        inner = nodes && use_bounds && (ld_node(nodes, e.na).z || ld_node(nodes, e.nb).z);
-        if (ta < ntris[e.na] && tb < ntris[e.nb]) {
-            const float* A = pm32 + 24 * (size_t)e.pair;
-            const float* B = A + 12;
-            const float4 sa = sph[(size_t)e.na * 8 + ta], sb = sph[(size_t)e.nb * 8 + tb];
-            const float dx = (A[0] * sa.x + A[1] * sa.y + A[2] * sa.z + A[3]) -
-                             (B[0] * sb.x + B[1] * sb.y + B[2] * sb.z + B[3]);
-            const float dy = (A[4] * sa.x + A[5] * sa.y + A[6] * sa.z + A[7]) -
-                             (B[4] * sb.x + B[5] * sb.y + B[6] * sb.z + B[7]);
-            const float dz = (A[8] * sa.x + A[9] * sa.y + A[10] * sa.z + A[11]) -
-                             (B[8] * sb.x + B[9] * sb.y + B[10] * sb.z + B[11]);
-            const float thr = search[e.pair] + eps_up[(size_t)e.na * 8 + ta] + eps_up[(size_t)e.nb * 8 + tb];
-            const float mag = fabsf(A[3]) + fabsf(A[7]) + fabsf(A[11]) + fabsf(B[3]) + fabsf(B[7]) + fabsf(B[11]) +
-                              fabsf(sa.x) + fabsf(sa.y) + fabsf(sa.z) + fabsf(sb.x) + fabsf(sb.y) + fabsf(sb.z) +
-                              sa.w + sb.w + thr;
-            float lb = sqrtf(dx * dx + dy * dy + dz * dz) - sa.w - sb.w;
-            const float lim = thr + (1e-3f + 4e-6f * mag);
-            keep = !use_bounds || !(lb > lim);  // NaN keeps the slot
-            if (keep) {
-                const float* va = tri32 + ((size_t)e.na * 8 + ta) * 9;
-                const float* vb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
+template <bool LEAF>
+__global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __restrict__ front,
+                                                      const float* __restrict__ pm32, const int32_t* __restrict__ ntris,
+                                                      const float4* __restrict__ sph, const float* __restrict__ tri32,
+                                                      const float* __restrict__ eps_up,
+                                                      const float* __restrict__ search,
+                                                      const int4* __restrict__ nodes, int use_bounds,
+                                                      uint32_t* __restrict__ mask, int32_t* __restrict__ cnt,
+                                                      int32_t* __restrict__ entry_hits, int32_t* __restrict__ list,
+                                                      int32_t* __restrict__ lc) {
+    __shared__ float s_v[kBlock / 32][16][9];
+    __shared__ float s_c[kBlock / 32][16][7];  // centre, radius, eps, magnitude, 1 for a triangle that is a point
+    const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    if (w >= n) return;  // uniform per warp
+    const Entry e = front[w];
+    if (!LEAF && !ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z) {
+        // a root pair of two leaves goes onto the list of leaf pairs as it is
+        if (lane == 0) {
+            entry_hits[w] = 1;
+            atomicAdd(lc + LC_ROOT, 1);
+        }
+        return;
+    }
+    const int na = ntris[e.na], nb = ntris[e.nb];
+    const float* PA = pm32 + 24 * (size_t)e.pair;
+    const float* PB = PA + 12;
+    if (lane < 16 && (lane & 7) < (lane < 8 ? na : nb)) {
+        const size_t t = (size_t)(lane < 8 ? e.na : e.nb) * 8 + (lane & 7);
+        const float* M = lane < 8 ? PA : PB;
+        const float* tv = tri32 + t * 9;
+        float* v = s_v[wi][lane];
+        float* c = s_c[wi][lane];
+        const float4 sp = sph[t];
 #pragma unroll
-                for (int v = 0; v < 3; v++)
+        for (int r = 0; r < 3; r++) {
+            const float m0 = M[4 * r], m1 = M[4 * r + 1], m2 = M[4 * r + 2], m3 = M[4 * r + 3];
+            c[r] = m0 * sp.x + m1 * sp.y + m2 * sp.z + m3;
 #pragma unroll
-                    for (int r = 0; r < 3; r++) {
-                        wa[v][r] = A[4 * r] * va[3 * v] + A[4 * r + 1] * va[3 * v + 1] + A[4 * r + 2] * va[3 * v + 2] +
-                                   A[4 * r + 3];
-                        wb[v][r] = B[4 * r] * vb[3 * v] + B[4 * r + 1] * vb[3 * v + 1] + B[4 * r + 2] * vb[3 * v + 2] +
-                                   B[4 * r + 3];
-                    }
-                if (use_bounds) {
-                    // the gap between the transformed triangles' boxes
-                    float gap2 = 0.f;
+            for (int k = 0; k < 3; k++) v[3 * k + r] = m0 * tv[3 * k] + m1 * tv[3 * k + 1] + m2 * tv[3 * k + 2] + m3;
+        }
+        c[3] = sp.w;
+        c[4] = eps_up[t];
+        c[5] = fabsf(sp.x) + fabsf(sp.y) + fabsf(sp.z) + sp.w;
+        float ext = 0.f;
 #pragma unroll
-                    for (int r = 0; r < 3; r++) {
-                        const float alo = fminf(fminf(wa[0][r], wa[1][r]), wa[2][r]);
-                        const float ahi = fmaxf(fmaxf(wa[0][r], wa[1][r]), wa[2][r]);
-                        const float blo = fminf(fminf(wb[0][r], wb[1][r]), wb[2][r]);
-                        const float bhi = fmaxf(fmaxf(wb[0][r], wb[1][r]), wb[2][r]);
-                        const float g = fmaxf(blo - ahi, alo - bhi);
-                        if (g > 0.f) gap2 += g * g;
-                    }
-                    keep = !(sqrtf(gap2) > lim);
-                }
-                // (a triangle that is almost a point has no edge that certainly returns a distance)
-                auto extent = [](const float(&q)[3][3]) {
-                    float m = 0.f;
+        for (int r = 0; r < 3; r++) ext = fmaxf(ext, fmaxf(fabsf(v[3 + r] - v[r]), fabsf(v[6 + r] - v[r])));
+        c[6] = ext > 1e-5f ? 0.f : 1.f;
+    }
+    if (lane == 0) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), na * nb);
+    const float se = search[e.pair];
+    const float tm = fabsf(PA[3]) + fabsf(PA[7]) + fabsf(PA[11]) + fabsf(PB[3]) + fabsf(PB[7]) + fabsf(PB[11]);
+    __syncwarp();
+    bool keep[2];
+    float lim[2], room[2];
 #pragma unroll
-                    for (int r = 0; r < 3; r++) m = fmaxf(m, fmaxf(fabsf(q[1][r] - q[0][r]), fabsf(q[2][r] - q[0][r])));
-                    return m;
-                };
-                room = extent(wa) > 1e-5f && extent(wb) > 1e-5f ? thr - (1e-3f + 4e-6f * mag) : -1.f;
-                if (keep && use_bounds && !(inner && vv_min(wa, wb) < room)) {
-                    // Separating axes: along any direction n the distance is at
-                    // least the gap between the projections divided by |n|,
-                    // whatever n is, so n computed in FP32 still bounds; the two
-                    // face normals and the nine edge-edge cross products.
-                    lb = 0.f;
-                    auto axis_gap = [&](float nx, float ny, float nz) {
-                        const float nn = sqrtf(nx * nx + ny * ny + nz * nz);
-                        if (!(nn > 1e-20f)) return 0.f;
-                        float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
+    for (int h = 0; h < 2; h++) {
+        const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
+        keep[h] = ta < na && tb < nb;
+        lim[h] = 0.f;
+        room[h] = -1.f;
+        if (!keep[h] || !use_bounds) continue;
+        const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb];
+        const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
+        const float thr = se + ca[4] + cb[4];
+        const float margin = 1e-3f + 4e-6f * (tm + ca[5] + cb[5] + thr);
+        lim[h] = thr + margin;
+        keep[h] = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim[h]) &&  // NaN keeps the slot
+                  !(box_gap9(s_v[wi][ta], s_v[wi][8 + tb]) > lim[h]);
+        if (keep[h] && ca[6] + cb[6] == 0.f) room[h] = thr - margin;
+    }
+    if (!LEAF && use_bounds) {
+        bool sure = false;
 #pragma unroll
-                        for (int v = 0; v < 3; v++) {
-                            const float pa = wa[v][0] * nx + wa[v][1] * ny + wa[v][2] * nz;
-                            const float pb = wb[v][0] * nx + wb[v][1] * ny + wb[v][2] * nz;
-                            a0 = fminf(a0, pa);
-                            a1 = fmaxf(a1, pa);
-                            b0 = fminf(b0, pb);
-                            b1 = fmaxf(b1, pb);
-                        }
-                        return fmaxf(b0 - a1, a0 - b1) / nn;
-                    };
-                    float ea[3][3], eb[3][3];
+        for (int h = 0; h < 2; h++)
+            if (room[h] > 0.f) sure = sure || vert_min(s_v[wi][(lane + 32 * h) >> 3], s_v[wi][8 + (lane & 7)]) < room[h];
+        sure = __any_sync(0xffffffffu, sure);
+        if (!sure) {
 #pragma unroll
-                    for (int k = 0; k < 3; k++)
+            for (int h = 0; h < 2; h++)
+                if (room[h] > 0.f)
+                    sure = sure || edge_min(s_v[wi][(lane + 32 * h) >> 3], s_v[wi][8 + (lane & 7)]) < room[h];
+            sure = __any_sync(0xffffffffu, sure);
+        }
+        if (lane == 0) entry_hits[w] = sure ? 1 : 0;
+        if (sure) return;
+    } else if (!LEAF) {
+        if (lane == 0) entry_hits[w] = 0;
+    }
 #pragma unroll
-                        for (int r = 0; r < 3; r++) {
-                            ea[k][r] = wa[(k + 1) % 3][r] - wa[k][r];
-                            eb[k][r] = wb[(k + 1) % 3][r] - wb[k][r];
-                        }
-                    lb = fmaxf(lb, axis_gap(ea[0][1] * ea[1][2] - ea[0][2] * ea[1][1],
-                                            ea[0][2] * ea[1][0] - ea[0][0] * ea[1][2],
-                                            ea[0][0] * ea[1][1] - ea[0][1] * ea[1][0]));
-                    lb = fmaxf(lb, axis_gap(eb[0][1] * eb[1][2] - eb[0][2] * eb[1][1],
-                                            eb[0][2] * eb[1][0] - eb[0][0] * eb[1][2],
-                                            eb[0][0] * eb[1][1] - eb[0][1] * eb[1][0]));
-#pragma unroll
-                    for (int x = 0; x < 3; x++)
-#pragma unroll
-                        for (int y = 0; y < 3; y++)
-                            lb = fmaxf(lb, axis_gap(ea[x][1] * eb[y][2] - ea[x][2] * eb[y][1],
-                                                    ea[x][2] * eb[y][0] - ea[x][0] * eb[y][2],
-                                                    ea[x][0] * eb[y][1] - ea[x][1] * eb[y][0]));
-                    keep = !(lb > lim);
-                }
+    for (int h = 0; h < 2; h++) {
+        if (keep[h] && use_bounds) keep[h] = !(sat_gap(s_v[wi][(lane + 32 * h) >> 3], s_v[wi][8 + (lane & 7)]) > lim[h]);
+        if (LEAF) {
+            const unsigned m = __ballot_sync(0xffffffffu, keep[h]);
+            if (lane == 0) {
+                mask[2 * (size_t)w + h] = m;
+                cnt[2 * (size_t)w + h] = __popc(m);
             }
+        } else {
+            warp_append(64 * w + lane + 32 * h, keep[h], list, lc + LC_LIST);
         }
-    }
-    // node pairs that certainly hit: by the vertices, else by the edges
-    __syncthreads();
-    int* const hit = s_hit + (threadIdx.x >> 6);
-    if (keep && inner && vv_min(wa, wb) < room) *hit = 1;
-    __syncthreads();
-    const bool open = !*(volatile int*)hit;
-    __syncthreads();
-    if (open && keep && inner && ee_min(wa, wb) < room) *hit = 1;
-    __syncthreads();
-    if (*hit) {
-        keep = false;
-        if ((threadIdx.x & 63) == 0) entry_hits[i >> 6] = 1;
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    if ((threadIdx.x & 31) == 0 && i < n_slots) {
-        mask[i >> 5] = m;
-        cnt[i >> 5] = __popc(m);
     }
 }
 
-// The valid slots (ta < ntris_a, tb < ntris_b) of a level, for the statistics.
-__global__ void k_count_slots(int n, const Entry* __restrict__ front, const int32_t* __restrict__ ntris,
-                              int32_t* __restrict__ total) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int v = 0;
-    if (i < n) {
-        const Entry e = front[i];
-        v = ntris[e.na] * ntris[e.nb];
+// The undecided slots of a descent's level: the FP64 test of each until its
+// node pair is marked.
+__global__ void __launch_bounds__(kBlock) k_np_level_tests(const int32_t* __restrict__ list,
+                                                           const int32_t* __restrict__ n_list,
+                                                           const Entry* __restrict__ front,
+                                                           const double* __restrict__ pm,
+                                                           const double* __restrict__ tris,
+                                                           const double* __restrict__ eps,
+                                                           const float* __restrict__ search, int32_t* entry_hits,
+                                                           int use_bounds) {
+    const int n = *n_list;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int slot = list[k];
+        if (((volatile int32_t*)entry_hits)[slot >> 6]) continue;
+        const Entry e = front[slot >> 6];
+        const int ta = (slot >> 3) & 7, tb = slot & 7;
+        const double* M = pm + 32 * (size_t)e.pair;
+        const Tri A = tri_xform_rigid(load_tri(tris + (size_t)e.na * 72 + ta * 9), M);
+        const Tri B = tri_xform_rigid(load_tri(tris + (size_t)e.nb * 72 + tb * 9), M + 16);
+        const double thr = ((double)search[e.pair] + eps[(size_t)e.na * 8 + ta]) + eps[(size_t)e.nb * 8 + tb];
+        V3 P, Q;
+        if (use_bounds ? tri_tri_below(A, B, thr) : tri_tri_dist(A, B, P, Q) < thr) entry_hits[slot >> 6] = 1;
     }
-    v = __reduce_add_sync(0xffffffffu, v);
-    if ((threadIdx.x & 31) == 0 && v) atomicAdd(total, v);
 }
 
 // Ordered compaction of the surviving slots (slot order = the reference's
-// triangle-pair order within each node pair).
-__global__ void k_np_items(int n_slots, const uint32_t* __restrict__ mask, const int32_t* __restrict__ off,
+// triangle-pair order within each node pair), a thread per mask word.
+__global__ void k_np_items(int n_words, const uint32_t* __restrict__ mask, const int32_t* __restrict__ off,
                            int32_t* __restrict__ items) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_slots) return;
-    const unsigned m = mask[i >> 5];
-    const int lane = i & 31;
-    if ((m >> lane) & 1u) items[off[i >> 5] + __popc(m & ((1u << lane) - 1u))] = i;
+    if (i >= n_words) return;
+    int o = off[i];
+    for (unsigned m = mask[i]; m; m &= m - 1) items[o++] = 32 * i + __ffs(m) - 1;
 }
 
 // One surviving slot a thread: the FP64 triangle distance and the hit test.
@@ -1882,127 +1895,76 @@ __global__ void k_emit(int n, const int32_t* __restrict__ flags, const int32_t* 
 
 // Expansion rule of full_tree_comparison.h:27-59: leaf-leaf keeps its hits,
 // otherwise the shallower inner side (b on ties, the inner one when the other
-// is a leaf) is replaced by its children.  `split` separates children into
-// the soup (some inner node) and connected (both leaves) frontiers.
+// is a leaf) is replaced by its children.
 __global__ void k_expand_count(int n, const Entry* __restrict__ front, const int32_t* __restrict__ entry_hits,
-                               const int4* __restrict__ nodes, int split, int32_t* __restrict__ cnt_s,
-                               int32_t* __restrict__ cnt_c) {
+                               const int4* __restrict__ nodes, int32_t* __restrict__ cnt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int s = 0, c = 0;
+    int s = 0;
     if (entry_hits[i] > 0) {
-        const Entry e = front[i];
-        const int4 A = ld_node(nodes, e.na), B = ld_node(nodes, e.nb);
-        int rule;
-        if (!A.z && !B.z)
-            rule = 0;
-        else if (!A.z)
-            rule = 2;
-        else if (!B.z)
-            rule = 1;
-        else
-            rule = A.w < B.w ? 1 : 2;
-        if (rule) {
-            const int4 P = rule == 1 ? A : B;
-            for (int ch = 0; ch < P.y; ch++) {
-                const int ga = rule == 1 ? P.x + ch : e.na;
-                const int gb = rule == 1 ? e.nb : P.x + ch;
-                const bool inner = ld_node(nodes, ga).z || ld_node(nodes, gb).z;
-                if (!split || inner)
-                    s++;
-                else
-                    c++;
-            }
-        }
+        const int4 A = ld_node(nodes, front[i].na), B = ld_node(nodes, front[i].nb);
+        if (A.z || B.z) s = A.z && (!B.z || A.w < B.w) ? A.y : B.y;
     }
-    cnt_s[i] = s;
-    cnt_c[i] = c;
+    cnt[i] = s;
 }
 
 __global__ void k_expand_write(int n, const Entry* __restrict__ front, const int32_t* __restrict__ entry_hits,
-                               const int4* __restrict__ nodes, int split, const int32_t* __restrict__ off_s,
-                               const int32_t* __restrict__ off_c, Entry* __restrict__ next_s,
-                               Entry* __restrict__ next_c) {
+                               const int4* __restrict__ nodes, const int32_t* __restrict__ off,
+                               Entry* __restrict__ next) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || entry_hits[i] <= 0) return;
     const Entry e = front[i];
     const int4 A = ld_node(nodes, e.na), B = ld_node(nodes, e.nb);
-    int rule;
-    if (!A.z && !B.z)
-        rule = 0;
-    else if (!A.z)
-        rule = 2;
-    else if (!B.z)
-        rule = 1;
-    else
-        rule = A.w < B.w ? 1 : 2;
-    if (!rule) return;
-    const int4 P = rule == 1 ? A : B;
-    int s = off_s[i], c = off_c[i];
+    if (!A.z && !B.z) return;
+    const bool open_a = A.z && (!B.z || A.w < B.w);
+    const int4 P = open_a ? A : B;
+    Entry* o = next + off[i];
     for (int ch = 0; ch < P.y; ch++) {
         Entry x;
         x.pair = e.pair;
-        x.na = rule == 1 ? P.x + ch : e.na;
-        x.nb = rule == 1 ? e.nb : P.x + ch;
-        const bool inner = ld_node(nodes, x.na).z || ld_node(nodes, x.nb).z;
-        if (!split || inner)
-            next_s[s++] = x;
-        else
-            next_c[c++] = x;
+        x.na = open_a ? P.x + ch : e.na;
+        x.nb = open_a ? e.nb : P.x + ch;
+        *o++ = x;
     }
 }
 
-// k_expand_count, its prefix sums and k_expand_write in one block for a level
-// of up to kExpandOneBlock node pairs (a launch instead of three; 6 us against
-// 18 at 2,700 node pairs): each thread takes a run of consecutive node pairs.
-// Children with an inner node go to next[0 ..), leaf pairs to leaf[lc[LC_LEAF]
-// ..); the totals go to lc and the level's list is emptied for the next one.
-constexpr int kExpandThreads = 1024, kExpandOneBlock = 24576;
-__device__ __forceinline__ int expand_rule(int4 A, int4 B) {  // 1: open a, 2: open b, 0: two leaves
-    if (!A.z && !B.z) return 0;
-    if (!A.z) return 2;
-    if (!B.z) return 1;
-    return A.w < B.w ? 1 : 2;
-}
-__global__ void __launch_bounds__(kExpandThreads) k_expand_level(int n, const Entry* __restrict__ front,
-                                                                 const int32_t* __restrict__ entry_hits,
-                                                                 const int4* __restrict__ nodes,
-                                                                 Entry* __restrict__ next, Entry* __restrict__ leaf,
-                                                                 int32_t* __restrict__ lc) {
-    __shared__ int2 wsum[32];
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int per = (n + kExpandThreads - 1) / kExpandThreads;
-    const int i0 = min(n, tid * per), i1 = min(n, i0 + per);
-    int s = 0, c = 0;
-    auto open = [&](int i, Entry& e, int4& P, int& rule) {
-        if (entry_hits[i] <= 0) return false;
-        e = front[i];
-        const int4 A = ld_node(nodes, e.na), B = ld_node(nodes, e.nb);
-        rule = expand_rule(A, B);
-        P = rule == 1 ? A : B;
-        return rule != 0;
-    };
-    auto child = [&](const Entry& e, const int4& P, int rule, int ch) {
-        Entry x;
-        x.pair = e.pair;
-        x.na = rule == 1 ? P.x + ch : e.na;
-        x.nb = rule == 1 ? e.nb : P.x + ch;
-        return x;
-    };
-    for (int i = i0; i < i1; i++) {
-        Entry e;
-        int4 P;
-        int rule;
-        if (!open(i, e, P, rule)) continue;
-        for (int ch = 0; ch < P.y; ch++) {
-            const Entry x = child(e, P, rule, ch);
-            if (ld_node(nodes, x.na).z || ld_node(nodes, x.nb).z)
-                s++;
-            else
-                c++;
-        }
+// A level's expansion for the descents: children with an inner node to next
+// [0 ..), leaf pairs to leaf [lc[LC_LEAF] ..) (with self_leaf also a marked pair
+// of two leaves itself), in order; the totals to lc, and the level's list is
+// emptied for the next one.  A thread per node pair.  Up to kExpandOneBlock
+// node pairs one block does it all; larger levels take two launches,
+// k_expand_sums for the blocks' totals and k_expand_level, whose blocks add up
+// the totals before theirs (three launches and a library scan before).
+constexpr int kExpandThreads = 256, kExpandOneBlock = 1024;
+struct Opened {
+    Entry e;
+    int4 P;           // the opened node (two leaves: y = self_leaf)
+    int rule;
+    unsigned leaves;  // bit per child: a leaf pair
+};
+__device__ __forceinline__ bool open_pair(const Entry& e, const int4* __restrict__ nodes, int self_leaf, Opened& o) {
+    const int4 A = ld_node(nodes, e.na), B = ld_node(nodes, e.nb);
+    o.e = e;
+    o.rule = !A.z && !B.z ? 0 : (!A.z ? 2 : (!B.z ? 1 : (A.w < B.w ? 1 : 2)));
+    o.P = o.rule == 1 ? A : B;
+    o.leaves = 0;
+    if (!o.rule) {
+        o.P.y = self_leaf;
+        o.leaves = 1;
+        return self_leaf != 0;
     }
-    int xs = s, xc = c;  // inclusive warp scans
+    if (!(o.rule == 1 ? B : A).z) {
+#pragma unroll
+        for (int ch = 0; ch < 8; ch++)
+            if (ch < o.P.y && !ld_node(nodes, o.P.x + ch).z) o.leaves |= 1u << ch;
+    }
+    return true;
+}
+// Exclusive prefix sums of (s, c) over the block, and its totals (every thread).
+__device__ __forceinline__ int2 block_scan2(int s, int c, int2& total) {
+    __shared__ int2 wsum[kExpandThreads / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int xs = s, xc = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int ys = __shfl_up_sync(0xffffffffu, xs, o), yc = __shfl_up_sync(0xffffffffu, xc, o);
@@ -2011,49 +1973,89 @@ __global__ void __launch_bounds__(kExpandThreads) k_expand_level(int n, const En
             xc += yc;
         }
     }
-    if (lane == 31) wsum[w] = make_int2(xs, xc);
-    const int leaf0 = lc[LC_LEAF];
     __syncthreads();
-    if (w == 0) {
-        int zs = wsum[lane].x, zc = wsum[lane].y;
+    if (lane == 31) wsum[w] = make_int2(xs, xc);
+    __syncthreads();
+    int2 before = make_int2(xs - s, xc - c);
+    total = make_int2(0, 0);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int ys = __shfl_up_sync(0xffffffffu, zs, o), yc = __shfl_up_sync(0xffffffffu, zc, o);
-            if (lane >= o) {
-                zs += ys;
-                zc += yc;
+    for (int k = 0; k < kExpandThreads / 32; k++) {
+        const int2 v = wsum[k];
+        if (k < w) {
+            before.x += v.x;
+            before.y += v.y;
+        }
+        total.x += v.x;
+        total.y += v.y;
+    }
+    return before;
+}
+__global__ void __launch_bounds__(kExpandThreads) k_expand_sums(int n, const Entry* __restrict__ front,
+                                                                const int32_t* __restrict__ entry_hits,
+                                                                const int4* __restrict__ nodes, int self_leaf,
+                                                                int2* __restrict__ sums) {
+    const int i = blockIdx.x * kExpandThreads + threadIdx.x;
+    Opened o;
+    int s = 0, c = 0;
+    if (i < n && entry_hits[i] > 0 && open_pair(front[i], nodes, self_leaf, o)) {
+        c = __popc(o.leaves);
+        s = o.P.y - c;
+    }
+    int2 total;
+    block_scan2(s, c, total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(kExpandThreads) k_expand_level(int n, const Entry* __restrict__ front,
+                                                                 const int32_t* __restrict__ entry_hits,
+                                                                 const int4* __restrict__ nodes, int self_leaf,
+                                                                 const int2* __restrict__ sums,
+                                                                 Entry* __restrict__ next, Entry* __restrict__ leaf,
+                                                                 int leaf0, int32_t* __restrict__ lc) {
+    int2 base = make_int2(0, leaf0);
+    if (sums) {  // the blocks before this one
+        int s = 0, c = 0;
+        for (int k = threadIdx.x; k < (int)blockIdx.x; k += kExpandThreads) {
+            s += sums[k].x;
+            c += sums[k].y;
+        }
+        int2 total;
+        block_scan2(s, c, total);
+        base.x += total.x;
+        base.y += total.y;
+    }
+    const int step = sums ? n : kExpandThreads;  // one block walks the level, else one pass
+    for (int i0 = sums ? blockIdx.x * kExpandThreads : 0; i0 < n; i0 += step) {
+        const int i = i0 + threadIdx.x;
+        Opened o;
+        int s = 0, c = 0;
+        if (i < n && entry_hits[i] > 0 && open_pair(front[i], nodes, self_leaf, o)) {
+            c = __popc(o.leaves);
+            s = o.P.y - c;
+        }
+        int2 total;
+        const int2 at = block_scan2(s, c, total);
+        if (s + c > 0) {
+            Entry* ps = next + base.x + at.x;
+            Entry* pc = leaf + base.y + at.y;
+            for (int ch = 0; ch < o.P.y; ch++) {
+                Entry x;
+                x.pair = o.e.pair;
+                x.na = o.rule == 1 ? o.P.x + ch : o.e.na;
+                x.nb = o.rule == 2 ? o.P.x + ch : o.e.nb;
+                if ((o.leaves >> ch) & 1u)
+                    *pc++ = x;
+                else
+                    *ps++ = x;
             }
         }
-        wsum[lane] = make_int2(zs, zc);
+        base.x += total.x;
+        base.y += total.y;
     }
-    __syncthreads();
-    int os = xs - s + (w ? wsum[w - 1].x : 0), oc = leaf0 + xc - c + (w ? wsum[w - 1].y : 0);
-    for (int i = i0; i < i1; i++) {
-        Entry e;
-        int4 P;
-        int rule;
-        if (!open(i, e, P, rule)) continue;
-        for (int ch = 0; ch < P.y; ch++) {
-            const Entry x = child(e, P, rule, ch);
-            if (ld_node(nodes, x.na).z || ld_node(nodes, x.nb).z)
-                next[os++] = x;
-            else
-                leaf[oc++] = x;
-        }
-    }
-    if (tid == 0) {
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) {
         lc[LC_LIST] = 0;
-        lc[LC_NEXT] = wsum[31].x;
-        lc[LC_LEAF] = leaf0 + wsum[31].y;
+        lc[LC_NEXT] = base.x;
+        lc[LC_LEAF] = base.y;
     }
-}
-
-// The totals of a larger level's prefix sums, as k_expand_level leaves them.
-__global__ void k_expand_totals(const int32_t* __restrict__ n_next, const int32_t* __restrict__ n_leaf,
-                                int32_t* __restrict__ lc) {
-    lc[LC_LIST] = 0;
-    lc[LC_NEXT] = *n_next;
-    lc[LC_LEAF] += *n_leaf;
 }
 
 // ---------------------------------------------------------- output sort ----
@@ -2155,26 +2157,18 @@ void prof_collect(d2g_ctx* ctx) {
     E.pending.clear();
 }
 
-// Exclusive prefix sum of in[0..n) into out[0..n], out[n] = total.
-// Exclusive prefix sums of up to two small int32 arrays in one launch, one
-// 1024-thread block per array: out[0..n] with out[n] = total.  The array is
+// Exclusive prefix sum of a small int32 array in one 1024-thread block:
+// out[0..n] with out[n] = total.  The array is
 // staged in shared memory in chunks of kScanChunk (coalesced), each thread
 // sums its kScanPer contiguous elements, and a shuffle scan over the thread
 // sums gives every thread its offset.
 constexpr int kScanThreads = 1024, kScanPer = 8, kScanChunk = kScanThreads * kScanPer;
 static_assert(kScanThreads == 32 * 32, "the warp-sum scan assumes 32 warps");
 constexpr int kScanOneBlock = 4 * kScanChunk;  // larger arrays go to cub
-struct ScanSeg {  // up to two independent scans, one block each
-    const int32_t* in[2];
-    int32_t* out[2];
-    int n[2];
-};
-__global__ void __launch_bounds__(kScanThreads) k_scan1(ScanSeg sg) {
+__global__ void __launch_bounds__(kScanThreads) k_scan1(const int32_t* __restrict__ in, int32_t* __restrict__ out,
+                                                        int n) {
     __shared__ int32_t buf[kScanChunk];
     __shared__ int32_t wsum[32];
-    const int32_t* in = sg.in[blockIdx.x];
-    int32_t* out = sg.out[blockIdx.x];
-    const int n = sg.n[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     int carry = 0;
     for (int base = 0; base < n; base += kScanChunk) {
@@ -2222,11 +2216,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan1(ScanSeg sg) {
 
 int scan_on(cudaStream_t st, DBuf<uint8_t>& tmp, const int32_t* in, int32_t* out, int n) {
     if (n <= kScanOneBlock) {
-        ScanSeg sg;
-        sg.in[0] = sg.in[1] = in;
-        sg.out[0] = sg.out[1] = out;
-        sg.n[0] = sg.n[1] = n;
-        k_scan1<<<1, kScanThreads, 0, st>>>(sg);
+        k_scan1<<<1, kScanThreads, 0, st>>>(in, out, n);
         return D2G_OK;
     }
     D2G_CUDA(cudaMemsetAsync(out, 0, sizeof(int32_t), st));
@@ -2240,24 +2230,6 @@ int scan(d2g_ctx* ctx, const int32_t* in, int32_t* out, int n) {
     if (n <= kScanOneBlock) ctx->eng.launches++;  // this library's scan kernel (larger ones are cub's)
     return scan_on(ctx->stream, ctx->eng.cub_tmp, in, out, n);
 }
-// Two independent scans on the context's stream (one launch when both are small).
-int scan2(d2g_ctx* ctx, const int32_t* in0, int32_t* out0, int n0, const int32_t* in1, int32_t* out1, int n1) {
-    if (n0 <= kScanOneBlock && n1 <= kScanOneBlock) {
-        ScanSeg sg;
-        sg.in[0] = in0;
-        sg.out[0] = out0;
-        sg.n[0] = n0;
-        sg.in[1] = in1;
-        sg.out[1] = out1;
-        sg.n[1] = n1;
-        k_scan1<<<2, kScanThreads, 0, ctx->stream>>>(sg);
-        ctx->eng.launches++;
-        return D2G_OK;
-    }
-    if (int rc = scan(ctx, in0, out0, n0)) return rc;
-    return scan(ctx, in1, out1, n1);
-}
-
 // Read k device int32 scalars (after the stream's pending work).
 int read_scalars(d2g_ctx* ctx, const int32_t* const* src, int k, int32_t* dst) {
     for (int i = 0; i < k; i++)
@@ -2346,6 +2318,19 @@ int soup_grid_size(d2g_ctx* ctx, int* grid) {
         E.soup_grid = std::max(1, dev_sms * std::max(1, per_sm));
     }
     *grid = E.soup_grid;
+    return D2G_OK;
+}
+
+// Grid of k_np_level_tests, likewise.
+int np_grid_size(d2g_ctx* ctx, int* grid) {
+    Engine& E = ctx->eng;
+    if (E.np_grid == 0) {
+        int dev_sms = 0, per_sm = 0;
+        D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
+        D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_np_level_tests, kBlock, 0));
+        E.np_grid = std::max(1, dev_sms * std::max(1, per_sm));
+    }
+    *grid = E.np_grid;
     return D2G_OK;
 }
 
@@ -2443,14 +2428,15 @@ struct Traversal {
     bool abandon = false;
     double peak = 0.0;
     int64_t nodes = 0, tri = 0, levels = 0;
-    int n_leaf = 0, n_root = 0;  // n_root: root pairs of two leaves with candidate slots
+    int n_leaf = 0, n_root = 0;  // n_root: root pairs of two leaves (CCD: with candidate slots)
 };
 
 // Descends from the n node pairs in E.soup: per level `decide` marks the node
 // pairs with a hit in E.entry_hits, and their children go to the next level
-// or, two leaves, onto E.conn.  One read of the counts per level.
+// or, two leaves, onto E.conn (with self_leaf also marked root pairs that are
+// two leaves).  One read of the counts per level.
 template <class F>
-int descend(d2g_ctx* ctx, int n, double budget, bool may_abandon, Traversal& T, F decide) {
+int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon, Traversal& T, F decide) {
     Engine& E = ctx->eng;
     cudaStream_t s = ctx->stream;
     RC(E.lc.ensure(LC_SIZE));
@@ -2471,22 +2457,18 @@ int descend(d2g_ctx* ctx, int n, double budget, bool may_abandon, Traversal& T, 
         RC(decide(n));
         RC(E.soup_next.ensure(8 * (size_t)n + 1));  // a node has at most 8 children
         RC(E.conn.ensure_keep((size_t)T.n_leaf + 8 * (size_t)n + 1, (size_t)T.n_leaf, s));
-        if (n <= kExpandOneBlock) {
-            k_expand_level<<<1, kExpandThreads, 0, s>>>(n, E.soup.p, E.entry_hits.p, ctx->nodes.p, E.soup_next.p,
-                                                        E.conn.p, E.lc.p);
-            E.launches++;
-        } else {
-            RC(E.cnt_a.ensure(n));
-            RC(E.cnt_b.ensure(n));
-            RC(E.off_a.ensure(n + 1));
-            RC(E.off_b.ensure(n + 1));
-            LAUNCH(k_expand_count, n, n, E.soup.p, E.entry_hits.p, ctx->nodes.p, 1, E.cnt_a.p, E.cnt_b.p);
-            RC(scan2(ctx, E.cnt_a.p, E.off_a.p, n, E.cnt_b.p, E.off_b.p, n));
-            LAUNCH(k_expand_write, n, n, E.soup.p, E.entry_hits.p, ctx->nodes.p, 1, E.off_a.p, E.off_b.p,
-                   E.soup_next.p, E.conn.p + T.n_leaf);
-            k_expand_totals<<<1, 1, 0, s>>>(E.off_a.p + n, E.off_b.p + n, E.lc.p);
+        const bool one = n <= kExpandOneBlock;
+        const int blocks = one ? 1 : nblocks(n, kExpandThreads);
+        if (!one) {
+            RC(E.sums.ensure(2 * (size_t)blocks));
+            k_expand_sums<<<blocks, kExpandThreads, 0, s>>>(n, E.soup.p, E.entry_hits.p, ctx->nodes.p,
+                                                            self_leaf ? 1 : 0, (int2*)E.sums.p);
             E.launches++;
         }
+        k_expand_level<<<blocks, kExpandThreads, 0, s>>>(n, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0,
+                                                         one ? (const int2*)nullptr : (const int2*)E.sums.p,
+                                                         E.soup_next.p, E.conn.p, T.n_leaf, E.lc.p);
+        E.launches++;
         D2G_CUDA(cudaMemcpyAsync(ctx->h_pinned, E.lc.p, sizeof(int32_t) * LC_SIZE, cudaMemcpyDeviceToHost, s));
         D2G_CUDA(cudaStreamSynchronize(s));
         prof_collect(ctx);
@@ -2498,7 +2480,9 @@ int descend(d2g_ctx* ctx, int n, double budget, bool may_abandon, Traversal& T, 
         for (int k = 0; k < LC_TRI_N; k++) T.tri += (uint32_t)ctx->h_pinned[LC_TRI + k];
         D2G_CUDA(cudaMemsetAsync(E.lc.p + LC_TRI, 0, sizeof(int32_t) * LC_TRI_N, s));
     }
-    if (new_leaf > 0) T.levels++;  // the last level's leaf pairs are a level of the reference's
+    // the last level's leaf pairs are a level of the reference's (root pairs of
+    // two leaves belong to the first)
+    if (new_leaf > (self_leaf && T.levels == 1 ? T.n_root : 0)) T.levels++;
     return D2G_OK;
 }
 
@@ -2703,7 +2687,7 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
         Traversal T;
         RC(E.soup.ensure((size_t)(p1 - p0) + 1));  // the frontiers swap every level: this one may be the smaller
         D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
-        RC(descend(ctx, p1 - p0, budget, p1 - p0 > 1, T, [&](int n_soup) -> int {
+        RC(descend(ctx, p1 - p0, false, budget, p1 - p0 > 1, T, [&](int n_soup) -> int {
             RC(E.ccd_list.ensure(64 * (size_t)n_soup));
             const int pff = prof_begin(ctx, PROF_SOUP_FILTER, 64LL * n_soup);
             const uint8_t* eskip = nullptr;
@@ -2771,119 +2755,105 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
     return D2G_OK;
 }
 
+// The surviving slots of n node pairs at `front` (k_np_filter), tested; the
+// item list, hit flags and results stay in E.items, E.hit, E.res and res_eps
+// (E.pfut).  One read, of the survivors' count.
+int np_slot_tests(d2g_ctx* ctx, const int32_t* d_pairs, const Entry* front, int n, int* n_items_out) {
+    Engine& E = ctx->eng;
+    DBuf<double>& res_eps = E.pfut;  // per-slot eps record buffer
+    const int n_slots = 64 * n, n_words = 2 * n;
+    RC(E.np_mask.ensure(n_words + 1));
+    RC(E.np_cnt.ensure(n_words + 1));
+    RC(E.np_off.ensure(n_words + 1));
+    RC(E.lc.ensure(LC_SIZE));
+    LAUNCH(k_np_filter<true>, 32LL * n, n, front, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p,
+           E.search.p, ctx->nodes.p, E.fp32_bounds ? 1 : 0, E.np_mask.p, E.np_cnt.p, (int32_t*)nullptr, (int32_t*)nullptr, E.lc.p);
+    RC(scan(ctx, E.np_cnt.p, E.np_off.p, n_words));
+    int32_t n_items = 0;
+    const int32_t* src = E.np_off.p + n_words;
+    RC(read_scalars(ctx, &src, 1, &n_items));
+    *n_items_out = n_items;
+    if (n_items == 0) return D2G_OK;
+    RC(E.items.ensure(n_items + 1));
+    RC(E.res.ensure(n_items));
+    RC(res_eps.ensure(4 * (size_t)n_items));
+    RC(E.hit.ensure(n_items));
+    LAUNCH(k_np_items, n_words, n_words, E.np_mask.p, E.np_off.p, E.items.p);
+    const int pf = prof_begin(ctx, PROF_NP, n_slots);
+    LAUNCH(k_np, n_items, n_items, front, d_pairs, E.pm.p, ctx->ntris.p, ctx->tris.p, ctx->eps.p, ctx->inner_eps.p,
+           ctx->geo_eps.p, E.search.p, E.res.p, res_eps.p, E.hit.p, E.entry_hits.p, E.items.p, E.fp32_bounds ? 1 : 0);
+    prof_end(ctx, pf);
+    return D2G_OK;
+}
+
 int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_out, int64_t* counters) {
     Engine& E = ctx->eng;
     cudaStream_t s = ctx->stream;
-    int64_t c_node = 0, c_tri = 0, c_leaf = 0, c_levels = 0;
+    int64_t c_node = 0, c_tri = 0, c_levels = 0;
     RC(E.pm.ensure(32 * (size_t)n_pairs + 1));
     RC(E.search.ensure(n_pairs + 1));
-    RC(E.soup.ensure(n_pairs + 1));
-    RC(E.np_tri.ensure(1));
-    D2G_CUDA(cudaMemsetAsync(E.np_tri.p, 0, sizeof(int32_t), s));
+    RC(E.roots.ensure(n_pairs + 1));
     RC(E.pm32.ensure(24 * (size_t)n_pairs + 1));
     if (n_pairs > 0)
-        LAUNCH(k_np_prep, n_pairs, n_pairs, d_pairs, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p,
-                                                     ctx->geo_eps.p, E.pm.p, E.search.p, E.soup.p, E.pm32.p);
-    int n_rec = 0;
-    DBuf<double>& res_eps = E.pfut;  // reused as the per-slot eps record buffer
-    // pair chunks, as in run_ccd: a level that would pass the byte budget
-    // (~110 bytes per slot, 64 slots per node pair, x1.5 growth slack)
-    // abandons its chunk, which is halved
-    RC(E.roots.ensure(n_pairs + 1));
-    if (n_pairs > 0)
-        D2G_CUDA(cudaMemcpyAsync(E.roots.p, E.soup.p, sizeof(Entry) * n_pairs, cudaMemcpyDeviceToDevice, s));
+        LAUNCH(k_np_prep, n_pairs, n_pairs, d_pairs, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p,
+               E.pm.p, E.search.p, E.roots.p, E.pm32.p);
+    int n_rec = 0, test_grid = 0;
+    RC(np_grid_size(ctx, &test_grid));
+    // pair chunks, as in run_ccd
     const double budget = level_budget(ctx);
-    int chunk = E.np_chunk > 0 ? std::min(n_pairs, E.np_chunk) : n_pairs;  // as in run_ccd
+    // a leaf pair's slots take ~110 bytes each (x1.5 growth slack)
+    const int range = (int)std::min(8.0e6, std::max(1024.0, budget / (1.5 * 110.0 * 64.0)));
+    int chunk = E.np_chunk > 0 ? std::min(n_pairs, E.np_chunk) : n_pairs;
     double peak = 0.0;
     for (int p0 = 0; p0 < n_pairs;) {
-    const int p1 = std::min(n_pairs, p0 + chunk);
-    const int rec_start = n_rec;
-    const int32_t tri_start = (int32_t)c_tri;  // the device counter's value before this chunk
-    int64_t k_node = 0, k_levels = 0;
-    bool abandon = false;
-    double chunk_peak = 0.0;
-    RC(E.soup.ensure((size_t)(p1 - p0) + 1));  // the frontiers swap every level: this one may be the smaller
-    D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
-    int n = p1 - p0;
-    while (n > 0) {
-        if ((1.5 * 110.0 * 64.0 * n > budget || 64LL * n > (long long)INT32_MAX / 2) && p1 - p0 > 1) {
-            abandon = true;
-            break;
+        const int p1 = std::min(n_pairs, p0 + chunk);
+        Traversal T;
+        RC(E.soup.ensure((size_t)(p1 - p0) + 1));
+        D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
+        RC(descend(ctx, p1 - p0, true, budget, p1 - p0 > 1, T, [&](int n) -> int {
+            RC(E.ccd_list.ensure(64 * (size_t)n));
+            LAUNCH(k_np_filter<false>, 32LL * n, n, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p,
+                   ctx->eps_up.p, E.search.p, ctx->nodes.p, E.fp32_bounds ? 1 : 0, (uint32_t*)nullptr, (int32_t*)nullptr,
+                   E.entry_hits.p, E.ccd_list.p, E.lc.p);
+            k_np_level_tests<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p,
+                                                          ctx->tris.p, ctx->eps.p, E.search.p, E.entry_hits.p,
+                                                          E.fp32_bounds ? 1 : 0);
+            E.launches++;
+            return D2G_OK;
+        }));
+        if (T.abandon) {
+            chunk = std::max(1, (p1 - p0) / 2);
+            continue;
         }
-        chunk_peak = std::max(chunk_peak, 1.5 * 110.0 * 64.0 * n / budget);
-        k_levels++;
-        k_node += n;
-        const int n_slots = 64 * n;
-        RC(E.res.ensure(n_slots));
-        RC(res_eps.ensure(4 * (size_t)n_slots));
-        RC(E.hit.ensure(n_slots));
-        RC(E.flags.ensure(n_slots));
-        RC(E.entry_hits.ensure(n));
-        D2G_CUDA(cudaMemsetAsync(E.entry_hits.p, 0, sizeof(int32_t) * n, s));
-        const int n_words = n_slots / 32;
-        RC(E.np_mask.ensure(n_words + 1));
-        RC(E.np_cnt.ensure(n_words + 1));
-        RC(E.np_off.ensure(n_words + 1));
-        RC(E.items.ensure(n_slots + 1));
-        LAUNCH(k_np_mask, n_slots, n_slots, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p,
-               E.search.p, ctx->nodes.p, E.np_mask.p, E.np_cnt.p, E.entry_hits.p, E.fp32_bounds ? 1 : 0);
-        LAUNCH(k_count_slots, n, n, E.soup.p, ctx->ntris.p, E.np_tri.p);
-        RC(scan(ctx, E.np_cnt.p, E.np_off.p, n_words));
-        LAUNCH(k_np_items, n_slots, n_slots, E.np_mask.p, E.np_off.p, E.items.p);
-        // the survivors' count sizes every later kernel of the level
-        int32_t n_items = 0;
-        {
-            const int32_t* src = E.np_off.p + n_words;
-            RC(read_scalars(ctx, &src, 1, &n_items));
+        // contacts of the leaf pairs, in level order, in ranges within the budget
+        for (int c0 = 0; c0 < T.n_leaf; c0 += range) {
+            const int n = std::min(range, T.n_leaf - c0);
+            const Entry* front = E.conn.p + c0;
+            RC(E.entry_hits.ensure(n + 1));  // (counted by k_np, read by the bucket comparison only)
+            int n_items = 0;
+            RC(np_slot_tests(ctx, d_pairs, front, n, &n_items));
+            if (n_items == 0) continue;
+            RC(E.flag_off.ensure(n_items + 1));
+            RC(scan(ctx, E.hit.p, E.flag_off.p, n_items));
+            RC(E.rec.ensure_keep(14 * (size_t)(n_rec + n_items + 1), 14 * (size_t)n_rec, s));
+            RC(E.rec_pair.ensure_keep((size_t)(n_rec + n_items + 1), (size_t)n_rec, s));
+            LAUNCH(k_emit, n_items, n_items, E.hit.p, E.flag_off.p, E.items.p, 6, front, (const int32_t*)nullptr,
+                   d_pairs, E.res.p, E.pfut.p, ctx->geo_eps.p, E.rec.p, E.rec_pair.p, n_rec);
+            int32_t hits = 0;
+            const int32_t* src = E.flag_off.p + n_items;
+            RC(read_scalars(ctx, &src, 1, &hits));
+            n_rec += hits;
         }
-        if (n_items > 0) {
-            const int pf = prof_begin(ctx, PROF_NP, n_slots);
-            LAUNCH(k_np, n_items, n_items, E.soup.p, d_pairs, E.pm.p, ctx->ntris.p, ctx->tris.p, ctx->eps.p,
-                   ctx->inner_eps.p, ctx->geo_eps.p, E.search.p, E.res.p, res_eps.p, E.hit.p, E.entry_hits.p,
-                   E.items.p, E.fp32_bounds ? 1 : 0);
-            prof_end(ctx, pf);
-            LAUNCH(k_final_flags, n_items, n_items, E.items.p, E.soup.p, ctx->nodes.p, E.hit.p, E.flags.p);
+        if (T.n_leaf > 0) {  // the leaf pairs' slots, counted by k_np_filter
+            D2G_CUDA(cudaMemcpyAsync(ctx->h_pinned, E.lc.p, sizeof(int32_t) * LC_SIZE, cudaMemcpyDeviceToHost, s));
+            D2G_CUDA(cudaStreamSynchronize(s));
+            for (int k = 0; k < LC_TRI_N; k++) T.tri += (uint32_t)ctx->h_pinned[LC_TRI + k];
         }
-        // final contacts: compacted now, counted with the level-end read
-        RC(E.flag_off.ensure(n_items + 1));
-        RC(scan(ctx, E.flags.p, E.flag_off.p, n_items));
-        RC(E.rec.ensure_keep(14 * (size_t)(n_rec + n_items + 1), 14 * (size_t)n_rec, s));
-        RC(E.rec_pair.ensure_keep((size_t)(n_rec + n_items + 1), (size_t)n_rec, s));
-        if (n_items > 0)
-            LAUNCH(k_emit, n_items, n_items, E.flags.p, E.flag_off.p, E.items.p, 6, E.soup.p, (const int32_t*)nullptr,
-                   d_pairs, E.res.p, res_eps.p, ctx->geo_eps.p, E.rec.p, E.rec_pair.p, n_rec);
-        RC(E.cnt_a.ensure(n));
-        RC(E.cnt_b.ensure(n));
-        RC(E.off_a.ensure(n + 1));
-        RC(E.off_b.ensure(n + 1));
-        LAUNCH(k_expand_count, n, n, E.soup.p, E.entry_hits.p, ctx->nodes.p, 0, E.cnt_a.p,
-                                                     E.cnt_b.p);
-        RC(scan(ctx, E.cnt_a.p, E.off_a.p, n));
-        D2G_CUDA(cudaMemsetAsync(E.off_b.p, 0, sizeof(int32_t) * (n + 1), s));
-        int32_t vals[3];
-        const int32_t* srcs[3] = {E.off_a.p + n, E.np_tri.p, E.flag_off.p + n_items};
-        RC(read_scalars(ctx, srcs, 3, vals));
-        const int32_t tot = vals[0];
-        c_tri = vals[1];
-        n_rec += vals[2];
-        RC(E.soup_next.ensure(tot + 1));
-        LAUNCH(k_expand_write, n, n, E.soup.p, E.entry_hits.p, ctx->nodes.p, 0, E.off_a.p,
-                                                     E.off_b.p, E.soup_next.p, E.conn_next.p);
-        std::swap(E.soup, E.soup_next);
-        n = tot;
-    }
-    if (abandon) {
-        n_rec = rec_start;
-        c_tri = tri_start;
-        ctx->h_pinned[0] = tri_start;  // stream-ordered before any later read into h_pinned
-        D2G_CUDA(cudaMemcpyAsync(E.np_tri.p, ctx->h_pinned, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-        chunk = std::max(1, (p1 - p0) / 2);
-        continue;
-    }
-    c_node += k_node;
-    c_levels += k_levels;
-    peak = std::max(peak, chunk_peak);
-    p0 = p1;
+        c_node += T.nodes + T.n_leaf - T.n_root;  // root pairs of two leaves are in both
+        c_tri += T.tri;
+        c_levels += T.levels;
+        peak = std::max(peak, T.peak);
+        p0 = p1;
     }
     if (n_pairs > 0) E.np_chunk = chunk >= n_pairs ? 0 : (peak < 1.0 / 3.0 ? 2 * chunk : chunk);
     RC(finish_records(ctx, n_pairs, n_rec));
@@ -2892,7 +2862,7 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
     if (counters) {
         counters[0] = c_node;
         counters[1] = c_tri;
-        counters[2] = c_leaf;
+        counters[2] = 0;
         counters[3] = c_levels;
     }
     return D2G_OK;
@@ -2912,8 +2882,6 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
     RC(E.search.ensure(2));
     RC(E.pm32.ensure(25));
     RC(E.roots.ensure(2));
-    RC(E.np_tri.ensure(1));
-    D2G_CUDA(cudaMemsetAsync(E.np_tri.p, 0, sizeof(int32_t), s));
     LAUNCH(k_np_prep, 1, 1, d_pair, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p, E.pm.p,
            E.search.p, E.roots.p, E.pm32.p);
     RC(E.soup.ensure(n + 1));
@@ -2926,33 +2894,8 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
         return D2G_OK;
     }
     LAUNCH(k_bucket_entries, n, n, d_node_pairs, E.soup.p);
-    const int n_slots = 64 * n;
-    const int n_words = n_slots / 32;
-    DBuf<double>& res_eps = E.pfut;  // as in run_narrowphase
-    RC(E.res.ensure(n_slots));
-    RC(res_eps.ensure(4 * (size_t)n_slots));
-    RC(E.hit.ensure(n_slots));
-    RC(E.np_mask.ensure(n_words + 1));
-    RC(E.np_cnt.ensure(n_words + 1));
-    RC(E.np_off.ensure(n_words + 1));
-    RC(E.items.ensure(n_slots + 1));
-    LAUNCH(k_np_mask, n_slots, n_slots, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p,
-           ctx->eps_up.p, E.search.p, (const int4*)nullptr, E.np_mask.p, E.np_cnt.p, E.entry_hits.p,
-           E.fp32_bounds ? 1 : 0);
-    RC(scan(ctx, E.np_cnt.p, E.np_off.p, n_words));
-    LAUNCH(k_np_items, n_slots, n_slots, E.np_mask.p, E.np_off.p, E.items.p);
-    int32_t n_items = 0;
-    {
-        const int32_t* src = E.np_off.p + n_words;
-        RC(read_scalars(ctx, &src, 1, &n_items));
-    }
-    if (n_items > 0) {
-        const int pf = prof_begin(ctx, PROF_NP, n_slots);
-        LAUNCH(k_np, n_items, n_items, E.soup.p, d_pair, E.pm.p, ctx->ntris.p, ctx->tris.p, ctx->eps.p,
-               ctx->inner_eps.p, ctx->geo_eps.p, E.search.p, E.res.p, res_eps.p, E.hit.p, E.entry_hits.p, E.items.p,
-               E.fp32_bounds ? 1 : 0);
-        prof_end(ctx, pf);
-    }
+    int n_items = 0;
+    RC(np_slot_tests(ctx, d_pair, E.soup.p, n, &n_items));
     RC(E.flag_off.ensure(n_items + 1));
     RC(scan(ctx, E.hit.p, E.flag_off.p, n_items));
     RC(scan(ctx, E.entry_hits.p, E.off_a.p, n));
@@ -2965,7 +2908,7 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
     RC(E.rec_pair.ensure((size_t)tot + 1));
     if (tot > 0)
         LAUNCH(k_emit, n_items, n_items, E.hit.p, E.flag_off.p, E.items.p, 6, E.soup.p, (const int32_t*)nullptr,
-               d_pair, E.res.p, res_eps.p, ctx->geo_eps.p, E.rec.p, E.rec_pair.p, 0);
+               d_pair, E.res.p, E.pfut.p, ctx->geo_eps.p, E.rec.p, E.rec_pair.p, 0);
     D2G_CUDA(cudaGetLastError());
     *n_hits = tot;
     return D2G_OK;
@@ -3119,9 +3062,7 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
     Entry* next = cv.take<Entry>(MN);
     int32_t* entry_hits = cv.take<int32_t>(MN);
     int32_t* cnt_a = cv.take<int32_t>(MN);
-    int32_t* cnt_b = cv.take<int32_t>(MN);
     int32_t* off_a = cv.take<int32_t>(MN + 1);
-    int32_t* off_b = cv.take<int32_t>(MN + 1);
     PrimResult* res = cv.take<PrimResult>(64 * (size_t)MN);
     double* res_eps = cv.take<double>(4 * 64 * (size_t)MN);
     int32_t* hit = cv.take<int32_t>(64 * (size_t)MN);
@@ -3177,9 +3118,8 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
             NA_LAUNCH(k_emit, n_slots, n_slots, flags, flag_off, nullptr, 6, front, nullptr, d_pairs, res, res_eps,
                       sc->geo_eps, rec, rec_pair, n_rec);
         n_rec += tot;
-        NA_LAUNCH(k_expand_count, n, n, front, entry_hits, nodes, 0, cnt_a, cnt_b);
+        NA_LAUNCH(k_expand_count, n, n, front, entry_hits, nodes, cnt_a);
         if (int rc = noalloc_scan(s, tmp, tmp_bytes, cnt_a, off_a, n)) return rc;
-        D2G_CUDA(cudaMemsetAsync(off_b, 0, sizeof(int32_t) * (n + 1), s));
         int32_t nn = 0;
         if (int rc = noalloc_read(s, off_a + n, &nn)) return rc;
         if (nn > MN) {
@@ -3187,7 +3127,7 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
                       std::to_string(level + 1) + " exceed the limit of " + std::to_string(MN));
             return D2G_ERR_INVALID;
         }
-        NA_LAUNCH(k_expand_write, n, n, front, entry_hits, nodes, 0, off_a, off_b, next, next);
+        NA_LAUNCH(k_expand_write, n, n, front, entry_hits, nodes, off_a, next);
         Entry* t = front;
         front = next;
         next = t;

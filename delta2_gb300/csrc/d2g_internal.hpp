@@ -136,7 +136,7 @@ struct Engine {
     // frontiers
     DBuf<Entry> soup, conn, soup_next, conn_next;
     // per-entry counters / offsets
-    DBuf<int32_t> entry_hits, cnt_a, cnt_b, off_a, off_b;
+    DBuf<int32_t> entry_hits, off_a;
     // items of a stage
     DBuf<int32_t> flags, flag_off, items;
     DBuf<PrimResult> res;
@@ -144,12 +144,12 @@ struct Engine {
     // flattened primitive tests of a CCD level: soup sub-test results, leaf-pair
     // results, their hit flags and offsets
     DBuf<PrimResult> sub, cres;
-    DBuf<int32_t> chit, cflag_off, nn_cnt, nn_off, tp, lc;  // tp: leaf pair of a triangle pair; lc: level counters
+    DBuf<int32_t> chit, cflag_off, nn_cnt, nn_off, tp, lc, sums;  // tp: leaf pair of a triangle pair; lc: level counters
     // time-step selection
     DBuf<double> st_mt, st_new_dt, st_step, st_out;
     DBuf<int32_t> st_has, st_cl_pair_off, st_cl_part_off, st_cl_parts, st_loc;
     // contact filtering
-    DBuf<int32_t> flt_idx, flt_order, flt_keep, flt_pos, flt_cnt, flt_off, np_tri;
+    DBuf<int32_t> flt_idx, flt_order, flt_keep, flt_pos, flt_cnt, flt_off;
     DBuf<unsigned long long> flt_keys, flt_keys_s;
     DBuf<double> flt_mid;
     // CCD candidates: FP32 poses (8 per pair), survivor counts and lists
@@ -205,7 +205,7 @@ struct Engine {
     // phased edge-edge CCD (d2g_engine.cu)
     DBuf<double> ee_rec;
     DBuf<int32_t> ee_work;
-    int ee_grid = 0, soup_grid = 0;  // k_ee_rest4 and k_soup_tests grids (every block resident)
+    int ee_grid = 0, soup_grid = 0, np_grid = 0;  // k_ee_rest4, k_soup_tests, k_np_level_tests grids (all resident)
     // traversal chunking: root entries of the call's pairs; a byte budget for
     // a level's buffers (0: a third of the device memory)
     DBuf<Entry> roots;
