@@ -227,8 +227,8 @@ __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restri
 // test with a distance below the search distance.  Every edge-edge test
 // returns at most its distance at the start (edgeEdgeCCD evaluates it first)
 // or at most 1e-8, so a slot whose triangles' vertices, or else edges, are
-// closer than the search distance there by a margin (1 mm plus 4e-6 of the
-// coordinates, FP32) certainly hits: the node pair is marked and done.  The
+// closer than the search distance there by a margin (20 um plus 4e-6 of the
+// coordinates, above their FP32 rounding) certainly hits: the node pair is marked and done.  The
 // slots of the others go onto `list` for k_soup_tests.  Two bodies that are
 // single leaves meet at the root: their slots are counted (`lc`) and tested
 // with the leaf pairs (k_soup_filter).  The box stage:
@@ -263,6 +263,8 @@ __device__ __forceinline__ void swept_slots(const Entry& e, const int32_t* __res
         const float* MS = pm32_of(pm32, e.pair, side_b ? P32_BS : P32_AS);
         const float* ME = pm32_of(pm32, e.pair, side_b ? P32_BE : P32_AE);
         float o[3], oe[3][3];
+        mag = fmaxf(fmaxf(fmaxf(fabsf(MS[3]), fabsf(MS[7])), fabsf(MS[11])),
+                    fmaxf(fmaxf(fabsf(ME[3]), fabsf(ME[7])), fabsf(ME[11])));
 #pragma unroll
         for (int v = 0; v < 3; v++) {
             box_add(b32, MS, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
@@ -368,17 +370,23 @@ __device__ __forceinline__ float vert_min(const float* a, const float* b) {
         }
     return sqrtf(m);
 }
-__device__ __forceinline__ float edge_min(const float* a, const float* b) {
+// The closest edge pair: its distance, and the vector between its points.
+__device__ __forceinline__ float edge_min(const float* a, const float* b, F3& dir) {
     float m = 3.4e38f;
+    dir = f3(0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             const int i1 = (i + 1) % 3, j1 = (j + 1) % 3;
             float d2;
-            seg_vector(f3(a[3 * i], a[3 * i + 1], a[3 * i + 2]), f3(a[3 * i1], a[3 * i1 + 1], a[3 * i1 + 2]),
-                       f3(b[3 * j], b[3 * j + 1], b[3 * j + 2]), f3(b[3 * j1], b[3 * j1 + 1], b[3 * j1 + 2]), d2);
-            m = fminf(m, d2);
+            const F3 d =
+                seg_vector(f3(a[3 * i], a[3 * i + 1], a[3 * i + 2]), f3(a[3 * i1], a[3 * i1 + 1], a[3 * i1 + 2]),
+                           f3(b[3 * j], b[3 * j + 1], b[3 * j + 2]), f3(b[3 * j1], b[3 * j1 + 1], b[3 * j1 + 2]), d2);
+            if (d2 < m) {
+                m = d2;
+                dir = d;
+            }
         }
     return sqrtf(m);
 }
@@ -415,7 +423,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
             const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
             room[h] = -1.f;
             if (!res[h] || !use_bounds || !(thr > 1e-6f)) continue;
-            room[h] = thr - (1e-3f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
+            room[h] = thr - (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
             sure = sure || vert_min(s_verts[wi][ta], s_verts[wi][8 + tb]) < room[h];
         }
         sure = __any_sync(0xffffffffu, sure);
@@ -423,7 +431,8 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
-                if (room[h] > 0.f) sure = sure || edge_min(s_verts[wi][ta], s_verts[wi][8 + tb]) < room[h];
+                F3 d;
+                if (room[h] > 0.f) sure = sure || edge_min(s_verts[wi][ta], s_verts[wi][8 + tb], d) < room[h];
             }
             sure = __any_sync(0xffffffffu, sure);
         }
@@ -946,9 +955,15 @@ __device__ __forceinline__ void warp_append(int j, bool keep, int32_t* list, int
     if (keep) list[base + __popc(m & ((1u << lane) - 1u))] = j;
 }
 
-// The FP32 box bound of a point-triangle test: certainly farther apart than thr.
-__device__ __forceinline__ bool pt_box_gap(const float* __restrict__ pm32, int pair, int mC, int mT, const float* pt,
-                                           const float* tv, float thr) {
+// FP32 bounds of a point-triangle test (pointTriCCDLinear): certainly no
+// distance below thr.  Either the boxes are apart; or the point keeps its side
+// of the triangle's plane, so that only its start and end count, and at each
+// its projection is outside the triangle or it is too far above the plane.
+// Both in FP32 with margins: the box's as for k_ccd_mask_ee; the plane's in
+// the triangle's frame (PlaneBound, which covers the reference's single-
+// precision barycentrics).
+__device__ __forceinline__ bool pt_apart(const float* __restrict__ pm32, int pair, int mC, int mT, const float* pt,
+                                         const float* tv, float thr) {
     const float *Cs = pm32_of(pm32, pair, mC), *Ce = pm32_of(pm32, pair, mC + 1);
     const float *tS = pm32_of(pm32, pair, mT), *tE = pm32_of(pm32, pair, mT + 1);
     float mag = 0.f, ps[3], pe[3], o[3];
@@ -958,6 +973,8 @@ __device__ __forceinline__ bool pt_box_gap(const float* __restrict__ pm32, int p
     box_init(scratch);
     box_add(scratch, Cs, pt[0], pt[1], pt[2], ps, mag);
     box_add(scratch, Ce, pt[0], pt[1], pt[2], pe, mag);
+    const float local = fmaxf(mag, fmaxf(fmaxf(fmaxf(fabsf(Cs[3]), fabsf(Cs[7])), fabsf(Cs[11])),
+                                         fmaxf(fmaxf(fabsf(Ce[3]), fabsf(Ce[7])), fabsf(Ce[11]))));
     box_add(bp, tS, ps[0], ps[1], ps[2], o, mag);
     box_add(bp, tS, pe[0], pe[1], pe[2], o, mag);
     box_add(bp, tE, ps[0], ps[1], ps[2], o, mag);
@@ -966,7 +983,25 @@ __device__ __forceinline__ bool pt_box_gap(const float* __restrict__ pm32, int p
         box_add(bq, tS, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
         box_add(bq, tE, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
     }
-    return box_gap(bp, bq) > thr + (1e-3f + 4e-6f * (mag + thr));  // NaN: not certain
+    if (box_gap(bp, bq) > thr + (1e-3f + 4e-6f * (mag + thr))) return true;  // NaN: not certain
+    const F3 T0 = f3(tv[0], tv[1], tv[2]), T1 = f3(tv[3], tv[4], tv[5]), T2 = f3(tv[6], tv[7], tv[8]);
+    const F3 p0 = f3(ps[0], ps[1], ps[2]), p1 = f3(pe[0], pe[1], pe[2]);
+    // the frame's coordinates carry an error of 4e-7 of their size, 1e-6 here
+    const float rho = fmaxf(fmaxf(local, fmaxf(maxabs3(T0), fmaxf(maxabs3(T1), maxabs3(T2)))), 1e-3f);
+    const PlaneBound P = plane_bound(T0, T1, T2, 8.f * rho);
+    if (!P.ok) return false;
+    const F3 q[2] = {p0 - T0, p1 - T0};
+    const float h0 = dot3(P.n, q[0]), h1 = dot3(P.n, q[1]);
+    const float err = 2.f * P.eh * 8.f * rho;
+    if (!((h0 > err && h1 > err) || (h0 < -err && h1 < -err))) return false;
+    const float lim = (thr + (2e-5f + 4e-6f * (8.f * rho + thr))) * P.len + err;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        float u, v, w;
+        plane_bary(P, q[k], u, v, w);
+        if (!(u < -P.mb || v < -P.mb || w < -P.mb) && !(fabsf(k ? h1 : h0) > lim)) return false;
+    }
+    return true;
 }
 
 __global__ void __launch_bounds__(kBlock) k_ccd_mask_pt(int n_tp, int n_total, const int32_t* __restrict__ items,
@@ -985,7 +1020,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_pt(int n_tp, int n_total, c
         const PtWork w = decode_pt(j, n_tp, items, soup, conn, nn_off, tp, ntris, sub, cres, chit);
         const float* pt = tri32 + ((size_t)w.pt_node * 8 + w.pt_tri) * 9 + 3 * w.pt_vert;
         const float* tv = tri32 + ((size_t)w.tri_node * 8 + w.tri_idx) * 9;
-        keep = !use_bounds || !pt_box_gap(pm32, w.pair, w.mC, w.mT, pt, tv, search[w.pair]);
+        keep = !use_bounds || !pt_apart(pm32, w.pair, w.mC, w.mT, pt, tv, search[w.pair]);
         if (!keep) record_no_contact(w.out, w.hit);
     }
     warp_append(j, keep, list, count);
@@ -1265,7 +1300,7 @@ __global__ void __launch_bounds__(kPrimBlock) k_soup_tests(
             if (use_bounds) {
                 const float* pt = (pb ? fb : fa) + 3 * i;
                 const float* tv = pb ? fa : fb;
-                if (pt_box_gap(pm32, e.pair, pb ? P32_BAS : P32_ABS, pb ? P32_AS : P32_BS, pt, tv, thr)) continue;
+                if (pt_apart(pm32, e.pair, pb ? P32_BAS : P32_ABS, pb ? P32_AS : P32_BS, pt, tv, thr)) continue;
             }
             const Tri A = load_tri(da), B = load_tri(db);
             const Ccd r = pb ? point_tri_ccd(tvert(B, i), M + PM_BAS, M + PM_BAE, A, M + PM_AS, M + PM_AE)
@@ -1568,12 +1603,12 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // thr = search + eps_a + eps_b.  Lower bounds on that distance: the bounding
 // spheres' |c_a - c_b| - r_a - r_b (centroid, radius rounded up), the gap
 // between the boxes of the transformed triangles and, for slots those keep,
-// the gaps along the eleven separating axes (two face normals, nine edge-edge
-// cross products).  The largest is evaluated in FP32 and a slot is dropped
+// the gaps along the two face normals and the direction between the closest
+// edges.  The largest is evaluated in FP32 and a slot is dropped
 // only when it exceeds thr by a margin
-// (1 mm plus 4e-6 of the magnitudes involved) far above the FP32 rounding of
-// the bound and the FP64 rounding of the exact test, so every slot that hits
-// survives.  Dropped slots produce nothing in the reference
+// (20 um plus 4e-6 of the magnitudes involved) far above the FP32 rounding of
+// the bound (3e-7 of them) and the FP64 rounding of the exact test, so every
+// slot that hits survives.  Dropped slots produce nothing in the reference
 // either.
 //
 // A warp per node pair: lanes 0-7 transform a's triangles, 8-15 b's, once each
@@ -1587,50 +1622,31 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // than thr by the same margin certainly hits (unless a triangle is almost a
 // point, whose edges return no distance); the pair is marked and done, and only
 // the survivors of the others go onto `list` for k_np_level_tests.
-__device__ __forceinline__ float sat_gap(const float* a, const float* b) {
-    // Separating axes: along any direction n the distance is at least the gap
-    // between the projections divided by |n|, whatever n is, so n computed in
-    // FP32 still bounds; the two face normals and the nine edge-edge cross
-    // products.
-    float wa[3][3], wb[3][3], ea[3][3], eb[3][3];
+// The gap between the triangles along d (d need not be a unit vector).
+__device__ __forceinline__ float axis_gap9(F3 d, const float* a, const float* b) {
+    const float nn = sqrtf(dot3(d, d));
+    if (!(nn > 1e-20f)) return 0.f;
+    float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
 #pragma unroll
-    for (int v = 0; v < 3; v++)
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            wa[v][r] = a[3 * v + r];
-            wb[v][r] = b[3 * v + r];
-        }
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            ea[k][r] = wa[(k + 1) % 3][r] - wa[k][r];
-            eb[k][r] = wb[(k + 1) % 3][r] - wb[k][r];
-        }
-    auto axis_gap = [&](float nx, float ny, float nz) {
-        const float nn = sqrtf(nx * nx + ny * ny + nz * nz);
-        if (!(nn > 1e-20f)) return 0.f;
-        float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
-#pragma unroll
-        for (int v = 0; v < 3; v++) {
-            const float pa = wa[v][0] * nx + wa[v][1] * ny + wa[v][2] * nz;
-            const float pb = wb[v][0] * nx + wb[v][1] * ny + wb[v][2] * nz;
-            a0 = fminf(a0, pa);
-            a1 = fmaxf(a1, pa);
-            b0 = fminf(b0, pb);
-            b1 = fmaxf(b1, pb);
-        }
-        return fmaxf(b0 - a1, a0 - b1) / nn;
-    };
-    auto cross_gap = [&](const float(&u)[3], const float(&v)[3]) {
-        return axis_gap(u[1] * v[2] - u[2] * v[1], u[2] * v[0] - u[0] * v[2], u[0] * v[1] - u[1] * v[0]);
-    };
-    float lb = fmaxf(cross_gap(ea[0], ea[1]), cross_gap(eb[0], eb[1]));
-#pragma unroll
-    for (int x = 0; x < 3; x++)
-#pragma unroll
-        for (int y = 0; y < 3; y++) lb = fmaxf(lb, cross_gap(ea[x], eb[y]));
-    return lb;
+    for (int v = 0; v < 3; v++) {
+        const float pa = dot3(d, f3(a[3 * v], a[3 * v + 1], a[3 * v + 2]));
+        const float pb = dot3(d, f3(b[3 * v], b[3 * v + 1], b[3 * v + 2]));
+        a0 = fminf(a0, pa);
+        a1 = fmaxf(a1, pa);
+        b0 = fminf(b0, pb);
+        b1 = fmaxf(b1, pb);
+    }
+    return fmaxf(b0 - a1, a0 - b1) / nn;
+}
+// A lower bound of the triangles' distance: along any direction the distance
+// is at least the gap between the projections, whatever the direction, so one
+// computed in FP32 still bounds.  Separate triangles are closest between two
+// edges, in the direction d of their closest edge pair, or between a vertex and
+// a face, along its normal.
+__device__ __forceinline__ float tri_gap(F3 d, const float* a, const float* b) {
+    const F3 na = cross3(f3(a[3] - a[0], a[4] - a[1], a[5] - a[2]), f3(a[6] - a[0], a[7] - a[1], a[8] - a[2]));
+    const F3 nb = cross3(f3(b[3] - b[0], b[4] - b[1], b[5] - b[2]), f3(b[6] - b[0], b[7] - b[1], b[8] - b[2]));
+    return fmaxf(axis_gap9(d, a, b), fmaxf(axis_gap9(na, a, b), axis_gap9(nb, a, b)));
 }
 __device__ __forceinline__ float box_gap9(const float* a, const float* b) {
     float gap2 = 0.f;
@@ -1709,33 +1725,40 @@ __global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __rest
         const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb];
         const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
         const float thr = se + ca[4] + cb[4];
-        const float margin = 1e-3f + 4e-6f * (tm + ca[5] + cb[5] + thr);
+        const float margin = 2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr);
         lim[h] = thr + margin;
         keep[h] = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim[h]) &&  // NaN keeps the slot
                   !(box_gap9(s_v[wi][ta], s_v[wi][8 + tb]) > lim[h]);
         if (keep[h] && ca[6] + cb[6] == 0.f) room[h] = thr - margin;
     }
-    if (!LEAF && use_bounds) {
+    const float* va[2] = {s_v[wi][lane >> 3], s_v[wi][(lane >> 3) + 4]};
+    const float* vb = s_v[wi][8 + (lane & 7)];
+    if (!LEAF) {
         bool sure = false;
 #pragma unroll
         for (int h = 0; h < 2; h++)
-            if (room[h] > 0.f) sure = sure || vert_min(s_v[wi][(lane + 32 * h) >> 3], s_v[wi][8 + (lane & 7)]) < room[h];
+            if (room[h] > 0.f) sure = sure || vert_min(va[h], vb) < room[h];
         sure = __any_sync(0xffffffffu, sure);
-        if (!sure) {
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-                if (room[h] > 0.f)
-                    sure = sure || edge_min(s_v[wi][(lane + 32 * h) >> 3], s_v[wi][8 + (lane & 7)]) < room[h];
-            sure = __any_sync(0xffffffffu, sure);
-        }
         if (lane == 0) entry_hits[w] = sure ? 1 : 0;
         if (sure) return;
-    } else if (!LEAF) {
-        if (lane == 0) entry_hits[w] = 0;
+    }
+    bool sure = false;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        if (!keep[h] || !use_bounds) continue;
+        F3 d;
+        if (edge_min(va[h], vb, d) < room[h]) {
+            sure = true;
+            if (!LEAF) break;
+        }
+        keep[h] = !(tri_gap(d, va[h], vb) > lim[h]);
+    }
+    if (!LEAF && __any_sync(0xffffffffu, sure)) {
+        if (lane == 0) entry_hits[w] = 1;
+        return;
     }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        if (keep[h] && use_bounds) keep[h] = !(sat_gap(s_v[wi][(lane + 32 * h) >> 3], s_v[wi][8 + (lane & 7)]) > lim[h]);
         if (LEAF) {
             const unsigned m = __ballot_sync(0xffffffffu, keep[h]);
             if (lane == 0) {
@@ -1935,7 +1958,7 @@ __global__ void k_expand_write(int n, const Entry* __restrict__ front, const int
 // node pairs one block does it all; larger levels take two launches,
 // k_expand_sums for the blocks' totals and k_expand_level, whose blocks add up
 // the totals before theirs (three launches and a library scan before).
-constexpr int kExpandThreads = 256, kExpandOneBlock = 1024;
+constexpr int kExpandThreads = 256, kExpandOneThreads = 1024, kExpandOneBlock = 2048;
 struct Opened {
     Entry e;
     int4 P;           // the opened node (two leaves: y = self_leaf)
@@ -1961,8 +1984,9 @@ __device__ __forceinline__ bool open_pair(const Entry& e, const int4* __restrict
     return true;
 }
 // Exclusive prefix sums of (s, c) over the block, and its totals (every thread).
+template <int THREADS>
 __device__ __forceinline__ int2 block_scan2(int s, int c, int2& total) {
-    __shared__ int2 wsum[kExpandThreads / 32];
+    __shared__ int2 wsum[THREADS / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int xs = s, xc = c;
 #pragma unroll
@@ -1979,7 +2003,7 @@ __device__ __forceinline__ int2 block_scan2(int s, int c, int2& total) {
     int2 before = make_int2(xs - s, xc - c);
     total = make_int2(0, 0);
 #pragma unroll
-    for (int k = 0; k < kExpandThreads / 32; k++) {
+    for (int k = 0; k < THREADS / 32; k++) {
         const int2 v = wsum[k];
         if (k < w) {
             before.x += v.x;
@@ -2002,10 +2026,11 @@ __global__ void __launch_bounds__(kExpandThreads) k_expand_sums(int n, const Ent
         s = o.P.y - c;
     }
     int2 total;
-    block_scan2(s, c, total);
+    block_scan2<kExpandThreads>(s, c, total);
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
-__global__ void __launch_bounds__(kExpandThreads) k_expand_level(int n, const Entry* __restrict__ front,
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_expand_level(int n, const Entry* __restrict__ front,
                                                                  const int32_t* __restrict__ entry_hits,
                                                                  const int4* __restrict__ nodes, int self_leaf,
                                                                  const int2* __restrict__ sums,
@@ -2014,17 +2039,17 @@ __global__ void __launch_bounds__(kExpandThreads) k_expand_level(int n, const En
     int2 base = make_int2(0, leaf0);
     if (sums) {  // the blocks before this one
         int s = 0, c = 0;
-        for (int k = threadIdx.x; k < (int)blockIdx.x; k += kExpandThreads) {
+        for (int k = threadIdx.x; k < (int)blockIdx.x; k += THREADS) {
             s += sums[k].x;
             c += sums[k].y;
         }
         int2 total;
-        block_scan2(s, c, total);
+        block_scan2<THREADS>(s, c, total);
         base.x += total.x;
         base.y += total.y;
     }
-    const int step = sums ? n : kExpandThreads;  // one block walks the level, else one pass
-    for (int i0 = sums ? blockIdx.x * kExpandThreads : 0; i0 < n; i0 += step) {
+    const int step = sums ? n : THREADS;  // one block walks the level, else one pass
+    for (int i0 = sums ? blockIdx.x * THREADS : 0; i0 < n; i0 += step) {
         const int i = i0 + threadIdx.x;
         Opened o;
         int s = 0, c = 0;
@@ -2033,7 +2058,7 @@ __global__ void __launch_bounds__(kExpandThreads) k_expand_level(int n, const En
             s = o.P.y - c;
         }
         int2 total;
-        const int2 at = block_scan2(s, c, total);
+        const int2 at = block_scan2<THREADS>(s, c, total);
         if (s + c > 0) {
             Entry* ps = next + base.x + at.x;
             Entry* pc = leaf + base.y + at.y;
@@ -2465,9 +2490,14 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
                                                             self_leaf ? 1 : 0, (int2*)E.sums.p);
             E.launches++;
         }
-        k_expand_level<<<blocks, kExpandThreads, 0, s>>>(n, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0,
-                                                         one ? (const int2*)nullptr : (const int2*)E.sums.p,
-                                                         E.soup_next.p, E.conn.p, T.n_leaf, E.lc.p);
+        if (one)
+            k_expand_level<kExpandOneThreads><<<1, kExpandOneThreads, 0, s>>>(
+                n, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0, nullptr, E.soup_next.p, E.conn.p,
+                T.n_leaf, E.lc.p);
+        else
+            k_expand_level<kExpandThreads><<<blocks, kExpandThreads, 0, s>>>(
+                n, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0, (const int2*)E.sums.p, E.soup_next.p,
+                E.conn.p, T.n_leaf, E.lc.p);
         E.launches++;
         D2G_CUDA(cudaMemcpyAsync(ctx->h_pinned, E.lc.p, sizeof(int32_t) * LC_SIZE, cudaMemcpyDeviceToHost, s));
         D2G_CUDA(cudaStreamSynchronize(s));
