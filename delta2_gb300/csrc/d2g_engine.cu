@@ -229,7 +229,7 @@ __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restri
 // or at most 1e-8, so a slot whose triangles' vertices, or else edges, are
 // closer than the search distance there by a margin (20 um plus 4e-6 of the
 // coordinates, above their FP32 rounding) certainly hits: the node pair is marked and done.  The
-// slots of the others go onto `list` for k_soup_tests.  Two bodies that are
+// slots of the others go onto `list` for k_soup_slots.  Two bodies that are
 // single leaves meet at the root: their slots are counted (`lc`) and tested
 // with the leaf pairs (k_soup_filter).  The box stage:
 // lanes 0-7 form the swept boxes of a's triangles, lanes 8-15 those of b's,
@@ -1120,23 +1120,26 @@ __global__ void __launch_bounds__(kPrimBlock) k_prim_pt(int n_tp, int n_total, c
     chit[item] = r.dist < (double)search[e.pair] ? 1 : 0;
 }
 
-// Edge-edge CCD in two kernels over the level's surviving tests.  GB300's
-// FP64 pipe takes one warp instruction per 64 cycles per SM sub-partition
-// (SMSP), dependent or not and whatever the number of active lanes (a
-// division costs ~9 such slots, a square root ~10), and a level has only a
-// few thousand surviving tests, so a warp's time is the instruction count of
-// its longest lane and the level's time that of its slowest warp.  62% of the
-// tests end within two Newton iterations and 20% run all ten, so:
-//   k_ee_first   one test per lane: edges, FP64 box-gap skip, the bisection
-//                (its cost is about two Newton iterations) or at most two
-//                Newton iterations; the tests still running are saved and
-//                listed.
-//   k_ee_rest4   the listed tests on four lanes each (below): the remaining
-//                iterations with about half the instructions per iteration,
-//                on few enough warps that each has an SMSP to itself.
+// Edge-edge CCD in two passes over the surviving tests.  GB300's FP64 pipe
+// takes one warp instruction per 64 cycles per SM sub-partition (SMSP),
+// dependent or not and whatever the number of active lanes (a division costs
+// ~9 such slots, a square root ~10), so a warp's time is the instruction count
+// of its longest lane.  62% of the tests end within two Newton iterations (~330
+// slots each on one lane) and 20% run all ten; 0.5% bisect (~1,300 slots, which
+// would double the first pass for every warp that has one).  So:
+//   k_ee_first   one test per lane: edges, FP64 box-gap skip and at most two
+//                Newton iterations; the tests still running and those that
+//                bisect are saved and listed.
+//   k_ee_rest4   the listed tests on four lanes each (below), ~230 slots an
+//                iteration: while the list gives each SMSP at most a warp or
+//                two, latency is what counts.
+//   k_ee_rest1   the listed tests on one lane each, when there are more than
+//                kRestWide: a quarter of the warps at 1.4 times the slots (noisy
+//                spheres, 71,000 listed tests: 1,225 us on four lanes).
 // Each test performs exactly the operations of edge_edge_ccd, in order.
 // The first pass's iteration cap is the context setting D2G_TUNE_EE_FIRST_ITERS (default 2).
-constexpr int kEeRec = 10;  // saved test: t, min_dist, P, Q, toc, iterations done (the edges are recomputed)
+constexpr int kRestWide = 7000;
+constexpr int kEeRec = 10;  // saved test: t, min_dist, P, Q, toc, iterations done or -1: bisect (the edges are recomputed)
 struct EeArgs {
     int n_tp;
     const int32_t* items;
@@ -1196,18 +1199,137 @@ __device__ __forceinline__ bool ee_steady(const Edge& S, const Edge& E) {
 // The undecided slots of a level (list of node pair * 64 + slot): whether any
 // of their 15 sub-tests (continuous_comparison.h:692-777) returns a distance
 // below the search distance; a hit marks the node pair and ends its other
-// tests.  A thread a test, edge-edge tests first, in grid-stride order over
-// the list's device count.  FP32 bounds as in k_ccd_mask_pt / ee drop most
-// tests, and for edges also the gap along the closest points' direction at
-// the start, the smaller of the start's and the end's (the gap of linearly
-// moving points is concave in time).  An edge-edge test's distance at the
-// start decides it when it is a hit, or when it is beyond the search distance
-// by more than the motion (ee_motion_bound); only the rest runs edgeEdgeCCD.
-__global__ void __launch_bounds__(kPrimBlock) k_soup_tests(
-    const int32_t* __restrict__ list, const int32_t* __restrict__ n_list, const Entry* __restrict__ soup,
-    const double* __restrict__ pm, const float* __restrict__ pm32, const double* __restrict__ tris,
-    const float* __restrict__ tri32, const float* __restrict__ search, int32_t* entry_hits, int use_bounds,
-    int certificates, unsigned long long* ca_stats) {
+// slots.  A level leaves some ten to a few thousand slots, so the kernel lasts
+// as long as one slot's chain of FP64 instructions (64 cycles each): a warp a
+// slot, the vertices' start and end positions a component per lane, then the
+// nine edge pairs on lanes 0-8 and the six point-triangle tests on lanes
+// 16-21.  An edge pair is decided by its distance at the start (edgeEdgeCCD
+// evaluates it first, and returns no more than it or at most 1e-8), or by the
+// gap along the direction between its points there, the smaller of the start's
+// and the end's (the gap of linearly moving points is concave in time); the
+// rest runs edgeEdgeCCD's iterates until a distance is below the limit, and its
+// bisection (1,200 FP64 instructions) last.  A thread per sub-test took 51 us a
+// level on the 1,024-hull step.
+__global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict__ list,
+                                                       const int32_t* __restrict__ n_list,
+                                                       const Entry* __restrict__ soup, const double* __restrict__ pm,
+                                                       const float* __restrict__ pm32, const double* __restrict__ tris,
+                                                       const float* __restrict__ tri32,
+                                                       const float* __restrict__ search, int32_t* entry_hits,
+                                                       int certificates, unsigned long long* ca_stats) {
+    __shared__ double s_v[kBlock / 32][2][6][3];  // start, end; a's vertices, b's
+    const int n = *n_list;
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    double(*v)[6][3] = s_v[wi];
+    for (int k = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); k < n;
+         k += (int)((gridDim.x * (size_t)blockDim.x) >> 5)) {
+        const int slot = list[k];
+        if (__any_sync(0xffffffffu, ((volatile int32_t*)entry_hits)[slot >> 6] != 0)) continue;
+        const Entry e = soup[slot >> 6];
+        const int ta = (slot >> 3) & 7, tb = slot & 7;
+        const float thr = search[e.pair];
+        const double lim = (double)thr;
+        const double* M = pm + (size_t)PM_SIZE * e.pair;
+        const double* da = tris + (size_t)e.na * 72 + ta * 9;
+        const double* db = tris + (size_t)e.nb * 72 + tb * 9;
+        for (int r = lane; r < 36; r += 32) {  // xform_rigid, a row each
+            const int pose = r / 18, i = r % 18 / 3, c = r % 3;
+            const double* T = M + (i < 3 ? (pose ? PM_AE : PM_AS) : (pose ? PM_BE : PM_BS)) + 4 * c;
+            const double* p = i < 3 ? da + 3 * i : db + 3 * (i - 3);
+            v[pose][i][c] = ((T[0] * p[0] + T[1] * p[1]) + T[2] * p[2]) + T[3] * 1.0;
+        }
+        __syncwarp();
+        auto at = [&](int pose, int i) { return mk(v[pose][i][0], v[pose][i][1], v[pose][i][2]); };
+        Edge aS, aE, bS, bE;
+        bool hit = false, open = lane < 9, steady = false;
+        if (open) {
+            const int ia = lane / 3, ib = lane % 3, a1 = ia == 2 ? 0 : ia + 1, b1 = ib == 2 ? 0 : ib + 1;
+            aS.A = at(0, ia);
+            aS.B = at(0, a1);
+            aE.A = at(1, ia);
+            aE.B = at(1, a1);
+            bS.A = at(0, 3 + ib);
+            bS.B = at(0, 3 + b1);
+            bE.A = at(1, 3 + ib);
+            bE.B = at(1, 3 + b1);
+            // while no edge can vanish on its way every distance is a number, and
+            // any one below the limit makes the result one
+            steady = thr > 1e-6f && ee_steady(aS, aE) && ee_steady(bS, bE);
+            if (steady) {
+                V3 P, Q;
+                const double d0 = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q);
+                hit = d0 < lim;
+                const V3 d = Q - P;
+                const double g0 = fmin(dot(d, bS.A), dot(d, bS.B)) - fmax(dot(d, aS.A), dot(d, aS.B));
+                const double g1 = fmin(dot(d, bE.A), dot(d, bE.B)) - fmax(dot(d, aE.A), dot(d, aE.B));
+                const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
+                                        fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
+                open = !hit && !(fmin(g0, g1) >= ((lim + 1e-6) + 1e-9 * mag) * d0);
+            }
+        }
+        const unsigned cut = certificates ? __ballot_sync(0xffffffffu, lane < 9 && !hit && !open) : 0u;
+        if (lane == 0 && cut) {
+            atomicAdd(ca_stats, (unsigned long long)__popc(cut));
+            atomicAdd(ca_stats + 1, (unsigned long long)(__popc(cut) * (kEeNewtonIters - 1)));
+        }
+        bool any = __any_sync(0xffffffffu, hit);
+        double best = DBL_MAX;
+        if (!any && __any_sync(0xffffffffu, open)) {
+            if (open && steady) {  // edgeEdgeCCD's iterates, up to the first below the limit
+                Ccd r;
+                double t = 0.0;
+                for (int iter = 0; iter < kEeNewtonIters && !hit; iter++) {
+                    const bool last = ee_newton_iter(aS, aE, bS, bE, t, best, r);
+                    hit = best < lim;
+                    if (last) break;
+                }
+            }
+            any = __any_sync(0xffffffffu, hit);
+        }
+        if (!any && lane >= 16 && lane < 22) {
+            const int q = lane - 16, i = q >> 1;
+            const bool pb = (q & 1) != 0;  // a vertex of b against a, else of a against b
+            const float* fa = tri32 + ((size_t)e.na * 8 + ta) * 9;
+            const float* fb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
+            if (!pt_apart(pm32, e.pair, pb ? P32_BAS : P32_ABS, pb ? P32_AS : P32_BS, (pb ? fb : fa) + 3 * i,
+                          pb ? fa : fb, thr)) {
+                const double* p = (pb ? db : da) + 3 * i;
+                hit = point_tri_ccd(mk(p[0], p[1], p[2]), M + (pb ? PM_BAS : PM_ABS), M + (pb ? PM_BAE : PM_ABE),
+                                    load_tri(pb ? da : db), M + (pb ? PM_AS : PM_BS), M + (pb ? PM_AE : PM_BE))
+                          .dist < lim;
+            }
+        }
+        any = any || __any_sync(0xffffffffu, hit);
+        if (!any && __any_sync(0xffffffffu, open)) {
+            // the bisection's distance, and the whole of an unsteady test
+            if (open) {
+                Ccd r;
+                const double dot_start = ee_coplanarity(aS, bS);
+                const bool sign = dot_start * ee_coplanarity(aE, bE) < 0.0;
+                if (sign) best = ee_bisect(aS, aE, bS, bE, dot_start, r);
+                hit = best < lim;
+                if (!steady && !hit && best > 1e-8) {
+                    double t = 0.0;
+                    for (int iter = 0; iter < kEeNewtonIters; iter++)
+                        if (ee_newton_iter(aS, aE, bS, bE, t, best, r)) break;
+                    hit = best < lim;
+                }
+            }
+            any = __any_sync(0xffffffffu, hit);
+        }
+        if (any && lane == 0) entry_hits[slot >> 6] = 1;
+        __syncwarp();
+    }
+}
+
+// The same without FP32 bounds (the list holds every slot of the level), a
+// thread a test.
+__global__ void __launch_bounds__(kPrimBlock) k_soup_tests(const int32_t* __restrict__ list,
+                                                           const int32_t* __restrict__ n_list,
+                                                           const Entry* __restrict__ soup,
+                                                           const double* __restrict__ pm,
+                                                           const double* __restrict__ tris,
+                                                           const float* __restrict__ search, int32_t* entry_hits) {
     const int n = *n_list;
     const long long n_ee = 9LL * n, total = 15LL * n;
     for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < total;
@@ -1217,41 +1339,12 @@ __global__ void __launch_bounds__(kPrimBlock) k_soup_tests(
         const int slot = list[k];
         if (((volatile int32_t*)entry_hits)[slot >> 6]) continue;
         const Entry e = soup[slot >> 6];
-        const int ta = (slot >> 3) & 7, tb = slot & 7;
-        const float thr = search[e.pair];
-        const float* fa = tri32 + ((size_t)e.na * 8 + ta) * 9;
-        const float* fb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
         const double* M = pm + (size_t)PM_SIZE * e.pair;
-        const double* da = tris + (size_t)e.na * 72 + ta * 9;
-        const double* db = tris + (size_t)e.nb * 72 + tb * 9;
-        bool hit = false;
+        const Tri A = load_tri(tris + (size_t)e.na * 72 + ((slot >> 3) & 7) * 9);
+        const Tri B = load_tri(tris + (size_t)e.nb * 72 + (slot & 7) * 9);
+        double dist;
         if (ee) {
-            const int ia = q / 3, ib = q % 3;
-            if (use_bounds) {
-                const int a1 = ia == 2 ? 0 : ia + 1, b1 = ib == 2 ? 0 : ib + 1;
-                float mag = 0.f, o[2][4][3];  // [start, end][a0 a1 b0 b1]
-                Box32 ba, bb;
-                box_init(ba);
-                box_init(bb);
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    const float* MA = pm32_of(pm32, e.pair, P32_AS + m);
-                    const float* MB = pm32_of(pm32, e.pair, P32_BS + m);
-                    box_add(ba, MA, fa[3 * ia], fa[3 * ia + 1], fa[3 * ia + 2], o[m][0], mag);
-                    box_add(ba, MA, fa[3 * a1], fa[3 * a1 + 1], fa[3 * a1 + 2], o[m][1], mag);
-                    box_add(bb, MB, fb[3 * ib], fb[3 * ib + 1], fb[3 * ib + 2], o[m][2], mag);
-                    box_add(bb, MB, fb[3 * b1], fb[3 * b1 + 1], fb[3 * b1 + 2], o[m][3], mag);
-                }
-                const float lim = thr + (1e-3f + 4e-6f * (mag + thr));
-                if (box_gap(ba, bb) > lim) continue;  // NaN keeps the test
-                auto at = [&](int m, int v) { return f3(o[m][v][0], o[m][v][1], o[m][v][2]); };
-                float d2;
-                const F3 d = seg_vector(at(0, 0), at(0, 1), at(0, 2), at(0, 3), d2);
-                const float g0 = fminf(dot3(d, at(0, 2)), dot3(d, at(0, 3))) - fmaxf(dot3(d, at(0, 0)), dot3(d, at(0, 1)));
-                const float g1 = fminf(dot3(d, at(1, 2)), dot3(d, at(1, 3))) - fmaxf(dot3(d, at(1, 0)), dot3(d, at(1, 1)));
-                if (fminf(g0, g1) > lim * sqrtf(d2)) continue;
-            }
-            const Edge ea = tedge(load_tri(da), ia), eb = tedge(load_tri(db), ib);
+            const Edge ea = tedge(A, q / 3), eb = tedge(B, q % 3);
             Edge aS, aE, bS, bE;
             aS.A = xform_rigid(ea.A, M + PM_AS);
             aS.B = xform_rigid(ea.B, M + PM_AS);
@@ -1261,53 +1354,25 @@ __global__ void __launch_bounds__(kPrimBlock) k_soup_tests(
             aE.B = xform_rigid(ea.B, M + PM_AE);
             bE.A = xform_rigid(eb.A, M + PM_BE);
             bE.B = xform_rigid(eb.B, M + PM_BE);
-            // while no edge can vanish on its way every distance is a number
-            if (thr > 1e-6f && ee_steady(aS, aE) && ee_steady(bS, bE)) {
-                V3 P, Q;
-                const double d0 = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q), lim = (double)thr;
-                hit = d0 < lim;
-                bool open = !hit;
-                if (open && certificates) {
-                    const V3 d = Q - P;
-                    const double g0 = fmin(dot(d, bS.A), dot(d, bS.B)) - fmax(dot(d, aS.A), dot(d, aS.B));
-                    const double g1 = fmin(dot(d, bE.A), dot(d, bE.B)) - fmax(dot(d, aE.A), dot(d, aE.B));
-                    const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
-                                            fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
-                    if (fmin(g0, g1) >= ((lim + 1e-6) + 1e-9 * mag) * d0) {
-                        open = false;
-                        atomicAdd(ca_stats, 1ull);
-                        atomicAdd(ca_stats + 1, (unsigned long long)(kEeNewtonIters - 1));
-                    }
-                }
-                if (open) {  // edgeEdgeCCD up to its first distance below the limit
-                    Ccd r;
-                    const double dot_start = ee_coplanarity(aS, bS);
-                    double best = DBL_MAX, t = 0.0;
-                    if (dot_start * ee_coplanarity(aE, bE) < 0.0) best = ee_bisect(aS, aE, bS, bE, dot_start, r);
-                    hit = best < lim;
-                    for (int iter = 0; iter < kEeNewtonIters && !hit && best > 1e-8; iter++) {
-                        const bool last = ee_newton_iter(aS, aE, bS, bE, t, best, r);
-                        hit = best < lim;
-                        if (last) break;
-                    }
-                }
-            } else {
-                hit = edge_edge_ccd(aS, aE, bS, bE).dist < (double)thr;
+            V3 P, Q;
+            dist = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q);
+            const double lim = (double)search[e.pair];
+            if (!(lim > 1e-6 && ee_steady(aS, aE) && ee_steady(bS, bE))) {
+                dist = edge_edge_ccd(aS, aE, bS, bE).dist;
+            } else if (!(dist < lim)) {  // as in k_soup_slots
+                const V3 d = Q - P;
+                const double g0 = fmin(dot(d, bS.A), dot(d, bS.B)) - fmax(dot(d, aS.A), dot(d, aS.B));
+                const double g1 = fmin(dot(d, bE.A), dot(d, bE.B)) - fmax(dot(d, aE.A), dot(d, aE.B));
+                const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
+                                        fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
+                if (!(fmin(g0, g1) >= ((lim + 1e-6) + 1e-9 * mag) * dist)) dist = edge_edge_ccd(aS, aE, bS, bE).dist;
             }
+        } else if (q & 1) {
+            dist = point_tri_ccd(tvert(B, q >> 1), M + PM_BAS, M + PM_BAE, A, M + PM_AS, M + PM_AE).dist;
         } else {
-            const int i = q >> 1;
-            const bool pb = (q & 1) != 0;  // a vertex of b against a, else of a against b
-            if (use_bounds) {
-                const float* pt = (pb ? fb : fa) + 3 * i;
-                const float* tv = pb ? fa : fb;
-                if (pt_apart(pm32, e.pair, pb ? P32_BAS : P32_ABS, pb ? P32_AS : P32_BS, pt, tv, thr)) continue;
-            }
-            const Tri A = load_tri(da), B = load_tri(db);
-            const Ccd r = pb ? point_tri_ccd(tvert(B, i), M + PM_BAS, M + PM_BAE, A, M + PM_AS, M + PM_AE)
-                             : point_tri_ccd(tvert(A, i), M + PM_ABS, M + PM_ABE, B, M + PM_BS, M + PM_BE);
-            hit = r.dist < (double)thr;
+            dist = point_tri_ccd(tvert(A, q >> 1), M + PM_ABS, M + PM_ABE, B, M + PM_BS, M + PM_BE).dist;
         }
-        if (hit) entry_hits[slot >> 6] = 1;
+        if (dist < (double)search[e.pair]) entry_hits[slot >> 6] = 1;
     }
 }
 
@@ -1373,13 +1438,11 @@ __global__ void __launch_bounds__(kPrimBlock) k_ee_first(int n_total, const int3
             r.toc = 0.0;
             const double dot_start = ee_coplanarity(aS, bS);
             const double dot_end = ee_coplanarity(aE, bE);
-            bool bisected = false;
-            if (dot_start * dot_end < 0.0) {
-                min_dist = ee_bisect(aS, aE, bS, bE, dot_start, r);
-                bisected = true;
-            }
-            bool done = !(min_dist > 1e-8), cut = false;
-            if (!done && !bisected) {
+            const bool bisect = dot_start * dot_end < 0.0;
+            bool done = false, cut = false;
+            if (bisect) {
+                iters = -1;  // in the second pass
+            } else {
                 double V = 0.0, lim = 0.0;
                 if (a.certificates) {
                     V = ee_motion_bound(aS, aE, bS, bE);
@@ -1409,7 +1472,7 @@ __global__ void __launch_bounds__(kPrimBlock) k_ee_first(int n_total, const int3
                 r.dist = min_dist;
                 ee_store_at(a, o, thr, r);
             } else {
-                keep = true;  // the remaining iterations run in k_ee_rest4
+                keep = true;  // the rest runs in the second pass
             }
         }
     }
@@ -1493,8 +1556,16 @@ __device__ __forceinline__ double q_edge_closest(const Quad& q, double SA, doubl
     return sqrt(q_dot(q, d, d));
 }
 
+// ee_coplanarity of edges (aA, aB), (bA, bB), one component per lane
+__device__ __forceinline__ double q_coplanarity(const Quad& q, double aA, double aB, double bA, double bB) {
+    const int c1 = q.c == 1 ? 2 : (q.c == 2 ? 0 : 1), c2 = q.c == 1 ? 0 : (q.c == 2 ? 1 : 2);
+    const double u = aB - aA, v = bA - aA, w = bB - aA;
+    return q_dot(q, w, q_at(q, u, c1) * q_at(q, v, c2) - q_at(q, u, c2) * q_at(q, v, c1));
+}
+
 __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
     const int n = a.count[0];
+    if (n > kRestWide) return;  // k_ee_rest1
     Quad q;
     q.m = 0xFu << (threadIdx.x & 28);
     q.base = threadIdx.x & 28;
@@ -1524,7 +1595,31 @@ __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
         const double bEA = row(M + PM_BE, vb0), bEB = row(M + PM_BE, vb1);
         double t = R[0], min_dist = R[1];
         double rP = R[2 + comp], rQ = R[5 + comp], toc = R[8];
-        for (int iter = (int)R[9]; iter < kEeNewtonIters; iter++) {
+        int iter = (int)R[9];
+        if (iter < 0) {  // ee_bisect
+            iter = 0;
+            const double dot_start = q_coplanarity(q, aSA, aSB, bSA, bSB);
+            double lo = 0.0, hi = 1.0;
+            for (int k = 0; k < 20; k++) {
+                const double mid = (lo + hi) / 2.0;
+                const double dm = q_coplanarity(q, q_lerp(aSA, aEA, mid), q_lerp(aSB, aEB, mid), q_lerp(bSA, bEA, mid),
+                                                q_lerp(bSB, bEB, mid));
+                if (fabs(dm) < 1e-8) {
+                    lo = mid;
+                    hi = mid;
+                    break;
+                } else if (dot_start * dm < 0.0) {
+                    hi = mid;
+                } else {
+                    lo = mid;
+                }
+            }
+            toc = (lo + hi) / 2.0;
+            min_dist = q_edge_closest(q, q_lerp(aSA, aEA, toc), q_lerp(aSB, aEB, toc), q_lerp(bSA, bEA, toc),
+                                      q_lerp(bSB, bEB, toc), rP, rQ);
+            if (!(min_dist > 1e-8)) iter = kEeNewtonIters;
+        }
+        for (; iter < kEeNewtonIters; iter++) {
             const double atA = q_lerp(aSA, aEA, t), atB = q_lerp(aSB, aEB, t);
             const double btA = q_lerp(bSA, bEA, t), btB = q_lerp(bSB, bEB, t);
             double P, Qv;
@@ -1576,6 +1671,43 @@ __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
     }
 }
 
+__global__ void __launch_bounds__(kPrimBlock) k_ee_rest1(EeArgs a) {
+    const int n = a.count[0];
+    if (n <= kRestWide) return;  // k_ee_rest4
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double* R = a.rec + (size_t)kEeRec * i;
+        const EeWork w = decode_ee(a.work[i], a.n_tp, a.items, a.soup, a.conn, a.nn_off, a.tp, a.ntris, a.sub, a.cres,
+                                   a.chit);
+        const double* M = a.pm + (size_t)PM_SIZE * w.pair;
+        const Edge ea = tedge(load_tri(a.tris + (size_t)w.na * 72 + w.aTri * 9), w.aEdge);
+        const Edge eb = tedge(load_tri(a.tris + (size_t)w.nb * 72 + w.bTri * 9), w.bEdge);
+        Edge aS, aE, bS, bE;
+        aS.A = xform_rigid(ea.A, M + PM_AS);
+        aS.B = xform_rigid(ea.B, M + PM_AS);
+        aE.A = xform_rigid(ea.A, M + PM_AE);
+        aE.B = xform_rigid(ea.B, M + PM_AE);
+        bS.A = xform_rigid(eb.A, M + PM_BS);
+        bS.B = xform_rigid(eb.B, M + PM_BS);
+        bE.A = xform_rigid(eb.A, M + PM_BE);
+        bE.B = xform_rigid(eb.B, M + PM_BE);
+        double t = R[0], min_dist = R[1];
+        Ccd r;
+        r.P = mk(R[2], R[3], R[4]);
+        r.Q = mk(R[5], R[6], R[7]);
+        r.toc = R[8];
+        int iter = (int)R[9];
+        if (iter < 0) {
+            iter = 0;
+            min_dist = ee_bisect(aS, aE, bS, bE, ee_coplanarity(aS, bS), r);
+            if (!(min_dist > 1e-8)) iter = kEeNewtonIters;
+        }
+        for (; iter < kEeNewtonIters; iter++)
+            if (ee_newton_iter(aS, aE, bS, bE, t, min_dist, r)) break;
+        r.dist = min_dist;
+        ee_store_at(a, w.hit ? -1 - (int)(w.out - a.cres) : (int)(w.out - a.sub), a.search[w.pair], r);
+    }
+}
+
 // triTriCCDLinear's sequential (dist, toc) selection over its 15 sub-tests
 // (continuous_comparison.h:682-778), then the soup hit test (:817).
 __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entry* __restrict__ soup,
@@ -1621,7 +1753,7 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // that of any edge pair, so a slot whose vertices, or else edges, are closer
 // than thr by the same margin certainly hits (unless a triangle is almost a
 // point, whose edges return no distance); the pair is marked and done, and only
-// the survivors of the others go onto `list` for k_np_level_tests.
+// the survivors of the others go onto `list` for k_np_slots.
 // The gap between the triangles along d (d need not be a unit vector).
 __device__ __forceinline__ float axis_gap9(F3 d, const float* a, const float* b) {
     const float nn = sqrtf(dot3(d, d));
@@ -1771,16 +1903,94 @@ __global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __rest
     }
 }
 
-// The undecided slots of a descent's level: the FP64 test of each until its
-// node pair is marked.
+// The undecided slots of a descent's level: whether a triangle pair is closer
+// than its limit, until the node pair is marked.  As k_soup_slots: some ten to
+// a few hundred slots, a warp a slot (a thread a slot took 20 to 60 us a
+// level); the vertices a component per lane, then the nine edge pairs on lanes
+// 0-8 and, if none is below the limit, the six projections on lanes 9-14 and
+// the six edge crossings on lanes 16-21 that the FP32 bounds leave.
+__global__ void __launch_bounds__(kBlock) k_np_slots(const int32_t* __restrict__ list,
+                                                     const int32_t* __restrict__ n_list,
+                                                     const Entry* __restrict__ front, const double* __restrict__ pm,
+                                                     const double* __restrict__ tris, const double* __restrict__ eps,
+                                                     const float* __restrict__ search, int32_t* entry_hits) {
+    __shared__ double s_v[kBlock / 32][6][3];
+    const int n = *n_list;
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    double(*v)[3] = s_v[wi];
+    for (int k = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); k < n;
+         k += (int)((gridDim.x * (size_t)blockDim.x) >> 5)) {
+        const int slot = list[k];
+        if (__any_sync(0xffffffffu, ((volatile int32_t*)entry_hits)[slot >> 6] != 0)) continue;
+        const Entry e = front[slot >> 6];
+        const int ta = (slot >> 3) & 7, tb = slot & 7;
+        const double* M = pm + 32 * (size_t)e.pair;
+        if (lane < 18) {  // tri_xform_rigid, a row each
+            const int i = lane / 3, c = lane % 3;
+            const double* T = M + (i < 3 ? 0 : 16) + 4 * c;
+            const double* p = i < 3 ? tris + (size_t)e.na * 72 + ta * 9 + 3 * i : tris + (size_t)e.nb * 72 + tb * 9 + 3 * (i - 3);
+            v[i][c] = ((T[0] * p[0] + T[1] * p[1]) + T[2] * p[2]) + T[3] * 1.0;
+        }
+        __syncwarp();
+        const double thr = ((double)search[e.pair] + eps[(size_t)e.na * 8 + ta]) + eps[(size_t)e.nb * 8 + tb];
+        auto at = [&](int i) { return mk(v[i][0], v[i][1], v[i][2]); };
+        bool hit = false;
+        if (lane < 9) {
+            const int ia = lane / 3, ib = lane % 3;
+            V3 P, Q;
+            hit = edge_closest(at(ia), at(ia == 2 ? 0 : ia + 1), at(3 + ib), at(ib == 2 ? 3 : 4 + ib), P, Q) < thr;
+        }
+        bool any = __any_sync(0xffffffffu, hit);
+        if (!any && lane >= 9 && lane < 22 && lane != 15) {
+            // T: the triangle whose plane is used, the feature is the other's
+            const int q = lane < 15 ? lane - 9 : lane - 16;
+            const int t0 = q < 3 ? 0 : 3, o0 = 3 - t0, i = q < 3 ? q : q - 3, i1 = i == 2 ? 0 : i + 1;
+            const V3 o = at(0);
+            F3 r[6];
+            float rho = 0.f;
+#pragma unroll
+            for (int j = 0; j < 6; j++) {
+                r[j] = rel3(at(j < 3 ? t0 + j : o0 + j - 3), o);
+                rho = fmaxf(rho, maxabs3(r[j]));
+            }
+            const F3 ri = i == 0 ? r[3] : (i == 1 ? r[4] : r[5]), ri1 = i1 == 0 ? r[3] : (i1 == 1 ? r[4] : r[5]);
+            const PlaneBound p = plane_bound(r[0], r[1], r[2], rho);
+            const float h = dot3(p.n, ri - p.o);
+            const Tri T{at(t0), at(t0 + 1), at(t0 + 2)};
+            if (lane < 15) {
+                bool out = false;
+                if (p.ok) {
+                    float bu, bv, bw;
+                    plane_bary(p, ri - p.o, bu, bv, bw);
+                    out = bu < -p.mb || bv < -p.mb || bw < -p.mb;
+                }
+                if (!out) {
+                    const V3 pt = at(o0 + i);
+                    bool in;
+                    const V3 on = tri_project_to_plane(T, pt, in);
+                    hit = in && norm(on - pt) < thr;
+                }
+            } else if (!no_crossing(p, ri, ri1, h, dot3(p.n, ri1 - p.o))) {
+                double t;
+                bool t_inf;
+                tri_intersect_segment(T, at(o0 + i), at(o0 + i1), t, t_inf, hit);
+                hit = hit && 0.0 < thr;
+            }
+        }
+        any = any || __any_sync(0xffffffffu, hit);
+        if (any && lane == 0) entry_hits[slot >> 6] = 1;
+        __syncwarp();
+    }
+}
+
+// The same with the whole FP64 test of every slot (bounds off), a thread a slot.
 __global__ void __launch_bounds__(kBlock) k_np_level_tests(const int32_t* __restrict__ list,
                                                            const int32_t* __restrict__ n_list,
                                                            const Entry* __restrict__ front,
                                                            const double* __restrict__ pm,
                                                            const double* __restrict__ tris,
                                                            const double* __restrict__ eps,
-                                                           const float* __restrict__ search, int32_t* entry_hits,
-                                                           int use_bounds) {
+                                                           const float* __restrict__ search, int32_t* entry_hits) {
     const int n = *n_list;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int slot = list[k];
@@ -1792,7 +2002,7 @@ __global__ void __launch_bounds__(kBlock) k_np_level_tests(const int32_t* __rest
         const Tri B = tri_xform_rigid(load_tri(tris + (size_t)e.nb * 72 + tb * 9), M + 16);
         const double thr = ((double)search[e.pair] + eps[(size_t)e.na * 8 + ta]) + eps[(size_t)e.nb * 8 + tb];
         V3 P, Q;
-        if (use_bounds ? tri_tri_below(A, B, thr) : tri_tri_dist(A, B, P, Q) < thr) entry_hits[slot >> 6] = 1;
+        if (tri_tri_dist(A, B, P, Q) < thr) entry_hits[slot >> 6] = 1;
     }
 }
 
@@ -2333,29 +2543,16 @@ int ee_grid_size(d2g_ctx* ctx, int* grid) {
     return D2G_OK;
 }
 
-// Grid of k_soup_tests, which reads its list's length from device memory too.
-int soup_grid_size(d2g_ctx* ctx, int* grid) {
+// Grid of the kernels that test a level's undecided slots, whose number they
+// read from device memory too: a few warps per SM sub-partition.
+int slot_grid_size(d2g_ctx* ctx, int* grid) {
     Engine& E = ctx->eng;
-    if (E.soup_grid == 0) {
-        int dev_sms = 0, per_sm = 0;
+    if (E.slot_grid == 0) {
+        int dev_sms = 0;
         D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
-        D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_soup_tests, kPrimBlock, 0));
-        E.soup_grid = std::max(1, dev_sms * std::max(1, per_sm));
+        E.slot_grid = 3 * dev_sms;
     }
-    *grid = E.soup_grid;
-    return D2G_OK;
-}
-
-// Grid of k_np_level_tests, likewise.
-int np_grid_size(d2g_ctx* ctx, int* grid) {
-    Engine& E = ctx->eng;
-    if (E.np_grid == 0) {
-        int dev_sms = 0, per_sm = 0;
-        D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
-        D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_np_level_tests, kBlock, 0));
-        E.np_grid = std::max(1, dev_sms * std::max(1, per_sm));
-    }
-    *grid = E.np_grid;
+    *grid = E.slot_grid;
     return D2G_OK;
 }
 
@@ -2625,6 +2822,10 @@ int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, in
         k_ee_first<<<nblocks(n_ee, kPrimBlock), kPrimBlock, 0, s_ee>>>(n_ee, list_ee, cnt_ee, E.pm.p, ctx->tris.p,
                                                                       ea);
         k_ee_rest4<<<ee_grid, kBlock, 0, s_ee>>>(ea);
+        if (n_ee > kRestWide) {  // (the list is read on the device; a shorter one cannot be that long)
+            k_ee_rest1<<<2 * ee_grid, kPrimBlock, 0, s_ee>>>(ea);
+            ctx->eng.launches++;
+        }
         ctx->eng.launches += 3;
         prof_end(ctx, pfe, s_ee);
         LAUNCH(k_ccd_mask_pt, n_pt, K, n_pt, E.items.p, soup, conn, E.nn_off.p, E.tp.p, E.pm32c.p, ctx->ntris.p,
@@ -2671,7 +2872,7 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
     RC(E.search.ensure(n_pairs + 1));
     RC(E.soup.ensure(n_pairs + 1));
     int test_grid = 0;
-    RC(soup_grid_size(ctx, &test_grid));
+    RC(slot_grid_size(ctx, &test_grid));
     int n_rec = 0;
     long long n_streamed = 0;  // records handed to the sink
     if (n_pairs > 0)
@@ -2732,10 +2933,13 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
                    ctx->tri32.p, ctx->geo_eps.p, E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0,
                    E.entry_hits.p, E.ccd_list.p, E.lc.p);
             prof_end(ctx, pff);
-            k_soup_tests<<<test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p, E.pm32c.p,
+            if (E.fp32_bounds)
+                k_soup_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p, E.pm32c.p,
                                                           ctx->tris.p, ctx->tri32.p, E.search.p, E.entry_hits.p,
-                                                          E.fp32_bounds ? 1 : 0, E.certificates ? 1 : 0,
-                                                          E.ccd_stats.p);
+                                                          E.certificates ? 1 : 0, E.ccd_stats.p);
+            else
+                k_soup_tests<<<4 * test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p,
+                                                                  ctx->tris.p, E.search.p, E.entry_hits.p);
             E.launches++;
             if (E.witnesses) {
                 LAUNCH(k_witness_make, 32LL * n_soup, n_soup, E.soup.p, E.entry_hits.p, E.wt_flag.p, skip, d_pairs,
@@ -2828,7 +3032,7 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
         LAUNCH(k_np_prep, n_pairs, n_pairs, d_pairs, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p,
                E.pm.p, E.search.p, E.roots.p, E.pm32.p);
     int n_rec = 0, test_grid = 0;
-    RC(np_grid_size(ctx, &test_grid));
+    RC(slot_grid_size(ctx, &test_grid));
     // pair chunks, as in run_ccd
     const double budget = level_budget(ctx);
     // a leaf pair's slots take ~110 bytes each (x1.5 growth slack)
@@ -2845,9 +3049,13 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
             LAUNCH(k_np_filter<false>, 32LL * n, n, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p,
                    ctx->eps_up.p, E.search.p, ctx->nodes.p, E.fp32_bounds ? 1 : 0, (uint32_t*)nullptr, (int32_t*)nullptr,
                    E.entry_hits.p, E.ccd_list.p, E.lc.p);
-            k_np_level_tests<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p,
-                                                          ctx->tris.p, ctx->eps.p, E.search.p, E.entry_hits.p,
-                                                          E.fp32_bounds ? 1 : 0);
+            if (E.fp32_bounds)
+                k_np_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p, ctx->tris.p,
+                                                        ctx->eps.p, E.search.p, E.entry_hits.p);
+            else
+                k_np_level_tests<<<4 * test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p,
+                                                                  ctx->tris.p, ctx->eps.p, E.search.p,
+                                                                  E.entry_hits.p);
             E.launches++;
             return D2G_OK;
         }));

@@ -205,7 +205,7 @@ struct Engine {
     // phased edge-edge CCD (d2g_engine.cu)
     DBuf<double> ee_rec;
     DBuf<int32_t> ee_work;
-    int ee_grid = 0, soup_grid = 0, np_grid = 0;  // k_ee_rest4, k_soup_tests, k_np_level_tests grids (all resident)
+    int ee_grid = 0, slot_grid = 0;  // k_ee_rest4 grid (every block resident); grid of the level tests
     // traversal chunking: root entries of the call's pairs; a byte budget for
     // a level's buffers (0: a third of the device memory)
     DBuf<Entry> roots;

@@ -123,12 +123,8 @@ D2G_HD int lowest_bit(unsigned m) {
 }
 
 // tri_tri_dist(a, b, P, Q) where the result is below `limit`; else a distance
-// of at least `limit` (or NaN), with P and Q meaningless.  ANY: only whether
-// the result is below the limit is wanted: a distance below it (not the
-// smallest, P and Q meaningless) when it is, which FP32 settles except within
-// a few micrometres of the limit.
-template <bool ANY>
-D2G_HD double tri_tri_dist_bounded(const Tri& a, const Tri& b, double limit, V3& P, V3& Q) {
+// of at least `limit` (or NaN), with P and Q meaningless.
+D2G_HD double tri_tri_dist_below(const Tri& a, const Tri& b, double limit, V3& P, V3& Q) {
     const V3 o = a.A;
     F3 A[3], B[3];
     A[0] = f3(0.f, 0.f, 0.f);
@@ -150,23 +146,6 @@ D2G_HD double tri_tri_dist_bounded(const Tri& a, const Tri& b, double limit, V3&
         hA[i] = dot3(pb.n, A[i] - pb.o);
     }
     const float flimit = (float)limit * (1.f + 1e-6f);
-    if (ANY) {
-        // the distance is at most that of any edge pair whose edges are edges
-        // (a degenerate one returns no distance)
-        float up = 3.4e38f;
-        const bool solid = fminf(fminf(pa.d00, pa.d11), fminf(pb.d00, pb.d11)) > 1e-8f &&
-                           fminf(dot3(A[2] - A[1], A[2] - A[1]), dot3(B[2] - B[1], B[2] - B[1])) > 1e-8f;
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                float d2;
-                seg_vector(A[i], A[i == 2 ? 0 : i + 1], B[j], B[j == 2 ? 0 : j + 1], d2);
-                up = fminf(up, d2);
-            }
-        up = sqrtf(up) + margin;
-        if (solid && up < (float)limit * (1.f - 1e-6f)) return (double)up;
-    }
     // ---- intersections: the last one found decides
     unsigned cross = 0;
 #pragma unroll
@@ -188,7 +167,6 @@ D2G_HD double tri_tri_dist_bounded(const Tri& a, const Tri& b, double limit, V3&
         if (isInt) {
             X = lerp(e.A, e.B, t);
             any = true;
-            if (ANY) break;
         }
     }
     if (any) {
@@ -243,7 +221,6 @@ D2G_HD double tri_tri_dist_bounded(const Tri& a, const Tri& b, double limit, V3&
     int at = 15;
     unsigned todo = 1u << first, done = 0;
     for (int round = 0; round < 2; round++) {
-        if (ANY && dc < limit) break;
         if (round) {
             const float lim = fminf((float)dc * (1.f + 1e-6f), flimit);
             todo = 0;
@@ -293,14 +270,6 @@ D2G_HD double tri_tri_dist_bounded(const Tri& a, const Tri& b, double limit, V3&
     P = Pc;
     Q = Qc;
     return at < 15 ? norm(Pc - Qc) : 1.0 / 0.0;
-}
-D2G_HD double tri_tri_dist_below(const Tri& a, const Tri& b, double limit, V3& P, V3& Q) {
-    return tri_tri_dist_bounded<false>(a, b, limit, P, Q);
-}
-// tri_tri_dist(a, b, ...) < limit
-D2G_HD bool tri_tri_below(const Tri& a, const Tri& b, double limit) {
-    V3 P, Q;
-    return tri_tri_dist_bounded<true>(a, b, limit, P, Q) < limit;
 }
 
 }  // namespace d2g

@@ -55,7 +55,6 @@ int main(int argc, char** argv) {
         const double d = tri_tri_dist(a, b, P, Q);
         for (double lim : {0.25, 0.05, 1e9, d, d * (1 + 1e-15), d * (1 - 1e-15)}) {
             const double e = tri_tri_dist_below(a, b, lim, P2, Q2);
-            if (tri_tri_below(a, b, lim) != (d < lim) && bad++ < 5) std::printf("limit %.17g distance %.17g: below?\n", lim, d);
             bool ok = !(e < lim);
             if (d < lim) {
                 below++;
