@@ -228,8 +228,9 @@ __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restri
 // returns at most its distance at the start (edgeEdgeCCD evaluates it first)
 // or at most 1e-8, so a slot whose triangles' vertices, or else edges, are
 // closer than the search distance there by a margin (20 um plus 4e-6 of the
-// coordinates, above their FP32 rounding) certainly hits: the node pair is marked and done.  The
-// slots of the others go onto `list` for k_soup_slots.  Two bodies that are
+// coordinates, above their FP32 rounding) certainly hits: the node pair is
+// marked and done.  The slots of the others go onto `list` for k_soup_slots,
+// marked when a gap over the motion clears all their edge-edge tests.  Two bodies that are
 // single leaves meet at the root: their slots are counted (`lc`) and tested
 // with the leaf pairs (k_soup_filter).  The box stage:
 // lanes 0-7 form the swept boxes of a's triangles, lanes 8-15 those of b's,
@@ -241,13 +242,14 @@ __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restri
 // answer the FP64 boxes give; a warp with any slot inside the margin (or a
 // NaN) forms the FP64 boxes and decides those slots exactly.
 // res[h]: the swept boxes of slot lane + 32 h overlap.  verts: the warp's 16
-// triangles (a's, then b's) in FP32 at the start, [16][9]; mag: the largest
-// coordinate of each, for the margins.
+// triangles (a's, then b's) in FP32 at the start, [16][9], ends: at the end;
+// mags: the largest coordinate of each, for the margins (huge where a triangle
+// allows no certain hit).
 __device__ __forceinline__ void swept_slots(const Entry& e, const int32_t* __restrict__ pairs,
                                             const double* __restrict__ pm, const float* __restrict__ pm32,
                                             const int32_t* __restrict__ ntris, const double* __restrict__ tris,
                                             const float* __restrict__ tri32, const double* __restrict__ geo_eps,
-                                            int (&res)[2], float (*verts)[9], float* mags) {
+                                            int (&res)[2], float (*verts)[9], float (*ends)[9], float* mags) {
     const int lane = threadIdx.x & 31;
     const int na = ntris[e.na], nb = ntris[e.nb];
     const bool side_b = lane >= 8;
@@ -274,6 +276,11 @@ __device__ __forceinline__ void swept_slots(const Entry& e, const int32_t* __res
                 verts[lane][3 * v + 2] = o[2];
             }
             box_add(b32, ME, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], oe[v], mag);
+            if (verts) {
+                ends[lane][3 * v] = oe[v][0];
+                ends[lane][3 * v + 1] = oe[v][1];
+                ends[lane][3 * v + 2] = oe[v][2];
+            }
         }
         const float e32 = (float)geo_eps[body];
 #pragma unroll
@@ -391,6 +398,72 @@ __device__ __forceinline__ float edge_min(const float* a, const float* b, F3& di
     return sqrtf(m);
 }
 
+// The gap between the triangles along d (d need not be a unit vector).
+__device__ __forceinline__ float axis_gap9(F3 d, const float* a, const float* b) {
+    const float nn = sqrtf(dot3(d, d));
+    if (!(nn > 1e-20f)) return 0.f;
+    float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
+#pragma unroll
+    for (int v = 0; v < 3; v++) {
+        const float pa = dot3(d, f3(a[3 * v], a[3 * v + 1], a[3 * v + 2]));
+        const float pb = dot3(d, f3(b[3 * v], b[3 * v + 1], b[3 * v + 2]));
+        a0 = fminf(a0, pa);
+        a1 = fmaxf(a1, pa);
+        b0 = fminf(b0, pb);
+        b1 = fmaxf(b1, pb);
+    }
+    return fmaxf(b0 - a1, a0 - b1) / nn;
+}
+// A lower bound of the triangles' distance: along any direction the distance
+// is at least the gap between the projections, whatever the direction, so one
+// computed in FP32 still bounds.  Separate triangles are closest between two
+// edges, in the direction d of their closest edge pair, or between a vertex and
+// a face, along its normal.
+__device__ __forceinline__ float tri_gap(F3 d, const float* a, const float* b) {
+    const F3 na = cross3(f3(a[3] - a[0], a[4] - a[1], a[5] - a[2]), f3(a[6] - a[0], a[7] - a[1], a[8] - a[2]));
+    const F3 nb = cross3(f3(b[3] - b[0], b[4] - b[1], b[5] - b[2]), f3(b[6] - b[0], b[7] - b[1], b[8] - b[2]));
+    return fmaxf(axis_gap9(d, a, b), fmaxf(axis_gap9(na, a, b), axis_gap9(nb, a, b)));
+}
+// The same over a motion: points move on straight lines from their start to
+// their end positions, so the gap along a fixed direction is concave in time
+// and at least the smaller of the two ends'.  Bounds every distance between
+// points of the triangles at one time (every edge-edge distance of
+// edgeEdgeCCD).
+__device__ __forceinline__ float axis_gap_motion(F3 d, const float* a, const float* b, const float* ae,
+                                                 const float* be) {
+    const float nn = sqrtf(dot3(d, d));
+    if (!(nn > 1e-20f)) return 0.f;
+    float g[2][2];  // [pose][side]
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float *A = k ? ae : a, *B = k ? be : b;
+        float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
+#pragma unroll
+        for (int v = 0; v < 3; v++) {
+            const float pa = dot3(d, f3(A[3 * v], A[3 * v + 1], A[3 * v + 2]));
+            const float pb = dot3(d, f3(B[3 * v], B[3 * v + 1], B[3 * v + 2]));
+            a0 = fminf(a0, pa);
+            a1 = fmaxf(a1, pa);
+            b0 = fminf(b0, pb);
+            b1 = fmaxf(b1, pb);
+        }
+        g[k][0] = b0 - a1;
+        g[k][1] = a0 - b1;
+    }
+    return fmaxf(fminf(g[0][0], g[1][0]), fminf(g[0][1], g[1][1])) / nn;
+}
+__device__ __forceinline__ float tri_gap_motion(F3 d, const float* a, const float* b, const float* ae,
+                                                const float* be) {
+    const F3 na = cross3(f3(a[3] - a[0], a[4] - a[1], a[5] - a[2]), f3(a[6] - a[0], a[7] - a[1], a[8] - a[2]));
+    const F3 nb = cross3(f3(b[3] - b[0], b[4] - b[1], b[5] - b[2]), f3(b[6] - b[0], b[7] - b[1], b[8] - b[2]));
+    return fmaxf(axis_gap_motion(d, a, b, ae, be),
+                 fmaxf(axis_gap_motion(na, a, b, ae, be), axis_gap_motion(nb, a, b, ae, be)));
+}
+
+// Marks a slot of k_ccd_level's list whose edge-edge tests are all clear (slot
+// indices stay below 2^30).
+constexpr int kEdgesClear = 1 << 30;
+
 __global__ void __launch_bounds__(kBlock) k_ccd_level(
     int n_soup, const Entry* __restrict__ soup, const int32_t* __restrict__ pairs, const double* __restrict__ pm,
     const float* __restrict__ pm32, const int32_t* __restrict__ ntris, const double* __restrict__ tris,
@@ -398,6 +471,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
     const int4* __restrict__ nodes, const uint8_t* __restrict__ skip, const uint8_t* __restrict__ eskip,
     int use_bounds, int32_t* __restrict__ entry_hits, int32_t* __restrict__ list, int32_t* __restrict__ lc) {
     __shared__ float s_verts[kBlock / 32][16][9];
+    __shared__ float s_ends[kBlock / 32][16][9];
     __shared__ float s_mag[kBlock / 32][16];
     const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -410,7 +484,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
         return;
     }
     int res[2];
-    swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, s_verts[wi], s_mag[wi]);
+    swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, s_verts[wi], s_ends[wi], s_mag[wi]);
     const int k = __popc(__ballot_sync(0xffffffffu, res[0])) + __popc(__ballot_sync(0xffffffffu, res[1]));
     if (lane == 0 && k) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), k);
     bool sure = false;
@@ -428,17 +502,24 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
         }
         sure = __any_sync(0xffffffffu, sure);
         if (!sure) {
+            bool clear[2] = {false, false};
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
+                if (!res[h] || !use_bounds) continue;
                 F3 d;
-                if (room[h] > 0.f) sure = sure || edge_min(s_verts[wi][ta], s_verts[wi][8 + tb], d) < room[h];
+                const float m = edge_min(s_verts[wi][ta], s_verts[wi][8 + tb], d);
+                if (m < room[h]) sure = true;
+                // (s_mag is huge for an unsteady triangle: never clear either)
+                clear[h] = tri_gap_motion(d, s_verts[wi][ta], s_verts[wi][8 + tb], s_ends[wi][ta],
+                                          s_ends[wi][8 + tb]) >
+                           thr + (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
             }
             sure = __any_sync(0xffffffffu, sure);
-        }
-        if (!sure) {
-            warp_append(64 * w + lane, res[0] != 0, list, lc + LC_LIST);
-            warp_append(64 * w + lane + 32, res[1] != 0, list, lc + LC_LIST);
+            if (!sure) {
+                warp_append((64 * w + lane) | (clear[0] ? kEdgesClear : 0), res[0] != 0, list, lc + LC_LIST);
+                warp_append((64 * w + lane + 32) | (clear[1] ? kEdgesClear : 0), res[1] != 0, list, lc + LC_LIST);
+            }
         }
     } else if (lane == 0 && k) {
         atomicAdd(lc + LC_ROOT, 1);
@@ -460,7 +541,7 @@ __global__ void k_soup_filter(int n_soup, const Entry* __restrict__ soup, const 
     const Entry e = soup[w];
     int res[2] = {0, 0};
     if (!(skip && skip[e.pair]) && !ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z)
-        swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, nullptr, nullptr);
+        swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, nullptr, nullptr, nullptr);
     flags[64 * (size_t)w + lane] = res[0];
     flags[64 * (size_t)w + lane + 32] = res[1];
 }
@@ -1044,20 +1125,34 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_ee(int n_tp, int n_total, c
         const float* tb = tri32 + ((size_t)w.nb * 8 + w.bTri) * 9;
         const int a0 = w.aEdge, a1 = w.aEdge == 2 ? 0 : w.aEdge + 1;
         const int b0 = w.bEdge, b1 = w.bEdge == 2 ? 0 : w.bEdge + 1;
-        float mag = 0.f, o[3];
+        float mag = 0.f, o[2][4][3];  // [start, end][a0 a1 b0 b1]
         Box32 ba, bb;
         box_init(ba);
         box_init(bb);
+#pragma unroll
         for (int m = 0; m < 2; m++) {
             const float* MA = pm32_of(pm32, w.pair, P32_AS + m);
             const float* MB = pm32_of(pm32, w.pair, P32_BS + m);
-            box_add(ba, MA, ta[3 * a0], ta[3 * a0 + 1], ta[3 * a0 + 2], o, mag);
-            box_add(ba, MA, ta[3 * a1], ta[3 * a1 + 1], ta[3 * a1 + 2], o, mag);
-            box_add(bb, MB, tb[3 * b0], tb[3 * b0 + 1], tb[3 * b0 + 2], o, mag);
-            box_add(bb, MB, tb[3 * b1], tb[3 * b1 + 1], tb[3 * b1 + 2], o, mag);
+            mag = fmaxf(mag, fmaxf(fmaxf(fmaxf(fabsf(MA[3]), fabsf(MA[7])), fabsf(MA[11])),
+                                   fmaxf(fmaxf(fabsf(MB[3]), fabsf(MB[7])), fabsf(MB[11]))));
+            box_add(ba, MA, ta[3 * a0], ta[3 * a0 + 1], ta[3 * a0 + 2], o[m][0], mag);
+            box_add(ba, MA, ta[3 * a1], ta[3 * a1 + 1], ta[3 * a1 + 2], o[m][1], mag);
+            box_add(bb, MB, tb[3 * b0], tb[3 * b0 + 1], tb[3 * b0 + 2], o[m][2], mag);
+            box_add(bb, MB, tb[3 * b1], tb[3 * b1 + 1], tb[3 * b1 + 2], o[m][3], mag);
         }
         const float thr = search[w.pair];
-        keep = !use_bounds || !(box_gap(ba, bb) > thr + (1e-3f + 4e-6f * (mag + thr)));
+        const float lim = thr + (2e-5f + 4e-6f * (mag + thr));
+        keep = !use_bounds || !(box_gap(ba, bb) > lim);
+        if (keep && use_bounds) {
+            // the gap over the motion along the direction between the edges'
+            // closest points at the start (axis_gap_motion)
+            auto at = [&](int m, int v) { return f3(o[m][v][0], o[m][v][1], o[m][v][2]); };
+            float d2;
+            const F3 d = seg_vector(at(0, 0), at(0, 1), at(0, 2), at(0, 3), d2);
+            const float g0 = fminf(dot3(d, at(0, 2)), dot3(d, at(0, 3))) - fmaxf(dot3(d, at(0, 0)), dot3(d, at(0, 1)));
+            const float g1 = fminf(dot3(d, at(1, 2)), dot3(d, at(1, 3))) - fmaxf(dot3(d, at(1, 0)), dot3(d, at(1, 1)));
+            keep = !(fminf(g0, g1) > lim * sqrtf(d2));
+        }
         if (!keep) record_no_contact(w.out, w.hit);
     }
     warp_append(j, keep, list, count);
@@ -1127,7 +1222,7 @@ __global__ void __launch_bounds__(kPrimBlock) k_prim_pt(int n_tp, int n_total, c
 // of its longest lane.  62% of the tests end within two Newton iterations (~330
 // slots each on one lane) and 20% run all ten; 0.5% bisect (~1,300 slots, which
 // would double the first pass for every warp that has one).  So:
-//   k_ee_first   one test per lane: edges, FP64 box-gap skip and at most two
+//   k_ee_first   one test per lane: the edges and at most two
 //                Newton iterations; the tests still running and those that
 //                bisect are saved and listed.
 //   k_ee_rest4   the listed tests on four lanes each (below), ~230 slots an
@@ -1158,6 +1253,7 @@ struct EeArgs {
     int32_t* work;   // the listed test's work item
     int32_t* count;  // [0] listed tests
     int first_iters;  // Newton iterations in the first pass
+    int bounds;       // the FP32 bounds dropped tests before this
     int certificates;  // conservative-advancement cut-off of the first pass (results unchanged)
     unsigned long long* ca_stats;  // [0] tests cut, [1] Newton iterations they did not run
 };
@@ -1180,6 +1276,19 @@ __device__ __forceinline__ double ee_motion_bound(const Edge& aS, const Edge& aE
     return sqrt(m);
 }
 
+// The gap between the boxes of the two edges' endpoints, start and end, passes lim.
+__device__ __forceinline__ bool ee_boxes_apart(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE,
+                                               double lim) {
+    auto gap = [](double a0, double a1, double a2, double a3, double b0, double b1, double b2, double b3) {
+        return fmax(fmin(fmin(b0, b1), fmin(b2, b3)) - fmax(fmax(a0, a1), fmax(a2, a3)),
+                    fmin(fmin(a0, a1), fmin(a2, a3)) - fmax(fmax(b0, b1), fmax(b2, b3)));
+    };
+    const double gx = fmax(0.0, gap(aS.A.x, aS.B.x, aE.A.x, aE.B.x, bS.A.x, bS.B.x, bE.A.x, bE.B.x));
+    const double gy = fmax(0.0, gap(aS.A.y, aS.B.y, aE.A.y, aE.B.y, bS.A.y, bS.B.y, bE.A.y, bE.B.y));
+    const double gz = fmax(0.0, gap(aS.A.z, aS.B.z, aE.A.z, aE.B.z, bS.A.z, bS.B.z, bE.A.z, bE.B.z));
+    return (gx * gx + gy * gy) + gz * gz > lim * lim;
+}
+
 __device__ __forceinline__ void ee_store_at(const EeArgs& a, int o, float thr, const Ccd& r) {
     if (o < 0) {  // leaf-pair test: P and Q swapped (continuous_comparison.h:881-896)
         store_prim(a.cres + (-1 - o), r.dist, r.Q, r.P, r.toc);
@@ -1187,6 +1296,20 @@ __device__ __forceinline__ void ee_store_at(const EeArgs& a, int o, float thr, c
     } else {
         store_prim(a.sub + o, r.dist, r.P, r.Q, r.toc);
     }
+}
+
+// The gap between the edges along Q - P (of length d), at the start and at the
+// end, is at least lim plus a margin (1 um and 1e-9 of the coordinates): no
+// distance of the motion is below lim (the gap of linearly moving points is
+// concave in time).
+__device__ __forceinline__ bool ee_gap_clear(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE, V3 P,
+                                             V3 Q, double d, double lim) {
+    const V3 n = Q - P;
+    const double g0 = fmin(dot(n, bS.A), dot(n, bS.B)) - fmax(dot(n, aS.A), dot(n, aS.B));
+    const double g1 = fmin(dot(n, bE.A), dot(n, bE.B)) - fmax(dot(n, aE.A), dot(n, aE.B));
+    const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
+                            fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
+    return fmin(g0, g1) >= ((lim + 1e-6) + 1e-9 * mag) * d;
 }
 
 // No point of the motion shortens the edge to nothing: its change is less than
@@ -1223,7 +1346,8 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
     double(*v)[6][3] = s_v[wi];
     for (int k = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); k < n;
          k += (int)((gridDim.x * (size_t)blockDim.x) >> 5)) {
-        const int slot = list[k];
+        const int item = list[k], slot = item & ~kEdgesClear;
+        const bool edges = !(item & kEdgesClear);
         if (__any_sync(0xffffffffu, ((volatile int32_t*)entry_hits)[slot >> 6] != 0)) continue;
         const Entry e = soup[slot >> 6];
         const int ta = (slot >> 3) & 7, tb = slot & 7;
@@ -1232,6 +1356,17 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
         const double* M = pm + (size_t)PM_SIZE * e.pair;
         const double* da = tris + (size_t)e.na * 72 + ta * 9;
         const double* db = tris + (size_t)e.nb * 72 + tb * 9;
+        // the point-triangle tests the FP32 bounds leave
+        bool pt = false;
+        if (lane >= 16 && lane < 22) {
+            const int i = (lane - 16) >> 1;
+            const bool pb = (lane & 1) != 0;  // a vertex of b against a, else of a against b
+            const float* fa = tri32 + ((size_t)e.na * 8 + ta) * 9;
+            const float* fb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
+            pt = !pt_apart(pm32, e.pair, pb ? P32_BAS : P32_ABS, pb ? P32_AS : P32_BS, (pb ? fb : fa) + 3 * i,
+                           pb ? fa : fb, thr);
+        }
+        if (!edges && !__any_sync(0xffffffffu, pt)) continue;
         for (int r = lane; r < 36; r += 32) {  // xform_rigid, a row each
             const int pose = r / 18, i = r % 18 / 3, c = r % 3;
             const double* T = M + (i < 3 ? (pose ? PM_AE : PM_AS) : (pose ? PM_BE : PM_BS)) + 4 * c;
@@ -1241,7 +1376,8 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
         __syncwarp();
         auto at = [&](int pose, int i) { return mk(v[pose][i][0], v[pose][i][1], v[pose][i][2]); };
         Edge aS, aE, bS, bE;
-        bool hit = false, open = lane < 9, steady = false;
+        V3 P, Q;
+        bool hit = false, open = edges && lane < 9, steady = false;
         if (open) {
             const int ia = lane / 3, ib = lane % 3, a1 = ia == 2 ? 0 : ia + 1, b1 = ib == 2 ? 0 : ib + 1;
             aS.A = at(0, ia);
@@ -1256,57 +1392,54 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
             // any one below the limit makes the result one
             steady = thr > 1e-6f && ee_steady(aS, aE) && ee_steady(bS, bE);
             if (steady) {
-                V3 P, Q;
                 const double d0 = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q);
                 hit = d0 < lim;
-                const V3 d = Q - P;
-                const double g0 = fmin(dot(d, bS.A), dot(d, bS.B)) - fmax(dot(d, aS.A), dot(d, aS.B));
-                const double g1 = fmin(dot(d, bE.A), dot(d, bE.B)) - fmax(dot(d, aE.A), dot(d, aE.B));
-                const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
-                                        fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
-                open = !hit && !(fmin(g0, g1) >= ((lim + 1e-6) + 1e-9 * mag) * d0);
+                open = !hit && !ee_gap_clear(aS, aE, bS, bE, P, Q, d0, lim);
             }
         }
-        const unsigned cut = certificates ? __ballot_sync(0xffffffffu, lane < 9 && !hit && !open) : 0u;
+        const unsigned cut = certificates ? __ballot_sync(0xffffffffu, edges && lane < 9 && !hit && !open) : 0u;
         if (lane == 0 && cut) {
             atomicAdd(ca_stats, (unsigned long long)__popc(cut));
             atomicAdd(ca_stats + 1, (unsigned long long)(__popc(cut) * (kEeNewtonIters - 1)));
         }
         bool any = __any_sync(0xffffffffu, hit);
-        double best = DBL_MAX;
         if (!any && __any_sync(0xffffffffu, open)) {
-            if (open && steady) {  // edgeEdgeCCD's iterates, up to the first below the limit
-                Ccd r;
+            if (open && steady) {
+                // edgeEdgeCCD's iterates from the start's closest points, up to
+                // the first below the limit or one whose gap clears the test
                 double t = 0.0;
-                for (int iter = 0; iter < kEeNewtonIters && !hit; iter++) {
-                    const bool last = ee_newton_iter(aS, aE, bS, bE, t, best, r);
-                    hit = best < lim;
-                    if (last) break;
+                Edge a = aS, b = bS;
+                for (int iter = 1; iter < kEeNewtonIters && open; iter++) {
+                    const double t_prev = t;
+                    t = ee_newton_step(aS, aE, bS, bE, a, b, P, Q, t);
+                    if (t == t_prev || t != t) break;
+                    a.A = lerp(aS.A, aE.A, t);
+                    a.B = lerp(aS.B, aE.B, t);
+                    b.A = lerp(bS.A, bE.A, t);
+                    b.B = lerp(bS.B, bE.B, t);
+                    const double d = edge_closest(a.A, a.B, b.A, b.B, P, Q);
+                    hit = d < lim;
+                    open = !hit && !ee_gap_clear(aS, aE, bS, bE, P, Q, d, lim);
                 }
             }
             any = __any_sync(0xffffffffu, hit);
         }
-        if (!any && lane >= 16 && lane < 22) {
-            const int q = lane - 16, i = q >> 1;
-            const bool pb = (q & 1) != 0;  // a vertex of b against a, else of a against b
-            const float* fa = tri32 + ((size_t)e.na * 8 + ta) * 9;
-            const float* fb = tri32 + ((size_t)e.nb * 8 + tb) * 9;
-            if (!pt_apart(pm32, e.pair, pb ? P32_BAS : P32_ABS, pb ? P32_AS : P32_BS, (pb ? fb : fa) + 3 * i,
-                          pb ? fa : fb, thr)) {
-                const double* p = (pb ? db : da) + 3 * i;
-                hit = point_tri_ccd(mk(p[0], p[1], p[2]), M + (pb ? PM_BAS : PM_ABS), M + (pb ? PM_BAE : PM_ABE),
-                                    load_tri(pb ? da : db), M + (pb ? PM_AS : PM_BS), M + (pb ? PM_AE : PM_BE))
-                          .dist < lim;
-            }
+        if (!any && pt) {
+            const int i = (lane - 16) >> 1;
+            const bool pb = (lane & 1) != 0;
+            const double* p = (pb ? db : da) + 3 * i;
+            hit = point_tri_ccd(mk(p[0], p[1], p[2]), M + (pb ? PM_BAS : PM_ABS), M + (pb ? PM_BAE : PM_ABE),
+                                load_tri(pb ? da : db), M + (pb ? PM_AS : PM_BS), M + (pb ? PM_AE : PM_BE))
+                      .dist < lim;
         }
         any = any || __any_sync(0xffffffffu, hit);
         if (!any && __any_sync(0xffffffffu, open)) {
             // the bisection's distance, and the whole of an unsteady test
             if (open) {
                 Ccd r;
+                double best = DBL_MAX;
                 const double dot_start = ee_coplanarity(aS, bS);
-                const bool sign = dot_start * ee_coplanarity(aE, bE) < 0.0;
-                if (sign) best = ee_bisect(aS, aE, bS, bE, dot_start, r);
+                if (dot_start * ee_coplanarity(aE, bE) < 0.0) best = ee_bisect(aS, aE, bS, bE, dot_start, r);
                 hit = best < lim;
                 if (!steady && !hit && best > 1e-8) {
                     double t = 0.0;
@@ -1336,7 +1469,7 @@ __global__ void __launch_bounds__(kPrimBlock) k_soup_tests(const int32_t* __rest
          j += (long long)gridDim.x * blockDim.x) {
         const bool ee = j < n_ee;
         const int k = (int)(ee ? j / 9 : (j - n_ee) / 6), q = (int)(ee ? j % 9 : (j - n_ee) % 6);
-        const int slot = list[k];
+        const int slot = list[k] & ~kEdgesClear;
         if (((volatile int32_t*)entry_hits)[slot >> 6]) continue;
         const Entry e = soup[slot >> 6];
         const double* M = pm + (size_t)PM_SIZE * e.pair;
@@ -1360,12 +1493,7 @@ __global__ void __launch_bounds__(kPrimBlock) k_soup_tests(const int32_t* __rest
             if (!(lim > 1e-6 && ee_steady(aS, aE) && ee_steady(bS, bE))) {
                 dist = edge_edge_ccd(aS, aE, bS, bE).dist;
             } else if (!(dist < lim)) {  // as in k_soup_slots
-                const V3 d = Q - P;
-                const double g0 = fmin(dot(d, bS.A), dot(d, bS.B)) - fmax(dot(d, aS.A), dot(d, aS.B));
-                const double g1 = fmin(dot(d, bE.A), dot(d, bE.B)) - fmax(dot(d, aE.A), dot(d, aE.B));
-                const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
-                                        fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
-                if (!(fmin(g0, g1) >= ((lim + 1e-6) + 1e-9 * mag) * dist)) dist = edge_edge_ccd(aS, aE, bS, bE).dist;
+                if (!ee_gap_clear(aS, aE, bS, bE, P, Q, dist, lim)) dist = edge_edge_ccd(aS, aE, bS, bE).dist;
             }
         } else if (q & 1) {
             dist = point_tri_ccd(tvert(B, q >> 1), M + PM_BAS, M + PM_BAE, A, M + PM_AS, M + PM_AE).dist;
@@ -1405,32 +1533,11 @@ __global__ void __launch_bounds__(kPrimBlock) k_ee_first(int n_total, const int3
         bS.B = xform_rigid(eb.B, M + PM_BS);
         bE.A = xform_rigid(eb.A, M + PM_BE);
         bE.B = xform_rigid(eb.B, M + PM_BE);
-        // Every distance edgeEdgeCCD can return is between points of the two
-        // swept segments, which lie in the boxes of their four endpoint
-        // positions.  A box gap beyond the search distance (plus 1e-7 m, far
-        // above FP64 rounding at scene scale) means no hit, and such a
-        // sub-test can never be the best of a triangle pair that hits: skip
-        // it, recording +inf.
-        const double lim = (double)thr + 1e-7;
-        double gap2 = 0.0;
-        {
-            const double ax[4] = {aS.A.x, aS.B.x, aE.A.x, aE.B.x}, ay[4] = {aS.A.y, aS.B.y, aE.A.y, aE.B.y},
-                         az[4] = {aS.A.z, aS.B.z, aE.A.z, aE.B.z};
-            const double bx[4] = {bS.A.x, bS.B.x, bE.A.x, bE.B.x}, by[4] = {bS.A.y, bS.B.y, bE.A.y, bE.B.y},
-                         bz[4] = {bS.A.z, bS.B.z, bE.A.z, bE.B.z};
-            const double* av[3] = {ax, ay, az};
-            const double* bv[3] = {bx, by, bz};
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                const double alo = fmin(fmin(av[d][0], av[d][1]), fmin(av[d][2], av[d][3]));
-                const double ahi = fmax(fmax(av[d][0], av[d][1]), fmax(av[d][2], av[d][3]));
-                const double blo = fmin(fmin(bv[d][0], bv[d][1]), fmin(bv[d][2], bv[d][3]));
-                const double bhi = fmax(fmax(bv[d][0], bv[d][1]), fmax(bv[d][2], bv[d][3]));
-                const double g = fmax(blo - ahi, alo - bhi);
-                if (g > 0.0) gap2 = gap2 + g * g;
-            }
-        }
-        if (gap2 > lim * lim) {
+        // Without the FP32 bounds: every distance edgeEdgeCCD can return is
+        // between points of the two swept segments, which lie in the boxes of
+        // their four endpoint positions, so a box gap beyond the search distance
+        // (plus 1e-7 m, far above FP64 rounding at scene scale) means no hit.
+        if (!a.bounds && ee_boxes_apart(aS, aE, bS, bE, (double)thr + 1e-7)) {
             record_no_contact(w.out, w.hit);
         } else {
             r.P = mk(0, 0, 0);
@@ -1443,13 +1550,6 @@ __global__ void __launch_bounds__(kPrimBlock) k_ee_first(int n_total, const int3
             if (bisect) {
                 iters = -1;  // in the second pass
             } else {
-                double V = 0.0, lim = 0.0;
-                if (a.certificates) {
-                    V = ee_motion_bound(aS, aE, bS, bE);
-                    const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
-                                            fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
-                    lim = ((double)thr + 1e-6) + 1e-12 * (mag + V);
-                }
                 for (; iters < a.first_iters; iters++) {
                     const double t_at = t;
                     double d_at;
@@ -1457,10 +1557,16 @@ __global__ void __launch_bounds__(kPrimBlock) k_ee_first(int n_total, const int3
                         done = true;
                         break;
                     }
-                    if (a.certificates && min_dist >= lim && d_at - V * fmax(t_at, 1.0 - t_at) >= lim) {
-                        cut = true;
-                        iters++;
-                        break;
+                    if (a.certificates && min_dist >= (double)thr) {
+                        const double V = ee_motion_bound(aS, aE, bS, bE);
+                        const double mag = fmax(fmax(fmax(fabs(aS.A.x), fabs(aS.A.y)), fabs(aS.A.z)),
+                                                fmax(fmax(fabs(bS.A.x), fabs(bS.A.y)), fabs(bS.A.z)));
+                        const double lim = ((double)thr + 1e-6) + 1e-12 * (mag + V);
+                        if (min_dist >= lim && d_at - V * fmax(t_at, 1.0 - t_at) >= lim) {
+                            cut = true;
+                            iters++;
+                            break;
+                        }
                     }
                 }
             }
@@ -1754,32 +1860,6 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // than thr by the same margin certainly hits (unless a triangle is almost a
 // point, whose edges return no distance); the pair is marked and done, and only
 // the survivors of the others go onto `list` for k_np_slots.
-// The gap between the triangles along d (d need not be a unit vector).
-__device__ __forceinline__ float axis_gap9(F3 d, const float* a, const float* b) {
-    const float nn = sqrtf(dot3(d, d));
-    if (!(nn > 1e-20f)) return 0.f;
-    float a0 = 3.4e38f, a1 = -3.4e38f, b0 = 3.4e38f, b1 = -3.4e38f;
-#pragma unroll
-    for (int v = 0; v < 3; v++) {
-        const float pa = dot3(d, f3(a[3 * v], a[3 * v + 1], a[3 * v + 2]));
-        const float pb = dot3(d, f3(b[3 * v], b[3 * v + 1], b[3 * v + 2]));
-        a0 = fminf(a0, pa);
-        a1 = fmaxf(a1, pa);
-        b0 = fminf(b0, pb);
-        b1 = fmaxf(b1, pb);
-    }
-    return fmaxf(b0 - a1, a0 - b1) / nn;
-}
-// A lower bound of the triangles' distance: along any direction the distance
-// is at least the gap between the projections, whatever the direction, so one
-// computed in FP32 still bounds.  Separate triangles are closest between two
-// edges, in the direction d of their closest edge pair, or between a vertex and
-// a face, along its normal.
-__device__ __forceinline__ float tri_gap(F3 d, const float* a, const float* b) {
-    const F3 na = cross3(f3(a[3] - a[0], a[4] - a[1], a[5] - a[2]), f3(a[6] - a[0], a[7] - a[1], a[8] - a[2]));
-    const F3 nb = cross3(f3(b[3] - b[0], b[4] - b[1], b[5] - b[2]), f3(b[6] - b[0], b[7] - b[1], b[8] - b[2]));
-    return fmaxf(axis_gap9(d, a, b), fmaxf(axis_gap9(na, a, b), axis_gap9(nb, a, b)));
-}
 __device__ __forceinline__ float box_gap9(const float* a, const float* b) {
     float gap2 = 0.f;
 #pragma unroll
@@ -2817,6 +2897,7 @@ int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, in
         ea.work = E.ee_work.p;
         ea.count = cnt_rest;
         ea.first_iters = E.tune[D2G_TUNE_EE_FIRST_ITERS];
+        ea.bounds = E.fp32_bounds ? 1 : 0;
         ea.certificates = E.certificates ? 1 : 0;
         ea.ca_stats = E.ccd_stats.p;
         k_ee_first<<<nblocks(n_ee, kPrimBlock), kPrimBlock, 0, s_ee>>>(n_ee, list_ee, cnt_ee, E.pm.p, ctx->tris.p,

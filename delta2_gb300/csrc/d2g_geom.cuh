@@ -635,6 +635,17 @@ D2G_HD double ee_bisect(const Edge& aS, const Edge& aE, const Edge& bS, const Ed
     return d;
 }
 
+// The Newton step of edgeEdgeCCD (:621-637) from time t with the edges at t
+// and their closest points P, Q: t moves by -f'/f'' and is clamped to [0, 1].
+D2G_HD double ee_newton_step(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE, const Edge& a,
+                             const Edge& b, V3 P, V3 Q, double t) {
+    const double pa = edge_project(a.A, a.B, P);
+    const double pb = edge_project(b.A, b.B, Q);
+    double td, td2;
+    ee_newton_terms(aS, aE, bS, bE, pa, pb, t, td, td2);
+    return clamp01(t - td / td2);
+}
+
 // One Newton iteration from time t (:609-637): the closest points at t update
 // the best (min_dist, r), then t moves by -f'/f'' and is clamped to [0, 1].
 // Returns true when the iteration loop ends here: each iteration is a
@@ -654,13 +665,8 @@ D2G_HD bool ee_newton_iter(const Edge& aS, const Edge& aE, const Edge& bS, const
         r.Q = Q;
         r.toc = t;
     }
-    const double pa = edge_project(atA, atB, P);
-    const double pb = edge_project(btA, btB, Q);
-    double td, td2;
-    ee_newton_terms(aS, aE, bS, bE, pa, pb, t, td, td2);
     const double t_prev = t;
-    t = t - td / td2;
-    t = clamp01(t);
+    t = ee_newton_step(aS, aE, bS, bE, Edge{atA, atB}, Edge{btA, btB}, P, Q, t);
     return t == t_prev || t != t;
 }
 
