@@ -125,7 +125,7 @@ def main():
     p = argparse.ArgumentParser()
     p.add_argument("--out", default=DEFAULT_OUT)
     p.add_argument("--ee-values", default="0,1,2,3,4")
-    p.add_argument("--grid-values", default="64,512,1000000")
+    p.add_argument("--grid-values", default="64,768,1000000")
     a = p.parse_args()
     from delta2_gb300 import build as B
 

@@ -33,7 +33,7 @@ constexpr int kGridMinContacts = 128;    // a cluster this large may take a coop
 constexpr int kGridMaxClusters = 8;      // ... with more parts than D2G_TUNE_GRID_MIN_PARTS,
                                          // when at most this many clusters qualify
 constexpr int kClusterMinContacts = 32;  // a cluster this large may take a thread-block cluster
-constexpr int kPartsPerBlock = 32;       // particles of a cluster per block of its thread-block cluster
+constexpr int kOneBlockParts = 32;       // ... and more particles than this
 constexpr int kSolveSmemMax = 200 * 1024;  // dynamic shared memory of a solve block at most
 inline int nblocks(long long n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
@@ -148,6 +148,10 @@ __global__ void k_filter_offsets(int n, const int32_t* __restrict__ off, const i
 // FP64 instruction count, 28 for the velocity half and 20 for the position
 // half, against ~143 when one warp formed both with the quaternion integration
 // of two states.  A contact takes eight lanes of each (side A or B, component).
+// Where a block has a single task of at most four contacts in a wave its four
+// sub-partitions have room for sixteen lanes a contact: products, divisions and
+// the linear and angular sums run side by side, 20 instructions either half,
+// with the next wave's constants loaded before the barrier.
 // Bodies live in shared memory (spread over the blocks of a thread-block
 // cluster, read and written through distributed shared memory) and a contact
 // in the shared memory of the block that always processes it, both in global
@@ -354,6 +358,7 @@ struct SolveArgs {
 };
 
 constexpr int kStaticBit = 1 << 30;
+constexpr int kWaveCache = 1024;  // wave bounds kept in shared memory
 
 // Body p of the cluster: block p % G's shared memory, or global memory.
 template <int MODE>
@@ -444,6 +449,145 @@ __device__ __forceinline__ void velocity_half(ConS& C, bool act, int side, int c
             if (C.sd) C.sd[c] = neg_if(u, C.sneg != 0);
             if (c == 0) C.imp = imp1;
         }
+    }
+}
+
+// The sixteen-lane forms (a warp has two contacts): lane bits 0-1 component,
+// bit 2 k, bit 3 side, bit 4 contact.  Lanes that differ in k run different
+// operations of one instruction stream: x + y as fma(x, 1, y) and x y as
+// fma(x, y, -0), each the same single rounding, so an addition, a product or a
+// fused step of div_by can share an instruction: 20 FP64 instructions for the
+// velocity half instead of 28 and 15 instead of 18, 64 cycles each.  What no
+// other warp writes is loaded one interval ahead (HalfPre).  100 cubes on 16
+// blocks: 164 -> 140 us per iteration.
+struct HalfPre {
+    ConS* C;
+    BodyS* B;
+    double* sd;
+    bool act, moving, sneg;  // the lane's contact exists; its body is not static; the sign of sd
+    double q[9];
+};
+
+__device__ __forceinline__ HalfPre velocity16_load(ConS* task, int half) {
+    const int lane = threadIdx.x & 31, c = lane & 3, cc = c < 3 ? c : 0, k = (lane >> 2) & 1, side = (lane >> 3) & 1;
+    const int c1 = cc == 2 ? 0 : cc + 1, c2 = cc == 0 ? 2 : cc - 1;
+    HalfPre t;
+    ConS* C = task + 2 * half + (lane >> 4);
+    t.act = C->ci >= 0;
+    if (!t.act) C = task;  // (a task's first contact exists)
+    BodyS& B = *C->body[side];
+    t.C = C;
+    t.B = &B;
+    t.moving = t.act && c < 3 && !B.is_static;
+    t.sd = t.act && c < 3 && k && side == 0 ? C->sd : nullptr;
+    t.sneg = C->sneg != 0;
+    t.q[0] = C->n[k ? c2 : c1];
+    t.q[1] = C->n[cc];
+    t.q[2] = B.ii[3 * cc + k];
+    t.q[3] = B.ii[3 * cc + 2];
+    t.q[4] = C->m;
+    t.q[5] = B.fv[cc];
+    t.q[6] = B.fL[cc];
+    t.q[7] = B.m;
+    t.q[8] = B.rm;
+    return t;
+}
+__device__ __forceinline__ void velocity_half16(const HalfPre& t) {
+    const int lane = threadIdx.x & 31, c = lane & 3, cc = c < 3 ? c : 0, k = (lane >> 2) & 1, side = (lane >> 3) & 1;
+    const int c1 = cc == 2 ? 0 : cc + 1, c2 = cc == 0 ? 2 : cc - 1, base = lane & ~7;
+    ConS& C = *t.C;
+    BodyS& B = *t.B;
+    const double wx = B.w[k ? c2 : c1], rx = C.r[side][k ? c1 : c2], v = B.v[cc];
+    const double sum = k ? B.imp[cc] : B.rimp[cc], imp0 = C.imp;
+    const bool near_ = C.near_ != 0;
+    // (w1 r2 on k = 0) - (w2 r1 on k = 1)
+    const double p = wx * rx, po = shfl_d(p, lane ^ 4);
+    const double vs = v + ((k ? po : p) - (k ? p : po));
+    const double pr = vs * t.q[1];
+    const double dv = (shfl_d(pr, base) + shfl_d(pr, base | 1)) + shfl_d(pr, base | 2);
+    const double ot = shfl_d(dv, lane ^ 8);
+    const double v1 = (side ? ot : dv) - (side ? dv : ot);
+    const double dn = (v1 * t.q[4]) * 0.1;
+    const double imp1 = max0(imp0 + (near_ ? dn : neg_if(imp0, true)));
+    const double du = imp1 - imp0;
+    // nus = -us in component c1 (k = 0) or c2, times r2 or r1
+    const double nus = neg_if(neg_if(t.q[0], true) * du, !side);
+    const double g = nus * rx, go = shfl_d(g, lane ^ 4);
+    const double nn = neg_if(t.q[1], true);
+    const double x1 = fma(k ? nn : g, k ? du : 1.0, k ? -0.0 : neg_if(go, true));  // torque | u
+    const double x2 = sum + neg_if(x1, k & side);                                  // rimp | imp
+    const double x3 = fma(x2, k ? t.q[8] : 1.0, k ? -0.0 : t.q[6]);                // L | imp / m: q
+    const double La = shfl_d(x3, base | k), L2 = shfl_d(x3, base | 2);
+    const double P = t.q[2] * La;                                                  // i0 L0 | i1 L1
+    const double Po = shfl_d(P, lane ^ 4);
+    const double x4 = fma(k ? neg_if(x3, true) : t.q[3], k ? t.q[7] : L2, k ? x2 : -0.0);  // i2 L2 | residual
+    const double x5 = fma(k ? x4 : P, k ? t.q[8] : 1.0, k ? x3 : Po);              // i0 L0 + i1 L1 | imp / m
+    double im = x5;
+    if (k && t.moving) {  // div_by's range checks
+        const bool yok = (unsigned)(m_exp_field(t.q[7]) - 573) <= 900u;
+        if (!(yok && (unsigned)(m_exp_field(x3) - 573) <= 900u)) im = yok && m_is_zero(x2) ? x3 : x2 / t.q[7];
+    }
+    const double x6 = (k ? t.q[5] : x5) + (k ? im : x4);                           // w | v
+    __syncwarp();
+    if (t.moving) {
+        (k ? B.imp : B.rimp)[c] = x2;
+        (k ? B.v : B.w)[c] = x6;
+    }
+    if (t.sd) t.sd[c] = neg_if(x1, t.sneg);
+    if (t.act && (lane & 15) == 4) C.imp = imp1;
+}
+__device__ __forceinline__ HalfPre position16_load(ConS* task, int half) {
+    const int lane = threadIdx.x & 31, c = lane & 3, cc = c < 3 ? c : 0, side = (lane >> 3) & 1;
+    HalfPre t;
+    ConS* C = task + 2 * half + (lane >> 4);
+    t.act = C->ci >= 0;
+    if (!t.act) C = task;
+    BodyS& B = *C->body[side];
+    t.C = C;
+    t.B = &B;
+    t.moving = t.act && c < 3 && !B.is_static;
+    t.sd = nullptr;
+    t.sneg = false;
+    t.q[0] = C->rl[side][cc];
+    t.q[1] = C->n[cc];
+    t.q[2] = C->outer;
+    t.q[3] = C->slop;
+    t.q[4] = C->damp_m;
+    t.q[5] = B.fx[cc];
+    t.q[6] = B.m;
+    t.q[7] = B.rm;
+    t.q[8] = 0.0;
+    return t;
+}
+__device__ __forceinline__ void position_half16(const HalfPre& h, double t, double rt) {
+    const int lane = threadIdx.x & 31, c = lane & 3, cc = c < 3 ? c : 0, k = (lane >> 2) & 1, side = (lane >> 3) & 1;
+    const int base = lane & ~7;
+    ConS& C = *h.C;
+    BodyS& B = *h.B;
+    const double x = B.x[cc], ioff = B.ioff[cc], off0 = C.off;
+    const double p1 = h.q[0] + x;
+    const double y = fma(k ? x : p1, k ? -1.0 : h.q[1], k ? p1 : -0.0);  // p1 n | p1 - x
+    const double dv = (shfl_d(y, base) + shfl_d(y, base | 1)) + shfl_d(y, base | 2);
+    const double ot = shfl_d(dv, lane ^ 8);
+    const double d1 = (side ? dv : ot) - (side ? ot : dv);
+    const double pen = h.q[2] - d1;
+    const bool near_ = is_pos(pen);
+    const double e = pen - h.q[3];
+    const double dn = div_by(h.q[4] * (is_pos(e) ? e : 0.0), t, rt);
+    const double off1 = max0(off0 + (near_ ? dn : neg_if(off0, true)));
+    const double uo = neg_if(h.q[1], true) * (off1 - off0);
+    const double io = ioff + neg_if(uo, side);
+    const double xn = h.q[5] + div_by(io, h.q[6], h.q[7]) * t;
+    __syncwarp();
+    if (k) {
+        if (h.act && c < 3) C.r[side][c] = y;
+    } else if (h.moving) {
+        B.ioff[c] = io;
+        B.x[c] = xn;
+    }
+    if (h.act && (lane & 15) == 0) {
+        C.off = off1;
+        C.near_ = near_ ? 1 : 0;
     }
 }
 
@@ -800,6 +944,9 @@ __device__ void solve_body(int k, int gb, int G, const SolveSync& S, const Solve
     if (nc > 0) {
         const int levels = fl[kFlLevels], tasks = fl[kFlTasks];
         const int32_t* tl = a.tl + c0 + k;
+        __shared__ int32_t s_tl[kWaveCache];
+        if (levels < kWaveCache)
+            for (int l = threadIdx.x; l <= levels; l += kSolveBlock) s_tl[l] = tl[l];
         const bool cons_in = sizeof(ConS) * 4 * (size_t)((tasks + G - 1) / G) <= rest_bytes;
         ConS* cs = cons_in ? (ConS*)rest : a.cs + 4 * (size_t)c0;
         // place of task gt's first contact: tasks gb, gb + G, ... are this block's
@@ -850,13 +997,76 @@ __device__ void solve_body(int k, int gb, int G, const SolveSync& S, const Solve
         const bool vel = (warp & 2) == 0;
         const int rank = (warp & 1) | ((warp >> 1) & 2);
         const int grp = lane >> 3, side = (lane >> 2) & 1, c = lane & 3;
+        // The block's tasks of wave l: the first, and how many.
+        const int32_t* tls = levels < kWaveCache ? s_tl : tl;
+        auto wave_tasks = [&](int l, int& first, int& count) {
+            const int lo = tls[l], hi = tls[l + 1];
+            if (MODE == kSyncBlock) {
+                first = lo;
+                count = hi - lo;
+            } else {
+                int d = gb - lo % G;
+                if (d < 0) d += G;
+                first = lo + d;
+                count = first < hi ? (hi - 1 - first) / G + 1 : 0;
+            }
+        };
+        // Sixteen lanes a contact while a wave has hardly more than one task
+        // here: a single task's chain is then the interval's length (8 cubes:
+        // 61 -> 60 us per iteration, 100 cubes on 16 blocks 164 -> 140).  With
+        // more tasks the loads ahead and the dealing of waves cost more than
+        // the few narrow waves give (27 cubes, 1.5 tasks a wave: 123 -> 129).
+        const bool narrow = 4 * n_tasks <= 5 * levels;
         bool converged = false;
+        int p0w = 0, pcw = 0;  // wave 0's tasks
+        wave_tasks(0, p0w, pcw);
+        auto load16 = [&](int first) {
+            return vel ? velocity16_load(cs + place(first), rank) : position16_load(cs + place(first), rank);
+        };
+        HalfPre pre;
+        pre.act = false;
+        if (narrow && !vel && pcw == 1 && rank < 2) pre = load16(p0w);
         while (!converged && it_n < 1000) {
-            int t0 = 0, t1 = tl[0], t2 = tl[1];
-            for (int j = 0; j <= levels; j++) {
-                // position halves of wave j [t1, t2), velocity halves of wave j - 1 [t0, t1)
+            int pf = p0w, pc = pcw, vf = 0, vc = 0;
+            for (int j = 0; j <= levels && narrow; j++) {
+                // position halves of wave j (tasks pf, pc), velocity halves of
+                // wave j - 1 (vf, vc); then the next interval's constants
+                const int first = vel ? vf : pf, count = vel ? vc : pc;
+                if (count == 1) {
+                    if (rank < 2 && __any_sync(0xffffffffu, pre.act)) {
+                        if (vel)
+                            velocity_half16(pre);
+                        else
+                            position_half16(pre, t, rt);
+                    }
+                } else {
+                    for (int u = rank; u < count; u += 4) {
+                        ConS* C = cs + place(first + u * G);
+                        const bool act = C[grp].ci >= 0;
+                        ConS& Cg = C[act ? grp : 0];
+                        if (vel)
+                            velocity_half(Cg, act, side, c);
+                        else
+                            position_half(Cg, act, side, c, t, rt);
+                    }
+                }
+                vf = pf;
+                vc = pc;
+                pf = p0w;  // (after the last wave: the next iteration's first)
+                pc = pcw;
+                if (j + 1 < levels)
+                    wave_tasks(j + 1, pf, pc);
+                else if (j + 1 == levels)
+                    pc = 0;
+                if (rank < 2 && (vel ? vc : pc) == 1 && !(vel && j == levels)) pre = load16(vel ? vf : pf);
+                SYNC();
+            }
+            int t0 = 0, t1 = tls[0], t2 = tls[1];
+            for (int j = 0; j <= levels && !narrow; j++) {
+                // the same with eight lanes for each contact: wave j's tasks
+                // [t1, t2), wave j - 1's [t0, t1)
                 const int lo = vel ? t0 : t1, hi = vel ? t1 : t2;
-                const int t3 = j + 2 <= levels ? tl[j + 2] : t2;
+                const int t3 = j + 2 <= levels ? tls[j + 2] : t2;
                 int gt = lo + (gb - lo % G + G) % G + rank * G;
                 for (; gt < hi; gt += 4 * G) {
                     ConS* C = cs + place(gt);
@@ -1193,12 +1403,9 @@ int launch_solve_cl(d2g_ctx* ctx, int cs, int n, const int32_t* d_list, int32_t*
 
 // Blocks that serve a cluster of np particles best: a wave holds a seventh to
 // a quarter as many contacts as the cluster has particles, four to a task, and
-// a block runs two tasks at full rate (measured: the table in run_solve).
-int best_cluster_size(int np) {
-    int cs = 1;
-    while (cs < 16 && cs * kPartsPerBlock < np) cs *= 2;
-    return cs;
-}
+// a block that has a single task in a wave takes the faster form of the halves
+// (measured: the table in run_solve).
+int best_cluster_size(int np) { return np > kOneBlockParts ? 16 : 1; }
 
 // Solve clusters.  Contacts (14-double records in the reference's hit order,
 // clusters contiguous per d_con_off) with per-contact pair counts and warm
@@ -1278,21 +1485,23 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
         a.pair_warm = d_pair_warm;
         // Where each cluster is solved (us per iteration on GB300, normal and
         // friction; one block / thread-block cluster of 4 / 8 / 16 / grid):
-        //     8 cubes, 46 waves of 2.2 contacts     61 /   88 /   88 /  88 /    -
-        //    27 cubes, 89 waves of 5.0             123 /  167 /  166 / 166 /  240
-        //   100 cubes, one layer                   310 /  176 /  165 / 164 /  219
-        //   512 hulls, 24 waves of 71              353 /  113 /   82 /  71 /   85
-        // 1,024 hulls, 23 waves of 142             671 /  213 /  125 /  88 /   90
-        // 2,304 hulls                             1530 /  481 /  289 / 178 /  135
-        // 5,120 hulls                             3646 / 1115 /  683 / 467 /  268
-        // (before: 331 us for the 8 cubes, 257 for the 1,024 hulls).  A block
-        // barrier costs ~0.1 us, the cluster barrier with distributed shared
-        // memory ~0.5 us more, a grid barrier ~1.5 us, and a block runs two
-        // tasks at full rate: so one block up to kPartsPerBlock particles, then
-        // twice as many for every doubling (best_cluster_size) as long as all
-        // such clusters of the call are resident at once, and a cooperative
-        // grid for a cluster with at least kGridMinContacts contacts and more
-        // than D2G_TUNE_GRID_MIN_PARTS parts when at most kGridMaxClusters
+        //     8 cubes, 46 waves of 2.2 contacts     60 /   74 /   72 /  74 /    -
+        //    27 cubes, 89 waves of 5.0             124 /  141 /  136 / 140 /  223
+        //   100 cubes, one layer                   311 /  185 /  152 / 140 /  203
+        //   512 hulls, 24 waves of 71              357 /  118 /   79 /  67 /   77
+        // 1,024 hulls, 23 waves of 142             676 /  213 /  124 /  88 /   83
+        // 2,304 hulls                             1542 /  480 /  289 / 178 /  133
+        // (one to four contacts to a warp throughout, eight lanes each: 61 for
+        // the 8 cubes, 165 / 164 for the 100 on 8 / 16 blocks, 71 / 85 and 88 /
+        // 90 for 512 and 1,024 hulls on 16 blocks / a grid; the halves undivided,
+        // a contact on one warp: 331 for the 8 cubes, 257 for the 1,024 hulls.)
+        // A block barrier costs ~0.1 us, the cluster barrier with distributed
+        // shared memory ~0.5 us more, a grid barrier ~1.5 us: so one block up
+        // to kOneBlockParts particles, then 16 (best_cluster_size), or the most
+        // with which all such clusters of the call are resident at once, and a
+        // cooperative grid for a cluster with at least kGridMinContacts contacts
+        // and more than D2G_TUNE_GRID_MIN_PARTS parts (768 by default, between
+        // the 513 and the 1,025 of the table) when at most kGridMaxClusters
         // qualify (grids run one after another).  D2G_TUNE_SOLVE_CLUSTER fixes
         // the cluster's size.  Blocks and thread-block clusters run side by
         // side on two streams, the grids after them.
