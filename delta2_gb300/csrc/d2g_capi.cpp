@@ -435,6 +435,8 @@ void d2g_ctx_destroy(d2g_ctx* c) {
     E.nn_cnt.release();
     E.nn_off.release();
     E.st_mt.release();
+    E.st_spin.release();
+    E.st_best.release();
     E.st_new_dt.release();
     E.st_step.release();
     E.st_out.release();

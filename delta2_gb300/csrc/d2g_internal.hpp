@@ -146,7 +146,8 @@ struct Engine {
     DBuf<PrimResult> sub, cres;
     DBuf<int32_t> chit, cflag_off, nn_cnt, nn_off, tp, lc, sums;  // tp: leaf pair of a triangle pair; lc: level counters
     // time-step selection
-    DBuf<double> st_mt, st_new_dt, st_step, st_out;
+    DBuf<double> st_mt, st_new_dt, st_step, st_out, st_spin;
+    DBuf<unsigned long long> st_best;
     DBuf<int32_t> st_has, st_cl_pair_off, st_cl_part_off, st_cl_parts, st_loc;
     // contact filtering
     DBuf<int32_t> flt_idx, flt_order, flt_keep, flt_pos, flt_cnt, flt_off;

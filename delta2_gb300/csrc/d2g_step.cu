@@ -21,18 +21,32 @@ namespace {
 constexpr int kBlock = 128;
 inline int nblocks(long long n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
+// What a contact's step scale reads of its pair's bodies.
+struct StepBody {
+    V3 v, x;
+};
+
 // separate_clusters.cpp:497-554: the scale one continuous contact asks for
-// (Ia, Ib: the future world inverse inertias, Particle::futurePointVelocity).
-__device__ double contact_step_scale(const double* c, const State& fa, const double* Ia, const State& fb,
-                                     const double* Ib, double max_dt) {
+// (wa, wb: the future angular velocities, of Particle::futurePointVelocity).
+__device__ double contact_step_scale(const double* c, const StepBody& fa, const V3 wa, const StepBody& fb,
+                                     const V3 wb, double max_dt) {
     double scale = 1.0;
     const V3 A = mk(c[0], c[1], c[2]), B = mk(c[3], c[4], c[5]);
     const double toc = c[10];
     const V3 hit_normal = A - B;
+    // |hit_normal| above 1e-4 beyond rounding: a contact at the motion's end
+    // asks for nothing, nor does one whose sides part
+    const double h2 = dot(hit_normal, hit_normal);
+    const bool apart = h2 > 1.0001e-8;
+    if (apart && !(toc < 1.0)) return 1.0;
     const double interaction_dist = c[6] + c[7];
-    const V3 a_vel = fa.v + cross(m3_vec(Ia, fa.L), A - fa.x);
-    const V3 b_vel = fb.v + cross(m3_vec(Ib, fb.L), B - fb.x);
+    const V3 a_vel = fa.v + cross(wa, A - fa.x);
+    const V3 b_vel = fb.v + cross(wb, B - fb.x);
     const V3 rel = a_vel - b_vel;
+    // the test's dot of unit vectors is off by a few 1e-16 at most, so its sign
+    // is known when the cosine is above 1e-12 (near zero or out of range: below)
+    const double hr = dot(hit_normal, rel), r2 = dot(rel, rel);
+    if (apart && hr > 0.0 && r2 > 1e-200 && hr * hr > 1e-24 * (h2 * r2)) return 1.0;
     if (dot(normalized(hit_normal), normalized(rel)) <= 0.0 || norm(hit_normal) < 1e-4) {
         if (norm(hit_normal) < 1e-4) {
             if (toc == 0.0) return 1.0;
@@ -64,52 +78,84 @@ __device__ __forceinline__ double dmin_fast(double a, double b) {
     return b < a ? b : a;
 }
 
-// One warp per interaction (separate_clusters.cpp:494-562): every contact's
-// scale in parallel, then the reference's running minimum from 1.0, which
-// keeps the first of equal values and never takes a NaN, as a leftmost-
-// minimum reduction over (value, contact index).
-__global__ void k_pair_new_dt(int n_pairs, const int32_t* __restrict__ pairs, const double* __restrict__ max_time,
-                              const int32_t* __restrict__ off, const double* __restrict__ rec,
-                              const double* __restrict__ pfut, const double* __restrict__ ii,
-                              double* __restrict__ new_dt, int32_t* __restrict__ has) {
-    const int p = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (p >= n_pairs) return;  // uniform per warp
-    const int a = pairs[2 * p], b = pairs[2 * p + 1];
-    const int c0 = off[p], c1 = off[p + 1];
-    if (c1 <= c0) {
-        if (lane == 0) {
-            has[p] = 0;
-            new_dt[p] = 0.0;
+// The order of non-NaN doubles as unsigned integers.
+__device__ __forceinline__ unsigned long long order_bits(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return b >> 63 ? ~b : b | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double from_order_bits(unsigned long long b) {
+    return __longlong_as_double((long long)(b >> 63 ? b & 0x7fffffffffffffffull : ~b));
+}
+
+// Every interaction's new step (separate_clusters.cpp:494-562), in three
+// launches.  k_pair_spin: the future angular velocities of each pair's two
+// bodies, a thread per body, and the running minimum's start 1.0.
+// k_contact_scale: a thread per contact, whichever pair it belongs to, so a
+// pair with thousands of contacts spreads over the chip; the minimum over a
+// pair's contacts, which never takes a NaN, by integer atomics (scales are
+// positive, so equal values are equal bits and the order of arrival does not
+// matter).  FP64 issue bounds it; contacts whose sides part, most of a
+// resting pile's, leave after 45 of 200 operations.  One warp per pair took
+// 380 us for 64 piles of eight cubes, waiting for the pairs with the most
+// contacts.
+__global__ void k_pair_spin(int n_pairs, const int32_t* __restrict__ pairs, const double* __restrict__ pfut,
+                            const double* __restrict__ ii, double* __restrict__ spin,
+                            unsigned long long* __restrict__ best) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * n_pairs) return;
+    const State f = load_state(pfut + 14 * (size_t)i);
+    double I[9];
+    world_inv_inertia(f.q, ii + 9 * (size_t)pairs[i], I);
+    const V3 w = m3_vec(I, f.L);
+    spin[3 * (size_t)i] = w.x;
+    spin[3 * (size_t)i + 1] = w.y;
+    spin[3 * (size_t)i + 2] = w.z;
+    if (!(i & 1)) best[i >> 1] = order_bits(1.0);
+}
+
+__global__ void __launch_bounds__(kBlock) k_contact_scale(int n_pairs, const double* __restrict__ max_time,
+                                                          const int32_t* __restrict__ off,
+                                                          const double* __restrict__ rec,
+                                                          const double* __restrict__ pfut,
+                                                          const double* __restrict__ spin,
+                                                          unsigned long long* __restrict__ best) {
+    const int n = off[n_pairs], lane = threadIdx.x & 31;
+    for (int base = (int)(blockIdx.x * kBlock + (threadIdx.x & ~31)); base < n; base += (int)gridDim.x * kBlock) {
+        const int c = min(base + lane, n - 1);  // (a last one taken twice changes no minimum)
+        int lo = 0, hi = n_pairs;               // the pair with off[lo] <= c < off[lo + 1]
+        while (hi - lo > 1) {
+            const int m = (lo + hi) >> 1;
+            if (off[m] <= c)
+                lo = m;
+            else
+                hi = m;
         }
-        return;
-    }
-    const State fa = load_state(pfut + 28 * (size_t)p), fb = load_state(pfut + 28 * (size_t)p + 14);
-    const double mt = max_time[p];
-    double Ia[9], Ib[9];
-    world_inv_inertia(fa.q, ii + 9 * (size_t)a, Ia);
-    world_inv_inertia(fb.q, ii + 9 * (size_t)b, Ib);
-    double best = 1.0;
-    int best_i = -1;  // the running minimum's start value comes first
-    for (int c = c0 + lane; c < c1; c += 32) {
-        const double sc = contact_step_scale(rec + 14 * (size_t)c, fa, Ia, fb, Ib, mt);
-        if (sc < best) {
-            best = sc;
-            best_i = c;
+        const double *pa = pfut + 28 * (size_t)lo, *pb = pa + 14, *w = spin + 6 * (size_t)lo;
+        const State sa = load_state(pa), sb = load_state(pb);
+        const double sc = contact_step_scale(rec + 14 * (size_t)c, StepBody{sa.v, sa.x}, mk(w[0], w[1], w[2]),
+                                             StepBody{sb.v, sb.x}, mk(w[3], w[4], w[5]), max_time[lo]);
+        const bool nan = (__double_as_longlong(sc) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+        unsigned long long k = nan ? ~0ull : order_bits(sc);
+        if (__all_sync(0xffffffffu, lo == __shfl_sync(0xffffffffu, lo, 0))) {
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, o);
+                k = ok < k ? ok : k;
+            }
+            if (lane == 0) atomicMin(best + lo, k);
+        } else {
+            atomicMin(best + lo, k);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_down_sync(0xffffffffu, best, o);
-        const int oi = __shfl_down_sync(0xffffffffu, best_i, o);
-        if (ob < best || (ob == best && oi < best_i)) {
-            best = ob;
-            best_i = oi;
-        }
-    }
-    if (lane == 0) {
-        has[p] = 1;
-        new_dt[p] = mt * best;
-    }
+}
+
+__global__ void k_pair_new_dt(int n_pairs, const double* __restrict__ max_time, const int32_t* __restrict__ off,
+                              const unsigned long long* __restrict__ best, double* __restrict__ new_dt,
+                              int32_t* __restrict__ has) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n_pairs) return;
+    const bool any = off[p + 1] > off[p];
+    has[p] = any ? 1 : 0;
+    new_dt[p] = any ? max_time[p] * from_order_bits(best[p]) : 0.0;
 }
 
 // Leftmost minimum of (value, index) over a block (all threads call it; the
@@ -145,6 +191,7 @@ __device__ void block_lmin(double& v, int& i, double* red_v, int* red_i) {
 }
 
 constexpr int kStepsBlock = 256;
+constexpr int kScaleGrid = 152 * 4;  // a warp per sub-partition for the FP64 pipe, four to hide loads
 constexpr int kStepsChunk = 1024;  // interactions staged per pass
 
 // The reference's order-dependent propagation over a cluster's interactions
@@ -641,10 +688,16 @@ int run_select_steps(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, const in
         const int32_t* pr = static_cast<Use*>(u)->pairs;
         const int np = p1 - p0;
         if (np > 0) {
-            k_pair_new_dt<<<nblocks(32LL * np), kBlock, 0, c->stream>>>(
-                np, pr + 2 * (size_t)p0, En.st_mt.p + p0, En.out_off.p, En.rec_sorted.p, En.pfut.p + 28 * (size_t)p0,
-                c->inv_inertia.p, En.st_new_dt.p + p0, En.st_has.p + p0);
-            En.launches++;
+            RC(En.st_spin.ensure(6 * (size_t)np));
+            RC(En.st_best.ensure(np));
+            const double *fut = En.pfut.p + 28 * (size_t)p0, *mt = En.st_mt.p + p0;
+            k_pair_spin<<<nblocks(2LL * np), kBlock, 0, c->stream>>>(np, pr + 2 * (size_t)p0, fut, c->inv_inertia.p,
+                                                                     En.st_spin.p, En.st_best.p);
+            k_contact_scale<<<kScaleGrid, kBlock, 0, c->stream>>>(np, mt, En.out_off.p, En.rec_sorted.p, fut,
+                                                                    En.st_spin.p, En.st_best.p);
+            k_pair_new_dt<<<nblocks(np), kBlock, 0, c->stream>>>(np, mt, En.out_off.p, En.st_best.p,
+                                                                 En.st_new_dt.p + p0, En.st_has.p + p0);
+            En.launches += 3;
         }
         D2G_CUDA(cudaGetLastError());
         return D2G_OK;
