@@ -150,9 +150,8 @@ struct Engine {
     DBuf<unsigned long long> st_best;
     DBuf<int32_t> st_has, st_cl_pair_off, st_cl_part_off, st_cl_parts, st_loc;
     // contact filtering
-    DBuf<int32_t> flt_idx, flt_order, flt_keep, flt_pos, flt_cnt, flt_off;
+    DBuf<int32_t> flt_idx, flt_cnt, flt_off, flt_list;
     DBuf<unsigned long long> flt_keys, flt_keys_s;
-    DBuf<double> flt_mid;
     // CCD candidates: FP32 poses (8 per pair), survivor counts and lists
     DBuf<float> pm32c;
     DBuf<int32_t> ccd_cnt, ccd_list;  // CCD survivors: counts (point-triangle, edge-edge) and lists
@@ -162,11 +161,11 @@ struct Engine {
     DBuf<int32_t> np_cnt, np_off;
     DBuf<double> flt;
     // sequential-impulse solve
-    DBuf<unsigned long long> sv_keys, sv_keys_out;
-    DBuf<int32_t> sv_vals, sv_order, sv_slot, sv_part_int, sv_con_int, sv_tcon, sv_tl;
+    DBuf<unsigned long long> sv_keys;
+    DBuf<int32_t> sv_long, sv_order, sv_slot, sv_part_int, sv_con_int, sv_tcon, sv_tl;
     DBuf<double> sv_sdelta;
     DBuf<int32_t> sv_list, sv_grid, sv_cl_flags;
-    bool sv_smem_set = false;  // the solve kernels' shared memory limit was raised
+    bool sv_smem_set = false, seg_smem_set = false;  // the solve and sort kernels' shared memory limits were raised
     int sv_cl_fit[4] = {-1, -1, -1, -1};  // resident thread-block clusters of 16, 8, 4, 2 solve blocks
     int sv_layout[4] = {0, 0, 0, 0};  // the last solve call's layout (d2g_ctx_solve_layout)
     DBuf<unsigned char> sv_bg_raw, sv_bs_raw, sv_cg_raw, sv_cs_raw;

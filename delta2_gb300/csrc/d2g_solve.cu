@@ -37,96 +37,216 @@ constexpr int kOneBlockParts = 32;       // ... and more particles than this
 constexpr int kSolveSmemMax = 200 * 1024;  // dynamic shared memory of a solve block at most
 inline int nblocks(long long n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
-// ------------------------------------------------------------ filtering ---
-// Sort keys of compareContacts (contact.h:32-40): (eps_a + eps_b, |A - B|),
-// both non-negative doubles, whose bit patterns order like the values.
-__global__ void k_filter_keys(int n, const double* __restrict__ rec, unsigned long long* __restrict__ key_norm,
-                              int32_t* __restrict__ idx) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* c = rec + 14 * (size_t)i;
-    key_norm[i] = (unsigned long long)__double_as_longlong(norm(mk(c[0] - c[3], c[1] - c[4], c[2] - c[5])));
-    idx[i] = i;
-}
+// -------------------------------------------------------- segment sorts ---
+// Contacts are sorted within a body pair (the filter) or a cluster (the
+// solve), never across: a block sorts a segment where it lies, in shared
+// memory up to the kernel's capacity and in global memory above.  Ascending by
+// (a, b, id), or by (a, id) without TWO: ids are distinct, so ties keep their
+// input order.  A bitonic network whose merges start with a mirrored step, so
+// that all exchanges put the smaller element first and places from n on need
+// not exist.  A comparator t of a step within 64 elements belongs to the warp
+// that owns them, and needs no block barrier before the next such step.
+// (Library segmented sorts took 22 launches and ~175 us of a 296 us filter
+// call on 4,000 contacts in 300 pairs, and 12 launches in a solve.)
+constexpr int kSegSmall = 1024;        // elements of the 128-thread kernels' shared memory
+constexpr int kSegLarge = 8192;        // ... of the 1,024-thread kernels'
+constexpr int kSegSmallBlock = 128, kSegLargeBlock = 1024, kSegLargeGrid = 152;
+constexpr int kSegLargeSmem = 20 * kSegLarge, kOrderSmem = 12 * kSegLarge;
+typedef unsigned long long u64;
 
-__global__ void k_filter_eps_keys(int n, const double* __restrict__ rec, const int32_t* __restrict__ idx,
-                                  unsigned long long* __restrict__ key_eps) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* c = rec + 14 * (size_t)idx[i];
-    key_eps[i] = (unsigned long long)__double_as_longlong(c[6] + c[7]);
-}
-
-// The greedy pass of filterContacts (contact.h:49-66), one warp per body
-// pair over its contacts in sorted order: a contact is kept unless its
-// midpoint lies within eps_a + eps_b + margin (its own) of an already kept
-// contact's midpoint.  Contacts are taken 32 at a time: each lane tests its
-// contact against the pair's kept midpoints, then the chunk is resolved in
-// order (the lowest surviving lane is kept and eliminates the later lanes
-// near it).  kept_mid holds each pair's kept midpoints (from its first slot).
-__global__ void k_filter_dedupe(int n_pairs, const int32_t* __restrict__ off, const int32_t* __restrict__ order,
-                                const double* __restrict__ rec, double margin, int32_t* __restrict__ keep,
-                                int32_t* __restrict__ kept_cnt, double* __restrict__ kept_mid) {
-    const int warp = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (warp >= n_pairs) return;  // uniform per warp
-    const int c0 = off[warp], c1 = off[warp + 1];
-    int nk = 0;
-    for (int base = c0; base < c1; base += 32) {
-        const int j = base + lane;
-        const bool in = j < c1;
-        V3 mid = mk(0, 0, 0);
-        double search = 0.0;
-        if (in) {
-            const double* ct = rec + 14 * (size_t)order[j];
-            mid = mk((ct[0] + ct[3]) / 2, (ct[1] + ct[4]) / 2, (ct[2] + ct[5]) / 2);
-            search = (ct[6] + ct[7]) + margin;
+template <bool TWO>
+__device__ void sort_segment(int n, u64* a, u64* b, int32_t* id) {
+    const int nt = (int)blockDim.x;
+    int half = 1;  // comparators of a step: half the padded size
+    while (2 * half < n) half *= 2;
+    auto exchange = [&](int i, int j) {
+        if (j >= n) return;
+        const u64 ai = a[i], aj = a[j], bi = TWO ? b[i] : 0, bj = TWO ? b[j] : 0;
+        const int32_t di = id[i], dj = id[j];
+        if (ai < aj || (ai == aj && (bi < bj || (bi == bj && di < dj)))) return;
+        a[i] = aj;
+        a[j] = ai;
+        if (TWO) {
+            b[i] = bj;
+            b[j] = bi;
         }
-        bool alive = in;
-        for (int t = 0; t < nk && alive; t++) {
-            const double* h = kept_mid + 3 * (size_t)(c0 + t);
-            if (norm(mid - mk(h[0], h[1], h[2])) < search) alive = false;
+        id[i] = dj;
+        id[j] = di;
+    };
+    __syncthreads();
+    for (int h = 1; h <= half; h *= 2) {  // sorted runs of h become runs of 2 h
+        for (int t = threadIdx.x; t < half; t += nt) {
+            const int base = 2 * (t & ~(h - 1)), o = t & (h - 1);
+            exchange(base + o, base + 2 * h - 1 - o);
         }
-        unsigned kept = 0;
-        unsigned live = __ballot_sync(0xffffffffu, alive);
-        while (live) {
-            const int src = __ffs(live) - 1;
-            kept |= 1u << src;
-            const V3 h = mk(__shfl_sync(0xffffffffu, mid.x, src), __shfl_sync(0xffffffffu, mid.y, src),
-                            __shfl_sync(0xffffffffu, mid.z, src));
-            if (alive && lane > src && norm(mid - h) < search) alive = false;
-            live = __ballot_sync(0xffffffffu, alive) & ~((2u << src) - 1u);
+        if (h > 32)
+            __syncthreads();
+        else
+            __syncwarp();
+        for (int w = h / 2; w > 0; w /= 2) {
+            for (int t = threadIdx.x; t < half; t += nt) {
+                const int i = 2 * (t & ~(w - 1)) + (t & (w - 1));
+                exchange(i, i + w);
+            }
+            if (w > 32)
+                __syncthreads();
+            else
+                __syncwarp();
         }
-        const bool k = (kept >> lane) & 1u;
-        if (in) keep[j] = k ? 1 : 0;
-        if (k) {
-            double* o = kept_mid + 3 * (size_t)(c0 + nk + __popc(kept & ((1u << lane) - 1u)));
-            o[0] = mid.x;
-            o[1] = mid.y;
-            o[2] = mid.z;
-        }
-        nk += __popc(kept);
-        __syncwarp();
+        if (h >= 32) __syncthreads();  // the next merge crosses warps
     }
-    if (lane == 0) kept_cnt[warp] = nk;
+    __syncthreads();
 }
 
-// Kept contacts, in sorted order per pair, to their scanned positions.
-__global__ void k_filter_write(int n, const int32_t* __restrict__ order, const int32_t* __restrict__ keep,
-                               const int32_t* __restrict__ pos, const double* __restrict__ rec,
+// Segments above the small kernels' capacity go to the large ones' list
+// (list[0] counts them): true when the block is to leave segment p.
+__device__ __forceinline__ bool leave_segment(int p, int n, int32_t* list) {
+    if (n <= kSegSmall) return false;
+    if (threadIdx.x == 0) list[1 + atomicAdd(list, 1)] = p;
+    return true;
+}
+
+// ------------------------------------------------------------ filtering ---
+// The midpoint of a contact, and filterContacts' test (contact.h:49-66): h's
+// within eps_a + eps_b + margin (c's own) of c's.
+__device__ __forceinline__ V3 contact_mid(const double* c) {
+    return mk((c[0] + c[3]) / 2, (c[1] + c[4]) / 2, (c[2] + c[5]) / 2);
+}
+__device__ __noinline__ bool contact_near_exact(const double* c, const double* h, double margin) {
+    return norm(contact_mid(c) - contact_mid(h)) < (c[6] + c[7]) + margin;
+}
+
+// The same in FP32 on midpoints relative to the pair's first contact: a
+// distance further from the search radius than both roundings can move it (a
+// component of the difference by 2^-24 (|x| + |y| + |x - y|), the root by a
+// few 2^-24 of itself, the radius by 2^-24 of itself) decides; the rest, and
+// whatever is not finite, goes to the FP64 test.
+struct NearF {
+    float x, y, z, s;
+};
+__device__ __forceinline__ bool contact_near(const NearF& c, const NearF& h, const double* cr, const double* hr,
+                                             double margin) {
+    const float dx = c.x - h.x, dy = c.y - h.y, dz = c.z - h.z;
+    const float d = sqrtf(dx * dx + dy * dy + dz * dz);
+    const float m = 5e-7f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z) + fabsf(h.x) + fabsf(h.y) + fabsf(h.z)) + 1e-15f;
+    if (d + m < c.s * 0.999999f) return true;
+    if (d - m > c.s * 1.000001f && d < 1e18f) return false;
+    return contact_near_exact(cr, hr, margin);
+}
+
+// filterContacts of one body pair's contacts, one block: sorted by
+// compareContacts (contact.h:32-40: (eps_a + eps_b, |A - B|), both
+// non-negative doubles, whose bit patterns order like the values), then the
+// greedy pass (contact.h:49-66): a contact is kept unless near an already kept
+// one.  Contacts are taken 32 at a time: every warp tests them against its
+// share of the kept ones, then warp 0 resolves the 32 in order (the lowest
+// surviving lane is kept and eliminates the later lanes near it).  The kept
+// contacts' FP32 midpoints and ids are compacted to the segment's front.
+// Bounded by the serial chain of kept contacts, ~60 instructions each; with
+// FP64 distances it was ~20 FP64 instructions at 64 cycles.
+struct FilterArgs {
+    const int32_t* off;
+    const double* rec;
+    double margin;
+    u64 *ga, *gb;        // global working arrays of the largest segments
+    int32_t *order, *cnt, *list;
+};
+__device__ void filter_segment(const FilterArgs& f, int p, int n, u64* a, u64* b, int32_t* id) {
+    const int c0 = f.off[p], nt = (int)blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nt >> 5;
+    for (int i = threadIdx.x; i < n; i += nt) {
+        const double* c = f.rec + 14 * (size_t)(c0 + i);
+        a[i] = (u64)__double_as_longlong(c[6] + c[7]);
+        b[i] = (u64)__double_as_longlong(norm(mk(c[0] - c[3], c[1] - c[4], c[2] - c[5])));
+        id[i] = c0 + i;
+    }
+    sort_segment<true>(n, a, b, id);
+    const V3 o = n > 0 ? contact_mid(f.rec + 14 * (size_t)c0) : mk(0, 0, 0);
+    for (int i = threadIdx.x; i < n; i += nt) {  // the keys' places take the midpoints
+        const double* c = f.rec + 14 * (size_t)id[i];
+        const V3 m = contact_mid(c) - o;
+        *(float2*)(a + i) = make_float2((float)m.x, (float)m.y);
+        *(float2*)(b + i) = make_float2((float)m.z, (float)((c[6] + c[7]) + f.margin));
+    }
+    __shared__ unsigned s_dead[kSegLargeBlock / 32];
+    __shared__ int s_kept;
+    __syncthreads();
+    auto at = [&](int i) {
+        const float2 u = *(const float2*)(a + i), v = *(const float2*)(b + i);
+        return NearF{u.x, u.y, v.x, v.y};
+    };
+    int nk = 0;
+    for (int base = 0; base < n; base += 32) {
+        const int j = base + lane;
+        const bool in = j < n;
+        const NearF me = at(in ? j : base);
+        const int32_t my = id[in ? j : base];
+        const double* mr = f.rec + 14 * (size_t)my;
+        bool alive = in;
+        for (int t = warp; t < nk && alive; t += nw)
+            if (contact_near(me, at(t), mr, f.rec + 14 * (size_t)id[t], f.margin)) alive = false;
+        const unsigned dead = __ballot_sync(0xffffffffu, !alive);
+        if (lane == 0) s_dead[warp] = dead;
+        __syncthreads();  // every warp has read this chunk: kept contacts may take its places
+        if (warp == 0) {
+            unsigned d = lane < nw ? s_dead[lane] : 0u;
+            d = __reduce_or_sync(0xffffffffu, d);
+            alive = !((d >> lane) & 1u);
+            unsigned kept = 0, live = __ballot_sync(0xffffffffu, alive);
+            while (live) {
+                const int src = __ffs(live) - 1;
+                kept |= 1u << src;
+                const NearF h{__shfl_sync(0xffffffffu, me.x, src), __shfl_sync(0xffffffffu, me.y, src),
+                              __shfl_sync(0xffffffffu, me.z, src), 0.0f};
+                const int32_t hid = __shfl_sync(0xffffffffu, my, src);
+                if (alive && lane > src && contact_near(me, h, mr, f.rec + 14 * (size_t)hid, f.margin)) alive = false;
+                live = __ballot_sync(0xffffffffu, alive) & ~((2u << src) - 1u);
+            }
+            if ((kept >> lane) & 1u) {
+                const int k = nk + __popc(kept & ((1u << lane) - 1u));
+                *(float2*)(a + k) = make_float2(me.x, me.y);
+                *(float2*)(b + k) = make_float2(me.z, me.s);
+                id[k] = my;
+            }
+            if (lane == 0) s_kept = nk + __popc(kept);
+        }
+        __syncthreads();
+        nk = s_kept;
+    }
+    for (int i = threadIdx.x; i < nk; i += nt) f.order[c0 + i] = id[i];
+    if (threadIdx.x == 0) f.cnt[p] = nk;
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kSegSmallBlock) k_filter(FilterArgs f) {
+    __shared__ u64 a[kSegSmall], b[kSegSmall];
+    __shared__ int32_t id[kSegSmall];
+    const int p = blockIdx.x, n = f.off[p + 1] - f.off[p];
+    if (!leave_segment(p, n, f.list)) filter_segment(f, p, n, a, b, id);
+}
+__global__ void __launch_bounds__(kSegLargeBlock) k_filter_large(FilterArgs f) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    u64 *a = (u64*)dyn, *b = a + kSegLarge;
+    int32_t* id = (int32_t*)(b + kSegLarge);
+    for (int q = blockIdx.x; q < f.list[0]; q += gridDim.x) {
+        const int p = f.list[1 + q], c0 = f.off[p], n = f.off[p + 1] - c0;
+        if (n <= kSegLarge)
+            filter_segment(f, p, n, a, b, id);
+        else
+            filter_segment(f, p, n, f.ga + c0, f.gb + c0, f.order + c0);
+    }
+}
+
+// Kept contacts, in sorted order per pair, to their scanned positions: a warp
+// per pair copies its 14-double records in one run.
+__global__ void k_filter_write(int n_pairs, const int32_t* __restrict__ off, const int32_t* __restrict__ order,
+                               const int32_t* __restrict__ out_off, const double* __restrict__ rec,
                                double* __restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n || !keep[j]) return;
-    const double* s = rec + 14 * (size_t)order[j];
-    double* d = out + 14 * (size_t)pos[j];
-    for (int k = 0; k < 14; k++) d[k] = s[k];
-}
-
-// flt_off[p] = pos[off[p]] for p in [0, n].
-__global__ void k_filter_offsets(int n, const int32_t* __restrict__ off, const int32_t* __restrict__ pos,
-                                 int32_t* __restrict__ out) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p <= n) out[p] = pos[off[p]];
+    const int p = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    if (p >= n_pairs) return;
+    const int o0 = out_off[p], n = 14 * (out_off[p + 1] - o0);
+    const int32_t* ids = order + off[p];
+    double* d = out + 14 * (size_t)o0;
+    for (int e = threadIdx.x & 31; e < n; e += 32) d[e] = rec[14 * (size_t)ids[e / 14] + e % 14];
 }
 
 // ---------------------------------------------------------------- solve ---
@@ -1245,16 +1365,42 @@ __global__ void __launch_bounds__(kSolveBlock) k_solve_cl(const int32_t* __restr
     solve_body<kSyncCluster>(cl_list[cid], (int)rank, (int)nrank, S, a);
 }
 
-// Sort key of Contact::operator< (contact.h:17-21) as orderable bits
-// (proportions are >= +0).
-__global__ void k_prop_keys(int n, const double* __restrict__ rec, unsigned long long* __restrict__ keys,
-                            int32_t* __restrict__ vals) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* h = rec + 14 * (size_t)i;
-    const double prop = norm(mk(h[0] - h[3], h[1] - h[4], h[2] - h[5])) / (h[6] + h[7]);
-    keys[i] = (unsigned long long)__double_as_longlong(prop);
-    vals[i] = i;
+// A cluster's contacts in the order of Contact::operator< (contact.h:17-21): by
+// |A - B| / (eps_a + eps_b), a non-negative double, ties in input order.
+struct OrderArgs {
+    const int32_t* off;
+    const double* rec;
+    u64* keys;  // global working array of the largest clusters
+    int32_t *order, *list;
+};
+__device__ void order_segment(const OrderArgs& f, int k, int n, u64* key, int32_t* id) {
+    const int c0 = f.off[k];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double* h = f.rec + 14 * (size_t)(c0 + i);
+        const double prop = norm(mk(h[0] - h[3], h[1] - h[4], h[2] - h[5])) / (h[6] + h[7]);
+        key[i] = (u64)__double_as_longlong(prop);
+        id[i] = c0 + i;
+    }
+    sort_segment<false>(n, key, nullptr, id);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) f.order[c0 + i] = id[i];
+    __syncthreads();
+}
+__global__ void __launch_bounds__(kSegSmallBlock) k_order(OrderArgs f) {
+    __shared__ u64 key[kSegSmall];
+    __shared__ int32_t id[kSegSmall];
+    const int k = blockIdx.x, n = f.off[k + 1] - f.off[k];
+    if (!leave_segment(k, n, f.list)) order_segment(f, k, n, key, id);
+}
+__global__ void __launch_bounds__(kSegLargeBlock) k_order_large(OrderArgs f) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    u64* key = (u64*)dyn;
+    for (int q = blockIdx.x; q < f.list[0]; q += gridDim.x) {
+        const int k = f.list[1 + q], c0 = f.off[k], n = f.off[k + 1] - c0;
+        if (n <= kSegLarge)
+            order_segment(f, k, n, key, (int32_t*)(key + kSegLarge));
+        else
+            order_segment(f, k, n, f.keys + c0, f.order + c0);
+    }
 }
 
 #define VLAUNCH(kern, n, ...)                                        \
@@ -1269,6 +1415,17 @@ __global__ void k_prop_keys(int n, const double* __restrict__ rec, unsigned long
 
 }  // namespace
 
+int allow_segment_smem(d2g_ctx* ctx) {
+    Engine& E = ctx->eng;
+    if (E.seg_smem_set) return D2G_OK;
+    D2G_CUDA(cudaFuncSetAttribute((const void*)k_filter_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kSegLargeSmem));
+    D2G_CUDA(cudaFuncSetAttribute((const void*)k_order_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kOrderSmem));
+    E.seg_smem_set = true;
+    return D2G_OK;
+}
+
 // Per-pair filterContacts of contact records grouped by pair (d_rec /
 // d_off over n_pairs), into flt (records) / flt_off / flt_cnt (kept per pair).
 int run_filter(d2g_ctx* ctx, const int32_t* d_off, const double* d_rec, int n_pairs, int n_rec, double margin,
@@ -1276,50 +1433,33 @@ int run_filter(d2g_ctx* ctx, const int32_t* d_off, const double* d_rec, int n_pa
     Engine& E = ctx->eng;
     cudaStream_t s = ctx->stream;
     const size_t n = (size_t)n_rec;
-    RC(E.flt_keys.ensure(n + 1));
-    RC(E.flt_keys_s.ensure(n + 1));
     RC(E.flt_idx.ensure(n + 1));
-    RC(E.flt_order.ensure(n + 1));
-    RC(E.flt_keep.ensure(n + 1));
-    RC(E.flt_pos.ensure(n + 1));
-    RC(E.flt_mid.ensure(3 * n + 3));
     RC(E.flt_cnt.ensure(n_pairs + 1));
     RC(E.flt_off.ensure(n_pairs + 1));
     if (n_rec > 0 && n_pairs > 0) {
-        // stable sort by |A - B|, then stable by eps_a + eps_b: lexicographic, ties in input order
-        VLAUNCH(k_filter_keys, n_rec, n_rec, d_rec, E.flt_keys.p, E.flt_idx.p);
-        size_t bytes = 0;
-        D2G_CUDA(cub::DeviceSegmentedSort::StableSortPairs(nullptr, bytes, E.flt_keys.p, E.flt_keys_s.p, E.flt_idx.p,
-                                                          E.flt_order.p, n_rec, n_pairs, d_off, d_off + 1, s));
-        RC(E.cub_tmp.ensure(bytes + 16));
-        D2G_CUDA(cub::DeviceSegmentedSort::StableSortPairs(E.cub_tmp.p, bytes, E.flt_keys.p, E.flt_keys_s.p,
-                                                          E.flt_idx.p, E.flt_order.p, n_rec, n_pairs, d_off,
-                                                          d_off + 1, s));
-        VLAUNCH(k_filter_eps_keys, n_rec, n_rec, d_rec, E.flt_order.p, E.flt_keys.p);
-        bytes = 0;
-        D2G_CUDA(cub::DeviceSegmentedSort::StableSortPairs(nullptr, bytes, E.flt_keys.p, E.flt_keys_s.p,
-                                                          E.flt_order.p, E.flt_idx.p, n_rec, n_pairs, d_off,
-                                                          d_off + 1, s));
-        RC(E.cub_tmp.ensure(bytes + 16));
-        D2G_CUDA(cub::DeviceSegmentedSort::StableSortPairs(E.cub_tmp.p, bytes, E.flt_keys.p, E.flt_keys_s.p,
-                                                          E.flt_order.p, E.flt_idx.p, n_rec, n_pairs, d_off,
-                                                          d_off + 1, s));
-        // E.flt_idx now holds the sorted order
-        k_filter_dedupe<<<nblocks(32LL * n_pairs), kBlock, 0, s>>>(n_pairs, d_off, E.flt_idx.p, d_rec, margin,
-                                                                    E.flt_keep.p, E.flt_cnt.p, E.flt_mid.p);
+        RC(E.flt_list.ensure(n_pairs + 1));
+        FilterArgs f{d_off, d_rec, margin, nullptr, nullptr, E.flt_idx.p, E.flt_cnt.p, E.flt_list.p};
+        if (n_rec > kSegLarge) {
+            RC(E.flt_keys.ensure(n + 1));
+            RC(E.flt_keys_s.ensure(n + 1));
+            f.ga = E.flt_keys.p;
+            f.gb = E.flt_keys_s.p;
+        }
+        D2G_CUDA(cudaMemsetAsync(E.flt_list.p, 0, sizeof(int32_t), s));
+        D2G_CUDA(cudaMemsetAsync(E.flt_cnt.p + n_pairs, 0, sizeof(int32_t), s));
+        k_filter<<<n_pairs, kSegSmallBlock, 0, s>>>(f);
         ctx->eng.launches++;
-    } else if (n_pairs > 0) {
-        D2G_CUDA(cudaMemsetAsync(E.flt_cnt.p, 0, sizeof(int32_t) * n_pairs, s));
-    }
-    RC(E.flt_keep.ensure(n + 1));
-    if (n_rec > 0) {
+        if (n_rec > kSegSmall) {  // (else no pair has more)
+            RC(allow_segment_smem(ctx));
+            k_filter_large<<<kSegLargeGrid, kSegLargeBlock, kSegLargeSmem, s>>>(f);
+            ctx->eng.launches++;
+        }
         size_t bytes = 0;
-        D2G_CUDA(cudaMemsetAsync(E.flt_pos.p, 0, sizeof(int32_t), s));
-        D2G_CUDA(cub::DeviceScan::InclusiveSum(nullptr, bytes, E.flt_keep.p, E.flt_pos.p + 1, n_rec, s));
+        D2G_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, E.flt_cnt.p, E.flt_off.p, n_pairs + 1, s));
         RC(E.cub_tmp.ensure(bytes + 16));
-        D2G_CUDA(cub::DeviceScan::InclusiveSum(E.cub_tmp.p, bytes, E.flt_keep.p, E.flt_pos.p + 1, n_rec, s));
-        VLAUNCH(k_filter_offsets, n_pairs + 1, n_pairs, d_off, E.flt_pos.p, E.flt_off.p);
+        D2G_CUDA(cub::DeviceScan::ExclusiveSum(E.cub_tmp.p, bytes, E.flt_cnt.p, E.flt_off.p, n_pairs + 1, s));
     } else {
+        if (n_pairs > 0) D2G_CUDA(cudaMemsetAsync(E.flt_cnt.p, 0, sizeof(int32_t) * n_pairs, s));
         D2G_CUDA(cudaMemsetAsync(E.flt_off.p, 0, sizeof(int32_t) * (n_pairs + 1), s));
     }
     D2G_CUDA(cudaMemcpyAsync(ctx->h_pinned, E.flt_off.p + n_pairs, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -1327,7 +1467,7 @@ int run_filter(d2g_ctx* ctx, const int32_t* d_off, const double* d_rec, int n_pa
     prof_mark_collect(ctx);
     const int kept = ctx->h_pinned[0];
     RC(E.flt.ensure(14 * (size_t)kept + 14));
-    if (n_rec > 0) VLAUNCH(k_filter_write, n_rec, n_rec, E.flt_idx.p, E.flt_keep.p, E.flt_pos.p, d_rec, E.flt.p);
+    if (kept > 0) VLAUNCH(k_filter_write, 32LL * n_pairs, n_pairs, d_off, E.flt_idx.p, E.flt_off.p, d_rec, E.flt.p);
     *n_out = kept;
     D2G_CUDA(cudaGetLastError());
     return D2G_OK;
@@ -1419,10 +1559,8 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
     Engine& E = ctx->eng;
     cudaStream_t s = ctx->stream;
     const size_t n1 = (size_t)n_con + 1, np1 = (size_t)n_parts + 1;
-    RC(E.sv_keys.ensure(n1));
-    RC(E.sv_keys_out.ensure(n1));
-    RC(E.sv_vals.ensure(n1));
     RC(E.sv_order.ensure(n1));
+    RC(E.sv_long.ensure(n_clusters + 1));
     RC(E.sv_bg_raw.ensure(sizeof(BodyG) * np1));
     RC(E.sv_bs_raw.ensure(sizeof(BodyS) * np1));
     RC(E.sv_cg_raw.ensure(sizeof(ConG) * n1));
@@ -1434,16 +1572,20 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
     RC(E.sv_tl.ensure(n_con + n_clusters + 2));
     RC(E.sv_sdelta.ensure(6 * n1));
     RC(allow_solve_smem(ctx));
-    if (n_con > 0) {
-        VLAUNCH(k_prop_keys, n_con, n_con, d_rec, E.sv_keys.p, E.sv_vals.p);
-        size_t bytes = 0;
-        D2G_CUDA(cub::DeviceSegmentedRadixSort::SortPairs(nullptr, bytes, E.sv_keys.p, E.sv_keys_out.p, E.sv_vals.p,
-                                                          E.sv_order.p, n_con, n_clusters, d_con_off, d_con_off + 1,
-                                                          0, 64, s));
-        RC(E.cub_tmp.ensure(bytes + 16));
-        D2G_CUDA(cub::DeviceSegmentedRadixSort::SortPairs(E.cub_tmp.p, bytes, E.sv_keys.p, E.sv_keys_out.p,
-                                                          E.sv_vals.p, E.sv_order.p, n_con, n_clusters, d_con_off,
-                                                          d_con_off + 1, 0, 64, s));
+    if (n_con > 0 && n_clusters > 0) {
+        OrderArgs f{d_con_off, d_rec, nullptr, E.sv_order.p, E.sv_long.p};
+        if (n_con > kSegLarge) {
+            RC(E.sv_keys.ensure(n1));
+            f.keys = E.sv_keys.p;
+        }
+        D2G_CUDA(cudaMemsetAsync(E.sv_long.p, 0, sizeof(int32_t), s));
+        k_order<<<n_clusters, kSegSmallBlock, 0, s>>>(f);
+        ctx->eng.launches++;
+        if (n_con > kSegSmall) {
+            RC(allow_segment_smem(ctx));
+            k_order_large<<<kSegLargeGrid, kSegLargeBlock, kOrderSmem, s>>>(f);
+            ctx->eng.launches++;
+        }
     }
     if (n_clusters > 0) {
         SolveArgs a;

@@ -464,3 +464,26 @@ def test_solve_sizes_match_oracle(ctx, nx, ny, nz, cluster):
         solve_against_oracle(ctx, s.copy(), s)
     finally:
         ctx.set_tuning(D.TUNE_SOLVE_CLUSTER, 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[1, 0, 2, 31, 32, 33, 64, 65, 66], [0, 1024, 1025, 1, 2047], [8192, 3, 8193]])
+def test_filter_sizes_match_oracle(ctx, sizes):
+    """Groups at the edges of the sort's warp-local steps (64), of the small
+    and large kernels' shared memory (1,024 and 8,192 contacts) and beyond;
+    equal keys in both key words, midpoints whose distance is the search
+    radius to the last bits."""
+    rng = np.random.default_rng(sum(sizes))
+    n = sum(sizes)
+    con = np.zeros((n, 14))
+    mid = rng.integers(0, 14, (n, 3)) * 0.125 + rng.uniform(-1, 1, (n, 3)) * rng.choice([0.0, 1e-16, 1e-9, 0.02], (n, 1))
+    gap = rng.choice([0.0, 0.01, 0.02], (n, 1)) * np.array([1.0, 0.0, 0.0])
+    con[:, 0:3] = mid + gap
+    con[:, 3:6] = mid - gap
+    con[:, 6:8] = rng.choice([0.125, 0.1, 0.05], (n, 1))
+    con[:, 8] = np.arange(n)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    kept, koff = ctx.filter_contacts(con, off)
+    for p in range(len(sizes)):
+        ref = np.asarray(O.filter_contacts(con[off[p]:off[p + 1]])).reshape(-1, 14)
+        assert np.array_equal(kept[koff[p]:koff[p + 1]].view(np.uint64), ref.view(np.uint64))
