@@ -373,7 +373,7 @@ __device__ __forceinline__ float vert_min(const float* a, const float* b) {
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             const float dx = a[3 * i] - b[3 * j], dy = a[3 * i + 1] - b[3 * j + 1], dz = a[3 * i + 2] - b[3 * j + 2];
-            m = fminf(m, dx * dx + dy * dy + dz * dz);
+            m = fminf(m, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
         }
     return sqrtf(m);
 }
@@ -414,17 +414,11 @@ __device__ __forceinline__ float axis_gap9(F3 d, const float* a, const float* b)
     }
     return fmaxf(b0 - a1, a0 - b1) / nn;
 }
-// A lower bound of the triangles' distance: along any direction the distance
-// is at least the gap between the projections, whatever the direction, so one
-// computed in FP32 still bounds.  Separate triangles are closest between two
-// edges, in the direction d of their closest edge pair, or between a vertex and
-// a face, along its normal.
-__device__ __forceinline__ float tri_gap(F3 d, const float* a, const float* b) {
-    const F3 na = cross3(f3(a[3] - a[0], a[4] - a[1], a[5] - a[2]), f3(a[6] - a[0], a[7] - a[1], a[8] - a[2]));
-    const F3 nb = cross3(f3(b[3] - b[0], b[4] - b[1], b[5] - b[2]), f3(b[6] - b[0], b[7] - b[1], b[8] - b[2]));
-    return fmaxf(axis_gap9(d, a, b), fmaxf(axis_gap9(na, a, b), axis_gap9(nb, a, b)));
-}
-// The same over a motion: points move on straight lines from their start to
+// A lower bound of two triangles' distance: along any direction it is at least
+// the gap between the projections, whatever the direction, so one computed in
+// FP32 still bounds.  Separate triangles are closest between two edges, in the
+// direction d of their closest edge pair, or between a vertex and a face, along
+// its normal.  Over a motion: points move on straight lines from their start to
 // their end positions, so the gap along a fixed direction is concave in time
 // and at least the smaller of the two ends'.  Bounds every distance between
 // points of the triangles at one time (every edge-edge distance of
@@ -1850,8 +1844,14 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // either.
 //
 // A warp per node pair: lanes 0-7 transform a's triangles, 8-15 b's, once each
-// into shared memory, and every lane takes two of the 64 slots (a thread per
-// slot transformed both triangles of each: 870 us of a 1,024-hull call).
+// into shared memory, with their normals; every lane takes two of the 64 slots
+// through the spheres, boxes and normals; what is left is packed onto the first
+// lanes for the edges, ~400 instructions of the ~700.  Bounded by issue (67%)
+// at 34% occupancy: 1,024 hulls' 355,000 leaf pairs 258 us, their four levels
+// 207 us (323 and 257 with the edges before the normals, two slots a lane and
+// unfused products; a thread per slot, transforming both triangles of each:
+// 870 us).  Rejecting by spheres before the other bounds are prepared, or a
+// cap of 64 registers, gained nothing.
 //
 // LEAF: the node pair's contacts are wanted; the survivors as two mask words
 // and counts.  Otherwise the pair has an inner node and emits nothing: all the
@@ -1872,6 +1872,15 @@ __device__ __forceinline__ float box_gap9(const float* a, const float* b) {
     return sqrtf(gap2);
 }
 
+// The gap along a triangle's unit normal (n: the normal, the triangle's range
+// along it) to the triangle v.
+__device__ __forceinline__ float normal_gap(const float* n, const float* v) {
+    const F3 d = f3(n[0], n[1], n[2]);
+    const float p0 = dot3(d, f3(v[0], v[1], v[2])), p1 = dot3(d, f3(v[3], v[4], v[5])),
+                p2 = dot3(d, f3(v[6], v[7], v[8]));
+    return fmaxf(fminf(p0, fminf(p1, p2)) - n[4], n[3] - fmaxf(p0, fmaxf(p1, p2)));
+}
+
 template <bool LEAF>
 __global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __restrict__ front,
                                                       const float* __restrict__ pm32, const int32_t* __restrict__ ntris,
@@ -1883,7 +1892,10 @@ __global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __rest
                                                       int32_t* __restrict__ entry_hits, int32_t* __restrict__ list,
                                                       int32_t* __restrict__ lc) {
     __shared__ float s_v[kBlock / 32][16][9];
-    __shared__ float s_c[kBlock / 32][16][7];  // centre, radius, eps, magnitude, 1 for a triangle that is a point
+    // centre, radius, eps, magnitude, 1 for a triangle that is a point, unit
+    // normal, the triangle's own range along it
+    __shared__ float s_c[kBlock / 32][16][13];
+    __shared__ uint8_t s_slot[kBlock / 32][64];
     const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     if (w >= n) return;  // uniform per warp
@@ -1909,9 +1921,9 @@ __global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __rest
 #pragma unroll
         for (int r = 0; r < 3; r++) {
             const float m0 = M[4 * r], m1 = M[4 * r + 1], m2 = M[4 * r + 2], m3 = M[4 * r + 3];
-            c[r] = m0 * sp.x + m1 * sp.y + m2 * sp.z + m3;
+            c[r] = fmaf(m0, sp.x, fmaf(m1, sp.y, fmaf(m2, sp.z, m3)));
 #pragma unroll
-            for (int k = 0; k < 3; k++) v[3 * k + r] = m0 * tv[3 * k] + m1 * tv[3 * k + 1] + m2 * tv[3 * k + 2] + m3;
+            for (int k = 0; k < 3; k++) v[3 * k + r] = fmaf(m0, tv[3 * k], fmaf(m1, tv[3 * k + 1], fmaf(m2, tv[3 * k + 2], m3)));
         }
         c[3] = sp.w;
         c[4] = eps_up[t];
@@ -1920,65 +1932,86 @@ __global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __rest
 #pragma unroll
         for (int r = 0; r < 3; r++) ext = fmaxf(ext, fmaxf(fabsf(v[3 + r] - v[r]), fabsf(v[6 + r] - v[r])));
         c[6] = ext > 1e-5f ? 0.f : 1.f;
+        F3 nn = cross3(f3(v[3] - v[0], v[4] - v[1], v[5] - v[2]), f3(v[6] - v[0], v[7] - v[1], v[8] - v[2]));
+        const float len = sqrtf(dot3(nn, nn)), inv = len > 1e-20f ? 1.f / len : 0.f;
+        nn = f3(nn.x * inv, nn.y * inv, nn.z * inv);
+        const float p0 = dot3(nn, f3(v[0], v[1], v[2])), p1 = dot3(nn, f3(v[3], v[4], v[5])),
+                    p2 = dot3(nn, f3(v[6], v[7], v[8]));
+        c[7] = nn.x;
+        c[8] = nn.y;
+        c[9] = nn.z;
+        c[10] = fminf(p0, fminf(p1, p2));
+        c[11] = fmaxf(p0, fmaxf(p1, p2));
     }
     if (lane == 0) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), na * nb);
     const float se = search[e.pair];
     const float tm = fabsf(PA[3]) + fabsf(PA[7]) + fabsf(PA[11]) + fabsf(PB[3]) + fabsf(PB[7]) + fabsf(PB[11]);
     __syncwarp();
-    bool keep[2];
-    float lim[2], room[2];
+    // the bounds that each triangle's own data give, two slots a lane
+    const int ta0 = lane >> 3, tb0 = lane & 7;
+    unsigned m[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
-        keep[h] = ta < na && tb < nb;
-        lim[h] = 0.f;
-        room[h] = -1.f;
-        if (!keep[h] || !use_bounds) continue;
-        const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb];
-        const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
-        const float thr = se + ca[4] + cb[4];
-        const float margin = 2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr);
-        lim[h] = thr + margin;
-        keep[h] = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim[h]) &&  // NaN keeps the slot
-                  !(box_gap9(s_v[wi][ta], s_v[wi][8 + tb]) > lim[h]);
-        if (keep[h] && ca[6] + cb[6] == 0.f) room[h] = thr - margin;
-    }
-    const float* va[2] = {s_v[wi][lane >> 3], s_v[wi][(lane >> 3) + 4]};
-    const float* vb = s_v[wi][8 + (lane & 7)];
-    if (!LEAF) {
-        bool sure = false;
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-            if (room[h] > 0.f) sure = sure || vert_min(va[h], vb) < room[h];
-        sure = __any_sync(0xffffffffu, sure);
-        if (lane == 0) entry_hits[w] = sure ? 1 : 0;
-        if (sure) return;
-    }
-    bool sure = false;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        if (!keep[h] || !use_bounds) continue;
-        F3 d;
-        if (edge_min(va[h], vb, d) < room[h]) {
-            sure = true;
-            if (!LEAF) break;
+        const int ta = ta0 + 4 * h;
+        bool keep = ta < na && tb0 < nb;
+        if (keep && use_bounds) {
+            const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb0], *va = s_v[wi][ta], *vb = s_v[wi][8 + tb0];
+            const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
+            const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
+            keep = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
+                   !(box_gap9(va, vb) > lim) && !(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim);
         }
-        keep[h] = !(tri_gap(d, va[h], vb) > lim[h]);
+        m[h] = __ballot_sync(0xffffffffu, keep);
     }
-    if (!LEAF && __any_sync(0xffffffffu, sure)) {
-        if (lane == 0) entry_hits[w] = 1;
-        return;
+    const int k0 = __popc(m[0]), K = k0 + __popc(m[1]);
+    if (use_bounds && K > 0) {
+        // the others, packed, a slot a lane
+        const unsigned low = (1u << lane) - 1u;
+        if ((m[0] >> lane) & 1u) s_slot[wi][__popc(m[0] & low)] = (uint8_t)lane;
+        if ((m[1] >> lane) & 1u) s_slot[wi][k0 + __popc(m[1] & low)] = (uint8_t)(32 + lane);
+        __syncwarp();
+        auto room = [&](const float* ca, const float* cb) {
+            const float thr = se + ca[4] + cb[4];
+            return ca[6] + cb[6] == 0.f ? thr - (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr)) : -1.f;
+        };
+        if (!LEAF) {
+            bool sure = false;
+            for (int k = lane; k < K; k += 32) {
+                const int ta = s_slot[wi][k] >> 3, tb = 8 + (s_slot[wi][k] & 7);
+                const float rm = room(s_c[wi][ta], s_c[wi][tb]);
+                sure = sure || (rm > 0.f && vert_min(s_v[wi][ta], s_v[wi][tb]) < rm);
+            }
+            if (__any_sync(0xffffffffu, sure)) {
+                if (lane == 0) entry_hits[w] = 1;
+                return;
+            }
+        }
+        m[0] = m[1] = 0;
+        for (int base = 0; base < K; base += 32) {
+            const int k = min(base + lane, K - 1), sl = s_slot[wi][k], ta = sl >> 3, tb = 8 + (sl & 7);
+            const float *ca = s_c[wi][ta], *cb = s_c[wi][tb], *va = s_v[wi][ta], *vb = s_v[wi][tb];
+            F3 d;
+            const float dist = edge_min(va, vb, d);
+            if (!LEAF && __any_sync(0xffffffffu, dist < room(ca, cb))) {
+                if (lane == 0) entry_hits[w] = 1;
+                return;
+            }
+            const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
+            const unsigned bit = !(axis_gap9(d, va, vb) > lim) ? 1u << (sl & 31) : 0u;
+            m[0] |= __reduce_or_sync(0xffffffffu, sl < 32 ? bit : 0u);
+            m[1] |= __reduce_or_sync(0xffffffffu, sl < 32 ? 0u : bit);
+        }
     }
+    if (!LEAF && lane == 0) entry_hits[w] = 0;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         if (LEAF) {
-            const unsigned m = __ballot_sync(0xffffffffu, keep[h]);
             if (lane == 0) {
-                mask[2 * (size_t)w + h] = m;
-                cnt[2 * (size_t)w + h] = __popc(m);
+                mask[2 * (size_t)w + h] = m[h];
+                cnt[2 * (size_t)w + h] = __popc(m[h]);
             }
         } else {
-            warp_append(64 * w + lane + 32 * h, keep[h], list, lc + LC_LIST);
+            warp_append(64 * w + lane + 32 * h, (m[h] >> lane) & 1u, list, lc + LC_LIST);
         }
     }
 }

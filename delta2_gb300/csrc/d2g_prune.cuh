@@ -35,9 +35,20 @@ D2G_HD F3 f3(float x, float y, float z) {
     return r;
 }
 D2G_HD F3 operator-(F3 a, F3 b) { return f3(a.x - b.x, a.y - b.y, a.z - b.z); }
-D2G_HD F3 fma3(F3 d, float s, F3 p) { return f3(p.x + d.x * s, p.y + d.y * s, p.z + d.z * s); }
-D2G_HD float dot3(F3 a, F3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-D2G_HD F3 cross3(F3 a, F3 b) { return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x); }
+// Fused where that saves an instruction: only a bound's quality depends on it.
+D2G_HD F3 fma3(F3 d, float s, F3 p) { return f3(fmaf(d.x, s, p.x), fmaf(d.y, s, p.y), fmaf(d.z, s, p.z)); }
+D2G_HD float dot3(F3 a, F3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
+D2G_HD F3 cross3(F3 a, F3 b) {
+    return f3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
+}
+// x / y to a few ulps.
+D2G_HD float div_fast(float x, float y) {
+#ifdef __CUDA_ARCH__
+    return __fdividef(x, y);
+#else
+    return x / y;
+#endif
+}
 D2G_HD float clampf01(float t) { return t > 0.f ? (t < 1.f ? t : 1.f) : 0.f; }  // NaN: 0
 D2G_HD F3 rel3(V3 p, V3 o) { return f3((float)(p.x - o.x), (float)(p.y - o.y), (float)(p.z - o.z)); }
 D2G_HD float maxabs3(F3 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)); }
@@ -47,9 +58,9 @@ D2G_HD float maxabs3(F3 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a
 D2G_HD F3 seg_vector(F3 S0, F3 S1, F3 E0, F3 E1, float& d2) {
     const F3 u = S1 - S0, v = E1 - E0, w = S0 - E0;
     const float a = dot3(u, u), b = dot3(u, v), c = dot3(v, v), d = dot3(u, w), e = dot3(v, w);
-    const float s = clampf01((b * e - c * d) / (a * c - b * b));
-    const float t = clampf01((b * s + e) / c);
-    const float s2 = clampf01((b * t - d) / a);
+    const float s = clampf01(div_fast(fmaf(b, e, -(c * d)), fmaf(a, c, -(b * b))));
+    const float t = clampf01(div_fast(fmaf(b, s, e), c));
+    const float s2 = clampf01(div_fast(fmaf(b, t, -d), a));
     const F3 n = fma3(v, t, E0) - fma3(u, s2, S0);
     d2 = dot3(n, n);
     return n;
