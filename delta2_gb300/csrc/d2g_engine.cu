@@ -1371,6 +1371,7 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
         auto at = [&](int pose, int i) { return mk(v[pose][i][0], v[pose][i][1], v[pose][i][2]); };
         Edge aS, aE, bS, bE;
         V3 P, Q;
+        EdgeDiv div;
         bool hit = false, open = edges && lane < 9, steady = false;
         if (open) {
             const int ia = lane / 3, ib = lane % 3, a1 = ia == 2 ? 0 : ia + 1, b1 = ib == 2 ? 0 : ib + 1;
@@ -1386,7 +1387,7 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
             // any one below the limit makes the result one
             steady = thr > 1e-6f && ee_steady(aS, aE) && ee_steady(bS, bE);
             if (steady) {
-                const double d0 = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q);
+                const double d0 = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q, div);
                 hit = d0 < lim;
                 open = !hit && !ee_gap_clear(aS, aE, bS, bE, P, Q, d0, lim);
             }
@@ -1405,13 +1406,13 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
                 Edge a = aS, b = bS;
                 for (int iter = 1; iter < kEeNewtonIters && open; iter++) {
                     const double t_prev = t;
-                    t = ee_newton_step(aS, aE, bS, bE, a, b, P, Q, t);
+                    t = ee_newton_step(aS, aE, bS, bE, a, b, P, Q, div, t);
                     if (t == t_prev || t != t) break;
                     a.A = lerp(aS.A, aE.A, t);
                     a.B = lerp(aS.B, aE.B, t);
                     b.A = lerp(bS.A, bE.A, t);
                     b.B = lerp(bS.B, bE.B, t);
-                    const double d = edge_closest(a.A, a.B, b.A, b.B, P, Q);
+                    const double d = edge_closest(a.A, a.B, b.A, b.B, P, Q, div);
                     hit = d < lim;
                     open = !hit && !ee_gap_clear(aS, aE, bS, bE, P, Q, d, lim);
                 }
@@ -1623,24 +1624,31 @@ __device__ __forceinline__ double q_lerp(double A, double B, double t) {
 }
 // components differ anywhere (vne)
 __device__ __forceinline__ bool q_ne(const Quad& q, double a, double b) {
-    const unsigned bal = __ballot_sync(q.m, q.c < 3 && a != b);
+    const unsigned bal = __ballot_sync(q.m, q.c < 3 && m_ne(a, b));
     return ((bal >> q.base) & 7u) != 0u;
 }
-// edge_constrain(A, B, pos)
-__device__ __forceinline__ double q_constrain(const Quad& q, double A, double B, double pos) {
-    const double ba = B - A;
-    const double t = q_dot(q, pos - A, ba) / q_dot(q, ba, ba);
-    return q_lerp(A, B, clamp01(t));
+// m_div_recip by the squared length of an edge (rl: its reciprocal), clamped.
+__device__ __forceinline__ double q_lerp_at(double A, double B, double n, double l, double rl) {
+    return q_lerp(A, B, clamp01(m_div_recip(n, l, rl)));
 }
-// edge_closest(SA, SB, EA, EB, P, Q): one component per lane
+// edge_closest(SA, SB, EA, EB, P, Q): one component per lane.  The squared
+// lengths of the edges and their reciprocals (one division, on different
+// lanes) serve all five divisions by them.
+struct QuadDiv {
+    double S, rS, E, rE;  // of (SA, SB) and (EA, EB)
+};
 __device__ __forceinline__ double q_edge_closest(const Quad& q, double SA, double SB, double EA, double EB, double& P,
-                                                 double& Qo) {
-    const double segDC = EB - EA;
-    const double lineDirSqrMag = q_dot(q, segDC, segDC);
+                                                 double& Qo, QuadDiv& d) {
+    const double segDC = EB - EA, segAB = SB - SA;
+    d.E = q_dot(q, segDC, segDC);
+    d.S = q_dot(q, segAB, segAB);
+    const double rl = 1.0 / ((q.c & 1) ? d.S : d.E);
+    d.rE = q_at(q, rl, 0);
+    d.rS = q_at(q, rl, 1);
     const double segAC = SA - EA;
     const double segBC = SB - EA;
     const double nA = q_dot(q, segAC, segDC), nB = q_dot(q, segBC, segDC);
-    const double s2 = ((q.c & 1) ? nB : nA) / lineDirSqrMag;  // lanes 0, 2: A; 1, 3: B
+    const double s2 = m_div_recip((q.c & 1) ? nB : nA, d.E, d.rE);  // lanes 0, 2: A; 1, 3: B
     const double sA = q_at(q, s2, 0), sB = q_at(q, s2, 1);
     const double inPlaneA = SA - sA * segDC;
     const double inPlaneB = SB - sB * segDC;
@@ -1648,12 +1656,10 @@ __device__ __forceinline__ double q_edge_closest(const Quad& q, double SA, doubl
     double t = q_dot(q, EA - inPlaneA, inPlaneBA) / q_dot(q, inPlaneBA, inPlaneBA);
     t = q_ne(q, inPlaneA, inPlaneB) ? t : 0.0;
     const double segABtoLineCD = q_lerp(SA, SB, clamp01(t));
-    const double segCDtoSegAB = q_constrain(q, EA, EB, segABtoLineCD);
-    const double segABtoSegCD = q_constrain(q, SA, SB, segCDtoSegAB);
-    Qo = segCDtoSegAB;
-    P = segABtoSegCD;
-    const double d = Qo - P;
-    return sqrt(q_dot(q, d, d));
+    Qo = q_lerp_at(EA, EB, q_dot(q, segABtoLineCD - EA, segDC), d.E, d.rE);
+    P = q_lerp_at(SA, SB, q_dot(q, Qo - SA, segAB), d.S, d.rS);
+    const double v = Qo - P;
+    return sqrt(q_dot(q, v, v));
 }
 
 // ee_coplanarity of edges (aA, aB), (bA, bB), one component per lane
@@ -1661,6 +1667,29 @@ __device__ __forceinline__ double q_coplanarity(const Quad& q, double aA, double
     const int c1 = q.c == 1 ? 2 : (q.c == 2 ? 0 : 1), c2 = q.c == 1 ? 0 : (q.c == 2 ? 1 : 2);
     const double u = aB - aA, v = bA - aA, w = bB - aA;
     return q_dot(q, w, q_at(q, u, c1) * q_at(q, v, c2) - q_at(q, u, c2) * q_at(q, v, c1));
+}
+
+// ee_cubic, one component per lane.
+__device__ __forceinline__ EeCubic q_cubic(const Quad& q, double aSA, double aSB, double bSA, double bSB, double aEA,
+                                           double aEB, double bEA, double bEB) {
+    const int c1 = q.c == 1 ? 2 : (q.c == 2 ? 0 : 1), c2 = q.c == 1 ? 0 : (q.c == 2 ? 1 : 2);
+    const double u0 = aSB - aSA, v0 = bSA - aSA, w0 = bSB - aSA;
+    const double uE = aEB - aEA, vE = bEA - aEA, wE = bEB - aEA;
+    const double u1 = uE - u0, v1 = vE - v0, w1 = wE - w0;
+    const double u01 = q_at(q, u0, c1), u02 = q_at(q, u0, c2), v01 = q_at(q, v0, c1), v02 = q_at(q, v0, c2);
+    const double u11 = q_at(q, u1, c1), u12 = q_at(q, u1, c2), v11 = q_at(q, v1, c1), v12 = q_at(q, v1, c2);
+    const double n0 = u01 * v02 - u02 * v01, n2 = u11 * v12 - u12 * v11;
+    const double n1 = (u01 * v12 - u02 * v11) + (u11 * v02 - u12 * v01);
+    auto sum = [&](double p) { return (q_at(q, p, 0) + q_at(q, p, 1)) + q_at(q, p, 2); };
+    EeCubic c;
+    c.c0 = sum(w0 * n0);
+    c.c1 = sum(w0 * n1 + w1 * n0);
+    c.c2 = sum(w0 * n2 + w1 * n1);
+    c.c3 = sum(w1 * n2);
+    const uint32_t l = max_hi3(max_hi3(0, mk(u0, v0, w0)), mk(uE, vE, wE));
+    const uint32_t m = m_max_hi(m_max_hi(max_hi3(max_hi3(0, mk(aSA, aSB, bSA)), mk(aEA, aEB, bEA)), bSB), bEB);
+    c.err = ee_cubic_err(__reduce_max_sync(q.m, m), __reduce_max_sync(q.m, l));
+    return c;
 }
 
 __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
@@ -1696,19 +1725,25 @@ __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
         double t = R[0], min_dist = R[1];
         double rP = R[2 + comp], rQ = R[5 + comp], toc = R[8];
         int iter = (int)R[9];
+        QuadDiv div;
         if (iter < 0) {  // ee_bisect
             iter = 0;
             const double dot_start = q_coplanarity(q, aSA, aSB, bSA, bSB);
+            const EeCubic cubic = q_cubic(q, aSA, aSB, bSA, bSB, aEA, aEB, bEA, bEB);
             double lo = 0.0, hi = 1.0;
             for (int k = 0; k < 20; k++) {
                 const double mid = (lo + hi) / 2.0;
-                const double dm = q_coplanarity(q, q_lerp(aSA, aEA, mid), q_lerp(aSB, aEB, mid), q_lerp(bSA, bEA, mid),
-                                                q_lerp(bSB, bEB, mid));
-                if (fabs(dm) < 1e-8) {
+                int side = ee_bisect_side(cubic.at(mid), cubic.err, dot_start);
+                if (side < 0) {
+                    const double dm = q_coplanarity(q, q_lerp(aSA, aEA, mid), q_lerp(aSB, aEB, mid),
+                                                    q_lerp(bSA, bEA, mid), q_lerp(bSB, bEB, mid));
+                    side = fabs(dm) < 1e-8 ? 1 : (dot_start * dm < 0.0 ? 2 : 0);
+                }
+                if (side == 1) {
                     lo = mid;
                     hi = mid;
                     break;
-                } else if (dot_start * dm < 0.0) {
+                } else if (side == 2) {
                     hi = mid;
                 } else {
                     lo = mid;
@@ -1716,14 +1751,14 @@ __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
             }
             toc = (lo + hi) / 2.0;
             min_dist = q_edge_closest(q, q_lerp(aSA, aEA, toc), q_lerp(aSB, aEB, toc), q_lerp(bSA, bEA, toc),
-                                      q_lerp(bSB, bEB, toc), rP, rQ);
+                                      q_lerp(bSB, bEB, toc), rP, rQ, div);
             if (!(min_dist > 1e-8)) iter = kEeNewtonIters;
         }
         for (; iter < kEeNewtonIters; iter++) {
             const double atA = q_lerp(aSA, aEA, t), atB = q_lerp(aSB, aEB, t);
             const double btA = q_lerp(bSA, bEA, t), btB = q_lerp(bSB, bEB, t);
             double P, Qv;
-            const double dist = q_edge_closest(q, atA, atB, btA, btB, P, Qv);
+            const double dist = q_edge_closest(q, atA, atB, btA, btB, P, Qv, div);
             if (dist < min_dist) {
                 min_dist = dist;
                 rP = P;
@@ -1731,18 +1766,23 @@ __global__ void __launch_bounds__(kBlock) k_ee_rest4(EeArgs a) {
                 toc = t;
             }
             // edge_project(atA, atB, P) and edge_project(btA, btB, Q), divided on lanes 0 / 1
-            const double AB = atB - atA, CD = btB - btA;
-            const double na = q_dot(q, P - atA, AB), da = q_dot(q, AB, AB);
-            const double nb = q_dot(q, Qv - btA, CD), db = q_dot(q, CD, CD);
-            const double pr = ((q.c & 1) ? nb : na) / ((q.c & 1) ? db : da);
+            const double na = q_dot(q, P - atA, atB - atA), nb = q_dot(q, Qv - btA, btB - btA);
+            const double pr = m_div_recip((q.c & 1) ? nb : na, (q.c & 1) ? div.E : div.S, (q.c & 1) ? div.rE : div.rS);
             const double pa = q_at(q, pr, 0), pb = q_at(q, pr, 1);
             // ee_newton_terms, component per lane
             const double omt = 1 - t, ompa = 1 - pa, ompb = 1 - pb, pbm1 = pb - 1;
-            const double f = ((pa * (aEB + aSB * omt) - pb * (bEB + bSB * omt)) + ompa * (aEA * t + aSA * omt)) -
-                             ompb * (bEA * t + bSA * omt);
-            const double g = ((-2 * aSB * pa + 2 * bSB * pb) + 2 * ompa * (aEA - aSA)) + 2 * (bEA - bSA) * pbm1;
-            const double h = ((-aSB * pa / 2 + bSB * pb / 2) + ompa * (aEA - aSA) / 2) + (bEA - bSA) * pbm1 / 2;
-            const double gf2 = g * f / 2, gh = g * h, ff = f * f;
+            const double f = ((pa * (aEB + aSB * omt) - pb * (bEB + bSB * omt)) + ompa * atA) - ompb * btA;
+            const double p1 = aSB * pa, p2 = bSB * pb, p3 = ompa * (aEA - aSA), p4 = (bEA - bSA) * pbm1;
+            const double G = ((p2 - p1) + p3) + p4;
+            double gf2 = G * f, gh = G * G;
+            const double ff = f * f;
+            if (__any_sync(q.m, !(m_scalable(p1) && m_scalable(p2) && m_scalable(p3) && m_scalable(p4) &&
+                                  m_scalable(gf2) && (!m_is_zero(gf2) || m_is_zero(G) || m_is_zero(f))))) {
+                const double g = ((-2 * aSB * pa + 2 * bSB * pb) + 2 * ompa * (aEA - aSA)) + 2 * (bEA - bSA) * pbm1;
+                const double h = ((-aSB * pa / 2 + bSB * pb / 2) + ompa * (aEA - aSA) / 2) + (bEA - bSA) * pbm1 / 2;
+                gf2 = g * f / 2;
+                gh = g * h;
+            }
             const double gf = (q_at(q, gf2, 0) + q_at(q, gf2, 1)) + q_at(q, gf2, 2);
             const double S = (q_at(q, ff, 0) + q_at(q, ff, 1)) + q_at(q, ff, 2);
             const double GH = (q_at(q, gh, 0) + q_at(q, gh, 1)) + q_at(q, gh, 2);

@@ -36,7 +36,12 @@ D2G_HD V3 operator-(V3 a) { return mk(-a.x, -a.y, -a.z); }
 D2G_HD V3 operator*(V3 a, double s) { return mk(a.x * s, a.y * s, a.z * s); }
 D2G_HD V3 operator*(double s, V3 a) { return mk(s * a.x, s * a.y, s * a.z); }
 D2G_HD V3 operator/(V3 a, double s) { return mk(a.x / s, a.y / s, a.z / s); }
-D2G_HD bool vne(V3 a, V3 b) { return a.x != b.x || a.y != b.y || a.z != b.z; }
+// a != b by integer instructions (an FP64 compare takes the FP64 pipe).
+D2G_HD bool m_ne(double a, double b) {
+    const uint64_t x = m_bits(a), y = m_bits(b);
+    return x == y ? (x << 1) > 0xffe0000000000000ull : ((x | y) << 1) != 0;
+}
+D2G_HD bool vne(V3 a, V3 b) { return m_ne(a.x, b.x) || m_ne(a.y, b.y) || m_ne(a.z, b.z); }
 D2G_HD double dot(V3 a, V3 b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
 D2G_HD V3 cross(V3 a, V3 b) { return mk(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x); }
 D2G_HD double norm(V3 a) { return sqrt(dot(a, a)); }
@@ -51,10 +56,12 @@ D2G_HD V3 normalized(V3 a) {
 D2G_HD double dmin(double a, double b) { return (b < a) ? b : a; }
 D2G_HD double dmax(double a, double b) { return (a < b) ? b : a; }
 D2G_HD double dclamp(double v, double lo, double hi) { return (v < lo) ? lo : ((hi < v) ? hi : v); }
+// t < 0 ? 0 : t > 1 ? 1 : t, likewise.
 D2G_HD double clamp01(double t) {
-    if (t < 0) return 0;
-    if (t > 1) return 1;
-    return t;
+    const uint64_t b = m_bits(t), m = b << 1;
+    if (m > 0xffe0000000000000ull) return t;  // NaN
+    if (b >> 63) return m ? 0.0 : t;
+    return b > 0x3ff0000000000000ull ? 1.0 : t;
 }
 D2G_HD V3 lerp(V3 A, V3 B, double t) {
     const double u = 1 - t;
@@ -413,22 +420,45 @@ D2G_HD V3 edge_constrain(V3 A, V3 B, V3 pos) {
     const double t = dot(pos - A, ba) / dot(ba, ba);
     return lerp(A, B, clamp01(t));
 }
-// common/edge.h:40-59, this = (SA,SB), other = (EA,EB)
-D2G_HD double edge_closest(V3 SA, V3 SB, V3 EA, V3 EB, V3& P_out, V3& Q_out) {
-    const V3 segDC = EB - EA;
-    const double lineDirSqrMag = dot(segDC, segDC);
+// The squared lengths edge_closest divides by, and their reciprocals.
+struct EdgeDiv {
+    double S, rS, E, rE;  // of (SA, SB) and (EA, EB)
+};
+// common/edge.h:40-59, this = (SA,SB), other = (EA,EB); m_div_recip gives the
+// bits of the divisions.
+D2G_HD double edge_closest(V3 SA, V3 SB, V3 EA, V3 EB, V3& P_out, V3& Q_out, EdgeDiv& d) {
+    const V3 segDC = EB - EA, segAB = SB - SA;
+    d.E = dot(segDC, segDC);
+    d.rE = 1.0 / d.E;
     const V3 segAC = SA - EA;
     const V3 segBC = SB - EA;
-    const V3 inPlaneA = SA - (dot(segAC, segDC) / lineDirSqrMag) * segDC;
-    const V3 inPlaneB = SB - (dot(segBC, segDC) / lineDirSqrMag) * segDC;
+    const V3 inPlaneA = SA - m_div_recip(dot(segAC, segDC), d.E, d.rE) * segDC;
+    const V3 inPlaneB = SB - m_div_recip(dot(segBC, segDC), d.E, d.rE) * segDC;
     const V3 inPlaneBA = inPlaneB - inPlaneA;
     double t = dot(EA - inPlaneA, inPlaneBA) / dot(inPlaneBA, inPlaneBA);
     t = vne(inPlaneA, inPlaneB) ? t : 0.0;
     const V3 segABtoLineCD = lerp(SA, SB, clamp01(t));
-    const V3 segCDtoSegAB = edge_constrain(EA, EB, segABtoLineCD);
-    const V3 segABtoSegCD = edge_constrain(SA, SB, segCDtoSegAB);
-    Q_out = segCDtoSegAB;
-    P_out = segABtoSegCD;
+    // edge_constrain onto (EA, EB), then back onto (SA, SB)
+    Q_out = lerp(EA, EB, clamp01(m_div_recip(dot(segABtoLineCD - EA, segDC), d.E, d.rE)));
+    d.S = dot(segAB, segAB);
+    d.rS = 1.0 / d.S;
+    P_out = lerp(SA, SB, clamp01(m_div_recip(dot(Q_out - SA, segAB), d.S, d.rS)));
+    return norm(Q_out - P_out);
+}
+D2G_HD double edge_closest(V3 SA, V3 SB, V3 EA, V3 EB, V3& P_out, V3& Q_out) {
+    const V3 segDC = EB - EA;
+    const double lineDirSqrMag = dot(segDC, segDC);
+    const double r = 1.0 / lineDirSqrMag;
+    const V3 segAC = SA - EA;
+    const V3 segBC = SB - EA;
+    const V3 inPlaneA = SA - m_div_recip(dot(segAC, segDC), lineDirSqrMag, r) * segDC;
+    const V3 inPlaneB = SB - m_div_recip(dot(segBC, segDC), lineDirSqrMag, r) * segDC;
+    const V3 inPlaneBA = inPlaneB - inPlaneA;
+    double t = dot(EA - inPlaneA, inPlaneBA) / dot(inPlaneBA, inPlaneBA);
+    t = vne(inPlaneA, inPlaneB) ? t : 0.0;
+    const V3 segABtoLineCD = lerp(SA, SB, clamp01(t));
+    Q_out = lerp(EA, EB, clamp01(m_div_recip(dot(segABtoLineCD - EA, segDC), lineDirSqrMag, r)));
+    P_out = edge_constrain(SA, SB, Q_out);
     return norm(Q_out - P_out);
 }
 D2G_HD double edge_project(V3 A, V3 B, V3 V) {
@@ -569,8 +599,13 @@ D2G_HD Ccd point_tri_ccd(V3 pt, const double* Cs, const double* Ce, const Tri& t
 
 // Newton quantities of edgeEdgeCCD (continuous_comparison.h:630-631), the
 // generated expressions restated with shared sub-expressions f, g, h.
-D2G_HD void ee_newton_terms(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE, double pa, double pb,
-                            double t, double& t_diff, double& t_diff2) {
+#ifdef __CUDA_ARCH__
+static __device__ __noinline__
+#else
+inline
+#endif
+void ee_newton_terms_plain(Edge aS, Edge aE, Edge bS, Edge bE, double pa, double pb, double t, double& t_diff,
+                           double& t_diff2) {
     const double omt = 1 - t, ompa = 1 - pa, ompb = 1 - pb, pbm1 = pb - 1;
     double gf2[3], gh[3], ff[3];
 #pragma unroll
@@ -599,6 +634,49 @@ D2G_HD void ee_newton_terms(const Edge& aS, const Edge& aE, const Edge& bS, cons
     t_diff2 = GH / sS + ((-gf) * gf) / m_pow15(S);
 }
 
+// The same with half the FP64 operations, at and bt the edges at t.  g, h and
+// the halves are the same sum at 2, 1/2 and 1 times the scale, so with
+// G = ((p2 - p1) + p3) + p4 at scale 1: g f / 2 = G f and g h = G G to the last
+// bit as long as no product is near the ends of the exponent range (otherwise
+// the plain form); and f's two interpolated points are the edges' own.
+D2G_HD void ee_newton_terms(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE, const Edge& at,
+                            const Edge& bt, double pa, double pb, double t, double& t_diff, double& t_diff2) {
+    const double omt = 1 - t, ompa = 1 - pa, ompb = 1 - pb, pbm1 = pb - 1;
+    double GF[3], GG[3], ff[3];
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double aSA = k == 0 ? aS.A.x : (k == 1 ? aS.A.y : aS.A.z);
+        const double aSB = k == 0 ? aS.B.x : (k == 1 ? aS.B.y : aS.B.z);
+        const double aEA = k == 0 ? aE.A.x : (k == 1 ? aE.A.y : aE.A.z);
+        const double aEB = k == 0 ? aE.B.x : (k == 1 ? aE.B.y : aE.B.z);
+        const double bSA = k == 0 ? bS.A.x : (k == 1 ? bS.A.y : bS.A.z);
+        const double bSB = k == 0 ? bS.B.x : (k == 1 ? bS.B.y : bS.B.z);
+        const double bEA = k == 0 ? bE.A.x : (k == 1 ? bE.A.y : bE.A.z);
+        const double bEB = k == 0 ? bE.B.x : (k == 1 ? bE.B.y : bE.B.z);
+        const double atA = k == 0 ? at.A.x : (k == 1 ? at.A.y : at.A.z);
+        const double btA = k == 0 ? bt.A.x : (k == 1 ? bt.A.y : bt.A.z);
+        const double f = ((pa * (aEB + aSB * omt) - pb * (bEB + bSB * omt)) + ompa * atA) - ompb * btA;
+        const double p1 = aSB * pa, p2 = bSB * pb, p3 = ompa * (aEA - aSA), p4 = (bEA - bSA) * pbm1;
+        const double G = ((p2 - p1) + p3) + p4;
+        GF[k] = G * f;
+        GG[k] = G * G;
+        ff[k] = f * f;
+        ok = ok && m_scalable(p1) && m_scalable(p2) && m_scalable(p3) && m_scalable(p4) && m_scalable(GF[k]) &&
+             (!m_is_zero(GF[k]) || m_is_zero(G) || m_is_zero(f));
+    }
+    if (!ok) {
+        ee_newton_terms_plain(aS, aE, bS, bE, pa, pb, t, t_diff, t_diff2);
+        return;
+    }
+    const double gf = (GF[0] + GF[1]) + GF[2];
+    const double S = (ff[0] + ff[1]) + ff[2];
+    const double sS = sqrt(S), rS = 1.0 / sS;
+    const double GH = (GG[0] + GG[1]) + GG[2];
+    t_diff = m_div_recip(gf, sS, rS);
+    t_diff2 = m_div_recip(GH, sS, rS) + ((-gf) * gf) / (S * sS);  // (m_pow15(S))
+}
+
 // The pieces of collision_detection/continuous_comparison.h:565-673
 // edgeEdgeCCD, shared by edge_edge_ccd below and the phased kernels.
 // Coplanarity triple product of two edges (:570-573).
@@ -607,21 +685,75 @@ D2G_HD double ee_coplanarity(const Edge& a, const Edge& b) {
     return dot(b.B - a.A, n);
 }
 
+// ee_coplanarity of the edges at time t.
+#ifdef __CUDA_ARCH__
+static __device__ __noinline__
+#else
+inline
+#endif
+double ee_coplanarity_at(Edge aS, Edge aE, Edge bS, Edge bE, double t) {
+    const V3 atA = lerp(aS.A, aE.A, t), atB = lerp(aS.B, aE.B, t);
+    const V3 btA = lerp(bS.A, bE.A, t), btB = lerp(bS.B, bE.B, t);
+    return dot(btB - atA, cross(atB - atA, btA - atA));
+}
+
+// The triple product as a cubic of t, for the bisection's decisions.  Points
+// move on straight lines, so it is one; cubic and ee_coplanarity_at both differ
+// from the exact value by rounding, by less than `err` together: with L above
+// every component of the three vectors at both ends and M above every
+// coordinate, 1.6e-12 L^3 for the cubic (its terms sum to at most 729 L^3), and
+// 3.6e-14 M L^2 + 3e-14 L^3 for the points interpolated at M's scale.
+struct EeCubic {
+    double c0, c1, c2, c3, err;
+    D2G_HD double at(double t) const { return m_fma(m_fma(m_fma(c3, t, c2), t, c1), t, c0); }
+};
+D2G_HD uint32_t max_hi3(uint32_t hi, V3 v) { return m_max_hi(m_max_hi(m_max_hi(hi, v.x), v.y), v.z); }
+D2G_HD double ee_cubic_err(uint32_t m, uint32_t l) {
+    const double M = m_above_hi(m), L = m_above_hi(l);
+    return (4e-12 * L + 1e-13 * M) * (L * L);
+}
+D2G_HD EeCubic ee_cubic(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE) {
+    const V3 u0 = aS.B - aS.A, v0 = bS.A - aS.A, w0 = bS.B - aS.A;
+    const V3 uE = aE.B - aE.A, vE = bE.A - aE.A, wE = bE.B - aE.A;
+    const V3 u1 = uE - u0, v1 = vE - v0, w1 = wE - w0;
+    const V3 n0 = cross(u0, v0), n1 = cross(u0, v1) + cross(u1, v0), n2 = cross(u1, v1);
+    EeCubic c;
+    c.c0 = dot(w0, n0);
+    c.c1 = dot(w0, n1) + dot(w1, n0);
+    c.c2 = dot(w0, n2) + dot(w1, n1);
+    c.c3 = dot(w1, n2);
+    const uint32_t l = max_hi3(max_hi3(max_hi3(max_hi3(max_hi3(max_hi3(0, u0), v0), w0), uE), vE), wE);
+    const uint32_t m = max_hi3(max_hi3(max_hi3(max_hi3(0, aS.A), aS.B), bS.A), bS.B);
+    c.err = ee_cubic_err(max_hi3(max_hi3(max_hi3(max_hi3(m, aE.A), aE.B), bE.A), bE.B), l);
+    return c;
+}
+// A bisection step's decision from the cubic's value p: 1 the triple product is
+// below 1e-8, 2 it has not dot_start's sign, 0 it has, -1 not certain.
+D2G_HD int ee_bisect_side(double p, double err, double dot_start) {
+    const double a = fabs(p);
+    if (a < 1e-8 - err) return 1;
+    if (a > 1e-8 + err && fabs(dot_start) > 1e-290) return (m_bits(p) ^ m_bits(dot_start)) >> 63 ? 2 : 0;
+    return -1;
+}
+
 // The bisection on a sign change of the triple product (:574-607): 20 halvings,
-// then the closest points at the middle time.  Returns the distance.
+// then the closest points at the middle time.  Returns the distance.  A
+// halving is 7 FP64 operations on the cubic instead of 60.
 D2G_HD double ee_bisect(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE, double dot_start, Ccd& r) {
+    const EeCubic cubic = ee_cubic(aS, aE, bS, bE);
     double t_lower = 0.0, t_upper = 1.0;
     for (int iter = 0; iter < 20; iter++) {
         const double t_mid = (t_lower + t_upper) / 2.0;
-        const V3 atA = lerp(aS.A, aE.A, t_mid), atB = lerp(aS.B, aE.B, t_mid);
-        const V3 btA = lerp(bS.A, bE.A, t_mid), btB = lerp(bS.B, bE.B, t_mid);
-        const V3 n_mid = cross(atB - atA, btA - atA);
-        const double dot_mid = dot(btB - atA, n_mid);
-        if (fabs(dot_mid) < 1e-8) {
+        int side = ee_bisect_side(cubic.at(t_mid), cubic.err, dot_start);
+        if (side < 0) {
+            const double dot_mid = ee_coplanarity_at(aS, aE, bS, bE, t_mid);
+            side = fabs(dot_mid) < 1e-8 ? 1 : (dot_start * dot_mid < 0.0 ? 2 : 0);
+        }
+        if (side == 1) {
             t_lower = t_mid;
             t_upper = t_mid;
             break;
-        } else if (dot_start * dot_mid < 0.0) {
+        } else if (side == 2) {
             t_upper = t_mid;
         } else {
             t_lower = t_mid;
@@ -636,13 +768,15 @@ D2G_HD double ee_bisect(const Edge& aS, const Edge& aE, const Edge& bS, const Ed
 }
 
 // The Newton step of edgeEdgeCCD (:621-637) from time t with the edges at t
-// and their closest points P, Q: t moves by -f'/f'' and is clamped to [0, 1].
+// and their closest points P, Q (d: from edge_closest(a, b)): t moves by
+// -f'/f'' and is clamped to [0, 1].
 D2G_HD double ee_newton_step(const Edge& aS, const Edge& aE, const Edge& bS, const Edge& bE, const Edge& a,
-                             const Edge& b, V3 P, V3 Q, double t) {
-    const double pa = edge_project(a.A, a.B, P);
-    const double pb = edge_project(b.A, b.B, Q);
+                             const Edge& b, V3 P, V3 Q, const EdgeDiv& d, double t) {
+    // edge_project
+    const double pa = m_div_recip(dot(P - a.A, a.B - a.A), d.S, d.rS);
+    const double pb = m_div_recip(dot(Q - b.A, b.B - b.A), d.E, d.rE);
     double td, td2;
-    ee_newton_terms(aS, aE, bS, bE, pa, pb, t, td, td2);
+    ee_newton_terms(aS, aE, bS, bE, a, b, pa, pb, t, td, td2);
     return clamp01(t - td / td2);
 }
 
@@ -657,7 +791,8 @@ D2G_HD bool ee_newton_iter(const Edge& aS, const Edge& aE, const Edge& bS, const
     const V3 atA = lerp(aS.A, aE.A, t), atB = lerp(aS.B, aE.B, t);
     const V3 btA = lerp(bS.A, bE.A, t), btB = lerp(bS.B, bE.B, t);
     V3 P, Q;
-    const double dist = edge_closest(atA, atB, btA, btB, P, Q);
+    EdgeDiv div;
+    const double dist = edge_closest(atA, atB, btA, btB, P, Q, div);
     if (dist_out) *dist_out = dist;
     if (dist < min_dist) {
         min_dist = dist;
@@ -666,7 +801,7 @@ D2G_HD bool ee_newton_iter(const Edge& aS, const Edge& aE, const Edge& bS, const
         r.toc = t;
     }
     const double t_prev = t;
-    t = ee_newton_step(aS, aE, bS, bE, Edge{atA, atB}, Edge{btA, btB}, P, Q, t);
+    t = ee_newton_step(aS, aE, bS, bE, Edge{atA, atB}, Edge{btA, btB}, P, Q, div, t);
     return t == t_prev || t != t;
 }
 

@@ -196,6 +196,27 @@ D2G_HD int m_exp_field(double v) { return (int)((m_bits(v) >> 52) & 0x7ff); }
 
 D2G_HD bool m_is_zero(double v) { return (m_bits(v) << 1) == 0; }
 
+// Zero, or within [2^-1020, 2^1018): twice and half of it are exact, and a sum
+// of a few such values is as exact at twice and at half the scale.
+D2G_HD bool m_scalable(double v) { return (unsigned)(m_exp_field(v) - 3) <= 2037u || m_is_zero(v); }
+
+// The larger of a bound on |v| kept as a high word, and v's.
+D2G_HD uint32_t m_max_hi(uint32_t hi, double v) {
+    const uint32_t h = (uint32_t)(m_bits(v) >> 32) & 0x7fffffffu;
+    return h > hi ? h : hi;
+}
+// A value above every v that went into hi (NaN or infinity if one was).
+D2G_HD double m_above_hi(uint32_t hi) {
+    const uint64_t b = (uint64_t)(hi + 1) << 32;
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)b);
+#else
+    double v;
+    std::memcpy(&v, &b, sizeof v);
+    return v;
+#endif
+}
+
 // x / y rounded to nearest, given ry = 1 / y rounded to nearest (P. W.
 // Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. Res. Dev. 34(1), 1990): q = RN(x ry) lies
@@ -205,13 +226,20 @@ D2G_HD bool m_is_zero(double v) { return (m_bits(v) << 1) == 0; }
 // r neither underflows nor overflows): for others it divides.  A zero x
 // gives q, which carries the quotient's sign.  Three FP64 operations in
 // place of a division when a divisor repeats (masses, time steps, counts).
+// (Out of line on the GPU, whose compiler hoists a division's instructions out
+// of a branch that is hardly ever taken.)
+#ifdef __CUDA_ARCH__
+static __device__ __noinline__ double m_div_out_of_line(double x, double y) { return x / y; }
+#else
+inline double m_div_out_of_line(double x, double y) { return x / y; }
+#endif
 D2G_HD double m_div_recip(double x, double y, double ry) {
     const double q = x * ry;
     const int ey = m_exp_field(y);
-    if (ey < 573 || ey > 1473) return x / y;  // |y| outside [2^-450, 2^451)
+    if (ey < 573 || ey > 1473) return m_div_out_of_line(x, y);  // |y| outside [2^-450, 2^451)
     if (m_is_zero(x)) return q;
     const int eq = m_exp_field(q);
-    if (eq < 573 || eq > 1473) return x / y;
+    if (eq < 573 || eq > 1473) return m_div_out_of_line(x, y);
 #ifdef __CUDA_ARCH__
     const double r = fma(-q, y, x);
     return fma(r, ry, q);
