@@ -86,9 +86,9 @@ __global__ void k_ccd_prep(int n, const int32_t* __restrict__ pairs, const doubl
 __global__ void k_np_prep(int n, const int32_t* __restrict__ pairs, const double* __restrict__ fut,
                           const int32_t* __restrict__ mesh, const int32_t* __restrict__ mesh_node_off,
                           const double* __restrict__ geo_eps, double* __restrict__ pm, float* __restrict__ search,
-                          Entry* __restrict__ front, float* __restrict__ pm32) {
+                          Entry* __restrict__ front, float* __restrict__ pm32, const int32_t* __restrict__ err) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
+    if (p >= n || (err && *err)) return;
     const int a = pairs[2 * p], b = pairs[2 * p + 1];
     const State fa = load_state(fut + 14 * (size_t)a);
     const State fb = load_state(fut + 14 * (size_t)b);
@@ -2182,11 +2182,10 @@ __global__ void __launch_bounds__(kBlock) k_np(int n_slots, const Entry* __restr
                                                double* __restrict__ res_eps, int32_t* __restrict__ hit,
                                                int32_t* __restrict__ entry_hits, const int32_t* __restrict__ items,
                                                int use_bounds) {
-    // Work item k tests slot items[k] (all slots when items is null); results
-    // are stored per item.
+    // Work item k tests slot items[k]; results are stored per item.
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n_slots) return;
-    const int i = items ? items[k] : k;
+    const int i = items[k];
     const Entry e = front[i >> 6];
     const int ta = (i >> 3) & 7, tb = i & 7;
     int h = 0;
@@ -2224,48 +2223,20 @@ __global__ void k_bucket_entries(int n, const int32_t* __restrict__ node_pairs, 
 }
 
 // --------------------------------------------------- finals / expansion ----
-// Final-contact flag of each result: a hit inside a leaf-leaf node pair.
-// `slot_entry` maps a result to its entry: item >> 6 through `items` when
-// given (soup stage), else the slot index >> 6 (discrete stage).
-__global__ void k_final_flags(int n, const int32_t* __restrict__ items, const Entry* __restrict__ front,
-                              const int4* __restrict__ nodes, const int32_t* __restrict__ hit,
-                              int32_t* __restrict__ flags) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int slot = items ? items[k] : k;
-    int f = 0;
-    if (hit[k]) {
-        const Entry e = front[slot >> 6];
-        f = (!ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z) ? 1 : 0;
-    }
-    flags[k] = f;
-}
-
-// Append flagged results as contact records (collision_detection/contact.h).
-__global__ void k_emit(int n, const int32_t* __restrict__ flags, const int32_t* __restrict__ off,
-                       const int32_t* __restrict__ items, int slot_shift, const Entry* __restrict__ front,
-                       const int32_t* __restrict__ tp, const int32_t* __restrict__ pairs,
-                       const PrimResult* __restrict__ res, const double* __restrict__ res_eps,
-                       const double* __restrict__ geo_eps, double* __restrict__ rec, int32_t* __restrict__ rec_pair,
-                       int base) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || !flags[k]) return;
-    const int ei = tp ? tp[k / 15] : (items ? items[k] : k) >> slot_shift;
-    const Entry e = front[ei];
-    const int a = pairs[2 * e.pair], b = pairs[2 * e.pair + 1];
-    const PrimResult& r = res[k];
-    double* o = rec + 14 * (size_t)(base + off[k]);
+// A result as a contact record (collision_detection/contact.h).
+__device__ __forceinline__ void write_record(const PrimResult& r, const double* re, int a, int b,
+                                             const double* __restrict__ geo_eps, double* __restrict__ o) {
     o[0] = r.P[0];
     o[1] = r.P[1];
     o[2] = r.P[2];
     o[3] = r.Q[0];
     o[4] = r.Q[1];
     o[5] = r.Q[2];
-    if (res_eps) {
-        o[6] = res_eps[4 * (size_t)k + 0];
-        o[7] = res_eps[4 * (size_t)k + 1];
-        o[8] = res_eps[4 * (size_t)k + 2];
-        o[9] = res_eps[4 * (size_t)k + 3];
+    if (re) {
+        o[6] = re[0];
+        o[7] = re[1];
+        o[8] = re[2];
+        o[9] = re[3];
     } else {
         o[6] = geo_eps[a];
         o[7] = geo_eps[b];
@@ -2276,44 +2247,27 @@ __global__ void k_emit(int n, const int32_t* __restrict__ flags, const int32_t* 
     o[11] = (double)a;
     o[12] = (double)b;
     o[13] = 0.0;
+}
+
+// Append flagged results as contact records.
+__global__ void k_emit(int n, const int32_t* __restrict__ flags, const int32_t* __restrict__ off,
+                       const int32_t* __restrict__ items, int slot_shift, const Entry* __restrict__ front,
+                       const int32_t* __restrict__ tp, const int32_t* __restrict__ pairs,
+                       const PrimResult* __restrict__ res, const double* __restrict__ res_eps,
+                       const double* __restrict__ geo_eps, double* __restrict__ rec, int32_t* __restrict__ rec_pair,
+                       int base) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n || !flags[k]) return;
+    const int ei = tp ? tp[k / 15] : (items ? items[k] : k) >> slot_shift;
+    const Entry e = front[ei];
+    write_record(res[k], res_eps ? res_eps + 4 * (size_t)k : nullptr, pairs[2 * e.pair], pairs[2 * e.pair + 1],
+                 geo_eps, rec + 14 * (size_t)(base + off[k]));
     rec_pair[base + off[k]] = e.pair;
 }
 
 // Expansion rule of full_tree_comparison.h:27-59: leaf-leaf keeps its hits,
 // otherwise the shallower inner side (b on ties, the inner one when the other
 // is a leaf) is replaced by its children.
-__global__ void k_expand_count(int n, const Entry* __restrict__ front, const int32_t* __restrict__ entry_hits,
-                               const int4* __restrict__ nodes, int32_t* __restrict__ cnt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int s = 0;
-    if (entry_hits[i] > 0) {
-        const int4 A = ld_node(nodes, front[i].na), B = ld_node(nodes, front[i].nb);
-        if (A.z || B.z) s = A.z && (!B.z || A.w < B.w) ? A.y : B.y;
-    }
-    cnt[i] = s;
-}
-
-__global__ void k_expand_write(int n, const Entry* __restrict__ front, const int32_t* __restrict__ entry_hits,
-                               const int4* __restrict__ nodes, const int32_t* __restrict__ off,
-                               Entry* __restrict__ next) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || entry_hits[i] <= 0) return;
-    const Entry e = front[i];
-    const int4 A = ld_node(nodes, e.na), B = ld_node(nodes, e.nb);
-    if (!A.z && !B.z) return;
-    const bool open_a = A.z && (!B.z || A.w < B.w);
-    const int4 P = open_a ? A : B;
-    Entry* o = next + off[i];
-    for (int ch = 0; ch < P.y; ch++) {
-        Entry x;
-        x.pair = e.pair;
-        x.na = open_a ? P.x + ch : e.na;
-        x.nb = open_a ? e.nb : P.x + ch;
-        *o++ = x;
-    }
-}
-
 // A level's expansion for the descents: children with an inner node to next
 // [0 ..), leaf pairs to leaf [lc[LC_LEAF] ..) (with self_leaf also a marked pair
 // of two leaves itself), in order; the totals to lc, and the level's list is
@@ -3184,7 +3138,7 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
     RC(E.pm32.ensure(24 * (size_t)n_pairs + 1));
     if (n_pairs > 0)
         LAUNCH(k_np_prep, n_pairs, n_pairs, d_pairs, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p,
-               E.pm.p, E.search.p, E.roots.p, E.pm32.p);
+               E.pm.p, E.search.p, E.roots.p, E.pm32.p, nullptr);
     int n_rec = 0, test_grid = 0;
     RC(slot_grid_size(ctx, &test_grid));
     // pair chunks, as in run_ccd
@@ -3275,7 +3229,7 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
     RC(E.pm32.ensure(25));
     RC(E.roots.ensure(2));
     LAUNCH(k_np_prep, 1, 1, d_pair, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p, E.pm.p,
-           E.search.p, E.roots.p, E.pm32.p);
+           E.search.p, E.roots.p, E.pm32.p, nullptr);
     RC(E.soup.ensure(n + 1));
     RC(E.off_a.ensure(n + 1));
     RC(E.entry_hits.ensure(n + 1));
@@ -3400,23 +3354,162 @@ __global__ void k_noalloc_validate(int n_pairs, const int32_t* __restrict__ pair
     }
 }
 
-int noalloc_read(cudaStream_t s, const int32_t* src, int32_t* dst) {
-    D2G_CUDA(cudaMemcpyAsync(dst, src, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    D2G_CUDA(cudaStreamSynchronize(s));
-    return D2G_OK;
+// A level of the allocation-free traversal in three launches and one read of
+// its sizes (before: 13 launches and copies, two reads; 8 cubes 448 us).
+// k_na_slots: 64 threads per node pair, a slot each.  They first transform the
+// two buckets' 48 vertices into shared memory, one each: transforming both
+// triangles in every slot was 216 FP64 instructions of a node pair's two
+// warps, 46 of 70 us a level of 2,048 node pairs, instead of 36.  Contacts are
+// wanted of leaf pairs only: their hits go into a mask word per warp.
+__global__ void __launch_bounds__(kBlock) k_na_slots(int n, const int32_t* __restrict__ err,
+                                                     const Entry* __restrict__ front,
+                                                     const int32_t* __restrict__ pairs, const double* __restrict__ pm,
+                                                     const int4* __restrict__ nodes,
+                                                     const int32_t* __restrict__ ntris,
+                                                     const double* __restrict__ tris, const double* __restrict__ eps,
+                                                     const double* __restrict__ inner_eps,
+                                                     const double* __restrict__ geo_eps,
+                                                     const float* __restrict__ search, PrimResult* __restrict__ res,
+                                                     double* __restrict__ res_eps, uint32_t* __restrict__ mask,
+                                                     int32_t* __restrict__ any) {
+    __shared__ double s_v[kBlock / 64][48][3];
+    const int w = (int)(blockIdx.x * (kBlock / 64) + (threadIdx.x >> 6)), l = threadIdx.x & 63;
+    const bool in = w < n && !*err;
+    Entry e{0, 0, 0};
+    int na = 0, nb = 0;
+    double(*v)[3] = s_v[threadIdx.x >> 6];
+    if (in) {
+        e = front[w];
+        na = ntris[e.na];
+        nb = ntris[e.nb];
+        const int t = l % 24 / 3, node = l < 24 ? e.na : e.nb;
+        if (l < 48 && t < (l < 24 ? na : nb)) {
+            const double* p = tris + (size_t)node * 72 + 3 * (l % 24);
+            const V3 x = xform_rigid(mk(p[0], p[1], p[2]), pm + 32 * (size_t)e.pair + (l < 24 ? 0 : 16));
+            v[l][0] = x.x;
+            v[l][1] = x.y;
+            v[l][2] = x.z;
+        }
+    }
+    __syncthreads();
+    const int ta = l >> 3, tb = l & 7;
+    bool h = false, leaf = false;
+    if (in && ta < na && tb < nb) {
+        auto at = [&](int i) { return mk(v[i][0], v[i][1], v[i][2]); };
+        const Tri A{at(3 * ta), at(3 * ta + 1), at(3 * ta + 2)};
+        const Tri B{at(24 + 3 * tb), at(24 + 3 * tb + 1), at(24 + 3 * tb + 2)};
+        const double ea = eps[(size_t)e.na * 8 + ta], eb = eps[(size_t)e.nb * 8 + tb];
+        const double thr = ((double)search[e.pair] + ea) + eb;
+        V3 P, Q;
+        const double d = tri_tri_dist_below(A, B, thr, P, Q);
+        h = d < thr;
+        leaf = !ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z;
+        if (h && leaf) {
+            const size_t k = 64 * (size_t)w + l;
+            put_result(res[k], d, P, Q, 0.0);
+            res_eps[4 * k + 0] = geo_eps[pairs[2 * e.pair]] + ea;
+            res_eps[4 * k + 1] = geo_eps[pairs[2 * e.pair + 1]] + eb;
+            res_eps[4 * k + 2] = inner_eps[(size_t)e.na * 8 + ta];
+            res_eps[4 * k + 3] = inner_eps[(size_t)e.nb * 8 + tb];
+        }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, h && leaf), hits = __ballot_sync(0xffffffffu, h);
+    if (w < n && (l & 31) == 0) {
+        mask[2 * (size_t)w + (l >> 5)] = m;
+        any[2 * (size_t)w + (l >> 5)] = hits ? 1 : 0;
+    }
 }
 
-int noalloc_scan(cudaStream_t s, void* tmp, size_t tmp_bytes, const int32_t* in, int32_t* out, int n) {
-    D2G_CUDA(cudaMemsetAsync(out, 0, sizeof(int32_t), s));
-    if (n == 0) return D2G_OK;
-    size_t need = 0;
-    D2G_CUDA(cub::DeviceScan::InclusiveSum(nullptr, need, in, out + 1, n, s));
-    if (need > tmp_bytes) {
-        set_error("allocation-free scratch: prefix-sum temporary storage too small");
-        return D2G_ERR_INVALID;
+// One block: the records' offsets and the next level's node pairs
+// (full_tree_comparison.h:27-59, as k_expand_level), both from one scan, two
+// node pairs a thread.  out: records, node pairs (written when they fit), err.
+constexpr int kNaLevel = 1024;
+__global__ void __launch_bounds__(kNaLevel) k_na_level(int n, const int32_t* __restrict__ err,
+                                                       const Entry* __restrict__ front,
+                                                       const int4* __restrict__ nodes,
+                                                       const uint32_t* __restrict__ mask,
+                                                       const int32_t* __restrict__ any, int32_t* __restrict__ off,
+                                                       Entry* __restrict__ next, int max_next,
+                                                       int32_t* __restrict__ out) {
+    static_assert(2 * kNaLevel >= D2G_NOALLOC_MAX_NODE_PAIRS, "two node pairs a thread");
+    __shared__ unsigned long long s_sum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (*err) {
+        if (threadIdx.x < 3) out[threadIdx.x] = threadIdx.x == 2 ? 1 : 0;
+        return;
     }
-    size_t avail = tmp_bytes;
-    D2G_CUDA(cub::DeviceScan::InclusiveSum(tmp, avail, in, out + 1, n, s));
+    int cnt[2][2], kids[2] = {0, 0}, first[2] = {0, 0};
+    bool open_a[2] = {false, false};
+    unsigned long long sum = 0;  // records, and node pairs in the high half
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int w = 2 * threadIdx.x + q;
+        cnt[q][0] = w < n ? __popc(mask[2 * w]) : 0;
+        cnt[q][1] = w < n ? __popc(mask[2 * w + 1]) : 0;
+        if (w < n && (any[2 * w] | any[2 * w + 1])) {
+            const int4 A = ld_node(nodes, front[w].na), B = ld_node(nodes, front[w].nb);
+            if (A.z || B.z) {
+                open_a[q] = A.z && (!B.z || A.w < B.w);
+                kids[q] = open_a[q] ? A.y : B.y;
+                first[q] = open_a[q] ? A.x : B.x;
+            }
+        }
+        sum += (unsigned long long)(cnt[q][0] + cnt[q][1]) + ((unsigned long long)kids[q] << 32);
+    }
+    unsigned long long inc = sum;
+    for (int o = 1; o < 32; o *= 2) {
+        const unsigned long long x = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += x;
+    }
+    if (lane == 31) s_sum[warp] = inc;
+    __syncthreads();
+    unsigned long long before = inc - sum, total = 0;
+    for (int i = 0; i < 32; i++) {
+        if (i < warp) before += s_sum[i];
+        total += s_sum[i];
+    }
+    const int nn = (int)(total >> 32);
+    int at = (int)(unsigned)before, to = (int)(before >> 32);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int w = 2 * threadIdx.x + q;
+        if (w >= n) break;
+        off[2 * w] = at;
+        off[2 * w + 1] = at + cnt[q][0];
+        at += cnt[q][0] + cnt[q][1];
+        if (nn > max_next) continue;
+        Entry x = front[w];
+        for (int c = 0; c < kids[q]; c++) {
+            (open_a[q] ? x.na : x.nb) = first[q] + c;
+            next[to++] = x;
+        }
+    }
+    if (threadIdx.x == 0) {
+        out[0] = (int)(unsigned)total;
+        out[1] = nn;
+        out[2] = 0;
+    }
+}
+
+__global__ void k_na_emit(int n_slots, const uint32_t* __restrict__ mask, const int32_t* __restrict__ off,
+                          const Entry* __restrict__ front, const int32_t* __restrict__ pairs,
+                          const PrimResult* __restrict__ res, const double* __restrict__ res_eps,
+                          const double* __restrict__ geo_eps, double* __restrict__ rec, int32_t* __restrict__ rec_pair,
+                          int base) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n_slots) return;
+    const uint32_t m = mask[k >> 5], bit = 1u << (k & 31);
+    if (!(m & bit)) return;
+    const int o = base + off[k >> 5] + __popc(m & (bit - 1u));
+    const Entry e = front[k >> 6];
+    write_record(res[k], res_eps + 4 * (size_t)k, pairs[2 * e.pair], pairs[2 * e.pair + 1], geo_eps,
+                 rec + 14 * (size_t)o);
+    rec_pair[o] = e.pair;
+}
+
+int noalloc_read(cudaStream_t s, const int32_t* src, int32_t* dst, int n) {
+    D2G_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    D2G_CUDA(cudaStreamSynchronize(s));
     return D2G_OK;
 }
 
@@ -3452,23 +3545,21 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
     float* search = cv.take<float>(MP);
     Entry* front = cv.take<Entry>(MN);
     Entry* next = cv.take<Entry>(MN);
-    int32_t* entry_hits = cv.take<int32_t>(MN);
-    int32_t* cnt_a = cv.take<int32_t>(MN);
-    int32_t* off_a = cv.take<int32_t>(MN + 1);
+    uint32_t* mask = cv.take<uint32_t>(2 * (size_t)MN);
+    int32_t* any = cv.take<int32_t>(2 * (size_t)MN);
+    int32_t* off = cv.take<int32_t>(2 * (size_t)MN);
     PrimResult* res = cv.take<PrimResult>(64 * (size_t)MN);
     double* res_eps = cv.take<double>(4 * 64 * (size_t)MN);
-    int32_t* hit = cv.take<int32_t>(64 * (size_t)MN);
-    int32_t* flags = cv.take<int32_t>(64 * (size_t)MN);
-    int32_t* flag_off = cv.take<int32_t>(64 * (size_t)MN + 1);
     double* rec = cv.take<double>(14 * (size_t)MR);
     int32_t* rec_pair = cv.take<int32_t>(MR);
     int32_t* rec_pair_sorted = cv.take<int32_t>(MR);
     int32_t* rec_idx = cv.take<int32_t>(MR);
     int32_t* rec_idx_sorted = cv.take<int32_t>(MR);
     int32_t* err = cv.take<int32_t>(1);
+    int32_t* out = cv.take<int32_t>(3);
     const size_t tmp_bytes = kNoAllocBytes - ((cv.used + 255) & ~(size_t)255) - 256;
     void* tmp = cv.take<unsigned char>(tmp_bytes);
-    if (!tmp || !err) {
+    if (!tmp || !err || !out) {
         set_error("allocation-free scratch layout does not fit");
         return D2G_ERR_INVALID;
     }
@@ -3479,47 +3570,41 @@ extern "C" int d2g_compare_trees_full_noalloc(const d2g_device_scene* sc, const 
     nv = nv > sc->n_meshes ? nv : sc->n_meshes;
     NA_LAUNCH(k_noalloc_validate, nv, n_pairs, d_pairs, sc->n_bodies, sc->mesh, sc->n_meshes, sc->mesh_node_off,
               sc->n_nodes, nodes, sc->ntris, err);
-    if (int rc = noalloc_read(s, err, &h_err)) return rc;
-    if (h_err) {
+    // (the kernels below do nothing once err is set: its read comes with the
+    // first level's)
+    auto refused = [&]() {
         set_error("allocation-free narrow phase: a body, mesh or node index is out of range");
         return D2G_ERR_INVALID;
-    }
-    if (n_pairs > 0)
+    };
+    if (n_pairs > 0) {
         NA_LAUNCH(k_np_prep, n_pairs, n_pairs, d_pairs, sc->fut, sc->mesh, sc->mesh_node_off, sc->geo_eps, pm, search,
-                  front, nullptr);
+                  front, nullptr, err);
+    } else {
+        if (int rc = noalloc_read(s, err, &h_err, 1)) return rc;
+        if (h_err) return refused();
+    }
     int n = n_pairs, n_rec = 0, level = 0;
     while (n > 0) {
-        if (n > MN) {
-            set_error("allocation-free narrow phase: " + std::to_string(n) + " node pairs at level " +
-                      std::to_string(level) + " exceed the limit of " + std::to_string(MN));
-            return D2G_ERR_INVALID;
-        }
-        const int n_slots = 64 * n;
-        D2G_CUDA(cudaMemsetAsync(entry_hits, 0, sizeof(int32_t) * n, s));
-        NA_LAUNCH(k_np, n_slots, n_slots, front, d_pairs, pm, sc->ntris, sc->tris, sc->eps, sc->inner_eps,
-                  sc->geo_eps, search, res, res_eps, hit, entry_hits, nullptr, 1);
-        NA_LAUNCH(k_final_flags, n_slots, n_slots, nullptr, front, nodes, hit, flags);
-        if (int rc = noalloc_scan(s, tmp, tmp_bytes, flags, flag_off, n_slots)) return rc;
-        int32_t tot = 0;
-        if (int rc = noalloc_read(s, flag_off + n_slots, &tot)) return rc;
+        NA_LAUNCH(k_na_slots, 64 * n, n, err, front, d_pairs, pm, nodes, sc->ntris, sc->tris, sc->eps, sc->inner_eps,
+                  sc->geo_eps, search, res, res_eps, mask, any);
+        k_na_level<<<1, kNaLevel, 0, s>>>(n, err, front, nodes, mask, any, off, next, MN, out);
+        int32_t got[3] = {0, 0, 0};
+        if (int rc = noalloc_read(s, out, got, 3)) return rc;
+        if (got[2]) return refused();
+        const int tot = got[0], nn = got[1];
         if (n_rec + tot > MR) {
             set_error("allocation-free narrow phase: contacts exceed the limit of " + std::to_string(MR));
             return D2G_ERR_INVALID;
         }
         if (tot > 0)
-            NA_LAUNCH(k_emit, n_slots, n_slots, flags, flag_off, nullptr, 6, front, nullptr, d_pairs, res, res_eps,
-                      sc->geo_eps, rec, rec_pair, n_rec);
+            NA_LAUNCH(k_na_emit, 64 * n, 64 * n, mask, off, front, d_pairs, res, res_eps, sc->geo_eps, rec, rec_pair,
+                      n_rec);
         n_rec += tot;
-        NA_LAUNCH(k_expand_count, n, n, front, entry_hits, nodes, cnt_a);
-        if (int rc = noalloc_scan(s, tmp, tmp_bytes, cnt_a, off_a, n)) return rc;
-        int32_t nn = 0;
-        if (int rc = noalloc_read(s, off_a + n, &nn)) return rc;
         if (nn > MN) {
             set_error("allocation-free narrow phase: " + std::to_string(nn) + " node pairs at level " +
                       std::to_string(level + 1) + " exceed the limit of " + std::to_string(MN));
             return D2G_ERR_INVALID;
         }
-        NA_LAUNCH(k_expand_write, n, n, front, entry_hits, nodes, off_a, next);
         Entry* t = front;
         front = next;
         next = t;
