@@ -380,7 +380,7 @@ int d2g_ctx_create(int32_t device, d2g_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_pinned, 64 * sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_pinned, 256 * sizeof(int32_t));
     if (e != cudaSuccess) {
         set_error(std::string("context creation: ") + cudaGetErrorString(e));
         delete c;
@@ -550,6 +550,8 @@ int d2g_ctx_set_trees(d2g_ctx* c, const d2g_trees* t) {
     D2G_CUDA(cudaStreamSynchronize(c->stream));
     c->n_meshes = t->n_meshes;
     c->n_nodes = N;
+    c->max_depth = 0;
+    for (int i = 0; i < N; i++) c->max_depth = std::max(c->max_depth, (int)t->nodes[4 * (size_t)i + 3]);
     return D2G_OK;
 }
 

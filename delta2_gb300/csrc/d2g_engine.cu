@@ -463,62 +463,66 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
     const float* __restrict__ pm32, const int32_t* __restrict__ ntris, const double* __restrict__ tris,
     const float* __restrict__ tri32, const double* __restrict__ geo_eps, const float* __restrict__ search,
     const int4* __restrict__ nodes, const uint8_t* __restrict__ skip, const uint8_t* __restrict__ eskip,
-    int use_bounds, int32_t* __restrict__ entry_hits, int32_t* __restrict__ list, int32_t* __restrict__ lc) {
+    int use_bounds, int32_t* __restrict__ entry_hits, int32_t* __restrict__ list, int32_t* __restrict__ lc,
+    const int32_t* __restrict__ n_dev) {
     __shared__ float s_verts[kBlock / 32][16][9];
     __shared__ float s_ends[kBlock / 32][16][9];
     __shared__ float s_mag[kBlock / 32][16];
-    const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    if (w >= n_soup) return;  // uniform per warp
-    const Entry e = soup[w];
-    // a pair the root certificate proved contact-free, or a node pair its
-    // separation witness proved clear: no slot goes on
-    if ((skip && skip[e.pair]) || (eskip && eskip[w])) {
-        if (lane == 0) entry_hits[w] = 0;
-        return;
-    }
-    int res[2];
-    swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, s_verts[wi], s_ends[wi], s_mag[wi]);
-    const int k = __popc(__ballot_sync(0xffffffffu, res[0])) + __popc(__ballot_sync(0xffffffffu, res[1]));
-    if (lane == 0 && k) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), k);
-    bool sure = false;
-    if (ld_node(nodes, e.na).z || ld_node(nodes, e.nb).z) {
+    if (n_dev) n_soup = *n_dev;
+    for (int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); w < n_soup;  // uniform per warp
+         w += (int)((gridDim.x * (size_t)blockDim.x) >> 5)) {
         __syncwarp();
-        const float thr = search[e.pair];
-        float room[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
-            room[h] = -1.f;
-            if (!res[h] || !use_bounds || !(thr > 1e-6f)) continue;
-            room[h] = thr - (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
-            sure = sure || vert_min(s_verts[wi][ta], s_verts[wi][8 + tb]) < room[h];
+        const Entry e = soup[w];
+        // a pair the root certificate proved contact-free, or a node pair its
+        // separation witness proved clear: no slot goes on
+        if ((skip && skip[e.pair]) || (eskip && eskip[w])) {
+            if (lane == 0) entry_hits[w] = 0;
+            continue;
         }
-        sure = __any_sync(0xffffffffu, sure);
-        if (!sure) {
-            bool clear[2] = {false, false};
+        int res[2];
+        swept_slots(e, pairs, pm, pm32, ntris, tris, tri32, geo_eps, res, s_verts[wi], s_ends[wi], s_mag[wi]);
+        const int k = __popc(__ballot_sync(0xffffffffu, res[0])) + __popc(__ballot_sync(0xffffffffu, res[1]));
+        if (lane == 0 && k) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), k);
+        bool sure = false;
+        if (ld_node(nodes, e.na).z || ld_node(nodes, e.nb).z) {
+            __syncwarp();
+            const float thr = search[e.pair];
+            float room[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
-                if (!res[h] || !use_bounds) continue;
-                F3 d;
-                const float m = edge_min(s_verts[wi][ta], s_verts[wi][8 + tb], d);
-                if (m < room[h]) sure = true;
-                // (s_mag is huge for an unsteady triangle: never clear either)
-                clear[h] = tri_gap_motion(d, s_verts[wi][ta], s_verts[wi][8 + tb], s_ends[wi][ta],
-                                          s_ends[wi][8 + tb]) >
-                           thr + (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
+                room[h] = -1.f;
+                if (!res[h] || !use_bounds || !(thr > 1e-6f)) continue;
+                room[h] = thr - (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
+                sure = sure || vert_min(s_verts[wi][ta], s_verts[wi][8 + tb]) < room[h];
             }
             sure = __any_sync(0xffffffffu, sure);
             if (!sure) {
-                warp_append((64 * w + lane) | (clear[0] ? kEdgesClear : 0), res[0] != 0, list, lc + LC_LIST);
-                warp_append((64 * w + lane + 32) | (clear[1] ? kEdgesClear : 0), res[1] != 0, list, lc + LC_LIST);
+                bool clear[2] = {false, false};
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int sl = lane + 32 * h, ta = sl >> 3, tb = sl & 7;
+                    if (!res[h] || !use_bounds) continue;
+                    F3 d;
+                    const float m = edge_min(s_verts[wi][ta], s_verts[wi][8 + tb], d);
+                    if (m < room[h]) sure = true;
+                    // (s_mag is huge for an unsteady triangle: never clear either)
+                    clear[h] = tri_gap_motion(d, s_verts[wi][ta], s_verts[wi][8 + tb], s_ends[wi][ta],
+                                              s_ends[wi][8 + tb]) >
+                               thr + (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
+                }
+                sure = __any_sync(0xffffffffu, sure);
+                if (!sure) {
+                    warp_append((64 * w + lane) | (clear[0] ? kEdgesClear : 0), res[0] != 0, list, lc + LC_LIST);
+                    warp_append((64 * w + lane + 32) | (clear[1] ? kEdgesClear : 0), res[1] != 0, list, lc + LC_LIST);
+                }
             }
+        } else if (lane == 0 && k) {
+            atomicAdd(lc + LC_ROOT, 1);
         }
-    } else if (lane == 0 && k) {
-        atomicAdd(lc + LC_ROOT, 1);
+        if (lane == 0) entry_hits[w] = sure ? 1 : 0;
     }
-    if (lane == 0) entry_hits[w] = sure ? 1 : 0;
 }
 
 // The swept-box flags of the root node pairs that are two leaves (the soup
@@ -1922,7 +1926,7 @@ __device__ __forceinline__ float normal_gap(const float* n, const float* v) {
 }
 
 template <bool LEAF>
-__global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __restrict__ front,
+__global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const Entry* __restrict__ front,
                                                       const float* __restrict__ pm32, const int32_t* __restrict__ ntris,
                                                       const float4* __restrict__ sph, const float* __restrict__ tri32,
                                                       const float* __restrict__ eps_up,
@@ -1930,129 +1934,138 @@ __global__ void __launch_bounds__(kBlock) k_np_filter(int n, const Entry* __rest
                                                       const int4* __restrict__ nodes, int use_bounds,
                                                       uint32_t* __restrict__ mask, int32_t* __restrict__ cnt,
                                                       int32_t* __restrict__ entry_hits, int32_t* __restrict__ list,
-                                                      int32_t* __restrict__ lc) {
+                                                      int32_t* __restrict__ lc, const int32_t* __restrict__ n_dev) {
     __shared__ float s_v[kBlock / 32][16][9];
     // centre, radius, eps, magnitude, 1 for a triangle that is a point, unit
     // normal, the triangle's own range along it
     __shared__ float s_c[kBlock / 32][16][13];
     __shared__ uint8_t s_slot[kBlock / 32][64];
-    const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    if (w >= n) return;  // uniform per warp
-    const Entry e = front[w];
-    if (!LEAF && !ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z) {
-        // a root pair of two leaves goes onto the list of leaf pairs as it is
-        if (lane == 0) {
-            entry_hits[w] = 1;
-            atomicAdd(lc + LC_ROOT, 1);
-        }
-        return;
-    }
-    const int na = ntris[e.na], nb = ntris[e.nb];
-    const float* PA = pm32 + 24 * (size_t)e.pair;
-    const float* PB = PA + 12;
-    if (lane < 16 && (lane & 7) < (lane < 8 ? na : nb)) {
-        const size_t t = (size_t)(lane < 8 ? e.na : e.nb) * 8 + (lane & 7);
-        const float* M = lane < 8 ? PA : PB;
-        const float* tv = tri32 + t * 9;
-        float* v = s_v[wi][lane];
-        float* c = s_c[wi][lane];
-        const float4 sp = sph[t];
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            const float m0 = M[4 * r], m1 = M[4 * r + 1], m2 = M[4 * r + 2], m3 = M[4 * r + 3];
-            c[r] = fmaf(m0, sp.x, fmaf(m1, sp.y, fmaf(m2, sp.z, m3)));
-#pragma unroll
-            for (int k = 0; k < 3; k++) v[3 * k + r] = fmaf(m0, tv[3 * k], fmaf(m1, tv[3 * k + 1], fmaf(m2, tv[3 * k + 2], m3)));
-        }
-        c[3] = sp.w;
-        c[4] = eps_up[t];
-        c[5] = fabsf(sp.x) + fabsf(sp.y) + fabsf(sp.z) + sp.w;
-        float ext = 0.f;
-#pragma unroll
-        for (int r = 0; r < 3; r++) ext = fmaxf(ext, fmaxf(fabsf(v[3 + r] - v[r]), fabsf(v[6 + r] - v[r])));
-        c[6] = ext > 1e-5f ? 0.f : 1.f;
-        F3 nn = cross3(f3(v[3] - v[0], v[4] - v[1], v[5] - v[2]), f3(v[6] - v[0], v[7] - v[1], v[8] - v[2]));
-        const float len = sqrtf(dot3(nn, nn)), inv = len > 1e-20f ? 1.f / len : 0.f;
-        nn = f3(nn.x * inv, nn.y * inv, nn.z * inv);
-        const float p0 = dot3(nn, f3(v[0], v[1], v[2])), p1 = dot3(nn, f3(v[3], v[4], v[5])),
-                    p2 = dot3(nn, f3(v[6], v[7], v[8]));
-        c[7] = nn.x;
-        c[8] = nn.y;
-        c[9] = nn.z;
-        c[10] = fminf(p0, fminf(p1, p2));
-        c[11] = fmaxf(p0, fmaxf(p1, p2));
-    }
-    if (lane == 0) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), na * nb);
-    const float se = search[e.pair];
-    const float tm = fabsf(PA[3]) + fabsf(PA[7]) + fabsf(PA[11]) + fabsf(PB[3]) + fabsf(PB[7]) + fabsf(PB[11]);
-    __syncwarp();
-    // the bounds that each triangle's own data give, two slots a lane
-    const int ta0 = lane >> 3, tb0 = lane & 7;
-    unsigned m[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int ta = ta0 + 4 * h;
-        bool keep = ta < na && tb0 < nb;
-        if (keep && use_bounds) {
-            const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb0], *va = s_v[wi][ta], *vb = s_v[wi][8 + tb0];
-            const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
-            const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
-            keep = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
-                   !(box_gap9(va, vb) > lim) && !(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim);
-        }
-        m[h] = __ballot_sync(0xffffffffu, keep);
-    }
-    const int k0 = __popc(m[0]), K = k0 + __popc(m[1]);
-    if (use_bounds && K > 0) {
-        // the others, packed, a slot a lane
-        const unsigned low = (1u << lane) - 1u;
-        if ((m[0] >> lane) & 1u) s_slot[wi][__popc(m[0] & low)] = (uint8_t)lane;
-        if ((m[1] >> lane) & 1u) s_slot[wi][k0 + __popc(m[1] & low)] = (uint8_t)(32 + lane);
+    if (!LEAF && n_dev) n = *n_dev;
+    for (int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); w < n;  // uniform per warp
+         w += (int)((gridDim.x * (size_t)blockDim.x) >> 5)) {
         __syncwarp();
-        auto room = [&](const float* ca, const float* cb) {
-            const float thr = se + ca[4] + cb[4];
-            return ca[6] + cb[6] == 0.f ? thr - (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr)) : -1.f;
-        };
-        if (!LEAF) {
-            bool sure = false;
-            for (int k = lane; k < K; k += 32) {
-                const int ta = s_slot[wi][k] >> 3, tb = 8 + (s_slot[wi][k] & 7);
-                const float rm = room(s_c[wi][ta], s_c[wi][tb]);
-                sure = sure || (rm > 0.f && vert_min(s_v[wi][ta], s_v[wi][tb]) < rm);
-            }
-            if (__any_sync(0xffffffffu, sure)) {
-                if (lane == 0) entry_hits[w] = 1;
-                return;
-            }
-        }
-        m[0] = m[1] = 0;
-        for (int base = 0; base < K; base += 32) {
-            const int k = min(base + lane, K - 1), sl = s_slot[wi][k], ta = sl >> 3, tb = 8 + (sl & 7);
-            const float *ca = s_c[wi][ta], *cb = s_c[wi][tb], *va = s_v[wi][ta], *vb = s_v[wi][tb];
-            F3 d;
-            const float dist = edge_min(va, vb, d);
-            if (!LEAF && __any_sync(0xffffffffu, dist < room(ca, cb))) {
-                if (lane == 0) entry_hits[w] = 1;
-                return;
-            }
-            const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
-            const unsigned bit = !(axis_gap9(d, va, vb) > lim) ? 1u << (sl & 31) : 0u;
-            m[0] |= __reduce_or_sync(0xffffffffu, sl < 32 ? bit : 0u);
-            m[1] |= __reduce_or_sync(0xffffffffu, sl < 32 ? 0u : bit);
-        }
-    }
-    if (!LEAF && lane == 0) entry_hits[w] = 0;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        if (LEAF) {
+        const Entry e = front[w];
+        if (!LEAF && !ld_node(nodes, e.na).z && !ld_node(nodes, e.nb).z) {
+            // a root pair of two leaves goes onto the list of leaf pairs as it is
             if (lane == 0) {
-                mask[2 * (size_t)w + h] = m[h];
-                cnt[2 * (size_t)w + h] = __popc(m[h]);
+                entry_hits[w] = 1;
+                atomicAdd(lc + LC_ROOT, 1);
             }
-        } else {
-            warp_append(64 * w + lane + 32 * h, (m[h] >> lane) & 1u, list, lc + LC_LIST);
+            continue;
         }
+        const int na = ntris[e.na], nb = ntris[e.nb];
+        const float* PA = pm32 + 24 * (size_t)e.pair;
+        const float* PB = PA + 12;
+        if (lane < 16 && (lane & 7) < (lane < 8 ? na : nb)) {
+            const size_t t = (size_t)(lane < 8 ? e.na : e.nb) * 8 + (lane & 7);
+            const float* M = lane < 8 ? PA : PB;
+            const float* tv = tri32 + t * 9;
+            float* v = s_v[wi][lane];
+            float* c = s_c[wi][lane];
+            const float4 sp = sph[t];
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const float m0 = M[4 * r], m1 = M[4 * r + 1], m2 = M[4 * r + 2], m3 = M[4 * r + 3];
+                c[r] = fmaf(m0, sp.x, fmaf(m1, sp.y, fmaf(m2, sp.z, m3)));
+#pragma unroll
+                for (int k = 0; k < 3; k++) v[3 * k + r] = fmaf(m0, tv[3 * k], fmaf(m1, tv[3 * k + 1], fmaf(m2, tv[3 * k + 2], m3)));
+            }
+            c[3] = sp.w;
+            c[4] = eps_up[t];
+            c[5] = fabsf(sp.x) + fabsf(sp.y) + fabsf(sp.z) + sp.w;
+            float ext = 0.f;
+#pragma unroll
+            for (int r = 0; r < 3; r++) ext = fmaxf(ext, fmaxf(fabsf(v[3 + r] - v[r]), fabsf(v[6 + r] - v[r])));
+            c[6] = ext > 1e-5f ? 0.f : 1.f;
+            F3 nn = cross3(f3(v[3] - v[0], v[4] - v[1], v[5] - v[2]), f3(v[6] - v[0], v[7] - v[1], v[8] - v[2]));
+            const float len = sqrtf(dot3(nn, nn)), inv = len > 1e-20f ? 1.f / len : 0.f;
+            nn = f3(nn.x * inv, nn.y * inv, nn.z * inv);
+            const float p0 = dot3(nn, f3(v[0], v[1], v[2])), p1 = dot3(nn, f3(v[3], v[4], v[5])),
+                        p2 = dot3(nn, f3(v[6], v[7], v[8]));
+            c[7] = nn.x;
+            c[8] = nn.y;
+            c[9] = nn.z;
+            c[10] = fminf(p0, fminf(p1, p2));
+            c[11] = fmaxf(p0, fmaxf(p1, p2));
+        }
+        if (lane == 0) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), na * nb);
+        const float se = search[e.pair];
+        const float tm = fabsf(PA[3]) + fabsf(PA[7]) + fabsf(PA[11]) + fabsf(PB[3]) + fabsf(PB[7]) + fabsf(PB[11]);
+        __syncwarp();
+        // the bounds that each triangle's own data give, two slots a lane
+        const int ta0 = lane >> 3, tb0 = lane & 7;
+        unsigned m[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int ta = ta0 + 4 * h;
+            bool keep = ta < na && tb0 < nb;
+            if (keep && use_bounds) {
+                const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb0], *va = s_v[wi][ta], *vb = s_v[wi][8 + tb0];
+                const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
+                const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
+                keep = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
+                       !(box_gap9(va, vb) > lim) && !(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim);
+            }
+            m[h] = __ballot_sync(0xffffffffu, keep);
+        }
+        const int k0 = __popc(m[0]), K = k0 + __popc(m[1]);
+        if (use_bounds && K > 0) {
+            // the others, packed, a slot a lane
+            const unsigned low = (1u << lane) - 1u;
+            if ((m[0] >> lane) & 1u) s_slot[wi][__popc(m[0] & low)] = (uint8_t)lane;
+            if ((m[1] >> lane) & 1u) s_slot[wi][k0 + __popc(m[1] & low)] = (uint8_t)(32 + lane);
+            __syncwarp();
+            auto room = [&](const float* ca, const float* cb) {
+                const float thr = se + ca[4] + cb[4];
+                return ca[6] + cb[6] == 0.f ? thr - (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr)) : -1.f;
+            };
+            if (!LEAF) {
+                bool sure = false;
+                for (int k = lane; k < K; k += 32) {
+                    const int ta = s_slot[wi][k] >> 3, tb = 8 + (s_slot[wi][k] & 7);
+                    const float rm = room(s_c[wi][ta], s_c[wi][tb]);
+                    sure = sure || (rm > 0.f && vert_min(s_v[wi][ta], s_v[wi][tb]) < rm);
+                }
+                if (__any_sync(0xffffffffu, sure)) {
+                    if (lane == 0) entry_hits[w] = 1;
+                    continue;
+                }
+            }
+            m[0] = m[1] = 0;
+            bool sure = false;
+            for (int base = 0; base < K; base += 32) {
+                const int k = min(base + lane, K - 1), sl = s_slot[wi][k], ta = sl >> 3, tb = 8 + (sl & 7);
+                const float *ca = s_c[wi][ta], *cb = s_c[wi][tb], *va = s_v[wi][ta], *vb = s_v[wi][tb];
+                F3 d;
+                const float dist = edge_min(va, vb, d);
+                if (!LEAF && __any_sync(0xffffffffu, dist < room(ca, cb))) {
+                    sure = true;
+                    break;
+                }
+                const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
+                const unsigned bit = !(axis_gap9(d, va, vb) > lim) ? 1u << (sl & 31) : 0u;
+                m[0] |= __reduce_or_sync(0xffffffffu, sl < 32 ? bit : 0u);
+                m[1] |= __reduce_or_sync(0xffffffffu, sl < 32 ? 0u : bit);
+            }
+            if (!LEAF && sure) {
+                if (lane == 0) entry_hits[w] = 1;
+                continue;
+            }
+        }
+        if (!LEAF && lane == 0) entry_hits[w] = 0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (LEAF) {
+                if (lane == 0) {
+                    mask[2 * (size_t)w + h] = m[h];
+                    cnt[2 * (size_t)w + h] = __popc(m[h]);
+                }
+            } else {
+                warp_append(64 * w + lane + 32 * h, (m[h] >> lane) & 1u, list, lc + LC_LIST);
+            }
+        }
+        if (LEAF) break;  // a warp a node pair
     }
 }
 
@@ -2269,9 +2282,10 @@ __global__ void k_emit(int n, const int32_t* __restrict__ flags, const int32_t* 
 // otherwise the shallower inner side (b on ties, the inner one when the other
 // is a leaf) is replaced by its children.
 // A level's expansion for the descents: children with an inner node to next
-// [0 ..), leaf pairs to leaf [lc[LC_LEAF] ..) (with self_leaf also a marked pair
-// of two leaves itself), in order; the totals to lc, and the level's list is
-// emptied for the next one.  A thread per node pair.  Up to kExpandOneBlock
+// [0 ..), leaf pairs to leaf [leaf0 ..) (with self_leaf also a marked pair of
+// two leaves itself), in order; the totals to lc.  prev: the counters of the
+// level before, when the host does not know them yet (n and leaf0 are its
+// totals, the launch is for a bound).  A thread per node pair.  Up to kExpandOneBlock
 // node pairs one block does it all; larger levels take two launches,
 // k_expand_sums for the blocks' totals and k_expand_level, whose blocks add up
 // the totals before theirs (three launches and a library scan before).
@@ -2334,7 +2348,9 @@ __device__ __forceinline__ int2 block_scan2(int s, int c, int2& total) {
 __global__ void __launch_bounds__(kExpandThreads) k_expand_sums(int n, const Entry* __restrict__ front,
                                                                 const int32_t* __restrict__ entry_hits,
                                                                 const int4* __restrict__ nodes, int self_leaf,
-                                                                int2* __restrict__ sums) {
+                                                                int2* __restrict__ sums,
+                                                                const int32_t* __restrict__ prev) {
+    if (prev) n = prev[LC_NEXT];
     const int i = blockIdx.x * kExpandThreads + threadIdx.x;
     Opened o;
     int s = 0, c = 0;
@@ -2352,7 +2368,12 @@ __global__ void __launch_bounds__(THREADS) k_expand_level(int n, const Entry* __
                                                                  const int4* __restrict__ nodes, int self_leaf,
                                                                  const int2* __restrict__ sums,
                                                                  Entry* __restrict__ next, Entry* __restrict__ leaf,
-                                                                 int leaf0, int32_t* __restrict__ lc) {
+                                                                 int leaf0, int32_t* __restrict__ lc,
+                                                                 const int32_t* __restrict__ prev) {
+    if (prev) {
+        n = prev[LC_NEXT];
+        leaf0 = prev[LC_LEAF];
+    }
     int2 base = make_int2(0, leaf0);
     if (sums) {  // the blocks before this one
         int s = 0, c = 0;
@@ -2365,8 +2386,9 @@ __global__ void __launch_bounds__(THREADS) k_expand_level(int n, const Entry* __
         base.x += total.x;
         base.y += total.y;
     }
-    const int step = sums ? n : THREADS;  // one block walks the level, else one pass
-    for (int i0 = sums ? blockIdx.x * THREADS : 0; i0 < n; i0 += step) {
+    // one block walks the level, else one pass (with n from the device some
+    // blocks have nothing)
+    for (int i0 = sums ? blockIdx.x * THREADS : 0; i0 < n; i0 += sums ? INT32_MAX / 2 : THREADS) {
         const int i = i0 + threadIdx.x;
         Opened o;
         int s = 0, c = 0;
@@ -2394,7 +2416,6 @@ __global__ void __launch_bounds__(THREADS) k_expand_level(int n, const Entry* __
         base.y += total.y;
     }
     if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) {
-        lc[LC_LIST] = 0;
         lc[LC_NEXT] = base.x;
         lc[LC_LEAF] = base.y;
     }
@@ -2763,14 +2784,25 @@ struct Traversal {
 // Descends from the n node pairs in E.soup: per level `decide` marks the node
 // pairs with a hit in E.entry_hits, and their children go to the next level
 // or, two leaves, onto E.conn (with self_leaf also marked root pairs that are
-// two leaves).  One read of the counts per level.
+// two leaves).
+//
+// Reading a level's counts drains the GPU for the launches of the next (~30 us
+// a level of an icosphere descent's 8), so up to kAhead levels are launched per
+// read: for the first the host knows the node pairs, the others take the count
+// from the level before on the device and are launched for a bound, eight
+// children a node pair.  Levels run ahead only while the bound is below
+// kAheadPairs, whose buffers (~2.4 KB a node pair) fit the budget, and while
+// the meshes' depths allow another level; levels above are long enough to
+// hide the read.  decide gets the level's bound, its counters and, running
+// ahead, where its count is.
+constexpr int kAhead = 4, kAheadPairs = 1 << 16;
 template <class F>
 int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon, Traversal& T, F decide) {
     Engine& E = ctx->eng;
     cudaStream_t s = ctx->stream;
-    RC(E.lc.ensure(LC_SIZE));
-    D2G_CUDA(cudaMemsetAsync(E.lc.p, 0, sizeof(int32_t) * LC_SIZE, s));
+    RC(E.lc.ensure(kAhead * LC_SIZE));
     int new_leaf = 0;
+    const int max_levels = 2 * ctx->max_depth;  // a level opens one side, and stops at two leaves
     while (n > 0) {
         // past the budget (768 bytes a node pair: its slot list and its
         // children), or past 32-bit slot indices (64 slots per node pair)
@@ -2779,46 +2811,71 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
             T.abandon = true;
             return D2G_OK;
         }
-        T.peak = std::max(T.peak, need / budget);
-        T.levels++;
-        T.nodes += n;
-        RC(E.entry_hits.ensure(n + 1));
-        RC(decide(n));
-        RC(E.soup_next.ensure(8 * (size_t)n + 1));  // a node has at most 8 children
-        RC(E.conn.ensure_keep((size_t)T.n_leaf + 8 * (size_t)n + 1, (size_t)T.n_leaf, s));
-        const bool one = n <= kExpandOneBlock;
-        const int blocks = one ? 1 : nblocks(n, kExpandThreads);
-        if (!one) {
-            RC(E.sums.ensure(2 * (size_t)blocks));
-            k_expand_sums<<<blocks, kExpandThreads, 0, s>>>(n, E.soup.p, E.entry_hits.p, ctx->nodes.p,
-                                                            self_leaf ? 1 : 0, (int2*)E.sums.p);
-            E.launches++;
+        // (profiling counts slots, witnesses keep a table a level)
+        const int most = E.profiling || E.witnesses ? 1 : std::min<int64_t>(kAhead, max_levels - T.levels);
+        int bound[kAhead] = {n}, K = 1;
+        for (; K < most; K++) {
+            const long long b = 8LL * bound[K - 1];
+            if (b > kAheadPairs || 2400.0 * 1.5 * (double)b > budget) break;
+            bound[K] = (int)b;
         }
-        if (one)
-            k_expand_level<kExpandOneThreads><<<1, kExpandOneThreads, 0, s>>>(
-                n, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0, nullptr, E.soup_next.p, E.conn.p,
-                T.n_leaf, E.lc.p);
-        else
-            k_expand_level<kExpandThreads><<<blocks, kExpandThreads, 0, s>>>(
-                n, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0, (const int2*)E.sums.p, E.soup_next.p,
-                E.conn.p, T.n_leaf, E.lc.p);
-        E.launches++;
-        D2G_CUDA(cudaMemcpyAsync(ctx->h_pinned, E.lc.p, sizeof(int32_t) * LC_SIZE, cudaMemcpyDeviceToHost, s));
+        const size_t top = (size_t)bound[K - 1];
+        size_t leaves = (size_t)T.n_leaf + 1;
+        for (int k = 0; k < K; k++) leaves += 8 * (size_t)bound[k];  // a node has at most 8 children
+        RC(E.entry_hits.ensure(top + 1));
+        RC(E.ccd_list.ensure(64 * top));
+        RC(E.soup_next.ensure(8 * top + 1));
+        RC(E.soup.ensure_keep(K > 1 ? 8 * top + 1 : (size_t)n + 1, (size_t)n, s));
+        RC(E.conn.ensure_keep(leaves, (size_t)T.n_leaf, s));
+        D2G_CUDA(cudaMemsetAsync(E.lc.p, 0, sizeof(int32_t) * LC_SIZE * K, s));
+        for (int k = 0; k < K; k++) {
+            int32_t* lc = E.lc.p + k * LC_SIZE;
+            const int32_t* prev = k ? lc - LC_SIZE : nullptr;
+            const int m = bound[k];
+            RC(decide(m, lc, k ? prev + LC_NEXT : nullptr));
+            const bool one = m <= kExpandOneBlock;
+            const int blocks = one ? 1 : nblocks(m, kExpandThreads);
+            if (!one) {
+                RC(E.sums.ensure(2 * (size_t)blocks));
+                k_expand_sums<<<blocks, kExpandThreads, 0, s>>>(m, E.soup.p, E.entry_hits.p, ctx->nodes.p,
+                                                                self_leaf ? 1 : 0, (int2*)E.sums.p, prev);
+                E.launches++;
+            }
+            if (one)
+                k_expand_level<kExpandOneThreads><<<1, kExpandOneThreads, 0, s>>>(
+                    m, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0, nullptr, E.soup_next.p, E.conn.p,
+                    T.n_leaf, lc, prev);
+            else
+                k_expand_level<kExpandThreads><<<blocks, kExpandThreads, 0, s>>>(
+                    m, E.soup.p, E.entry_hits.p, ctx->nodes.p, self_leaf ? 1 : 0, (const int2*)E.sums.p,
+                    E.soup_next.p, E.conn.p, T.n_leaf, lc, prev);
+            E.launches++;
+            std::swap(E.soup, E.soup_next);
+        }
+        D2G_CUDA(cudaMemcpyAsync(ctx->h_pinned, E.lc.p, sizeof(int32_t) * LC_SIZE * K, cudaMemcpyDeviceToHost, s));
         D2G_CUDA(cudaStreamSynchronize(s));
         prof_collect(ctx);
-        std::swap(E.soup, E.soup_next);
-        n = ctx->h_pinned[LC_NEXT];
-        new_leaf = ctx->h_pinned[LC_LEAF] - T.n_leaf;
-        T.n_leaf = ctx->h_pinned[LC_LEAF];
-        T.n_root = ctx->h_pinned[LC_ROOT];
-        for (int k = 0; k < LC_TRI_N; k++) T.tri += (uint32_t)ctx->h_pinned[LC_TRI + k];
-        D2G_CUDA(cudaMemsetAsync(E.lc.p + LC_TRI, 0, sizeof(int32_t) * LC_TRI_N, s));
+        for (int k = 0; k < K && n > 0; k++) {
+            const int32_t* lc = ctx->h_pinned + k * LC_SIZE;
+            T.peak = std::max(T.peak, 64.0 * 8.0 * 1.5 * n / budget);
+            if (T.levels == 0) T.n_root = lc[LC_ROOT];
+            T.levels++;
+            T.nodes += n;
+            n = lc[LC_NEXT];
+            new_leaf = lc[LC_LEAF] - T.n_leaf;
+            T.n_leaf = lc[LC_LEAF];
+            for (int q = 0; q < LC_TRI_N; q++) T.tri += (uint32_t)lc[LC_TRI + q];
+        }
     }
+    D2G_CUDA(cudaMemsetAsync(E.lc.p + LC_TRI, 0, sizeof(int32_t) * LC_TRI_N, s));
     // the last level's leaf pairs are a level of the reference's (root pairs of
     // two leaves belong to the first)
     if (new_leaf > (self_leaf && T.levels == 1 ? T.n_root : 0)) T.levels++;
     return D2G_OK;
 }
+// Blocks for a level's kernels, a warp a node pair: running ahead, as many as
+// are resident at once (the kernels stride).
+int level_blocks(int n, bool ahead) { return ahead ? std::min(nblocks(32LL * n), 152 * 8) : nblocks(32LL * n); }
 
 // The FP64 tests of the descent's leaf pairs (E.conn, in level order), and of
 // the chunk's root pairs that are two leaves (soup stage: the best of a
@@ -3026,8 +3083,7 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
         Traversal T;
         RC(E.soup.ensure((size_t)(p1 - p0) + 1));  // the frontiers swap every level: this one may be the smaller
         D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
-        RC(descend(ctx, p1 - p0, false, budget, p1 - p0 > 1, T, [&](int n_soup) -> int {
-            RC(E.ccd_list.ensure(64 * (size_t)n_soup));
+        RC(descend(ctx, p1 - p0, false, budget, p1 - p0 > 1, T, [&](int n_soup, int32_t* lc, const int32_t* n_dev) -> int {
             const int pff = prof_begin(ctx, PROF_SOUP_FILTER, 64LL * n_soup);
             const uint8_t* eskip = nullptr;
             if (E.witnesses) {
@@ -3037,16 +3093,17 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
                        E.wt_table.p, E.wt_log2cap, E.wt_flag.p, E.ccd_stats.p);
                 eskip = E.wt_flag.p;
             }
-            LAUNCH(k_ccd_level, 32LL * n_soup, n_soup, E.soup.p, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p,
-                   ctx->tri32.p, ctx->geo_eps.p, E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0,
-                   E.entry_hits.p, E.ccd_list.p, E.lc.p);
+            k_ccd_level<<<level_blocks(n_soup, n_dev != nullptr), kBlock, 0, s>>>(
+                n_soup, E.soup.p, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p, ctx->tri32.p, ctx->geo_eps.p,
+                E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0, E.entry_hits.p, E.ccd_list.p, lc, n_dev);
+            E.launches++;
             prof_end(ctx, pff);
             if (E.fp32_bounds)
-                k_soup_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p, E.pm32c.p,
+                k_soup_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p, E.pm32c.p,
                                                           ctx->tris.p, ctx->tri32.p, E.search.p, E.entry_hits.p,
                                                           E.certificates ? 1 : 0, E.ccd_stats.p);
             else
-                k_soup_tests<<<4 * test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p,
+                k_soup_tests<<<4 * test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p,
                                                                   ctx->tris.p, E.search.p, E.entry_hits.p);
             E.launches++;
             if (E.witnesses) {
@@ -3107,9 +3164,10 @@ int np_slot_tests(d2g_ctx* ctx, const int32_t* d_pairs, const Entry* front, int 
     RC(E.np_mask.ensure(n_words + 1));
     RC(E.np_cnt.ensure(n_words + 1));
     RC(E.np_off.ensure(n_words + 1));
-    RC(E.lc.ensure(LC_SIZE));
+    RC(E.lc.ensure(kAhead * LC_SIZE));
     LAUNCH(k_np_filter<true>, 32LL * n, n, front, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p,
-           E.search.p, ctx->nodes.p, E.fp32_bounds ? 1 : 0, E.np_mask.p, E.np_cnt.p, (int32_t*)nullptr, (int32_t*)nullptr, E.lc.p);
+           E.search.p, ctx->nodes.p, E.fp32_bounds ? 1 : 0, E.np_mask.p, E.np_cnt.p, (int32_t*)nullptr, (int32_t*)nullptr, E.lc.p,
+           (const int32_t*)nullptr);
     RC(scan(ctx, E.np_cnt.p, E.np_off.p, n_words));
     int32_t n_items = 0;
     const int32_t* src = E.np_off.p + n_words;
@@ -3152,16 +3210,16 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
         Traversal T;
         RC(E.soup.ensure((size_t)(p1 - p0) + 1));
         D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
-        RC(descend(ctx, p1 - p0, true, budget, p1 - p0 > 1, T, [&](int n) -> int {
-            RC(E.ccd_list.ensure(64 * (size_t)n));
-            LAUNCH(k_np_filter<false>, 32LL * n, n, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p,
-                   ctx->eps_up.p, E.search.p, ctx->nodes.p, E.fp32_bounds ? 1 : 0, (uint32_t*)nullptr, (int32_t*)nullptr,
-                   E.entry_hits.p, E.ccd_list.p, E.lc.p);
+        RC(descend(ctx, p1 - p0, true, budget, p1 - p0 > 1, T, [&](int n, int32_t* lc, const int32_t* n_dev) -> int {
+            k_np_filter<false><<<level_blocks(n, n_dev != nullptr), kBlock, 0, s>>>(
+                n, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p, E.search.p,
+                ctx->nodes.p, E.fp32_bounds ? 1 : 0, nullptr, nullptr, E.entry_hits.p, E.ccd_list.p, lc, n_dev);
+            E.launches++;
             if (E.fp32_bounds)
-                k_np_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p, ctx->tris.p,
+                k_np_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p, ctx->tris.p,
                                                         ctx->eps.p, E.search.p, E.entry_hits.p);
             else
-                k_np_level_tests<<<4 * test_grid, kBlock, 0, s>>>(E.ccd_list.p, E.lc.p + LC_LIST, E.soup.p, E.pm.p,
+                k_np_level_tests<<<4 * test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p,
                                                                   ctx->tris.p, ctx->eps.p, E.search.p,
                                                                   E.entry_hits.p);
             E.launches++;

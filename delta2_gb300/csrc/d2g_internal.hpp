@@ -262,6 +262,7 @@ struct d2g_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // trees
     int n_meshes = 0, n_nodes = 0;
+    int max_depth = 0;  // of the meshes' trees (a root is 0)
     d2g::DBuf<int32_t> mesh_node_off, ntris;
     d2g::DBuf<int4> nodes;
     d2g::DBuf<double> tris, eps, inner_eps;
