@@ -295,3 +295,41 @@ def test_work_saving_modes_keep_the_ccd_exact(ctx, case):
     assert len(ref) > 0
     assert stats[0]["pairs_seen"] == len(pairs)
     print(case, stats)
+
+
+@pytest.mark.parametrize("config, n, spacing, mt", [
+    (1, (2, 1, 1), 1.05, 0.05),    # roots and their leaf pairs only
+    (2, (2, 2, 1), 1.05, 0.04),    # levels within the one-block expansion
+    (2, (10, 10, 8), 1.2, 0.04),   # first levels above it, launched for a bound
+    (5, (3, 2, 3), 1.2, 0.05),     # eight levels; edge-edge lists for one lane each
+])
+def test_traversal_launch_forms_agree(ctx, config, n, spacing, mt):
+    """Levels launched ahead for a bound, read one by one (profiling), in
+    small chunks, and without the FP32 bounds: the same contacts and counters;
+    the smaller scenes also against the oracle."""
+    s = project_futures(D.make_scene(config, nx=n[0], ny=n[1], nz=n[2], spacing=spacing, speed_sigma=1.0, seed=6))
+    pairs = broad_pairs(s)
+    t = np.full(len(pairs), mt)
+    if np.prod(n) <= 4:
+        ccd_parity(ctx, s, pairs, t)
+        np_parity(ctx, s, pairs)
+    out = []
+    try:
+        for form in ("ahead", "each", "chunks", "plain"):
+            ctx.set_profiling(form == "each")
+            ctx.set_level_budget(3_000_000 if form == "chunks" else 0)
+            ctx.set_fp32_bounds(form != "plain")
+            ctx.set_scene(s.copy())
+            c1, o1, k1 = ctx.compare_trees_full_continuous(pairs, t)
+            c2, o2, k2 = ctx.compare_trees_full(pairs)
+            out.append((form, c1, o1, c2, o2, k1, k2))
+    finally:
+        ctx.set_profiling(False)
+        ctx.set_level_budget(0)
+        ctx.set_fp32_bounds(True)
+    for form, c1, o1, c2, o2, k1, k2 in out[1:]:
+        assert_bits_equal(c1, out[0][1], f"{form} ccd")
+        assert_bits_equal(c2, out[0][3], f"{form} narrow phase")
+        assert np.array_equal(o1, out[0][2]) and np.array_equal(o2, out[0][4]), form
+        if form == "each":
+            assert tuple(k1) == tuple(out[0][5]) and tuple(k2) == tuple(out[0][6])
