@@ -1217,18 +1217,19 @@ __global__ void __launch_bounds__(kPrimBlock) k_prim_pt(int n_tp, int n_total, c
 // takes one warp instruction per 64 cycles per SM sub-partition (SMSP),
 // dependent or not and whatever the number of active lanes (a division costs
 // ~9 such slots, a square root ~10), so a warp's time is the instruction count
-// of its longest lane.  62% of the tests end within two Newton iterations (~330
-// slots each on one lane) and 20% run all ten; 0.5% bisect (~1,300 slots, which
-// would double the first pass for every warp that has one).  So:
+// of its longest lane.  62% of the tests end within two Newton iterations (~230
+// slots each on one lane) and 20% run all ten; 0.5% bisect (~370 slots, which
+// every warp of the first pass that has one would wait for).  So:
 //   k_ee_first   one test per lane: the edges and at most two
 //                Newton iterations; the tests still running and those that
 //                bisect are saved and listed.
-//   k_ee_rest4   the listed tests on four lanes each (below), ~230 slots an
+//   k_ee_rest4   the listed tests on four lanes each (below), ~190 slots an
 //                iteration: while the list gives each SMSP at most a warp or
 //                two, latency is what counts.
 //   k_ee_rest1   the listed tests on one lane each, when there are more than
-//                kRestWide: a quarter of the warps at 1.4 times the slots (noisy
-//                spheres, 71,000 listed tests: 1,225 us on four lanes).
+//                kRestWide: a quarter of the warps at 1.2 times the slots (noisy
+//                spheres, 71,000 listed tests: 1,225 us on four lanes, 636 on
+//                one; 520 with the shortened iteration).
 // Each test performs exactly the operations of edge_edge_ccd, in order.
 // The first pass's iteration cap is the context setting D2G_TUNE_EE_FIRST_ITERS (default 2).
 constexpr int kRestWide = 7000;
@@ -1329,7 +1330,7 @@ __device__ __forceinline__ bool ee_steady(const Edge& S, const Edge& E) {
 // gap along the direction between its points there, the smaller of the start's
 // and the end's (the gap of linearly moving points is concave in time); the
 // rest runs edgeEdgeCCD's iterates until a distance is below the limit, and its
-// bisection (1,200 FP64 instructions) last.  A thread per sub-test took 51 us a
+// bisection (~370 FP64 instructions) last.  A thread per sub-test took 51 us a
 // level on the 1,024-hull step.
 __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict__ list,
                                                        const int32_t* __restrict__ n_list,
@@ -2184,8 +2185,8 @@ __global__ void k_np_items(int n_words, const uint32_t* __restrict__ mask, const
 
 // One surviving slot a thread: the FP64 triangle distance and the hit test.
 // Bound by the FP64 pipe; tri_tri_dist_below evaluates 2 to 3 of the 21
-// features (1,024 packed hulls: 825 us a level with all of them, the whole
-// call 5.60 -> 2.35 ms with that and the node pairs marked by k_np_mask).
+// features (1,024 packed hulls' leaf pairs: 352 us with the pipe 80% busy;
+// with all features, 825 us a level).
 __global__ void __launch_bounds__(kBlock) k_np(int n_slots, const Entry* __restrict__ front,
                                                const int32_t* __restrict__ pairs, const double* __restrict__ pm,
                                                const int32_t* __restrict__ ntris, const double* __restrict__ tris,
