@@ -1886,7 +1886,10 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // (20 um plus 4e-6 of the magnitudes involved) far above the FP32 rounding of
 // the bound (3e-7 of them) and the FP64 rounding of the exact test, so every
 // slot that hits survives.  Dropped slots produce nothing in the reference
-// either.
+// either.  (A triangle that is a point, or not finite, is the exception: the
+// reference's distance to it can be 0 with no feature at all (d2g_prune.cuh),
+// wherever the other triangle is.  Such slots are kept within 1 mm of the limit
+// by the spheres, boxes and normals, and decided by the whole distance.)
 //
 // A warp per node pair: lanes 0-7 transform a's triangles, 8-15 b's, once each
 // into shared memory, with their normals; every lane takes two of the 64 slots
@@ -1926,6 +1929,12 @@ __device__ __forceinline__ float normal_gap(const float* n, const float* v) {
     return fmaxf(fminf(p0, fminf(p1, p2)) - n[4], n[3] - fmaxf(p0, fmaxf(p1, p2)));
 }
 
+// Marks a slot of k_np_filter's list that only the whole distance decides: a
+// triangle that is a point or not finite, or poses (metres) so far out that a
+// small triangle could become a point there.
+constexpr int kWholeTest = 1 << 30;
+constexpr float kWorldMax = 1e6f;
+
 template <bool LEAF>
 __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const Entry* __restrict__ front,
                                                       const float* __restrict__ pm32, const int32_t* __restrict__ ntris,
@@ -1937,8 +1946,8 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                                                       int32_t* __restrict__ entry_hits, int32_t* __restrict__ list,
                                                       int32_t* __restrict__ lc, const int32_t* __restrict__ n_dev) {
     __shared__ float s_v[kBlock / 32][16][9];
-    // centre, radius, eps, magnitude, 1 for a triangle that is a point, unit
-    // normal, the triangle's own range along it
+    // centre, radius, eps, magnitude, 1 for a triangle that is a point or not
+    // finite, unit normal, the triangle's own range along it
     __shared__ float s_c[kBlock / 32][16][13];
     __shared__ uint8_t s_slot[kBlock / 32][64];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -1978,7 +1987,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
             float ext = 0.f;
 #pragma unroll
             for (int r = 0; r < 3; r++) ext = fmaxf(ext, fmaxf(fabsf(v[3 + r] - v[r]), fabsf(v[6 + r] - v[r])));
-            c[6] = ext > 1e-5f ? 0.f : 1.f;
+            c[6] = ext > 1e-5f && ext < 1e15f ? 0.f : 1.f;
             F3 nn = cross3(f3(v[3] - v[0], v[4] - v[1], v[5] - v[2]), f3(v[6] - v[0], v[7] - v[1], v[8] - v[2]));
             const float len = sqrtf(dot3(nn, nn)), inv = len > 1e-20f ? 1.f / len : 0.f;
             nn = f3(nn.x * inv, nn.y * inv, nn.z * inv);
@@ -2004,7 +2013,8 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
             if (keep && use_bounds) {
                 const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb0], *va = s_v[wi][ta], *vb = s_v[wi][8 + tb0];
                 const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
-                const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
+                const float thr = se + ca[4] + cb[4];
+                const float lim = thr + ((ca[6] + cb[6] == 0.f ? 2e-5f : 1e-3f) + 4e-6f * (tm + ca[5] + cb[5] + thr));
                 keep = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
                        !(box_gap9(va, vb) > lim) && !(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim);
             }
@@ -2045,7 +2055,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                     break;
                 }
                 const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
-                const unsigned bit = !(axis_gap9(d, va, vb) > lim) ? 1u << (sl & 31) : 0u;
+                const unsigned bit = ca[6] + cb[6] != 0.f || !(axis_gap9(d, va, vb) > lim) ? 1u << (sl & 31) : 0u;
                 m[0] |= __reduce_or_sync(0xffffffffu, sl < 32 ? bit : 0u);
                 m[1] |= __reduce_or_sync(0xffffffffu, sl < 32 ? 0u : bit);
             }
@@ -2063,7 +2073,10 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                     cnt[2 * (size_t)w + h] = __popc(m[h]);
                 }
             } else {
-                warp_append(64 * w + lane + 32 * h, (m[h] >> lane) & 1u, list, lc + LC_LIST);
+                const bool keep = (m[h] >> lane) & 1u;
+                const bool whole = keep && use_bounds &&
+                                   !(s_c[wi][ta0 + 4 * h][6] + s_c[wi][8 + tb0][6] == 0.f && tm < kWorldMax);
+                warp_append((64 * w + lane + 32 * h) | (whole ? kWholeTest : 0), keep, list, lc + LC_LIST);
             }
         }
         if (LEAF) break;  // a warp a node pair
@@ -2075,7 +2088,8 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
 // a few hundred slots, a warp a slot (a thread a slot took 20 to 60 us a
 // level); the vertices a component per lane, then the nine edge pairs on lanes
 // 0-8 and, if none is below the limit, the six projections on lanes 9-14 and
-// the six edge crossings on lanes 16-21 that the FP32 bounds leave.
+// the six edge crossings on lanes 16-21 that the FP32 bounds leave.  A marked
+// slot's distance is the reference's whole one, on one lane.
 __global__ void __launch_bounds__(kBlock) k_np_slots(const int32_t* __restrict__ list,
                                                      const int32_t* __restrict__ n_list,
                                                      const Entry* __restrict__ front, const double* __restrict__ pm,
@@ -2087,7 +2101,7 @@ __global__ void __launch_bounds__(kBlock) k_np_slots(const int32_t* __restrict__
     double(*v)[3] = s_v[wi];
     for (int k = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); k < n;
          k += (int)((gridDim.x * (size_t)blockDim.x) >> 5)) {
-        const int slot = list[k];
+        const int item = list[k], slot = item & ~kWholeTest;
         if (__any_sync(0xffffffffu, ((volatile int32_t*)entry_hits)[slot >> 6] != 0)) continue;
         const Entry e = front[slot >> 6];
         const int ta = (slot >> 3) & 7, tb = slot & 7;
@@ -2101,13 +2115,21 @@ __global__ void __launch_bounds__(kBlock) k_np_slots(const int32_t* __restrict__
         __syncwarp();
         const double thr = ((double)search[e.pair] + eps[(size_t)e.na * 8 + ta]) + eps[(size_t)e.nb * 8 + tb];
         auto at = [&](int i) { return mk(v[i][0], v[i][1], v[i][2]); };
-        bool hit = false;
+        bool hit = false, any;
+        if (item & kWholeTest) {
+            V3 P, Q;
+            if (lane == 0) hit = tri_tri_dist_plain(Tri{at(0), at(1), at(2)}, Tri{at(3), at(4), at(5)}, P, Q) < thr;
+            any = __any_sync(0xffffffffu, hit);
+            if (any && lane == 0) entry_hits[slot >> 6] = 1;
+            __syncwarp();
+            continue;
+        }
         if (lane < 9) {
             const int ia = lane / 3, ib = lane % 3;
             V3 P, Q;
             hit = edge_closest(at(ia), at(ia == 2 ? 0 : ia + 1), at(3 + ib), at(ib == 2 ? 3 : 4 + ib), P, Q) < thr;
         }
-        bool any = __any_sync(0xffffffffu, hit);
+        any = __any_sync(0xffffffffu, hit);
         if (!any && lane >= 9 && lane < 22 && lane != 15) {
             // T: the triangle whose plane is used, the feature is the other's
             const int q = lane < 15 ? lane - 9 : lane - 16;

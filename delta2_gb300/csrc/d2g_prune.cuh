@@ -19,6 +19,11 @@
 // of equal distances), so P, Q and the distance are the same bits whenever the
 // distance is below the limit; otherwise the returned distance is only known
 // to be no smaller than the limit (or NaN).
+//
+// tri_tri_dist of two triangles none of whose features has a distance (a
+// triangle that is a point, coordinates that are not finite) is 0 at the
+// origin: what all its comparisons leave.  Triangles that are not tri_regular
+// take the plain function, which alone knows.
 #pragma once
 #include "d2g_geom.cuh"
 
@@ -65,6 +70,20 @@ D2G_HD F3 seg_vector(F3 S0, F3 S1, F3 E0, F3 E1, float& d2) {
     d2 = dot3(n, n);
     return n;
 }
+
+// Two of the triangle's edges, taken from its vertices relative to the other's,
+// are neither points nor out of range: with another such triangle some edge
+// pair has a finite distance.  s: the squared lengths of the edges at the first
+// vertex.
+D2G_HD bool tri_regular(float s) { return s > 1e-30f && s < 1e30f; }  // false for NaN
+
+// tri_tri_dist, out of line: hardly ever called beside the bounds.
+#ifdef __CUDA_ARCH__
+static __device__ __noinline__
+#else
+inline
+#endif
+double tri_tri_dist_plain(const Tri& a, const Tri& b, V3& P, V3& Q) { return tri_tri_dist(a, b, P, Q); }
 
 // What the bounds read of a triangle's plane.
 struct PlaneBound {
@@ -150,6 +169,14 @@ D2G_HD double tri_tri_dist_below(const Tri& a, const Tri& b, double limit, V3& P
     const float mag = (float)(fabs(o.x) + fabs(o.y) + fabs(o.z));
     const float margin = 4e-6f * rho + 1e-13f * mag + 1e-30f;
     const PlaneBound pa = plane_bound(A[0], A[1], A[2], rho), pb = plane_bound(B[0], B[1], B[2], rho);
+    if (!(tri_regular(pa.d00 + pa.d11) && tri_regular(pb.d00 + pb.d11))) {
+        const Tri ca = a, cb = b;  // (in memory for the call; a, b, P and Q stay in registers)
+        V3 p, q;
+        const double d = tri_tri_dist_plain(ca, cb, p, q);
+        P = p;
+        Q = q;
+        return d;
+    }
     float hB[3], hA[3];  // heights of b's vertices over a's plane and of a's over b's
 #pragma unroll
     for (int i = 0; i < 3; i++) {
