@@ -23,6 +23,7 @@
 
 #include "d2g_geom.cuh"
 #include "d2g_internal.hpp"
+#include "d2g_limits.hpp"
 #include "d2g_prune.cuh"
 
 namespace d2g {
@@ -454,9 +455,8 @@ __device__ __forceinline__ float tri_gap_motion(F3 d, const float* a, const floa
                  fmaxf(axis_gap_motion(na, a, b, ae, be), axis_gap_motion(nb, a, b, ae, be)));
 }
 
-// Marks a slot of k_ccd_level's list whose edge-edge tests are all clear (slot
-// indices stay below 2^30).
-constexpr int kEdgesClear = 1 << 30;
+// Marks a slot of k_ccd_level's list whose edge-edge tests are all clear.
+constexpr int kEdgesClear = kSlotMark;
 
 __global__ void __launch_bounds__(kBlock) k_ccd_level(
     int n_soup, const Entry* __restrict__ soup, const int32_t* __restrict__ pairs, const double* __restrict__ pm,
@@ -1932,7 +1932,7 @@ __device__ __forceinline__ float normal_gap(const float* n, const float* v) {
 // Marks a slot of k_np_filter's list that only the whole distance decides: a
 // triangle that is a point or not finite, or poses (metres) so far out that a
 // small triangle could become a point there.
-constexpr int kWholeTest = 1 << 30;
+constexpr int kWholeTest = kSlotMark;
 constexpr float kWorldMax = 1e6f;
 
 template <bool LEAF>
@@ -2816,8 +2816,10 @@ struct Traversal {
 // children a node pair.  Levels run ahead only while the bound is below
 // kAheadPairs, whose buffers (~2.4 KB a node pair) fit the budget, and while
 // the meshes' depths allow another level; levels above are long enough to
-// hide the read.  decide gets the level's bound, its counters and, running
-// ahead, where its count is.
+// hide the read.  decide gets the level's first node pair and their number (or
+// a bound), its counters and, running ahead, where its count is; a single body
+// pair's level that a slot list cannot number, or that passes the budget, is
+// decided in ranges (level_range).
 constexpr int kAhead = 4, kAheadPairs = 1 << 16;
 template <class F>
 int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon, Traversal& T, F decide) {
@@ -2828,11 +2830,17 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
     const int max_levels = 2 * ctx->max_depth;  // a level opens one side, and stops at two leaves
     while (n > 0) {
         // past the budget (768 bytes a node pair: its slot list and its
-        // children), or past 32-bit slot indices (64 slots per node pair)
+        // children), or past what a slot list numbers
         const double need = 64.0 * 8.0 * 1.5 * n;
-        if ((need > budget || 64LL * n > (long long)INT32_MAX / 2) && may_abandon) {
+        const bool wide = 8LL * n + T.n_leaf > (long long)INT32_MAX;  // counts are 32-bit
+        if ((need > budget || n > kMaxListPairs || wide) && may_abandon) {
             T.abandon = true;
             return D2G_OK;
+        }
+        if (wide) {
+            set_error("a traversal level of one body pair with " + std::to_string(n) +
+                      " node pairs exceeds the 32-bit node pair count");
+            return D2G_ERR_INVALID;
         }
         // (profiling counts slots, witnesses keep a table a level)
         const int most = E.profiling || E.witnesses ? 1 : std::min<int64_t>(kAhead, max_levels - T.levels);
@@ -2843,10 +2851,11 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
             bound[K] = (int)b;
         }
         const size_t top = (size_t)bound[K - 1];
+        const int range = K > 1 ? bound[K - 1] : level_range(n, budget);
         size_t leaves = (size_t)T.n_leaf + 1;
         for (int k = 0; k < K; k++) leaves += 8 * (size_t)bound[k];  // a node has at most 8 children
         RC(E.entry_hits.ensure(top + 1));
-        RC(E.ccd_list.ensure(64 * top));
+        RC(E.ccd_list.ensure(64 * (size_t)range));
         RC(E.soup_next.ensure(8 * top + 1));
         RC(E.soup.ensure_keep(K > 1 ? 8 * top + 1 : (size_t)n + 1, (size_t)n, s));
         RC(E.conn.ensure_keep(leaves, (size_t)T.n_leaf, s));
@@ -2855,7 +2864,10 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
             int32_t* lc = E.lc.p + k * LC_SIZE;
             const int32_t* prev = k ? lc - LC_SIZE : nullptr;
             const int m = bound[k];
-            RC(decide(m, lc, k ? prev + LC_NEXT : nullptr));
+            for (int r0 = 0; r0 < m; r0 += range) {
+                if (r0 > 0) D2G_CUDA(cudaMemsetAsync(lc + LC_LIST, 0, sizeof(int32_t), s));
+                RC(decide(r0, std::min(range, m - r0), lc, k ? prev + LC_NEXT : nullptr));
+            }
             const bool one = m <= kExpandOneBlock;
             const int blocks = one ? 1 : nblocks(m, kExpandThreads);
             if (!one) {
@@ -3106,31 +3118,34 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
         Traversal T;
         RC(E.soup.ensure((size_t)(p1 - p0) + 1));  // the frontiers swap every level: this one may be the smaller
         D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
-        RC(descend(ctx, p1 - p0, false, budget, p1 - p0 > 1, T, [&](int n_soup, int32_t* lc, const int32_t* n_dev) -> int {
+        RC(descend(ctx, p1 - p0, false, budget, p1 - p0 > 1, T, [&](int r0, int n_soup, int32_t* lc,
+                                                                    const int32_t* n_dev) -> int {
+            const Entry* soup = E.soup.p + r0;
+            int32_t* hits = E.entry_hits.p + r0;
             const int pff = prof_begin(ctx, PROF_SOUP_FILTER, 64LL * n_soup);
             const uint8_t* eskip = nullptr;
             if (E.witnesses) {
                 RC(E.wt_flag.ensure(n_soup + 1));
-                LAUNCH(k_witness_check, 32LL * n_soup, n_soup, E.soup.p, d_pairs, E.pm.p, E.pm32c.p, ctx->tri32.p,
+                LAUNCH(k_witness_check, 32LL * n_soup, n_soup, soup, d_pairs, E.pm.p, E.pm32c.p, ctx->tri32.p,
                        ctx->mesh.p, ctx->mesh_node_off.p, ctx->ntris.p, ctx->tris.p, ctx->geo_eps.p, E.search.p,
                        E.wt_table.p, E.wt_log2cap, E.wt_flag.p, E.ccd_stats.p);
                 eskip = E.wt_flag.p;
             }
             k_ccd_level<<<level_blocks(n_soup, n_dev != nullptr), kBlock, 0, s>>>(
-                n_soup, E.soup.p, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p, ctx->tri32.p, ctx->geo_eps.p,
-                E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0, E.entry_hits.p, E.ccd_list.p, lc, n_dev);
+                n_soup, soup, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p, ctx->tri32.p, ctx->geo_eps.p,
+                E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0, hits, E.ccd_list.p, lc, n_dev);
             E.launches++;
             prof_end(ctx, pff);
             if (E.fp32_bounds)
-                k_soup_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p, E.pm32c.p,
-                                                          ctx->tris.p, ctx->tri32.p, E.search.p, E.entry_hits.p,
+                k_soup_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, soup, E.pm.p, E.pm32c.p,
+                                                          ctx->tris.p, ctx->tri32.p, E.search.p, hits,
                                                           E.certificates ? 1 : 0, E.ccd_stats.p);
             else
-                k_soup_tests<<<4 * test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p,
-                                                                  ctx->tris.p, E.search.p, E.entry_hits.p);
+                k_soup_tests<<<4 * test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, soup, E.pm.p,
+                                                                  ctx->tris.p, E.search.p, hits);
             E.launches++;
             if (E.witnesses) {
-                LAUNCH(k_witness_make, 32LL * n_soup, n_soup, E.soup.p, E.entry_hits.p, E.wt_flag.p, skip, d_pairs,
+                LAUNCH(k_witness_make, 32LL * n_soup, n_soup, soup, hits, E.wt_flag.p, skip, d_pairs,
                        E.pm.p, E.pm32c.p, ctx->tri32.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->ntris.p, ctx->tris.p,
                        ctx->geo_eps.p, E.search.p, E.wt_table.p, E.wt_log2cap, E.ccd_stats.p);
                 E.wt_inserts += n_soup;
@@ -3233,18 +3248,21 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
         Traversal T;
         RC(E.soup.ensure((size_t)(p1 - p0) + 1));
         D2G_CUDA(cudaMemcpyAsync(E.soup.p, E.roots.p + p0, sizeof(Entry) * (p1 - p0), cudaMemcpyDeviceToDevice, s));
-        RC(descend(ctx, p1 - p0, true, budget, p1 - p0 > 1, T, [&](int n, int32_t* lc, const int32_t* n_dev) -> int {
+        RC(descend(ctx, p1 - p0, true, budget, p1 - p0 > 1, T, [&](int r0, int n, int32_t* lc,
+                                                                   const int32_t* n_dev) -> int {
+            const Entry* front = E.soup.p + r0;
+            int32_t* hits = E.entry_hits.p + r0;
             k_np_filter<false><<<level_blocks(n, n_dev != nullptr), kBlock, 0, s>>>(
-                n, E.soup.p, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p, E.search.p,
-                ctx->nodes.p, E.fp32_bounds ? 1 : 0, nullptr, nullptr, E.entry_hits.p, E.ccd_list.p, lc, n_dev);
+                n, front, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p, E.search.p,
+                ctx->nodes.p, E.fp32_bounds ? 1 : 0, nullptr, nullptr, hits, E.ccd_list.p, lc, n_dev);
             E.launches++;
             if (E.fp32_bounds)
-                k_np_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p, ctx->tris.p,
-                                                        ctx->eps.p, E.search.p, E.entry_hits.p);
+                k_np_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, front, E.pm.p, ctx->tris.p,
+                                                        ctx->eps.p, E.search.p, hits);
             else
-                k_np_level_tests<<<4 * test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, E.soup.p, E.pm.p,
+                k_np_level_tests<<<4 * test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, front, E.pm.p,
                                                                   ctx->tris.p, ctx->eps.p, E.search.p,
-                                                                  E.entry_hits.p);
+                                                                  hits);
             E.launches++;
             return D2G_OK;
         }));
