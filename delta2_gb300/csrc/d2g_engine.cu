@@ -1142,14 +1142,12 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_ee(int n_tp, int n_total, c
         const float lim = thr + (2e-5f + 4e-6f * (mag + thr));
         keep = !use_bounds || !(box_gap(ba, bb) > lim);
         if (keep && use_bounds) {
-            // the gap over the motion along the direction between the edges'
-            // closest points at the start (axis_gap_motion)
-            auto at = [&](int m, int v) { return f3(o[m][v][0], o[m][v][1], o[m][v][2]); };
-            float d2;
-            const F3 d = seg_vector(at(0, 0), at(0, 1), at(0, 2), at(0, 3), d2);
-            const float g0 = fminf(dot3(d, at(0, 2)), dot3(d, at(0, 3))) - fmaxf(dot3(d, at(0, 0)), dot3(d, at(0, 1)));
-            const float g1 = fminf(dot3(d, at(1, 2)), dot3(d, at(1, 3))) - fmaxf(dot3(d, at(1, 0)), dot3(d, at(1, 1)));
-            keep = !(fminf(g0, g1) > lim * sqrtf(d2));
+            F3 p[2][4];
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int v = 0; v < 4; v++) p[m][v] = f3(o[m][v][0], o[m][v][1], o[m][v][2]);
+            keep = !edges_stay_apart(p, lim);
         }
         if (!keep) record_no_contact(w.out, w.hit);
     }

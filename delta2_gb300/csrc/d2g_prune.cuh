@@ -71,6 +71,19 @@ D2G_HD F3 seg_vector(F3 S0, F3 S1, F3 E0, F3 E1, float& d2) {
     return n;
 }
 
+// Edges p[][0] p[][1] and p[][2] p[][3] at the start and at the end of a motion
+// on straight lines: further apart than lim all along, because the gap along
+// the direction between their closest points at the start, concave in time, is
+// so at both ends.  Closest points within 1e-15 give no direction: the length
+// of one below 1e-20 underflows, and any gap would pass for a large one.
+D2G_HD bool edges_stay_apart(const F3 (&p)[2][4], float lim) {
+    float d2, g[2];
+    const F3 d = seg_vector(p[0][0], p[0][1], p[0][2], p[0][3], d2);
+    for (int m = 0; m < 2; m++)
+        g[m] = fminf(dot3(d, p[m][2]), dot3(d, p[m][3])) - fmaxf(dot3(d, p[m][0]), dot3(d, p[m][1]));
+    return d2 > 1e-30f && fminf(g[0], g[1]) > lim * sqrtf(d2);
+}
+
 // Two of the triangle's edges, taken from its vertices relative to the other's,
 // are neither points nor out of range: with another such triangle some edge
 // pair has a finite distance.  s: the squared lengths of the edges at the first
@@ -247,7 +260,7 @@ D2G_HD double tri_tri_dist_below(const Tri& a, const Tri& b, double limit, V3& P
             const F3 n = seg_vector(S0, S1, E0, E1, d2);
             const float d = sqrtf(d2);
             const float gap = (fminf(dot3(n, E0), dot3(n, E1)) - fmaxf(dot3(n, S0), dot3(n, S1))) / d;
-            lb[6 + 3 * i + j] = gap > 0.f ? gap - margin : 0.f;  // NaN: 0
+            lb[6 + 3 * i + j] = gap > 0.f && d2 > 1e-30f ? gap - margin : 0.f;  // NaN: 0 (edges_stay_apart)
             if (d < best_est) {
                 best_est = d;
                 first = 6 + 3 * i + j;
