@@ -2828,8 +2828,8 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
     const int max_levels = 2 * ctx->max_depth;  // a level opens one side, and stops at two leaves
     while (n > 0) {
         // past the budget (768 bytes a node pair: its slot list and its
-        // children), or past what a slot list numbers
-        const double need = 64.0 * 8.0 * 1.5 * n;
+        // children; 18 a leaf pair so far), or past what a slot list numbers
+        const double need = 64.0 * 8.0 * 1.5 * n + 1.5 * sizeof(Entry) * T.n_leaf;
         const bool wide = 8LL * n + T.n_leaf > (long long)INT32_MAX;  // counts are 32-bit
         if ((need > budget || n > kMaxListPairs || wide) && may_abandon) {
             T.abandon = true;
@@ -2890,7 +2890,7 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
         prof_collect(ctx);
         for (int k = 0; k < K && n > 0; k++) {
             const int32_t* lc = ctx->h_pinned + k * LC_SIZE;
-            T.peak = std::max(T.peak, 64.0 * 8.0 * 1.5 * n / budget);
+            T.peak = std::max(T.peak, (64.0 * 8.0 * 1.5 * n + 1.5 * sizeof(Entry) * T.n_leaf) / budget);
             if (T.levels == 0) T.n_root = lc[LC_ROOT];
             T.levels++;
             T.nodes += n;
@@ -2913,14 +2913,15 @@ int level_blocks(int n, bool ahead) { return ahead ? std::min(nblocks(32LL * n),
 // The FP64 tests of the descent's leaf pairs (E.conn, in level order), and of
 // the chunk's root pairs that are two leaves (soup stage: the best of a
 // triangle pair's 15 tests); their contacts are appended to E.rec.  Large lists
-// run in ranges that keep the test buffers within the budget.
-int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, int p0, int p1, const Traversal& T,
-                   double budget, int* n_rec_io, long long* n_pp, bool* abandon) {
+// run in ranges that keep the test buffers within the budget; `full` is called
+// between ranges with the records so far, and may take them.
+template <class F>
+int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, int p0, int p1, Traversal& T,
+                   double budget, int& n_rec, long long* n_pp, bool* abandon, F full) {
     Engine& E = ctx->eng;
     cudaStream_t s = ctx->stream;
     int ee_grid = 0;
     RC(ee_grid_size(ctx, &ee_grid));
-    int n_rec = *n_rec_io;
     // ~1900 bytes of test buffers per triangle pair (x1.5 growth slack), at most 64 in a leaf pair
     const int range = (int)std::min(1.0e6, std::max(256.0, budget / (1.5 * 1900.0 * 64.0)));
     for (int c0 = T.n_root > 0 ? -1 : 0; c0 < T.n_leaf; c0 = c0 < 0 ? 0 : c0 + range) {
@@ -2964,6 +2965,7 @@ int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, in
                 return D2G_ERR_INVALID;
             }
         }
+        T.peak = std::max(T.peak, 1.5 * 1900.0 * K / budget);
         if (K + P == 0) continue;
         RC(E.items.ensure(K + 1));
         RC(E.sub.ensure(15 * (size_t)K + 1));
@@ -3053,8 +3055,8 @@ int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, in
         else if (fin > 0)
             emit_records(ctx, 15 * P, E.chit.p, E.cflag_off.p, nullptr, 0, conn, E.tp.p, d_pairs, E.cres.p, n_rec);
         n_rec += fin;
+        RC(full());
     }
-    *n_rec_io = n_rec;
     return D2G_OK;
 }
 
@@ -3152,7 +3154,21 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
         }));
         bool abandon = T.abandon;
         long long n_pp = 0;  // leaf pairs' triangle pairs
-        if (!abandon) RC(ccd_leaf_tests(ctx, d_pairs, skip, p0, p1, T, budget, &n_rec, &n_pp, &abandon));
+        bool first = true;
+        // the records so far, sorted by pair, go to the consumer and are dropped
+        auto hand_over = [&]() -> int {
+            RC(finish_records(ctx, p1 - p0, n_rec, p0));
+            RC(sink->consume(ctx, sink->user, p0, p1, first));
+            first = false;
+            n_streamed += n_rec;
+            n_rec = 0;
+            return D2G_OK;
+        };
+        // ~240 bytes a record with its sorted copy (x1.5 growth slack): a
+        // streamed chunk keeps about half the budget of them
+        auto full = [&]() -> int { return sink && 360.0 * n_rec > 0.5 * budget ? hand_over() : D2G_OK; };
+        if (!abandon)
+            RC(ccd_leaf_tests(ctx, d_pairs, skip, p0, p1, T, budget, n_rec, &n_pp, &abandon, full));
         if (abandon) {
             n_rec = rec_start;
             chunk = std::max(1, (p1 - p0) / 2);
@@ -3163,12 +3179,7 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
         c_leaf += T.n_leaf;
         c_levels += T.levels;
         peak = std::max(peak, T.peak);
-        if (sink) {  // the chunk's records, sorted by pair, go to the consumer and are dropped
-            RC(finish_records(ctx, p1 - p0, n_rec, p0));
-            RC(sink->consume(ctx, sink->user, p0, p1));
-            n_streamed += n_rec;
-            n_rec = 0;
-        }
+        if (sink) RC(hand_over());
         p0 = p1;
     }
     if (n_pairs > 0) E.ccd_chunk = chunk >= n_pairs ? 0 : (peak < 1.0 / 3.0 ? 2 * chunk : chunk);

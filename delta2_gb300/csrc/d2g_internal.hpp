@@ -297,10 +297,12 @@ void prof_mark_collect(d2g_ctx* ctx);
 // Consumer of a CCD call's records chunk by chunk (pairs [p0, p1)): when run_ccd
 // is given one, each chunk's records are sorted into rec_sorted with offsets
 // out_off[0 .. p1 - p0], handed over, and dropped, so the call never holds
-// every record at once.
+// every record at once.  A chunk with more records than its share of the level
+// budget is handed over in parts, each with some of a pair's records (`first`:
+// the chunk's first part).
 struct CcdSink {
     void* user;
-    int (*consume)(d2g_ctx* ctx, void* user, int p0, int p1);
+    int (*consume)(d2g_ctx* ctx, void* user, int p0, int p1, bool first);
 };
 int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int n_pairs, int* n_out,
             int64_t* counters, const CcdSink* sink = nullptr);

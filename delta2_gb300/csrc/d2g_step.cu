@@ -89,7 +89,8 @@ __device__ __forceinline__ double from_order_bits(unsigned long long b) {
 
 // Every interaction's new step (separate_clusters.cpp:494-562), in three
 // launches.  k_pair_spin: the future angular velocities of each pair's two
-// bodies, a thread per body, and the running minimum's start 1.0.
+// bodies, a thread per body, and the running minimum's start 1.0; once per
+// chunk, whose records may come in parts.
 // k_contact_scale: a thread per contact, whichever pair it belongs to, so a
 // pair with thousands of contacts spreads over the chip; the minimum over a
 // pair's contacts, which never takes a NaN, by integer atomics (scales are
@@ -150,10 +151,10 @@ __global__ void __launch_bounds__(kBlock) k_contact_scale(int n_pairs, const dou
 
 __global__ void k_pair_new_dt(int n_pairs, const double* __restrict__ max_time, const int32_t* __restrict__ off,
                               const unsigned long long* __restrict__ best, double* __restrict__ new_dt,
-                              int32_t* __restrict__ has) {
+                              int32_t* __restrict__ has, int first) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n_pairs) return;
-    const bool any = off[p + 1] > off[p];
+    const bool any = off[p + 1] > off[p] || (!first && has[p]);
     has[p] = any ? 1 : 0;
     new_dt[p] = any ? max_time[p] * from_order_bits(best[p]) : 0.0;
 }
@@ -683,7 +684,7 @@ int run_select_steps(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, const in
     } use{d_pairs};
     CcdSink sink;
     sink.user = &use;
-    sink.consume = [](d2g_ctx* c, void* u, int p0, int p1) -> int {
+    sink.consume = [](d2g_ctx* c, void* u, int p0, int p1, bool first) -> int {
         Engine& En = c->eng;
         const int32_t* pr = static_cast<Use*>(u)->pairs;
         const int np = p1 - p0;
@@ -691,13 +692,16 @@ int run_select_steps(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, const in
             RC(En.st_spin.ensure(6 * (size_t)np));
             RC(En.st_best.ensure(np));
             const double *fut = En.pfut.p + 28 * (size_t)p0, *mt = En.st_mt.p + p0;
-            k_pair_spin<<<nblocks(2LL * np), kBlock, 0, c->stream>>>(np, pr + 2 * (size_t)p0, fut, c->inv_inertia.p,
-                                                                     En.st_spin.p, En.st_best.p);
+            if (first) {
+                k_pair_spin<<<nblocks(2LL * np), kBlock, 0, c->stream>>>(np, pr + 2 * (size_t)p0, fut,
+                                                                         c->inv_inertia.p, En.st_spin.p, En.st_best.p);
+                En.launches++;
+            }
             k_contact_scale<<<kScaleGrid, kBlock, 0, c->stream>>>(np, mt, En.out_off.p, En.rec_sorted.p, fut,
                                                                     En.st_spin.p, En.st_best.p);
             k_pair_new_dt<<<nblocks(np), kBlock, 0, c->stream>>>(np, mt, En.out_off.p, En.st_best.p,
-                                                                 En.st_new_dt.p + p0, En.st_has.p + p0);
-            En.launches += 3;
+                                                                 En.st_new_dt.p + p0, En.st_has.p + p0, first ? 1 : 0);
+            En.launches += 2;
         }
         D2G_CUDA(cudaGetLastError());
         return D2G_OK;

@@ -288,8 +288,9 @@ int d2g_ctx_solve_layout(d2g_ctx* ctx, int32_t* layout, int32_t n);
  * traversal (discrete narrow phase or CCD) may use for its buffers; 0 (the
  * default) means a sixth of the device memory.  A call whose level would
  * exceed it traverses its body pairs in chunks (halving a chunk that still
- * exceeds it), with identical results.  The contact records themselves are
- * output and are not capped. */
+ * exceeds it), with identical results.  The contact records that a call
+ * returns are output and are not capped; those that only feed a time-step
+ * selection are consumed whenever they pass half of it. */
 int d2g_ctx_set_level_budget(d2g_ctx* ctx, int64_t bytes);
 /* Instrumentation (no reference counterpart): the number of kernels this
  * library launched on the context, and, with profiling on, CUDA-event times
