@@ -463,8 +463,8 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
     const float* __restrict__ pm32, const int32_t* __restrict__ ntris, const double* __restrict__ tris,
     const float* __restrict__ tri32, const double* __restrict__ geo_eps, const float* __restrict__ search,
     const int4* __restrict__ nodes, const uint8_t* __restrict__ skip, const uint8_t* __restrict__ eskip,
-    int use_bounds, int32_t* __restrict__ entry_hits, int32_t* __restrict__ list, int32_t* __restrict__ lc,
-    const int32_t* __restrict__ n_dev) {
+    int use_bounds, int certificates, int32_t* __restrict__ entry_hits, int32_t* __restrict__ list,
+    int32_t* __restrict__ lc, const int32_t* __restrict__ n_dev) {
     __shared__ float s_verts[kBlock / 32][16][9];
     __shared__ float s_ends[kBlock / 32][16][9];
     __shared__ float s_mag[kBlock / 32][16];
@@ -508,9 +508,10 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
                     const float m = edge_min(s_verts[wi][ta], s_verts[wi][8 + tb], d);
                     if (m < room[h]) sure = true;
                     // (s_mag is huge for an unsteady triangle: never clear either)
-                    clear[h] = tri_gap_motion(d, s_verts[wi][ta], s_verts[wi][8 + tb], s_ends[wi][ta],
+                    clear[h] = certificates &&
+                               tri_gap_motion(d, s_verts[wi][ta], s_verts[wi][8 + tb], s_ends[wi][ta],
                                               s_ends[wi][8 + tb]) >
-                               thr + (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
+                                   thr + (2e-5f + 4e-6f * (fmaxf(s_mag[wi][ta], s_mag[wi][8 + tb]) + thr));
                 }
                 sure = __any_sync(0xffffffffu, sure);
                 if (!sure) {
@@ -1114,9 +1115,10 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_ee(int n_tp, int n_total, c
                                                         const float* __restrict__ search, PrimResult* __restrict__ sub,
                                                         PrimResult* __restrict__ cres, int32_t* __restrict__ chit,
                                                         int32_t* __restrict__ list, int32_t* __restrict__ count,
-                                                        int use_bounds) {
+                                                        int use_bounds, int certificates,
+                                                        unsigned long long* __restrict__ cut_counts) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    bool keep = false;
+    bool keep = false, cut = false;
     if (j < n_total) {
         const EeWork w = decode_ee(j, n_tp, items, soup, conn, nn_off, tp, ntris, sub, cres, chit);
         const float* ta = tri32 + ((size_t)w.na * 8 + w.aTri) * 9;
@@ -1141,16 +1143,20 @@ __global__ void __launch_bounds__(kBlock) k_ccd_mask_ee(int n_tp, int n_total, c
         const float thr = search[w.pair];
         const float lim = thr + (2e-5f + 4e-6f * (mag + thr));
         keep = !use_bounds || !(box_gap(ba, bb) > lim);
-        if (keep && use_bounds) {
+        if (keep && use_bounds && certificates) {
             F3 p[2][4];
 #pragma unroll
             for (int m = 0; m < 2; m++)
 #pragma unroll
                 for (int v = 0; v < 4; v++) p[m][v] = f3(o[m][v][0], o[m][v][1], o[m][v][2]);
-            keep = !edges_stay_apart(p, lim);
+            cut = edges_stay_apart(p, lim);
+            keep = !cut;
         }
         if (!keep) record_no_contact(w.out, w.hit);
     }
+    const unsigned n_cut = __popc(__ballot_sync(0xffffffffu, cut));
+    if (n_cut && (threadIdx.x & 31) == 0)
+        atomicAdd(cut_counts + (blockIdx.x % kCutCounters), (unsigned long long)n_cut);
     warp_append(j, keep, list, count);
 }
 
@@ -1324,7 +1330,8 @@ __device__ __forceinline__ bool ee_steady(const Edge& S, const Edge& E) {
 // slot, the vertices' start and end positions a component per lane, then the
 // nine edge pairs on lanes 0-8 and the six point-triangle tests on lanes
 // 16-21.  An edge pair is decided by its distance at the start (edgeEdgeCCD
-// evaluates it first, and returns no more than it or at most 1e-8), or by the
+// evaluates it first, and returns no more than it or at most 1e-8), or, as a
+// certificate, by the
 // gap along the direction between its points there, the smaller of the start's
 // and the end's (the gap of linearly moving points is concave in time); the
 // rest runs edgeEdgeCCD's iterates until a distance is below the limit, and its
@@ -1336,7 +1343,7 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
                                                        const float* __restrict__ pm32, const double* __restrict__ tris,
                                                        const float* __restrict__ tri32,
                                                        const float* __restrict__ search, int32_t* entry_hits,
-                                                       int certificates, unsigned long long* ca_stats) {
+                                                       int certificates) {
     __shared__ double s_v[kBlock / 32][2][6][3];  // start, end; a's vertices, b's
     const int n = *n_list;
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -1392,13 +1399,8 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
             if (steady) {
                 const double d0 = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q, div);
                 hit = d0 < lim;
-                open = !hit && !ee_gap_clear(aS, aE, bS, bE, P, Q, d0, lim);
+                open = !hit && !(certificates && ee_gap_clear(aS, aE, bS, bE, P, Q, d0, lim));
             }
-        }
-        const unsigned cut = certificates ? __ballot_sync(0xffffffffu, edges && lane < 9 && !hit && !open) : 0u;
-        if (lane == 0 && cut) {
-            atomicAdd(ca_stats, (unsigned long long)__popc(cut));
-            atomicAdd(ca_stats + 1, (unsigned long long)(__popc(cut) * (kEeNewtonIters - 1)));
         }
         bool any = __any_sync(0xffffffffu, hit);
         if (!any && __any_sync(0xffffffffu, open)) {
@@ -1417,7 +1419,7 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
                     b.B = lerp(bS.B, bE.B, t);
                     const double d = edge_closest(a.A, a.B, b.A, b.B, P, Q, div);
                     hit = d < lim;
-                    open = !hit && !ee_gap_clear(aS, aE, bS, bE, P, Q, d, lim);
+                    open = !hit && !(certificates && ee_gap_clear(aS, aE, bS, bE, P, Q, d, lim));
                 }
             }
             any = __any_sync(0xffffffffu, hit);
@@ -1454,13 +1456,14 @@ __global__ void __launch_bounds__(kBlock) k_soup_slots(const int32_t* __restrict
 }
 
 // The same without FP32 bounds (the list holds every slot of the level), a
-// thread a test.
+// thread a test; without the certificates too, each the reference's whole one.
 __global__ void __launch_bounds__(kPrimBlock) k_soup_tests(const int32_t* __restrict__ list,
                                                            const int32_t* __restrict__ n_list,
                                                            const Entry* __restrict__ soup,
                                                            const double* __restrict__ pm,
                                                            const double* __restrict__ tris,
-                                                           const float* __restrict__ search, int32_t* entry_hits) {
+                                                           const float* __restrict__ search, int32_t* entry_hits,
+                                                           int certificates) {
     const int n = *n_list;
     const long long n_ee = 9LL * n, total = 15LL * n;
     for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < total;
@@ -1485,14 +1488,13 @@ __global__ void __launch_bounds__(kPrimBlock) k_soup_tests(const int32_t* __rest
             aE.B = xform_rigid(ea.B, M + PM_AE);
             bE.A = xform_rigid(eb.A, M + PM_BE);
             bE.B = xform_rigid(eb.B, M + PM_BE);
-            V3 P, Q;
-            dist = edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q);
             const double lim = (double)search[e.pair];
-            if (!(lim > 1e-6 && ee_steady(aS, aE) && ee_steady(bS, bE))) {
+            V3 P, Q;
+            // as in k_soup_slots, else the whole test
+            const bool brief = certificates && lim > 1e-6 && ee_steady(aS, aE) && ee_steady(bS, bE);
+            dist = brief ? edge_closest(aS.A, aS.B, bS.A, bS.B, P, Q) : lim;
+            if (!(dist < lim) && !(brief && ee_gap_clear(aS, aE, bS, bE, P, Q, dist, lim)))
                 dist = edge_edge_ccd(aS, aE, bS, bE).dist;
-            } else if (!(dist < lim)) {  // as in k_soup_slots
-                if (!ee_gap_clear(aS, aE, bS, bE, P, Q, dist, lim)) dist = edge_edge_ccd(aS, aE, bS, bE).dist;
-            }
         } else if (q & 1) {
             dist = point_tri_ccd(tvert(B, q >> 1), M + PM_BAS, M + PM_BAE, A, M + PM_AS, M + PM_AE).dist;
         } else {
@@ -2775,8 +2777,9 @@ int check_device_pairs(d2g_ctx* ctx, const int32_t* d_pairs, int n) {
 int ensure_ccd_stats(d2g_ctx* ctx) {
     Engine& E = ctx->eng;
     if (!E.ccd_stats.p) {
-        RC(E.ccd_stats.ensure(kCcdStats));
-        D2G_CUDA(cudaMemsetAsync(E.ccd_stats.p, 0, sizeof(unsigned long long) * kCcdStats, ctx->stream));
+        RC(E.ccd_stats.ensure(kCcdStats + kCutCounters));
+        D2G_CUDA(cudaMemsetAsync(E.ccd_stats.p, 0, sizeof(unsigned long long) * (kCcdStats + kCutCounters),
+                                 ctx->stream));
     }
     return D2G_OK;
 }
@@ -2784,10 +2787,14 @@ int ensure_ccd_stats(d2g_ctx* ctx) {
 int read_ccd_stats(d2g_ctx* ctx, int64_t* out, int n, bool reset) {
     Engine& E = ctx->eng;
     RC(ensure_ccd_stats(ctx));
-    unsigned long long h[kCcdStats];
+    unsigned long long h[kCcdStats + kCutCounters];
     D2G_CUDA(cudaMemcpyAsync(h, E.ccd_stats.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     if (reset) D2G_CUDA(cudaMemsetAsync(E.ccd_stats.p, 0, sizeof(h), ctx->stream));
     D2G_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (int i = kCcdStats; i < kCcdStats + kCutCounters; i++) {  // cut before their first iterate
+        h[0] += h[i];
+        h[1] += kEeNewtonIters * h[i];
+    }
     for (int i = 0; i < n && i < kCcdStats; i++) out[i] = (int64_t)h[i];
     return D2G_OK;
 }
@@ -2996,7 +3003,8 @@ int ccd_leaf_tests(d2g_ctx* ctx, const int32_t* d_pairs, const uint8_t* skip, in
         D2G_CUDA(cudaStreamWaitEvent(s_ee, ctx->ev_fork, 0));
         k_ccd_mask_ee<<<nblocks(n_ee), kBlock, 0, s_ee>>>(K, n_ee, E.items.p, soup, conn, E.nn_off.p, E.tp.p,
                                                           E.pm32c.p, ctx->ntris.p, ctx->tri32.p, E.search.p, E.sub.p,
-                                                          E.cres.p, E.chit.p, list_ee, cnt_ee, E.fp32_bounds ? 1 : 0);
+                                                          E.cres.p, E.chit.p, list_ee, cnt_ee, E.fp32_bounds ? 1 : 0,
+                                                          E.certificates ? 1 : 0, E.ccd_stats.p + kCcdStats);
         const int pfe = prof_begin(ctx, PROF_CONN, n_ee, s_ee);
         EeArgs ea;
         ea.n_tp = K;
@@ -3133,16 +3141,18 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
             }
             k_ccd_level<<<level_blocks(n_soup, n_dev != nullptr), kBlock, 0, s>>>(
                 n_soup, soup, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p, ctx->tri32.p, ctx->geo_eps.p,
-                E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0, hits, E.ccd_list.p, lc, n_dev);
+                E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0, E.certificates ? 1 : 0, hits,
+                E.ccd_list.p, lc, n_dev);
             E.launches++;
             prof_end(ctx, pff);
             if (E.fp32_bounds)
                 k_soup_slots<<<test_grid, kBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, soup, E.pm.p, E.pm32c.p,
                                                           ctx->tris.p, ctx->tri32.p, E.search.p, hits,
-                                                          E.certificates ? 1 : 0, E.ccd_stats.p);
+                                                          E.certificates ? 1 : 0);
             else
                 k_soup_tests<<<4 * test_grid, kPrimBlock, 0, s>>>(E.ccd_list.p, lc + LC_LIST, soup, E.pm.p,
-                                                                  ctx->tris.p, E.search.p, hits);
+                                                                  ctx->tris.p, E.search.p, hits,
+                                                                  E.certificates ? 1 : 0);
             E.launches++;
             if (E.witnesses) {
                 LAUNCH(k_witness_make, 32LL * n_soup, n_soup, soup, hits, E.wt_flag.p, skip, d_pairs,

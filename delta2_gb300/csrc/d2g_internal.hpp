@@ -324,7 +324,9 @@ int run_mass_properties(d2g_ctx* ctx, const double* d_V, const int32_t* d_F, con
                         const int32_t* d_foff, const uint8_t* d_surface, int n_meshes, double thickness,
                         double* d_out);
 // CCD counters (D2G_CCD_STATS entries, see d2g_ctx_ccd_stats), read on the host.
-constexpr int kCcdStats = 8;
+// Behind them on the device, the edge-edge tests that k_ccd_mask_ee cut, over
+// several counters (a warp in two adds to one).
+constexpr int kCcdStats = 8, kCutCounters = 32;
 int read_ccd_stats(d2g_ctx* ctx, int64_t* out, int n, bool reset);
 // One level of one body pair's discrete traversal over the caller's node
 // pairs (d_pair: the pair's two bodies; d_node_pairs [n][2] global node ids):

@@ -194,13 +194,17 @@ int d2g_mass_properties(d2g_ctx* ctx, const double* V, int32_t n_vertices, const
  * above FP32 and FP64 rounding) and run the FP64 test only where a hit is
  * possible; with 0 every test runs in FP64.  Results are identical. */
 int d2g_ctx_set_fp32_bounds(d2g_ctx* ctx, int32_t enable);
-/* Conservative-advancement certificates (no reference counterpart): with
- * enable != 0 (the default) an edge-edge CCD test whose distance at a Newton
- * iterate, less the largest relative endpoint displacement times the time
- * still ahead, stays above the search distance (and whose distances so far
- * do too) is cut there: no later iterate can come closer, so it cannot hit and
- * is recorded as no contact, as the reference's min over its iterates would
- * leave it.  Results are identical; 0 runs every test to the end. */
+/* Certificates (no reference counterpart): with enable != 0 (the default) an
+ * edge-edge CCD test is cut, before its first Newton iterate, when the gap
+ * along the direction between the edges' closest points at the start stays
+ * above the search distance at both ends of the motion (it is concave in
+ * time); or at a Newton iterate when the distance there, less the largest
+ * relative endpoint displacement times the time still ahead, stays above it
+ * (and the distances so far do too).  No iterate can come closer, so the test
+ * cannot hit and is recorded as no contact, as the reference's min over its
+ * iterates would leave it.  Results are identical; 0 runs every test that the
+ * FP32 bounds leave to its end (a descent's tests until its node pair has a
+ * hit). */
 int d2g_ctx_set_ccd_certificates(d2g_ctx* ctx, int32_t enable);
 /* Learned proposal in the CCD (no reference counterpart): with a network of
  * this context (d2g_mlp_create), every CCD call (compareTreesFullContinuous,
@@ -231,8 +235,9 @@ int d2g_ccd_features(d2g_ctx* ctx, const int32_t* pairs, const double* max_time,
 int d2g_ctx_set_ccd_witnesses(d2g_ctx* ctx, int32_t enable);
 /* CCD counters since the context was created or last reset (reset != 0
  * clears them after reading), n of D2G_CCD_STATS entries:
- *   0 edge-edge tests cut by the certificates, 1 Newton iterations they did
- *   not run (of the reference's 10 per test), 2 pair queries the learned
+ *   0 edge-edge tests of leaf pairs cut by the certificates, 1 Newton
+ *   iterations they did not run (of the reference's 10 per test; a descent's
+ *   tests, which end with their node pair's first hit, are not counted), 2 pair queries the learned
  *   proposal predicted to have no contact, 3 of those the root certificate
  *   proved contact-free (skipped), 4 of those it could not prove (misses,
  *   traversed as usual), 5 pair queries seen by the proposal, 6 node pairs
