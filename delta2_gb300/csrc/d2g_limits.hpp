@@ -1,8 +1,11 @@
-// How many node pairs of a traversal level one slot list can number, and how
-// many are decided at once.
+// Small rules that both sides read and a host test can check: how many node
+// pairs of a traversal level are decided at once, and the lanes of the solve's
+// waves.
 #pragma once
 #include <algorithm>
 #include <cstdint>
+
+#include "d2g_math.cuh"
 
 namespace d2g {
 
@@ -20,6 +23,18 @@ constexpr int32_t kMinRangePairs = 256;
 inline int32_t level_range(int32_t n, double budget) {
     const double fit = std::max((double)kMinRangePairs, budget / (1.5 * 256.0));
     return (int32_t)std::min({(double)n, (double)kMaxListPairs, fit});
+}
+
+// The solve's normal loop on a block with n_tasks tasks (of four contacts) in
+// `levels` waves: sixteen lanes a contact in the waves where it has one task, or
+// eight (four a body side) throughout.  lanes: D2G_TUNE_SOLVE_LANES, 16 or 4
+// for the one or the other, 0 for sixteen while a wave has hardly more than one
+// task here: a single task's chain is then the interval's length (8 cubes: 61
+// -> 60 us per iteration, 100 cubes on 16 blocks 164 -> 140).  With more tasks
+// the loads ahead and the dealing of waves cost more than the few narrow waves
+// give (27 cubes, 1.5 tasks a wave: 123 -> 129).
+D2G_HD bool narrow_waves(int lanes, int n_tasks, int levels) {
+    return lanes ? lanes == 16 : 4LL * n_tasks <= 5LL * levels;
 }
 
 }  // namespace d2g

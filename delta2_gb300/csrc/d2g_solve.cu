@@ -22,6 +22,7 @@
 
 #include "d2g_geom.cuh"
 #include "d2g_internal.hpp"
+#include "d2g_limits.hpp"
 
 namespace d2g {
 
@@ -474,7 +475,8 @@ struct SolveArgs {
     int32_t* out_ab;
     const int32_t* con_pair;
     double* pair_warm;
-    int smem;  // dynamic shared memory, bytes
+    int smem;   // dynamic shared memory, bytes
+    int lanes;  // D2G_TUNE_SOLVE_LANES
 };
 
 constexpr int kStaticBit = 1 << 30;
@@ -1131,12 +1133,7 @@ __device__ void solve_body(int k, int gb, int G, const SolveSync& S, const Solve
                 count = first < hi ? (hi - 1 - first) / G + 1 : 0;
             }
         };
-        // Sixteen lanes a contact while a wave has hardly more than one task
-        // here: a single task's chain is then the interval's length (8 cubes:
-        // 61 -> 60 us per iteration, 100 cubes on 16 blocks 164 -> 140).  With
-        // more tasks the loads ahead and the dealing of waves cost more than
-        // the few narrow waves give (27 cubes, 1.5 tasks a wave: 123 -> 129).
-        const bool narrow = 4 * n_tasks <= 5 * levels;
+        const bool narrow = narrow_waves(a.lanes, n_tasks, levels);
         bool converged = false;
         int p0w = 0, pcw = 0;  // wave 0's tasks
         wave_tasks(0, p0w, pcw);
@@ -1625,6 +1622,7 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
         a.out_ab = d_out_ab;
         a.con_pair = d_con_pair;
         a.pair_warm = d_pair_warm;
+        a.lanes = E.tune[D2G_TUNE_SOLVE_LANES];
         // Where each cluster is solved (us per iteration on GB300, normal and
         // friction; one block / thread-block cluster of 4 / 8 / 16 / grid):
         //     8 cubes, 46 waves of 2.2 contacts     60 /   74 /   72 /  74 /    -

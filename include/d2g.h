@@ -252,9 +252,10 @@ int d2g_ctx_ccd_stats(d2g_ctx* ctx, int32_t reset, int64_t* stats, int32_t n);
  *   D2G_TUNE_GRID_MIN_PARTS (default 768, >= 0): a cluster with at least
  *     128 contacts and more parts than this is solved by a cooperative grid
  *     over the SMs, when at most 8 clusters of the solve call qualify.
- *   D2G_TUNE_SOLVE_LANES (default 0; 0, 4 or 16): has no effect any more (the
- *     solve takes 8 or 16 lanes a contact by its waves' widths); kept so that
- *     settings files still apply.
+ *   D2G_TUNE_SOLVE_LANES (default 0; 0, 4 or 16): lanes of the solve's
+ *     normal-impulse waves: 16 a contact wherever a block has at most four
+ *     contacts in a wave, 4 a body side of a contact throughout, or 0: by the
+ *     block's contacts per wave.
  *   D2G_TUNE_SPIN_LIMIT (default 33554432, >= 1): polls a block of the
  *     cooperative-grid solve makes at a grid barrier before it gives up
  *     (several seconds at the default); a call whose barrier gave up returns
