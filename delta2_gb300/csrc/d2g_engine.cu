@@ -2685,10 +2685,9 @@ void emit_records(d2g_ctx* ctx, int n, const int32_t* flags, const int32_t* off,
 int ee_grid_size(d2g_ctx* ctx, int* grid) {
     Engine& E = ctx->eng;
     if (E.ee_grid == 0) {
-        int dev_sms = 0, per_sm = 0;
-        D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
+        int per_sm = 0;
         D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ee_rest4, kBlock, 0));
-        E.ee_grid = std::max(1, dev_sms * std::max(1, per_sm));
+        E.ee_grid = std::max(1, ctx->n_sms * std::max(1, per_sm));
     }
     *grid = E.ee_grid;
     return D2G_OK;
@@ -2696,16 +2695,7 @@ int ee_grid_size(d2g_ctx* ctx, int* grid) {
 
 // Grid of the kernels that test a level's undecided slots, whose number they
 // read from device memory too: a few warps per SM sub-partition.
-int slot_grid_size(d2g_ctx* ctx, int* grid) {
-    Engine& E = ctx->eng;
-    if (E.slot_grid == 0) {
-        int dev_sms = 0;
-        D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
-        E.slot_grid = 3 * dev_sms;
-    }
-    *grid = E.slot_grid;
-    return D2G_OK;
-}
+int slot_grid_size(d2g_ctx* ctx) { return 3 * ctx->n_sms; }
 
 // Bytes a traversal level may use for its buffers: a sixth of the device
 // memory (the rest holds the scene, the contact records with their sorted
@@ -2913,9 +2903,11 @@ int descend(d2g_ctx* ctx, int n, bool self_leaf, double budget, bool may_abandon
     if (new_leaf > (self_leaf && T.levels == 1 ? T.n_root : 0)) T.levels++;
     return D2G_OK;
 }
-// Blocks for a level's kernels, a warp a node pair: running ahead, as many as
-// are resident at once (the kernels stride).
-int level_blocks(int n, bool ahead) { return ahead ? std::min(nblocks(32LL * n), 152 * 8) : nblocks(32LL * n); }
+// Blocks for a level's kernels, a warp a node pair: running ahead, eight an SM,
+// about what is resident at once (the kernels stride).
+int level_blocks(d2g_ctx* ctx, int n, bool ahead) {
+    return ahead ? std::min(nblocks(32LL * n), 8 * ctx->n_sms) : nblocks(32LL * n);
+}
 
 // The FP64 tests of the descent's leaf pairs (E.conn, in level order), and of
 // the chunk's root pairs that are two leaves (soup stage: the best of a
@@ -3079,8 +3071,7 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
     RC(E.pfut.ensure(28 * (size_t)n_pairs + 1));
     RC(E.search.ensure(n_pairs + 1));
     RC(E.soup.ensure(n_pairs + 1));
-    int test_grid = 0;
-    RC(slot_grid_size(ctx, &test_grid));
+    const int test_grid = slot_grid_size(ctx);
     int n_rec = 0;
     long long n_streamed = 0;  // records handed to the sink
     if (n_pairs > 0)
@@ -3139,7 +3130,7 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
                        E.wt_table.p, E.wt_log2cap, E.wt_flag.p, E.ccd_stats.p);
                 eskip = E.wt_flag.p;
             }
-            k_ccd_level<<<level_blocks(n_soup, n_dev != nullptr), kBlock, 0, s>>>(
+            k_ccd_level<<<level_blocks(ctx, n_soup, n_dev != nullptr), kBlock, 0, s>>>(
                 n_soup, soup, d_pairs, E.pm.p, E.pm32c.p, ctx->ntris.p, ctx->tris.p, ctx->tri32.p, ctx->geo_eps.p,
                 E.search.p, ctx->nodes.p, skip, eskip, E.fp32_bounds ? 1 : 0, E.certificates ? 1 : 0, hits,
                 E.ccd_list.p, lc, n_dev);
@@ -3254,8 +3245,8 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
     if (n_pairs > 0)
         LAUNCH(k_np_prep, n_pairs, n_pairs, d_pairs, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p,
                E.pm.p, E.search.p, E.roots.p, E.pm32.p, nullptr);
-    int n_rec = 0, test_grid = 0;
-    RC(slot_grid_size(ctx, &test_grid));
+    const int test_grid = slot_grid_size(ctx);
+    int n_rec = 0;
     // pair chunks, as in run_ccd
     const double budget = level_budget(ctx);
     // a leaf pair's slots take ~110 bytes each (x1.5 growth slack)
@@ -3271,7 +3262,7 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
                                                                    const int32_t* n_dev) -> int {
             const Entry* front = E.soup.p + r0;
             int32_t* hits = E.entry_hits.p + r0;
-            k_np_filter<false><<<level_blocks(n, n_dev != nullptr), kBlock, 0, s>>>(
+            k_np_filter<false><<<level_blocks(ctx, n, n_dev != nullptr), kBlock, 0, s>>>(
                 n, front, E.pm32.p, ctx->ntris.p, ctx->tri_sph.p, ctx->tri32.p, ctx->eps_up.p, E.search.p,
                 ctx->nodes.p, E.fp32_bounds ? 1 : 0, nullptr, nullptr, hits, E.ccd_list.p, lc, n_dev);
             E.launches++;

@@ -205,7 +205,7 @@ struct Engine {
     // phased edge-edge CCD (d2g_engine.cu)
     DBuf<double> ee_rec;
     DBuf<int32_t> ee_work;
-    int ee_grid = 0, slot_grid = 0;  // k_ee_rest4 grid (every block resident); grid of the level tests
+    int ee_grid = 0;  // k_ee_rest4 grid (every block resident)
     // traversal chunking: root entries of the call's pairs; a byte budget for
     // a level's buffers (0: a third of the device memory)
     DBuf<Entry> roots;
@@ -260,6 +260,7 @@ struct d2g_ctx {
     // joined back into `stream` by the two events)
     cudaStream_t stream2 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    int n_sms = 0;  // of the device
     // trees
     int n_meshes = 0, n_nodes = 0;
     int max_depth = 0;  // of the meshes' trees (a root is 0)

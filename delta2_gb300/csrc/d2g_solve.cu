@@ -51,7 +51,7 @@ inline int nblocks(long long n, int b = kBlock) { return (int)((n + b - 1) / b);
 // call on 4,000 contacts in 300 pairs, and 12 launches in a solve.)
 constexpr int kSegSmall = 1024;        // elements of the 128-thread kernels' shared memory
 constexpr int kSegLarge = 8192;        // ... of the 1,024-thread kernels'
-constexpr int kSegSmallBlock = 128, kSegLargeBlock = 1024, kSegLargeGrid = 152;
+constexpr int kSegSmallBlock = 128, kSegLargeBlock = 1024;
 constexpr int kSegLargeSmem = 20 * kSegLarge, kOrderSmem = 12 * kSegLarge;
 typedef unsigned long long u64;
 
@@ -1448,7 +1448,7 @@ int run_filter(d2g_ctx* ctx, const int32_t* d_off, const double* d_rec, int n_pa
         ctx->eng.launches++;
         if (n_rec > kSegSmall) {  // (else no pair has more)
             RC(allow_segment_smem(ctx));
-            k_filter_large<<<kSegLargeGrid, kSegLargeBlock, kSegLargeSmem, s>>>(f);
+            k_filter_large<<<ctx->n_sms, kSegLargeBlock, kSegLargeSmem, s>>>(f);
             ctx->eng.launches++;
         }
         size_t bytes = 0;
@@ -1580,7 +1580,7 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
         ctx->eng.launches++;
         if (n_con > kSegSmall) {
             RC(allow_segment_smem(ctx));
-            k_order_large<<<kSegLargeGrid, kSegLargeBlock, kOrderSmem, s>>>(f);
+            k_order_large<<<ctx->n_sms, kSegLargeBlock, kOrderSmem, s>>>(f);
             ctx->eng.launches++;
         }
     }
@@ -1730,11 +1730,10 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
             D2G_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
         }
         if (!big.empty()) {
-            int dev_sms = 0, per_sm = 0;
-            D2G_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
+            int per_sm = 0;
             a.smem = kSolveSmemMax;
             D2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_grid, kSolveBlock, a.smem));
-            const int G_max = std::max(1, std::min(dev_sms, dev_sms * per_sm));
+            const int G_max = std::max(1, std::min(ctx->n_sms, ctx->n_sms * per_sm));
             RC(E.sv_grid.ensure(16 * big.size() + 16));
             D2G_CUDA(cudaMemsetAsync(E.sv_grid.p, 0, (16 * big.size() + 16) * sizeof(int32_t), s));
             for (size_t b = 0; b < big.size(); b++) {

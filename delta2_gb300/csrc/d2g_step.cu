@@ -192,7 +192,7 @@ __device__ void block_lmin(double& v, int& i, double* red_v, int* red_i) {
 }
 
 constexpr int kStepsBlock = 256;
-constexpr int kScaleGrid = 152 * 4;  // a warp per sub-partition for the FP64 pipe, four to hide loads
+constexpr int kScaleBlocks = 4;  // blocks an SM: a warp per sub-partition for the FP64 pipe, four to hide loads
 constexpr int kStepsChunk = 1024;  // interactions staged per pass
 
 // The reference's order-dependent propagation over a cluster's interactions
@@ -697,7 +697,7 @@ int run_select_steps(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, const in
                                                                          c->inv_inertia.p, En.st_spin.p, En.st_best.p);
                 En.launches++;
             }
-            k_contact_scale<<<kScaleGrid, kBlock, 0, c->stream>>>(np, mt, En.out_off.p, En.rec_sorted.p, fut,
+            k_contact_scale<<<kScaleBlocks * c->n_sms, kBlock, 0, c->stream>>>(np, mt, En.out_off.p, En.rec_sorted.p, fut,
                                                                     En.st_spin.p, En.st_best.p);
             k_pair_new_dt<<<nblocks(np), kBlock, 0, c->stream>>>(np, mt, En.out_off.p, En.st_best.p,
                                                                  En.st_new_dt.p + p0, En.st_has.p + p0, first ? 1 : 0);
