@@ -121,6 +121,16 @@ def choose_grid_threshold(totals):
     return min(v for v, t in totals.items() if t <= 1.01 * best)
 
 
+EE_FIRST_ITERS = 2  # the library's default
+
+
+def choose_first_iters(ms):
+    """The library's default where it is within 1% of the fastest (what two
+    runs of one value differ by), else the fastest."""
+    best = min(ms, key=ms.get)
+    return EE_FIRST_ITERS if ms.get(EE_FIRST_ITERS, float("inf")) <= 1.01 * ms[best] else best
+
+
 def main():
     p = argparse.ArgumentParser()
     p.add_argument("--out", default=DEFAULT_OUT)
@@ -139,7 +149,7 @@ def main():
     for kind in {k for k, _ in world_dig}:
         if len({d for (k, _), d in world_dig.items() if k == kind}) != 1:
             raise SystemExit(f"grid_min_parts changed the {kind} states: {world_dig}")
-    best_ee = min(ccd_ms, key=ccd_ms.get)
+    best_ee = choose_first_iters(ccd_ms)
     totals = {v: sum(world_s[(k, v)] for k, vv in world_s if vv == v) for v in grid_values}
     best_grid = choose_grid_threshold(totals)
     import torch
