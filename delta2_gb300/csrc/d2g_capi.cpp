@@ -421,7 +421,6 @@ void d2g_ctx_destroy(d2g_ctx* c) {
     E.soup.release();
     E.conn.release();
     E.soup_next.release();
-    E.conn_next.release();
     E.entry_hits.release();
     E.off_a.release();
     E.flags.release();

@@ -1170,10 +1170,9 @@ __global__ void __launch_bounds__(kPrimBlock) k_prim_pt(int n_tp, int n_total, c
                                                         PrimResult* __restrict__ sub, PrimResult* __restrict__ cres,
                                                         int32_t* __restrict__ chit, const int32_t* __restrict__ list,
                                                         const int32_t* __restrict__ n_list) {
-    // work item list[kk] (every item when list is null)
     const int kk = blockIdx.x * blockDim.x + threadIdx.x;
-    if (kk >= n_total || (n_list && kk >= *n_list)) return;
-    const int j = list ? list[kk] : kk;
+    if (kk >= n_total || kk >= *n_list) return;
+    const int j = list[kk];
     if (j < 6 * n_tp) {
         const int k = j / 6, w = j % 6;
         const int slot = items[k];

@@ -134,7 +134,7 @@ struct PrimResult {
 
 struct Engine {
     // frontiers
-    DBuf<Entry> soup, conn, soup_next, conn_next;
+    DBuf<Entry> soup, conn, soup_next;
     // per-entry counters / offsets
     DBuf<int32_t> entry_hits, off_a;
     // items of a stage

@@ -1538,12 +1538,6 @@ int launch_solve_cl(d2g_ctx* ctx, int cs, int n, const int32_t* d_list, int32_t*
     return D2G_OK;
 }
 
-// Blocks that serve a cluster of np particles best: a wave holds a seventh to
-// a quarter as many contacts as the cluster has particles, four to a task, and
-// a block that has a single task in a wave takes the faster form of the halves
-// (measured: the table in run_solve).
-int best_cluster_size(int np) { return np > kOneBlockParts ? 16 : 1; }
-
 // Solve clusters.  Contacts (14-double records in the reference's hit order,
 // clusters contiguous per d_con_off) with per-contact pair counts and warm
 // values (NaN = none).  Outputs: status / iteration counts per cluster, the
@@ -1637,7 +1631,7 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
         // a contact on one warp: 331 for the 8 cubes, 257 for the 1,024 hulls.)
         // A block barrier costs ~0.1 us, the cluster barrier with distributed
         // shared memory ~0.5 us more, a grid barrier ~1.5 us: so one block up
-        // to kOneBlockParts particles, then 16 (best_cluster_size), or the most
+        // to kOneBlockParts particles, then 16, or the most
         // with which all such clusters of the call are resident at once, and a
         // cooperative grid for a cluster with at least kGridMinContacts contacts
         // and more than D2G_TUNE_GRID_MIN_PARTS parts (768 by default, between
@@ -1660,7 +1654,7 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
             }
             const int nck = h_con_off ? h_con_off[c + 1] - h_con_off[c] : 0;
             const int npk = h_con_off && h_part_off ? h_part_off[c + 1] - h_part_off[c] : 0;
-            const bool wide = cl_setting > 1 || (cl_setting == 0 && best_cluster_size(npk) > 1);
+            const bool wide = cl_setting > 1 || (cl_setting == 0 && npk > kOneBlockParts);
             if (h_con_off && wide && nck >= kClusterMinContacts)
                 mid.push_back(c);
             else
@@ -1671,10 +1665,7 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
             if (cl_setting > 1) {
                 cs = cl_setting;
             } else {
-                int most = 1;
-                for (int c : mid) most = std::max(most, best_cluster_size(h_part_off[c + 1] - h_part_off[c]));
                 for (int cand : {16, 8, 4, 2}) {
-                    if (cand > most) continue;
                     int fit = 0;
                     RC(max_solve_clusters(ctx, cand, &fit));
                     if (fit >= (int)mid.size()) {
