@@ -509,7 +509,7 @@ int d2g_ctx_set_trees(d2g_ctx* c, const d2g_trees* t) {
     for (int g = 0; g < N; g++) {
         const int32_t* nd = t->nodes + 4 * (size_t)g;
         if (t->ntris[g] < 0 || t->ntris[g] > 8 || nd[1] < 0 || nd[1] > 8 ||
-            (nd[2] && (nd[0] < 0 || nd[0] + nd[1] > N)) || (!nd[2] && nd[1] != 0)) {
+            (nd[2] && (nd[0] < 0 || nd[0] > N - nd[1])) || (!nd[2] && nd[1] != 0)) {
             set_error("invalid node " + std::to_string(g));
             return D2G_ERR_INVALID;
         }

@@ -3457,7 +3457,7 @@ __global__ void k_noalloc_validate(int n_pairs, const int32_t* __restrict__ pair
     }
     if (i < n_nodes) {
         const int4 nd = nodes[i];
-        if (ntris[i] < 0 || ntris[i] > 8 || nd.y < 0 || nd.y > 8 || (nd.z && (nd.x < 0 || nd.x + nd.y > n_nodes)))
+        if (ntris[i] < 0 || ntris[i] > 8 || nd.y < 0 || nd.y > 8 || (nd.z && (nd.x < 0 || nd.x > n_nodes - nd.y)))
             atomicExch(err, 1);
     }
 }

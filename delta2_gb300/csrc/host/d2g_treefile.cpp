@@ -153,7 +153,7 @@ bool load_trees(const char* path, TreeSet& t, std::string* err) {
         for (int i = a; i < b; i++) {
             const int child = t.nodes[4 * (size_t)i], count = t.nodes[4 * (size_t)i + 1];
             if (t.ntris[i] < 0 || t.ntris[i] > 8) return fail("bucket size out of range");
-            if (child != -1 && (child < a || child >= b || count < 0 || child + count > b))
+            if (child != -1 && (child < a || child >= b || count < 0 || count > b - child))
                 return fail("child link outside its mesh");
         }
     }
