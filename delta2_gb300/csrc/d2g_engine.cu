@@ -208,17 +208,31 @@ __device__ __forceinline__ float box_gap(const Box32& a, const Box32& b) {
     return sqrtf(g2);
 }
 
-// Indices of PM_* matrices in the FP32 pose block (8 x 12 floats per pair).
+// Indices of PM_* matrices in the FP32 pose block: 8 x 12 floats per pair, then
+// for the poses AS, AE, BS, BE whether they keep distances.
+constexpr int kPose32 = 100;
 __device__ __forceinline__ const float* pm32_of(const float* pm32, int pair, int which) {
-    return pm32 + (size_t)96 * pair + 12 * which;
+    return pm32 + (size_t)kPose32 * pair + 12 * which;
 }
 enum { P32_AS = 0, P32_AE, P32_BS, P32_BE, P32_ABS, P32_ABE, P32_BAS, P32_BAE };
 
+// A pose's rotation comes from the state's quaternion as it is, which a caller
+// may have set to any length: it keeps distances (to 3e-6 of themselves) when
+// its columns are orthonormal to 2e-6, FP32 rounding taking 3e-7 of that.
+__device__ __forceinline__ bool keeps_distances(const double* __restrict__ M) {
+    const F3 x = f3((float)M[0], (float)M[4], (float)M[8]), y = f3((float)M[1], (float)M[5], (float)M[9]),
+             z = f3((float)M[2], (float)M[6], (float)M[10]);
+    const float d = fmaxf(fmaxf(fabsf(dot3(x, y)), fabsf(dot3(y, z))), fabsf(dot3(z, x)));
+    const float l = fabsf(dot3(x, x) - 1.f) + fabsf(dot3(y, y) - 1.f) + fabsf(dot3(z, z) - 1.f);
+    return d < 2e-6f && l < 2e-6f;  // false for NaN: l is one then
+}
+
 __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restrict__ pm32) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * 96) return;
-    const int p = i / 96, w = (i % 96) / 12, r = i % 12;
-    pm32[i] = (float)pm[(size_t)PM_SIZE * p + 16 * w + r];
+    if (i >= n * kPose32) return;
+    const int p = i / kPose32, w = (i % kPose32) / 12, r = i % kPose32 - 12 * w;
+    const double* M = pm + (size_t)PM_SIZE * p;
+    pm32[i] = w < 8 ? (float)M[16 * w + r] : (keeps_distances(M + 16 * r) ? 1.f : 0.f);
 }
 
 // The swept-AABB prefilter of every (triangle of a, triangle of b) slot of a
@@ -1041,7 +1055,8 @@ __device__ __forceinline__ void warp_append(int j, bool keep, int32_t* list, int
 // its projection is outside the triangle or it is too far above the plane.
 // Both in FP32 with margins: the box's as for k_ccd_mask_ee; the plane's in
 // the triangle's frame (PlaneBound, which covers the reference's single-
-// precision barycentrics).
+// precision barycentrics), whose heights are distances only under poses that
+// keep them, and those come with the FP64 rounding of the world coordinates.
 __device__ __forceinline__ bool pt_apart(const float* __restrict__ pm32, int pair, int mC, int mT, const float* pt,
                                          const float* tv, float thr) {
     const float *Cs = pm32_of(pm32, pair, mC), *Ce = pm32_of(pm32, pair, mC + 1);
@@ -1064,6 +1079,8 @@ __device__ __forceinline__ bool pt_apart(const float* __restrict__ pm32, int pai
         box_add(bq, tE, tv[3 * v], tv[3 * v + 1], tv[3 * v + 2], o, mag);
     }
     if (box_gap(bp, bq) > thr + (1e-3f + 4e-6f * (mag + thr))) return true;  // NaN: not certain
+    const float* keeps = pm32_of(pm32, pair, 8);
+    if (keeps[mT] == 0.f || keeps[mT + 1] == 0.f) return false;
     const F3 T0 = f3(tv[0], tv[1], tv[2]), T1 = f3(tv[3], tv[4], tv[5]), T2 = f3(tv[6], tv[7], tv[8]);
     const F3 p0 = f3(ps[0], ps[1], ps[2]), p1 = f3(pe[0], pe[1], pe[2]);
     // the frame's coordinates carry an error of 4e-7 of their size, 1e-6 here
@@ -1074,7 +1091,7 @@ __device__ __forceinline__ bool pt_apart(const float* __restrict__ pm32, int pai
     const float h0 = dot3(P.n, q[0]), h1 = dot3(P.n, q[1]);
     const float err = 2.f * P.eh * 8.f * rho;
     if (!((h0 > err && h1 > err) || (h0 < -err && h1 < -err))) return false;
-    const float lim = (thr + (2e-5f + 4e-6f * (8.f * rho + thr))) * P.len + err;
+    const float lim = (thr + (2e-5f + 1e-13f * mag + 4e-6f * (8.f * rho + thr))) * P.len + err;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         float u, v, w;
@@ -3076,8 +3093,8 @@ int run_ccd(d2g_ctx* ctx, const int32_t* d_pairs, const double* d_max_time, int 
     if (n_pairs > 0)
         LAUNCH(k_ccd_prep, 4LL * n_pairs, n_pairs, d_pairs, d_max_time, ctx->cur.p, ctx->inv_inertia.p, ctx->mesh.p,
                ctx->mesh_node_off.p, ctx->geo_eps.p, E.pm.p, E.pfut.p, E.search.p, E.soup.p);
-    RC(E.pm32c.ensure((size_t)96 * n_pairs + 1));
-    if (n_pairs > 0) LAUNCH(k_ccd_pm32, 96LL * n_pairs, n_pairs, E.pm.p, E.pm32c.p);  // FP32 poses, once per call
+    RC(E.pm32c.ensure((size_t)kPose32 * n_pairs + 1));
+    if (n_pairs > 0) LAUNCH(k_ccd_pm32, (long long)kPose32 * n_pairs, n_pairs, E.pm.p, E.pm32c.p);  // FP32 poses, once per call
     // The learned proposal: the network predicts which queries have no
     // contact; the root certificate proves it for those it can, and the
     // proven ones are skipped (their outputs are empty either way).
