@@ -258,8 +258,9 @@ __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restri
 // NaN) forms the FP64 boxes and decides those slots exactly.
 // res[h]: the swept boxes of slot lane + 32 h overlap.  verts: the warp's 16
 // triangles (a's, then b's) in FP32 at the start, [16][9], ends: at the end;
-// mags: the largest coordinate of each, for the margins (huge where a triangle
-// allows no certain hit).
+// mags: the largest coordinate of each, for the margins (infinite where a
+// triangle's edges could vanish or its coordinates pass FP32's range: then
+// nothing is certain).
 __device__ __forceinline__ void swept_slots(const Entry& e, const int32_t* __restrict__ pairs,
                                             const double* __restrict__ pm, const float* __restrict__ pm32,
                                             const int32_t* __restrict__ ntris, const double* __restrict__ tris,
@@ -322,7 +323,7 @@ __device__ __forceinline__ void swept_slots(const Entry& e, const int32_t* __res
                 }
                 steady = steady && l2 > 1e-8f && c2 < 0.2f * l2;
             }
-            mags[lane] = steady ? mag : 3.4e38f;
+            mags[lane] = steady ? mag : INFINITY;
         }
     }
     bool border = false;
@@ -521,7 +522,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_level(
                     F3 d;
                     const float m = edge_min(s_verts[wi][ta], s_verts[wi][8 + tb], d);
                     if (m < room[h]) sure = true;
-                    // (s_mag is huge for an unsteady triangle: never clear either)
+                    // (s_mag is infinite for an unsteady triangle: never clear either)
                     clear[h] = certificates &&
                                tri_gap_motion(d, s_verts[wi][ta], s_verts[wi][8 + tb], s_ends[wi][ta],
                                               s_ends[wi][8 + tb]) >

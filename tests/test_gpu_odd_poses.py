@@ -1,6 +1,7 @@
 """Continuous queries of bodies whose orientation is not a unit quaternion: the
 pose's linear part scales and shears, and the reference measures distances
-after it.  Contacts, offsets and futures against the oracle, bit for bit."""
+after it; a huge one gives coordinates beyond FP32's range.  Contacts, offsets
+and futures against the oracle, bit for bit."""
 import numpy as np
 import pytest
 
@@ -52,3 +53,14 @@ def test_continuous_queries_match_oracle(ctx, config, mt, form):
         pairs = D.broad_phase(D.make_scene(config, nx=2, ny=2, nz=1, spacing=0.9, speed_sigma=0.0, seed=seed))
         total += ccd_against_oracle(ctx, s, pairs, np.full(len(pairs), mt))
     assert total > 0
+
+
+@pytest.mark.parametrize("seed", range(4))
+@pytest.mark.parametrize("value", [1e15, 1e18, 1e19, 1e20, 1e22, 1e100])
+def test_coordinates_beyond_fp32_match_oracle(ctx, value, seed):
+    for comp in range(1, 5):
+        s = D.make_scene(1, nx=2, ny=2, nz=1, spacing=1.2, speed_sigma=0.0, seed=seed)
+        moving = np.flatnonzero(s.is_static == 0)
+        s.cur[moving[seed], comp] = value
+        pairs = D.broad_phase(D.make_scene(1, nx=2, ny=2, nz=1, spacing=1.0, speed_sigma=0.0, seed=seed))
+        ccd_against_oracle(ctx, s, pairs, np.full(len(pairs), 0.02))
