@@ -1947,10 +1947,8 @@ __device__ __forceinline__ float normal_gap(const float* n, const float* v) {
 }
 
 // Marks a slot of k_np_filter's list that only the whole distance decides: a
-// triangle that is a point or not finite, or poses (metres) so far out that a
-// small triangle could become a point there.
+// triangle that is a point or not finite, or one that is kFarSizes away.
 constexpr int kWholeTest = kSlotMark;
-constexpr float kWorldMax = 1e6f;
 
 template <bool LEAF>
 __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const Entry* __restrict__ front,
@@ -1963,8 +1961,8 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                                                       int32_t* __restrict__ entry_hits, int32_t* __restrict__ list,
                                                       int32_t* __restrict__ lc, const int32_t* __restrict__ n_dev) {
     __shared__ float s_v[kBlock / 32][16][9];
-    // centre, radius, eps, magnitude, 1 for a triangle that is a point or not
-    // finite, unit normal, the triangle's own range along it
+    // centre, radius, eps, magnitude, size (0 for a triangle that is a point or
+    // not finite), unit normal, the triangle's own range along it
     __shared__ float s_c[kBlock / 32][16][13];
     __shared__ uint8_t s_slot[kBlock / 32][64];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -2004,7 +2002,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
             float ext = 0.f;
 #pragma unroll
             for (int r = 0; r < 3; r++) ext = fmaxf(ext, fmaxf(fabsf(v[3 + r] - v[r]), fabsf(v[6 + r] - v[r])));
-            c[6] = ext > 1e-5f && ext < 1e15f ? 0.f : 1.f;
+            c[6] = ext > 1e-5f && ext < 1e15f ? ext : 0.f;
             F3 nn = cross3(f3(v[3] - v[0], v[4] - v[1], v[5] - v[2]), f3(v[6] - v[0], v[7] - v[1], v[8] - v[2]));
             const float len = sqrtf(dot3(nn, nn)), inv = len > 1e-20f ? 1.f / len : 0.f;
             nn = f3(nn.x * inv, nn.y * inv, nn.z * inv);
@@ -2031,7 +2029,8 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                 const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb0], *va = s_v[wi][ta], *vb = s_v[wi][8 + tb0];
                 const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
                 const float thr = se + ca[4] + cb[4];
-                const float lim = thr + ((ca[6] + cb[6] == 0.f ? 2e-5f : 1e-3f) + 4e-6f * (tm + ca[5] + cb[5] + thr));
+                const float lim =
+                    thr + ((fminf(ca[6], cb[6]) > 0.f ? 2e-5f : 1e-3f) + 4e-6f * (tm + ca[5] + cb[5] + thr));
                 keep = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
                        !(box_gap9(va, vb) > lim) && !(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim);
             }
@@ -2046,7 +2045,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
             __syncwarp();
             auto room = [&](const float* ca, const float* cb) {
                 const float thr = se + ca[4] + cb[4];
-                return ca[6] + cb[6] == 0.f ? thr - (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr)) : -1.f;
+                return fminf(ca[6], cb[6]) > 0.f ? thr - (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr)) : -1.f;
             };
             if (!LEAF) {
                 bool sure = false;
@@ -2072,7 +2071,8 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                     break;
                 }
                 const float thr = se + ca[4] + cb[4], lim = thr + (2e-5f + 4e-6f * (tm + ca[5] + cb[5] + thr));
-                const unsigned bit = ca[6] + cb[6] != 0.f || !(axis_gap9(d, va, vb) > lim) ? 1u << (sl & 31) : 0u;
+                const bool kept = !(fminf(ca[6], cb[6]) > 0.f) || !(axis_gap9(d, va, vb) > lim);
+                const unsigned bit = kept ? 1u << (sl & 31) : 0u;
                 m[0] |= __reduce_or_sync(0xffffffffu, sl < 32 ? bit : 0u);
                 m[1] |= __reduce_or_sync(0xffffffffu, sl < 32 ? 0u : bit);
             }
@@ -2092,7 +2092,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
             } else {
                 const bool keep = (m[h] >> lane) & 1u;
                 const bool whole = keep && use_bounds &&
-                                   !(s_c[wi][ta0 + 4 * h][6] + s_c[wi][8 + tb0][6] == 0.f && tm < kWorldMax);
+                                   !(tm < 0.1f * kFarSizes * fminf(s_c[wi][ta0 + 4 * h][6], s_c[wi][8 + tb0][6]));
                 warp_append((64 * w + lane + 32 * h) | (whole ? kWholeTest : 0), keep, list, lc + LC_LIST);
             }
         }

@@ -22,8 +22,8 @@
 //
 // tri_tri_dist of two triangles none of whose features has a distance (a
 // triangle that is a point, coordinates that are not finite) is 0 at the
-// origin: what all its comparisons leave.  Triangles that are not tri_regular
-// take the plain function, which alone knows.
+// origin: what all its comparisons leave.  Triangles that are not tri_regular,
+// or kFarSizes away, take the plain function, which alone knows.
 #pragma once
 #include "d2g_geom.cuh"
 
@@ -89,6 +89,10 @@ D2G_HD bool edges_stay_apart(const F3 (&p)[2][4], float lim) {
 // pair has a finite distance.  s: the squared lengths of the edges at the first
 // vertex.
 D2G_HD bool tri_regular(float s) { return s > 1e-30f && s < 1e30f; }  // false for NaN
+// A triangle further from the origin than this many of its sizes: FP64 rounding
+// at its place, 1e-16 of the distance, comes near the bounds' margin of its
+// barycentric coordinates (1e-5).
+constexpr float kFarSizes = 1e10f;
 
 // tri_tri_dist, out of line: hardly ever called beside the bounds.
 #ifdef __CUDA_ARCH__
@@ -182,7 +186,8 @@ D2G_HD double tri_tri_dist_below(const Tri& a, const Tri& b, double limit, V3& P
     const float mag = (float)(fabs(o.x) + fabs(o.y) + fabs(o.z));
     const float margin = 4e-6f * rho + 1e-13f * mag + 1e-30f;
     const PlaneBound pa = plane_bound(A[0], A[1], A[2], rho), pb = plane_bound(B[0], B[1], B[2], rho);
-    if (!(tri_regular(pa.d00 + pa.d11) && tri_regular(pb.d00 + pb.d11))) {
+    const float sa = pa.d00 + pa.d11, sb = pb.d00 + pb.d11;
+    if (!(tri_regular(sa) && tri_regular(sb) && mag < kFarSizes * sqrtf(fminf(sa, sb)))) {
         const Tri ca = a, cb = b;  // (in memory for the call; a, b, P and Q stay in registers)
         V3 p, q;
         const double d = tri_tri_dist_plain(ca, cb, p, q);
