@@ -1906,7 +1906,7 @@ __global__ void k_soup_fold(int K, const int32_t* __restrict__ items, const Entr
 // either.  (A triangle that is a point, or not finite, is the exception: the
 // reference's distance to it can be 0 with no feature at all (d2g_prune.cuh),
 // wherever the other triangle is.  Such slots are kept within 1 mm of the limit
-// by the spheres, boxes and normals, and decided by the whole distance.)
+// by the spheres and boxes, and decided by the whole distance.)
 //
 // A warp per node pair: lanes 0-7 transform a's triangles, 8-15 b's, once each
 // into shared memory, with their normals; every lane takes two of the 64 slots
@@ -2029,10 +2029,11 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                 const float *ca = s_c[wi][ta], *cb = s_c[wi][8 + tb0], *va = s_v[wi][ta], *vb = s_v[wi][8 + tb0];
                 const float dx = ca[0] - cb[0], dy = ca[1] - cb[1], dz = ca[2] - cb[2];
                 const float thr = se + ca[4] + cb[4];
-                const float lim =
-                    thr + ((fminf(ca[6], cb[6]) > 0.f ? 2e-5f : 1e-3f) + 4e-6f * (tm + ca[5] + cb[5] + thr));
+                const bool plain = !(fminf(ca[6], cb[6]) > 0.f);
+                const float lim = thr + ((plain ? 1e-3f : 2e-5f) + 4e-6f * (tm + ca[5] + cb[5] + thr));
                 keep = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
-                       !(box_gap9(va, vb) > lim) && !(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim);
+                       !(box_gap9(va, vb) > lim) &&
+                       (plain || (!(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim)));
             }
             m[h] = __ballot_sync(0xffffffffu, keep);
         }

@@ -100,7 +100,8 @@ def _scene(inner, point, fut):
     s = SmallScene()
     s.add_leaf_mesh(FLAT)
     s.add_leaf_mesh([list(point) * 3])
-    s.add_body(0, 0.01)
+    tilt = TILTED if point[0] > 0.5 else state()
+    s.add_body(0, 0.01, cur=tilt, fut=tilt)
     s.add_body(1, 0.01, cur=fut, fut=fut)
     sc = s.build().to_product()
     if inner:
@@ -120,7 +121,9 @@ CASES = {
     "just beyond": ((-0.0204, 0.5, 0.0), state()),  # 0.4 mm past the limit of 20 mm
     "nan pose": ((0.1, 0.1, 0.005), NAN_X),
     "infinite pose": ((0.1, 0.1, 0.005), INF_X),
+    "beside a face": ((0.9, 0.6, 0.1), state()),  # in the tilted triangle's box, 0.35 m off its plane
 }
+TILTED = state(q=(np.cos(np.pi / 8), np.sin(np.pi / 8), 0, 0))
 
 
 @pytest.mark.gpu
