@@ -84,6 +84,20 @@ __global__ void k_ccd_prep(int n, const int32_t* __restrict__ pairs, const doubl
 }
 
 // Discrete narrow phase prep: future transforms of a and b (comparison_dist.h:225,229).
+// A pose's rotation comes from the state's quaternion as it is, which a caller
+// may have set to any length: it keeps distances (to 3e-6 of themselves) when
+// its columns are orthonormal to 2e-6, FP32 rounding taking 3e-7 of that.
+__device__ __forceinline__ bool keeps_distances(const double* __restrict__ M) {
+    const F3 x = f3((float)M[0], (float)M[4], (float)M[8]), y = f3((float)M[1], (float)M[5], (float)M[9]),
+             z = f3((float)M[2], (float)M[6], (float)M[10]);
+    const float d = fmaxf(fmaxf(fabsf(dot3(x, y)), fabsf(dot3(y, z))), fabsf(dot3(z, x)));
+    const float l = fabsf(dot3(x, x) - 1.f) + fabsf(dot3(y, y) - 1.f) + fabsf(dot3(z, z) - 1.f);
+    return d < 2e-6f && l < 2e-6f;  // false for NaN: l is one then
+}
+
+// The discrete phase's FP32 poses: rows 0-2 of both, then whether both keep
+// distances.
+constexpr int kNpPose32 = 25;
 __global__ void k_np_prep(int n, const int32_t* __restrict__ pairs, const double* __restrict__ fut,
                           const int32_t* __restrict__ mesh, const int32_t* __restrict__ mesh_node_off,
                           const double* __restrict__ geo_eps, double* __restrict__ pm, float* __restrict__ search,
@@ -96,11 +110,13 @@ __global__ void k_np_prep(int n, const int32_t* __restrict__ pairs, const double
     double* M = pm + 32 * (size_t)p;
     transformation(fa.q, fa.x, M);
     transformation(fb.q, fb.x, M + 16);
-    if (pm32)  // rows 0-2 of both poses in FP32, for the candidate prefilter
+    if (pm32) {
         for (int k = 0; k < 12; k++) {
-            pm32[24 * (size_t)p + k] = (float)M[k];
-            pm32[24 * (size_t)p + 12 + k] = (float)M[16 + k];
+            pm32[kNpPose32 * (size_t)p + k] = (float)M[k];
+            pm32[kNpPose32 * (size_t)p + 12 + k] = (float)M[16 + k];
         }
+        pm32[kNpPose32 * (size_t)p + 24] = keeps_distances(M) && keeps_distances(M + 16) ? 1.f : 0.f;
+    }
     search[p] = (float)(geo_eps[a] + geo_eps[b]);
     Entry e;
     e.pair = p;
@@ -215,17 +231,6 @@ __device__ __forceinline__ const float* pm32_of(const float* pm32, int pair, int
     return pm32 + (size_t)kPose32 * pair + 12 * which;
 }
 enum { P32_AS = 0, P32_AE, P32_BS, P32_BE, P32_ABS, P32_ABE, P32_BAS, P32_BAE };
-
-// A pose's rotation comes from the state's quaternion as it is, which a caller
-// may have set to any length: it keeps distances (to 3e-6 of themselves) when
-// its columns are orthonormal to 2e-6, FP32 rounding taking 3e-7 of that.
-__device__ __forceinline__ bool keeps_distances(const double* __restrict__ M) {
-    const F3 x = f3((float)M[0], (float)M[4], (float)M[8]), y = f3((float)M[1], (float)M[5], (float)M[9]),
-             z = f3((float)M[2], (float)M[6], (float)M[10]);
-    const float d = fmaxf(fmaxf(fabsf(dot3(x, y)), fabsf(dot3(y, z))), fabsf(dot3(z, x)));
-    const float l = fabsf(dot3(x, x) - 1.f) + fabsf(dot3(y, y) - 1.f) + fabsf(dot3(z, z) - 1.f);
-    return d < 2e-6f && l < 2e-6f;  // false for NaN: l is one then
-}
 
 __global__ void k_ccd_pm32(int n, const double* __restrict__ pm, float* __restrict__ pm32) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1980,7 +1985,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
             continue;
         }
         const int na = ntris[e.na], nb = ntris[e.nb];
-        const float* PA = pm32 + 24 * (size_t)e.pair;
+        const float* PA = pm32 + kNpPose32 * (size_t)e.pair;
         const float* PB = PA + 12;
         if (lane < 16 && (lane & 7) < (lane < 8 ? na : nb)) {
             const size_t t = (size_t)(lane < 8 ? e.na : e.nb) * 8 + (lane & 7);
@@ -2016,6 +2021,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
         }
         if (lane == 0) atomicAdd(lc + LC_TRI + (w & (LC_TRI_N - 1)), na * nb);
         const float se = search[e.pair];
+        const bool rigid = PA[24] != 0.f;  // else the spheres' radii are not the triangles'
         const float tm = fabsf(PA[3]) + fabsf(PA[7]) + fabsf(PA[11]) + fabsf(PB[3]) + fabsf(PB[7]) + fabsf(PB[11]);
         __syncwarp();
         // the bounds that each triangle's own data give, two slots a lane
@@ -2031,7 +2037,7 @@ __global__ void __launch_bounds__(kBlock, LEAF ? 7 : 6) k_np_filter(int n, const
                 const float thr = se + ca[4] + cb[4];
                 const bool plain = !(fminf(ca[6], cb[6]) > 0.f);
                 const float lim = thr + ((plain ? 1e-3f : 2e-5f) + 4e-6f * (tm + ca[5] + cb[5] + thr));
-                keep = !(sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
+                keep = !(rigid && sqrtf(dx * dx + dy * dy + dz * dz) - ca[3] - cb[3] > lim) &&  // NaN keeps the slot
                        !(box_gap9(va, vb) > lim) &&
                        (plain || (!(normal_gap(ca + 7, vb) > lim) && !(normal_gap(cb + 7, va) > lim)));
             }
@@ -3259,7 +3265,7 @@ int run_narrowphase(d2g_ctx* ctx, const int32_t* d_pairs, int n_pairs, int* n_ou
     RC(E.pm.ensure(32 * (size_t)n_pairs + 1));
     RC(E.search.ensure(n_pairs + 1));
     RC(E.roots.ensure(n_pairs + 1));
-    RC(E.pm32.ensure(24 * (size_t)n_pairs + 1));
+    RC(E.pm32.ensure(kNpPose32 * (size_t)n_pairs + 1));
     if (n_pairs > 0)
         LAUNCH(k_np_prep, n_pairs, n_pairs, d_pairs, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p,
                E.pm.p, E.search.p, E.roots.p, E.pm32.p, nullptr);
@@ -3353,7 +3359,7 @@ int run_bucket_comparison(d2g_ctx* ctx, const int32_t* d_pair, const int32_t* d_
     cudaStream_t s = ctx->stream;
     RC(E.pm.ensure(33));
     RC(E.search.ensure(2));
-    RC(E.pm32.ensure(25));
+    RC(E.pm32.ensure(kNpPose32));
     RC(E.roots.ensure(2));
     LAUNCH(k_np_prep, 1, 1, d_pair, ctx->fut.p, ctx->mesh.p, ctx->mesh_node_off.p, ctx->geo_eps.p, E.pm.p,
            E.search.p, E.roots.p, E.pm32.p, nullptr);

@@ -1,7 +1,8 @@
-"""Continuous queries of bodies whose orientation is not a unit quaternion: the
+"""Continuous and discrete queries of bodies whose orientation is not a unit quaternion: the
 pose's linear part scales and shears, and the reference measures distances
-after it; a huge one gives coordinates beyond FP32's range.  Contacts, offsets
-and futures against the oracle, bit for bit."""
+after it, while a triangle's bounding sphere does not follow; a huge one gives
+coordinates beyond FP32's range.  Contacts, offsets and futures against the
+oracle, bit for bit."""
 import numpy as np
 import pytest
 
@@ -64,3 +65,23 @@ def test_coordinates_beyond_fp32_match_oracle(ctx, value, seed):
         s.cur[moving[seed], comp] = value
         pairs = D.broad_phase(D.make_scene(1, nx=2, ny=2, nz=1, spacing=1.0, speed_sigma=0.0, seed=seed))
         ccd_against_oracle(ctx, s, pairs, np.full(len(pairs), 0.02))
+
+
+@pytest.mark.parametrize("config", [1, 2])
+@pytest.mark.parametrize("scale", [0.5, 0.999, 1.0001, 1.1, 1.3, 2.0])
+def test_discrete_queries_match_oracle(ctx, config, scale):
+    total = 0
+    for seed in range(4):
+        s = D.make_scene(config, nx=2, ny=2, nz=1, spacing=1.3, speed_sigma=0.0, seed=seed)
+        moving = np.flatnonzero(s.is_static == 0)
+        s.cur[moving, 1:5] *= scale
+        s.fut[...] = s.cur
+        pairs = D.broad_phase(D.make_scene(config, nx=2, ny=2, nz=1, spacing=0.9, speed_sigma=0.0, seed=seed))
+        ref, ref_off, ref_cnt = O.narrowphase(s.copy(), pairs)
+        ctx.set_scene(s.copy())
+        c, off, cnt = ctx.compare_trees_full(pairs, capacity=max(1024, 2 * len(ref)))
+        assert off.tolist() == ref_off.tolist()
+        assert np.array_equal(c.view(np.uint64), ref.view(np.uint64))
+        assert cnt[:2].tolist() == ref_cnt[:2].tolist()
+        total += len(ref)
+    assert total > 0 or scale < 1.0  # (smaller bodies no longer touch)
