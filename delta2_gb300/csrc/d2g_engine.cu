@@ -193,8 +193,8 @@ __device__ __forceinline__ void store_prim(PrimResult* __restrict__ r, double di
 // test cannot hit (a soup sub-test with such a distance can never be the best
 // of a triangle pair that hits), so the test is recorded as no contact (+inf)
 // and left out of the FP64 work list.  The gap is computed in FP32 and only
-// used beyond a margin (1 mm plus 4e-6 of the largest coordinate involved)
-// far above the FP32 and FP64 rounding at scene scale.
+// used beyond a margin (point-triangle 1 mm, edge-edge 20 um, plus 4e-6 of the
+// largest coordinate involved) far above the FP32 and FP64 rounding at scene scale.
 
 struct Box32 {
     float lo[3], hi[3];

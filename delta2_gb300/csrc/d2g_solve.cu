@@ -1,7 +1,7 @@
 // Contact filtering and the per-cluster sequential-impulse solve.
 //
-// filterContacts (collision_detection/contact.h:44-69): one thread per body
-// pair, stable insertion sort by (eps_a + eps_b, |A - B|) and the greedy
+// filterContacts (collision_detection/contact.h:44-69): one block per body
+// pair, a sort by (eps_a + eps_b, |A - B|, input order) and the greedy
 // de-duplication of contact midpoints.
 //
 // SequentialImpulses::solve (strategies/contact_force/sequential_impulses.cpp:
@@ -48,7 +48,12 @@ inline int nblocks(long long n, int b = kBlock) { return (int)((n + b - 1) / b);
 // not exist.  A comparator t of a step within 64 elements belongs to the warp
 // that owns them, and needs no block barrier before the next such step.
 // (Library segmented sorts took 22 launches and ~175 us of a 296 us filter
-// call on 4,000 contacts in 300 pairs, and 12 launches in a solve.)
+// call on 4,000 contacts in 300 pairs, and 12 launches in a solve.)  The filter
+// call by its groups, the caller's host copies included, before and now (ms):
+//   100,000 of 3                    5.1 / 5.1      1 of 20,000,  21 kept      7.8 / 1.6
+//   64 of 2,000, 983 kept each     27.5 / 1.4      1 of 20,000, 1,901 kept     575 / 8.2
+//   8 of 8,000, 1,600 kept each     198 / 2.5      1 of 262,144,   21 kept    95.5 / 23.4
+//   8 of 9,000 (global memory)      232 / 3.5      1 of 262,144, 2,549 kept  9,118 / 145
 constexpr int kSegSmall = 1024;        // elements of the 128-thread kernels' shared memory
 constexpr int kSegLarge = 8192;        // ... of the 1,024-thread kernels'
 constexpr int kSegSmallBlock = 128, kSegLargeBlock = 1024;
@@ -266,7 +271,7 @@ __global__ void k_filter_write(int n_pairs, const int32_t* __restrict__ off, con
 // The halves run on different warps, the position half one wave ahead:
 // GB300 issues an FP64 warp instruction every 64 cycles per SM sub-partition
 // whatever the number of active lanes, so a wave costs the longest warp's
-// FP64 instruction count, 28 for the velocity half and 20 for the position
+// FP64 instruction count, 28 for the velocity half and 21 for the position
 // half, against ~143 when one warp formed both with the quaternion integration
 // of two states.  A contact takes eight lanes of each (side A or B, component).
 // Where a block has a single task of at most four contacts in a wave its four
@@ -579,9 +584,9 @@ __device__ __forceinline__ void velocity_half(ConS& C, bool act, int side, int c
 // operations of one instruction stream: x + y as fma(x, 1, y) and x y as
 // fma(x, y, -0), each the same single rounding, so an addition, a product or a
 // fused step of div_by can share an instruction: 20 FP64 instructions for the
-// velocity half instead of 28 and 15 instead of 18, 64 cycles each.  What no
-// other warp writes is loaded one interval ahead (HalfPre).  100 cubes on 16
-// blocks: 164 -> 140 us per iteration.
+// velocity half instead of 28 and 20 for the position half instead of 21, 64
+// cycles each.  What no other warp writes is loaded one interval ahead
+// (HalfPre).  100 cubes on 16 blocks: 164 -> 140 us per iteration.
 struct HalfPre {
     ConS* C;
     BodyS* B;
@@ -963,8 +968,9 @@ __device__ void solve_body(int k, int gb, int G, const SolveSync& S, const Solve
         return;
     }
     // ---- every body's contacts in sorted order, a warp per body: a warp reads
-    // all of the cluster's contacts (a few thousand coalesced 8-byte loads),
-    // which needs neither a sort nor an order of arrival
+    // the cluster's contacts, coalesced 8-byte loads, up to the body's last one,
+    // which needs neither a sort nor an order of arrival (bodies times contacts:
+    // 4,096 hulls with 13,466 contacts on the grid solve in 35 ms, 86 before)
     for (int p = warp * G + gb; p < np; p += (kSolveBlock / 32) * G) {
         const int n = a.deg[p0 + p];
         int base = 0;
@@ -1620,25 +1626,37 @@ int run_solve(d2g_ctx* ctx, int n_clusters, const int32_t* d_part_off, const int
         // Where each cluster is solved (us per iteration on GB300, normal and
         // friction; one block / thread-block cluster of 4 / 8 / 16 / grid):
         //     8 cubes, 46 waves of 2.2 contacts     60 /   74 /   72 /  74 /    -
-        //    27 cubes, 89 waves of 5.0             124 /  141 /  136 / 140 /  223
-        //   100 cubes, one layer                   311 /  185 /  152 / 140 /  203
-        //   512 hulls, 24 waves of 71              357 /  118 /   79 /  67 /   77
-        // 1,024 hulls, 23 waves of 142             676 /  213 /  124 /  88 /   83
+        //    27 cubes, 89 waves of 5.0             123 /  141 /  136 / 136 /  214
+        //    32 cubes, two layers                  137 /    - /    - / 146 /  240
+        //    36 cubes, four layers                 145 /    - /    - / 158 /  253
+        //    48 cubes, four layers                 241 /    - /    - / 182 /  297
+        //    64 cubes, four layers                 274 /    - /    - / 185 /  308
+        //    64 cubes, one layer                   212 /    - /    - / 124 /  187
+        //    81 cubes, one layer                   261 /    - /    - / 130 /  196
+        //   100 cubes, one layer                   308 /  185 /  152 / 136 /  204
+        //   512 hulls, 24 waves of 71              352 /  118 /   79 /  67 /   78
+        //   576 hulls                              398 /    - /    - /  68 /   77
+        //   704 hulls                              479 /    - /    - /  74 /   74
+        //   768 hulls                              529 /    - /    - /  81 /   83
+        // 1,024 hulls, 23 waves of 142             666 /  213 /  124 /  87 /   82
         // 2,304 hulls                             1542 /  480 /  289 / 178 /  133
+        // (hull piles of 36 to 216 that converge at once: 16 blocks 0.33 to 0.47
+        // ms a call, one block 0.33 to 0.87.)
         // (one to four contacts to a warp throughout, eight lanes each: 61 for
         // the 8 cubes, 165 / 164 for the 100 on 8 / 16 blocks, 71 / 85 and 88 /
         // 90 for 512 and 1,024 hulls on 16 blocks / a grid; the halves undivided,
         // a contact on one warp: 331 for the 8 cubes, 257 for the 1,024 hulls.)
         // A block barrier costs ~0.1 us, the cluster barrier with distributed
         // shared memory ~0.5 us more, a grid barrier ~1.5 us: so one block up
-        // to kOneBlockParts particles, then 16, or the most
-        // with which all such clusters of the call are resident at once, and a
-        // cooperative grid for a cluster with at least kGridMinContacts contacts
-        // and more than D2G_TUNE_GRID_MIN_PARTS parts (768 by default, between
-        // the 513 and the 1,025 of the table) when at most kGridMaxClusters
-        // qualify (grids run one after another).  D2G_TUNE_SOLVE_CLUSTER fixes
-        // the cluster's size.  Blocks and thread-block clusters run side by
-        // side on two streams, the grids after them.
+        // to kOneBlockParts particles (one block is still 7 to 9% faster at 33 to
+        // 37, 16 are 24% faster at 49), then 16, or the most with which all such
+        // clusters of the call are resident at once, and a cooperative grid for a
+        // cluster with at least kGridMinContacts contacts and more than
+        // D2G_TUNE_GRID_MIN_PARTS parts (768 by default, where the table's two
+        // columns cross) when at most kGridMaxClusters qualify (grids run one
+        // after another).  D2G_TUNE_SOLVE_CLUSTER fixes the cluster's size.
+        // Blocks and thread-block clusters run side by side on two streams, the
+        // grids after them.
         const int cl_setting = E.tune[D2G_TUNE_SOLVE_CLUSTER];
         std::vector<int32_t> small, mid, big;
         if (h_con_off && h_part_off)

@@ -248,7 +248,7 @@ int d2g_ctx_ccd_stats(d2g_ctx* ctx, int32_t reset, int64_t* stats, int32_t n);
  * the work is spread over the GPU; every setting gives identical results.
  *   D2G_TUNE_EE_FIRST_ITERS (default 2, 0..10): Newton iterations an
  *     edge-edge CCD test runs on one lane before the tests still running
- *     continue on four lanes each.
+ *     are packed and continue on four lanes each (one when they are many).
  *   D2G_TUNE_GRID_MIN_PARTS (default 768, >= 0): a cluster with at least
  *     128 contacts and more parts than this is solved by a cooperative grid
  *     over the SMs, when at most 8 clusters of the solve call qualify.
@@ -269,10 +269,10 @@ int d2g_ctx_ccd_stats(d2g_ctx* ctx, int32_t reset, int64_t* stats, int32_t n);
  *   D2G_TUNE_SOLVE_CLUSTER (default 0; 0, 1, 2, 4, 8 or 16): a cluster with
  *     at least 32 contacts that does not take a grid is solved by a
  *     thread-block cluster of this many blocks (waves between them on the
- *     hardware cluster barrier); 0 chooses the size from the clusters'
- *     particles (one block up to 32, then doubling) as far as every such
- *     cluster of the call is resident at once (one block each when none is),
- *     1 solves them with one block each.
+ *     hardware cluster barrier); 0 takes 16 blocks for those of more than 32
+ *     particles, or the most with which all of them are resident at once (one
+ *     block each when not even two are), and one block for the others; 1 solves
+ *     them with one block each.
  * delta2_gb300/autotune.py measures candidate values on a workload and
  * writes them to a file that the Python layer applies. */
 #define D2G_TUNE_EE_FIRST_ITERS 0
